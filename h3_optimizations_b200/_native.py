@@ -60,6 +60,8 @@ PROTOTYPES = {
                                     c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "h3s_quant_v_fp8": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_int, c_int,
                                 c_int, c_int, c_float, c_void_p]),
+    "h3s_quant_v_fp8_half": (c_int, [c_void_p, c_int, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                     c_int, c_int, c_float, c_void_p]),
     "h3s_convrot_quant_rows": (c_int, [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "h3s_qkv_gemm_chunk": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
                                    c_int64, c_void_p, c_void_p]),
@@ -83,6 +85,10 @@ PROTOTYPES = {
     "h3s_sparse_attn_fwd_scatter": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                             c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
                                             c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "h3s_v_half": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p]),
+    "h3s_sparse_attn_half_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                         c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+                                         c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_void_p]),
     "h3s_sparse_attn_fwd_mma": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int64,
                                         c_int64, c_int, c_int, c_int, c_void_p]),

@@ -295,6 +295,7 @@ class B200SparseBackend:
             side = self._side_stream(q.device)
             k_mean, v_scale, scratch = ops.column_stats_buffers(heads, q.device, want_k_mean=self.smooth_k)
             v_carrier = ops.allocate_v_carrier(sequence, heads, v.device)
+            v_half = torch.empty(v_carrier.shape, dtype=torch.bfloat16, device=v.device)
             events = self.__dict__.setdefault("_stats_events", {})
             pair = events.get(side)
             if pair is None:
@@ -313,7 +314,7 @@ class B200SparseBackend:
                 with torch.cuda.stream(side):
                     if need_route:
                         side.wait_event(k_done)
-                    ops.quant_v_fp8_into(v, v_scale, v_carrier, v_bound=V_QUANT_BOUND)
+                    ops.quant_v_fp8_into(v, v_scale, v_carrier, v_bound=V_QUANT_BOUND, half=v_half)
                 if need_route:
                     route = self.router.build_route_from_summaries(
                         q_summary, k_summary, snapshot.layout, video_budget,
@@ -335,7 +336,7 @@ class B200SparseBackend:
             q_int8=q_int8, k_int8=k_int8, v_carrier=v_carrier, q_scale=q_scale, k_scale=k_scale,
             v_scale=v_scale, route=route, output_dtype=q.dtype, output_shape=tuple(q.shape),
             layer_index=int(layer_index), sequence=int(sequence), heads=int(heads),
-            metadata=self._metadata(route.metadata, layer_index, heads),
+            metadata=self._metadata(route.metadata, layer_index, heads), v_half=v_half,
         )
         sparse.metadata["smooth_k"] = bool(self.smooth_k)
         return PreparedHybrid(sparse=sparse)
@@ -378,6 +379,7 @@ class B200SparseBackend:
             q_scale=projected.q_scale, k_scale=projected.k_scale, v_scale=v_scale, route=route,
             output_dtype=projected.output_dtype, output_shape=(1, heads, sequence, projected.head_dim),
             layer_index=int(projected.layer_index), sequence=sequence, heads=heads, metadata=metadata,
+            v_half=projected.v_half if projected.v_carrier is not None else None,
         )
         return PreparedHybrid(sparse=sparse)
 
@@ -398,7 +400,7 @@ class B200SparseBackend:
                 sparse.q_int8, sparse.k_int8, sparse.v_carrier, sparse.q_scale, sparse.k_scale,
                 sparse.v_scale, route.indices,
                 q_start=geometry.pure_video_q_start, q_stop=geometry.pure_video_q_stop,
-                out=out, out_dtype=out_dtype, status=word, peer_out_ptrs=peer_out_ptrs,
+                out=out, out_dtype=out_dtype, status=word, peer_out_ptrs=peer_out_ptrs, v_half=sparse.v_half,
             )
             if not torch.cuda.is_current_stream_capturing():
                 # (an event recorded inside a capture could not be queried afterwards: replays are

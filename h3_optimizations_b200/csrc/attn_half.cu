@@ -1,0 +1,505 @@
+// Block-sparse attention on INT8 Q/K and a BF16 copy of the FP8 V carrier, for
+// sm_100a.
+//
+// One CTA owns one 128-row query tile of one head and walks that tile's list
+// of 64-row KV tiles:
+//   S = Q8 . K8^T      tcgen05.mma kind::i8, 128x64x128, Q8 in TMEM, int32 in TMEM
+//   P = exp2(c*S - m)  FP32 in registers, one thread per query row, m an integer
+//   O += P16 . V16     tcgen05.mma kind::f16, 128x128x64, P in TMEM, fp32 in TMEM
+// V16 holds the E4M3 codes as BF16 (exact), so the product is that of the FP8
+// carrier; P is rounded once to BF16 (relative error up to 2^-9, the two E4M3
+// terms of attn_tc.cu have 2^-8).
+//
+// Why BF16 P instead of two E4M3 terms: the tensor pipe takes the same time for
+// one 16-bit product as for two 8-bit products, but a softmax thread needs one
+// packed conversion per pair of scores instead of a mask, a residual and two
+// conversions per score, and BF16's exponent range makes the running maximum
+// unnecessary: m is the row maximum of the first tile and stays.  P may then
+// grow to 2^100 (70 nats above the first tile) before anything is lost; the row
+// sums tell, and a query tile where it happens is done again with the true row
+// maximum (one more pass over the scores to find it).
+//
+// Without a running maximum the tiles of a row are independent but for the sum:
+// the eight softmax warps form two groups, group g takes tiles g, g+2, ..., and
+// with two CTAs per SM four warps share a scheduler, each in its own phase of
+// wait / load / exponentials / store.  That is what keeps the ex2 pipe (512 cycles
+// per tile and SM) and the tensor pipe (384) busy; with one group, or with two
+// threads per row, the CTAs fall into step and both pipes idle a third of the
+// time.
+//
+// TMEM (256 columns per CTA, two CTAs per SM): O 128, Q8 32 (A operand of QK^T:
+// Q is read once instead of with every K tile, which takes a third off the
+// shared-memory traffic), and three 32-column slots A B C.  S(j) is 64 columns:
+// A+B for even j, B+C for odd j; P(j) is 32 columns: A for even, C for odd.
+// QK^T(j) needs S(j-1) in registers (slot B) and P.V(j-2) complete.
+//
+// Warp roles: warps 0-7 softmax/epilogue (TMEM lanes 32*(w%4).., group w/4), warp 8
+// TMA producer and QK^T issuer, warp 9 P.V issuer and TMEM owner.
+//
+// What bounds it: per tile and SM the ex2 pipe needs 512 cycles, the tensor pipe 453
+// (measured: 144 for QK^T with A in TMEM, 258 with A in shared memory, 309 for P.V),
+// the remaining softmax instructions about 290 issue slots; a tile takes 800.  24
+// heads x 33272 tokens at 30 %: 3.81 ms with two E4M3 terms -> 2.88 ms, and 4.20 ->
+// 3.33 ms once the board has reached its power cap (1 kW, 1.7 GHz), which it does
+// after half a second.  Tried and slower: a polynomial for a share of the
+// exponentials, two threads per row, one group per CTA, scores of the next tile
+// fetched between the halves of this one.
+#include "attn_common.cuh"
+#include "tma.cuh"
+
+namespace h3s {
+
+constexpr int kHStages = 4;  // tile i+2 is loaded when tile i-2 is done
+constexpr int kHSoftmaxWarps = 8;
+constexpr int kHThreads = (kHSoftmaxWarps + 2) * 32;
+constexpr int kHTmemCols = 256;
+constexpr uint32_t kHKBytes = H3S_KV_TILE * H3S_HEAD_DIM;      // 8192
+constexpr uint32_t kHVBytes = H3S_HEAD_DIM * H3S_KV_TILE * 2;  // 16384
+constexpr uint32_t kHOffK = 0;
+constexpr uint32_t kHOffV = kHOffK + kHStages * kHKBytes;
+constexpr uint32_t kHOffBar = kHOffV + kHStages * kHVBytes;
+constexpr uint32_t kHSmemBytes = kHOffBar + 4096 + 1024;  // barriers/scalars + alignment slack
+constexpr float kHSumLimit = 1.2676506e30f;  // 2^100: row sums above this send the query tile round again
+
+struct HalfShared {
+  uint64_t q_ready;            // four softmax warps have put the Q rows into TMEM
+  uint64_t kv_full[kHStages];
+  uint64_t s_full[2];          // QK^T of tile j has completed (one per group)
+  uint64_t s_taken[2];         // S(j) is in registers
+  uint64_t p_full[2];          // P(j) is in TMEM
+  uint64_t pv_done[2];         // P.V of tile j has completed: its stage and its slot are free
+  uint64_t first_max;          // group 0 has left the first tile's row maxima in `row`
+  uint64_t pass_end;           // row sums (or maxima) of a pass are in `row`, `again` is valid; all warps wait
+  uint64_t staged;             // softmax warps only: the output tile is in shared memory
+  uint32_t tmem_base;
+  int abort_word;
+  int again;                   // some row sum passed the limit
+  int tile_index[kHStages];    // KV tile held by each stage ...
+  float tile_scale[kHStages];  // ... and its k_scale, written by the producer
+  float v_scale[H3S_HEAD_DIM];
+  float first[H3S_Q_TILE];
+  float row[2][2][H3S_Q_TILE];  // values the two threads of a row give each other, in turn
+};
+static_assert(sizeof(HalfShared) <= 4096, "barrier block too large");
+
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+
+// Row sum and BF16 P of 64 scores.  The int32 scores become fp32 without a
+// conversion instruction: for |s| < 2^22, bits(12582912.0f) + s are the bits of
+// the float 12582912 + s exactly, and the offset is folded into the constants of
+// the FMA that follows: P = exp2(c*f + bias) = exp2(c*s - m).
+__device__ __forceinline__ float exp_pack(const uint32_t (&s)[H3S_KV_TILE], float c, float bias,
+                                          uint32_t (&packed)[H3S_KV_TILE / 2]) {
+  const float2 c2 = make_float2(c, c), bias2 = make_float2(bias, bias);
+  float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < H3S_KV_TILE / 2; ++i) {
+    const float2 f = make_float2(__uint_as_float(s[2 * i] + kIntBiasBits), __uint_as_float(s[2 * i + 1] + kIntBiasBits));
+    const float2 x = fma2(c2, f, bias2);
+    const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+    if (i & 1) sum_b = add2(sum_b, p); else sum_a = add2(sum_a, p);
+    packed[i] = pack_bf16x2(p.x, p.y);
+  }
+  sum_a = add2(sum_a, sum_b);
+  return sum_a.x + sum_a.y;
+}
+
+__device__ __forceinline__ int max_score(const uint32_t (&s)[H3S_KV_TILE]) {
+  int a = __vimax3_s32(s[0], s[1], s[2]), b = __vimax3_s32(s[3], s[4], s[5]);
+#pragma unroll
+  for (int i = 6; i + 3 < H3S_KV_TILE; i += 4) {
+    a = __vimax3_s32(a, s[i], s[i + 1]);
+    b = __vimax3_s32(b, s[i + 2], s[i + 3]);
+  }
+  return max(__vimax3_s32(a, s[H3S_KV_TILE - 2], s[H3S_KV_TILE - 1]), b);
+}
+
+template <typename OutT>
+__global__ void __launch_bounds__(kHThreads, 2)
+sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                        const int8_t *__restrict__ q8, const AttnParams prm) {
+  extern __shared__ unsigned char smem_dyn[];
+  // SWIZZLE_128B tiles need 1024-byte alignment
+  // (offset arithmetic, so that the compiler still sees shared memory)
+  unsigned char *smem = smem_dyn + ((1024u - (ptx::smem_u32(smem_dyn) & 1023u)) & 1023u);
+  HalfShared &sh = *reinterpret_cast<HalfShared *>(smem + kHOffBar);
+  volatile int *abort_word = &sh.abort_word;
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+
+  // ---- work item: dense (long) rows first, then the routed rows ----
+  const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
+  const int n_dense = prm.q_tiles - n_sparse;
+  int head, tq;
+  bool dense;
+  {
+    const int w = blockIdx.x;
+    const int dense_items = prm.heads * n_dense;
+    if (w < dense_items) {
+      dense = true;
+      head = w / n_dense;
+      const int i = w - head * n_dense;
+      tq = (n_sparse == 0 || i < prm.q_start) ? i : prm.q_stop + (i - prm.q_start);
+    } else {
+      dense = false;
+      const int v = w - dense_items;
+      head = v / n_sparse;
+      tq = prm.q_start + (v - head * n_sparse);
+    }
+  }
+  const int n_iter = dense ? prm.kv_tiles : prm.route_len;
+  const int32_t *route_row =
+      dense ? nullptr
+            : prm.route + (static_cast<int64_t>(head) * n_sparse + (tq - prm.q_start)) * prm.route_len;
+
+  // ---- setup ----
+  if (threadIdx.x == 0) {
+    ptx::mbar_init(&sh.q_ready, 4);
+    for (int i = 0; i < kHStages; ++i) ptx::mbar_init(&sh.kv_full[i], 1);
+    for (int g = 0; g < 2; ++g) {
+      ptx::mbar_init(&sh.s_full[g], 1);
+      ptx::mbar_init(&sh.s_taken[g], 4);
+      ptx::mbar_init(&sh.p_full[g], 4);
+      ptx::mbar_init(&sh.pv_done[g], 1);
+    }
+    ptx::mbar_init(&sh.first_max, 4);
+    ptx::mbar_init(&sh.pass_end, kHSoftmaxWarps);
+    ptx::mbar_init(&sh.staged, kHSoftmaxWarps);
+    sh.abort_word = 0;
+    sh.again = 0;
+    ptx::fence_mbar_init();
+  }
+  if (threadIdx.x < H3S_HEAD_DIM) sh.v_scale[threadIdx.x] = __ldg(prm.v_scale + head * H3S_HEAD_DIM + threadIdx.x);
+  if (warp == kHSoftmaxWarps + 1) {
+    ptx::tmem_alloc(&sh.tmem_base, kHTmemCols);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem_o = sh.tmem_base;         // 128 columns, fp32
+  const uint32_t tmem_q = tmem_o + 128;         // 32 columns, four int8 codes each
+  const uint32_t tmem_s = tmem_o + 160;         // slots A B C, 32 columns each
+
+  // Passes over the tile list: one, or three when a row sum passed the limit (the
+  // second only finds the row maxima).  Every warp waits for `pass_end`, so all
+  // agree on `again`.  `done` counts the tiles of earlier passes: stages and
+  // parities run on.
+  bool ok = true;
+  int done = 0;
+
+  // wait for tile j's use of one of a pair of barriers (tile j uses number j & 1)
+  auto wait_tile = [&](uint64_t (&bar)[2], int j, int code, int factor) {
+    return warp_wait(&bar[j & 1], static_cast<uint32_t>(j >> 1) & 1u, abort_word, code, factor * prm.wait_budget_ns);
+  };
+  auto wait_stage = [&](int j) {
+    return warp_wait(&sh.kv_full[j % kHStages], static_cast<uint32_t>(j / kHStages) & 1u, abort_word, kAbortKvFull,
+                     prm.wait_budget_ns);
+  };
+
+  if (warp == kHSoftmaxWarps) {
+    // =================== TMA producer and QK^T issuer ===================
+    // QK^T(j) waits for P.V(j-2), which also frees that tile's stage: tile j+2's
+    // loads go out behind it.  The whole warp fetches the tile indices and K scales
+    // of 32 tiles at a time, one block ahead of their use; lane 0 leaves each stage's
+    // index and scale in shared memory for the softmax warps.
+    constexpr uint32_t idesc_qk = ptx::umma_idesc(2, 1, 1, H3S_Q_TILE, H3S_KV_TILE);
+    const uint64_t k_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + kHOffK), 1024, ptx::kSwizzle128);
+    const float *k_scale = prm.k_scale + static_cast<int64_t>(head) * prm.kv_tiles;
+    if (lane == 0) {
+      ptx::prefetch_tensormap(&map_k);
+      ptx::prefetch_tensormap(&map_v);
+    }
+    int my_tile = 0, next_tile = 0, block = -1;  // tile list entries 32*block .. +31, one per lane, and the 32 after
+    float my_scale = 0.f, next_scale = 0.f;
+    auto fetch_block = [&](int b) {
+      const int mine = min(b * 32 + lane, n_iter - 1);
+      next_tile = dense ? mine : __ldg(route_row + mine);
+      next_scale = __ldg(k_scale + next_tile);
+    };
+    auto load = [&](int i) {      // tile i of the list, into the stage of its running number
+      if (i >= n_iter) return;
+      if ((i >> 5) != block) {
+        block = i >> 5;
+        my_tile = next_tile; my_scale = next_scale;
+        fetch_block(block + 1);
+      }
+      const int t = __shfl_sync(0xffffffffu, my_tile, i & 31);
+      const float ks = __shfl_sync(0xffffffffu, my_scale, i & 31);
+      if (lane == 0 && done + i != prm.drop_kv_load) {
+        const int s = (done + i) % kHStages;
+        sh.tile_index[s] = t;
+        sh.tile_scale[s] = ks;
+        ptx::mbar_arrive_expect_tx(&sh.kv_full[s], kHKBytes + kHVBytes);
+        ptx::tma_load_3d(smem + kHOffK + s * kHKBytes, &map_k, &sh.kv_full[s], 0, t * H3S_KV_TILE, head);
+        ptx::tma_load_3d(smem + kHOffV + s * kHVBytes, &map_v, &sh.kv_full[s], t * H3S_KV_TILE * 2, 0, head);
+      }
+      __syncwarp();
+    };
+    for (int pass = 0; ok; ++pass) {
+      block = -1;
+      fetch_block(0);
+      for (int i = 0; i < kHStages; ++i) load(i);
+      if (pass == 0) ok = warp_wait(&sh.q_ready, 0, abort_word, kAbortQFull, prm.wait_budget_ns);
+      for (int i = 0; ok && i < n_iter; ++i) {
+        const int j = done + i;
+        ok = wait_stage(j) && (i < 1 || wait_tile(sh.s_taken, j - 1, kAbortPEmpty, 3)) &&
+             (i < 2 || wait_tile(sh.pv_done, j - 2, kAbortPvDone, 4));
+        if (!ok) break;
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+          const uint64_t k_desc = k_desc0 + static_cast<uint64_t>((j % kHStages) * (kHKBytes >> 4));
+#pragma unroll
+          for (int k = 0; k < H3S_HEAD_DIM / 32; ++k)
+            ptx::umma_i8_ts(tmem_s + (j & 1) * 32, tmem_q + k * 8, k_desc + 2 * k, idesc_qk, k > 0);
+          ptx::tc_commit(&sh.s_full[j & 1]);
+        }
+        __syncwarp();
+        if (i >= 2) load(i + 2);
+      }
+      // (what the loop has not waited for, so that every barrier is one use behind at most)
+      const int last = done + n_iter - 1;
+      ok = ok && wait_tile(sh.s_taken, last, kAbortPEmpty, 3) && (n_iter < 2 || wait_tile(sh.pv_done, last - 1, kAbortFinal, 4)) &&
+           wait_tile(sh.pv_done, last, kAbortFinal, 4);
+      done += n_iter;
+      ok = ok && warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      if (pass == 2 || (pass == 0 && sh.again == 0)) break;
+    }
+  } else if (warp == kHSoftmaxWarps + 1) {
+    // =================== P.V issuer ===================
+    constexpr uint32_t idesc_pv = ptx::umma_idesc(1, 1, 1, H3S_Q_TILE, H3S_HEAD_DIM);
+    const uint64_t v_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + kHOffV), 1024, ptx::kSwizzle128);
+    for (int pass = 0; ok; ++pass) {
+      for (int j = done; j < done + n_iter; ++j) {
+        if (!wait_tile(sh.p_full, j, kAbortPFull, 3) || !wait_stage(j)) { ok = false; break; }
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+          const uint64_t v_desc = v_desc0 + static_cast<uint64_t>((j % kHStages) * (kHVBytes >> 4));
+#pragma unroll
+          for (int k = 0; k < H3S_KV_TILE / 16; ++k)
+            ptx::umma_f16_ts(tmem_o, tmem_s + (j & 1) * 64 + k * 8, v_desc + 2 * k, idesc_pv, (j > done || k > 0) ? 1u : 0u);
+          ptx::tc_commit(&sh.pv_done[j & 1]);
+        }
+        __syncwarp();
+      }
+      done += n_iter;
+      ok = ok && warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      if (pass == 2 || (pass == 0 && sh.again == 0)) break;
+    }
+  } else {
+    // =================== softmax + epilogue (warps 0-7) ===================
+    const int quarter = warp & 3, group = warp >> 2;
+    const int row = quarter * 32 + lane;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    if (group == 0) {
+      // this thread's Q row -> its TMEM lane
+      uint32_t q[32];
+      const int grow = tq * H3S_Q_TILE + row;
+      const uint4 *src = reinterpret_cast<const uint4 *>(q8 + (static_cast<int64_t>(head) * prm.sequence + grow) * H3S_HEAD_DIM);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint4 w = grow < prm.sequence ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+        q[4 * i] = w.x; q[4 * i + 1] = w.y; q[4 * i + 2] = w.z; q[4 * i + 3] = w.w;
+      }
+      H3S_TMEM_ST32(tmem_q + lane_addr, q);
+      ptx::tmem_wait_st();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.q_ready);
+    }
+    const float q_scale = __ldg(prm.q_scale + head * prm.q_tiles + tq) * (0.08838834764831845f * 1.4426950408889634f);
+    float m = 0.f, l = 0.f;
+
+    for (int pass = 0; ok; ++pass) {
+      const int last = done + n_iter - 1;
+      float top = -INFINITY;
+      l = 0.f;
+      for (int j = (done & 1) == group ? done : done + 1; j <= last; j += 2) {
+        if (!wait_tile(sh.s_full, j, kAbortSFull, 2)) { ok = false; break; }
+        ptx::tc_fence_after();
+        uint32_t s[H3S_KV_TILE];
+        H3S_TMEM_LD64(tmem_s + lane_addr + group * 32, s);
+        // index and K scale of this tile, left in shared memory by the producer
+        // before the stage was handed to the tensor pipe (free only after P.V(j))
+        const int n_valid = prm.sequence - sh.tile_index[j % kHStages] * H3S_KV_TILE;
+        const float c = q_scale * sh.tile_scale[j % kHStages];
+        ptx::tmem_wait_ld(s);
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&sh.s_taken[group]);
+
+        // Keys beyond the sequence (ragged last tile only): the integer whose biased
+        // bits are those of -inf, so that P becomes 0; it is also below every score.
+        if (n_valid < H3S_KV_TILE) {
+#pragma unroll
+          for (int i = 0; i < H3S_KV_TILE; ++i)
+            if (i >= n_valid) s[i] = 0xff800000u - kIntBiasBits;
+        }
+        if (j == 0) {
+          m = ceilf(c * static_cast<float>(max_score(s)));  // c > 0
+          sh.first[row] = m;
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&sh.first_max);
+        } else if (j == 1 && pass == 0) {
+          if (!warp_wait(&sh.first_max, 0, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
+          m = sh.first[row];
+        }
+        if (pass == 1) {
+          top = fmaxf(top, c * static_cast<float>(max_score(s)));
+        } else {
+          uint32_t packed[H3S_KV_TILE / 2];
+          l += exp_pack(s, c, -fmaf(c, kIntBias, m), packed);
+          // slot A or C: part of S(j), which is in registers
+          H3S_TMEM_ST32(tmem_s + lane_addr + group * 64, packed);
+          ptx::tmem_wait_st();
+          ptx::tc_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&sh.p_full[group]);
+      }
+      if (!ok) break;
+      done += n_iter;
+      // the row's two threads add up their sums (or agree on the maximum); two buffers,
+      // each written again only after every warp has passed the barrier in between
+      if (pass == 0 && __any_sync(0xffffffffu, !(l <= kHSumLimit)) && lane == 0) sh.again = 1;
+      float (&buffer)[2][H3S_Q_TILE] = sh.row[pass & 1];
+      buffer[group][row] = pass == 1 ? top : l;
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
+      ok = warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      if (pass == 1) m = ceilf(fmaxf(buffer[0][row], buffer[1][row])); else l = buffer[0][row] + buffer[1][row];
+      if (pass == 2 || (pass == 0 && *static_cast<volatile int *>(&sh.again) == 0)) break;
+    }
+
+    // every P.V of the last pass (one barrier per group)
+    if (ok && n_iter > 1) ok = wait_tile(sh.pv_done, done - 2, kAbortFinal, 4);
+    if (ok) ok = wait_tile(sh.pv_done, done - 1, kAbortFinal, 4);
+    if (ok) {
+      // Epilogue: O * v_scale / l -> OutT, staged through shared memory (the
+      // stage ring is free: every TMA load has been consumed).  A warp converts its
+      // 32 rows of one column half; the two warps of a row quarter then each write
+      // 16 of the quarter's rows as full contiguous lines.
+      ptx::tc_fence_after();
+      const float inv_l = 1.0f / l;
+      constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
+      static_assert(H3S_Q_TILE * kRowBytes <= kHOffBar, "output tile must fit the stage ring");
+      unsigned char *my_row = smem + row * kRowBytes;
+#pragma unroll 1
+      for (int cc = group * 2; cc < group * 2 + 2; ++cc) {
+        uint32_t o[32];
+        H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
+        ptx::tmem_wait_ld(o);
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            v[e] = __uint_as_float(o[i + e]) * sh.v_scale[cc * 32 + i + e] * inv_l;
+          // 8 values = one (bf16/fp16) or two (fp32) 16-byte chunks; the chunk index is
+          // XORed with the row so that the 32 rows of a warp do not collide on banks
+          constexpr int kChunks8 = 8 * static_cast<int>(sizeof(OutT)) / 16;
+          const int chunk0 = (cc * 32 + i) * static_cast<int>(sizeof(OutT)) / 16;
+          __align__(16) OutT tmp[8];
+          store_out8<OutT>(tmp, v);
+#pragma unroll
+          for (int k = 0; k < kChunks8; ++k)
+            *reinterpret_cast<uint4 *>(my_row + (((chunk0 + k) ^ (row & 15)) << 4)) =
+                reinterpret_cast<const uint4 *>(tmp)[k];
+        }
+      }
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.staged);
+      // both halves of the rows are staged
+      if (warp_wait(&sh.staged, 0, abort_word, kAbortFinal, 4 * prm.wait_budget_ns)) store_rows<OutT>(prm, smem, head, tq, quarter * 32 + group * 16, 16, lane);
+    }
+  }
+
+  // ---- teardown ----
+  __syncthreads();
+  const int code = sh.abort_word;
+  if (code != 0) {
+    // leave time for copies / MMAs still in flight before releasing TMEM and shared memory
+    __nanosleep(200000);
+    if (threadIdx.x == 0 && prm.status != nullptr) {
+      if (atomicCAS(prm.status, 0, code) == 0) {
+        prm.status[1] = blockIdx.x;
+        prm.status[2] = head;
+        prm.status[3] = tq;
+      }
+    }
+  }
+  if (warp == kHSoftmaxWarps + 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem_o, kHTmemCols);
+  }
+  // head-sharded run: the producer and MMA warps have nothing left to do and share the copy
+  if (code == 0 && prm.n_peer_out > 0) scatter_to_peers<OutT>(prm, smem, head, tq, kHThreads);
+}
+
+// E4M3 codes -> BF16 values: 16 per thread
+__global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v8, uint4 *__restrict__ v16, int64_t chunks) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= chunks) return;
+  uint4 out[2];
+  e4m3x16_to_bf16(__ldg(v8 + i), out);
+  v16[2 * i] = out[0];
+  v16[2 * i + 1] = out[1];
+}
+
+template <typename OutT>
+static int launch_attn_half(const CUtensorMap &mk, const CUtensorMap &mv, const int8_t *q8, const AttnParams &prm,
+                            cudaStream_t stream) {
+  H3S_CHECK_CUDA(cudaFuncSetAttribute(sparse_attn_half_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kHSmemBytes)));
+  sparse_attn_half_kernel<OutT><<<prm.heads * prm.q_tiles, kHThreads, kHSmemBytes, stream>>>(mk, mv, q8, prm);
+  H3S_CHECK_CUDA(cudaGetLastError());
+  return H3S_OK;
+}
+
+}  // namespace h3s
+
+extern "C" int h3s_v_half(const uint8_t *v8t, void *v16t, int heads, int sequence, h3s_stream_t stream) {
+  using namespace h3s;
+  H3S_CHECK_ARG(v8t != nullptr && v16t != nullptr, "v_half: NULL pointer");
+  H3S_CHECK_ARG(heads > 0 && sequence > 0, "v_half: empty problem (heads=%d sequence=%d)", heads, sequence);
+  H3S_CHECK_ARG(((reinterpret_cast<uintptr_t>(v8t) | reinterpret_cast<uintptr_t>(v16t)) & 15) == 0, "v_half: carriers must be 16-byte aligned");
+  const int64_t chunks = static_cast<int64_t>(heads) * H3S_HEAD_DIM * (ceil_div(sequence, 128) * 128) / 16;
+  v_half_kernel<<<static_cast<unsigned>((chunks + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const uint4 *>(v8t), static_cast<uint4 *>(v16t), chunks);
+  H3S_CHECK_CUDA(cudaGetLastError());
+  return H3S_OK;
+}
+
+extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, const void *v16t, const float *q_scale,
+                                        const float *k_scale, const float *v_scale, const int32_t *route,
+                                        int route_len, int q_start, int q_stop, void *out, void *const *peer_out,
+                                        int n_peer_out, int out_dtype, int64_t out_stride_h, int64_t out_stride_s,
+                                        int heads, int sequence, int flags, int32_t *status, h3s_stream_t stream) {
+  using namespace h3s;
+  AttnParams prm;
+  int rc = fill_attn_params(&prm, q8, k8, v16t, q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out,
+                            peer_out, n_peer_out, out_dtype, out_stride_h, out_stride_s, heads, sequence, flags, status,
+                            "sparse_attn_half_fwd");
+  if (rc) return rc;
+  const uint64_t S = static_cast<uint64_t>(sequence);
+  const uint64_t row_bytes = static_cast<uint64_t>(ceil_div(sequence, 128)) * 128 * 2;
+  CUtensorMap mk, mv;
+  rc = make_tensor_map_u8_3d(&mk, k8, H3S_HEAD_DIM, S, heads, H3S_HEAD_DIM, S * H3S_HEAD_DIM, H3S_HEAD_DIM,
+                             H3S_KV_TILE, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_half_fwd K map");
+  if (rc) return rc;
+  rc = make_tensor_map_u8_3d(&mv, v16t, row_bytes, H3S_HEAD_DIM, heads, row_bytes, row_bytes * H3S_HEAD_DIM,
+                             H3S_KV_TILE * 2, H3S_HEAD_DIM, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_half_fwd V map");
+  if (rc) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (out_dtype) {
+    case H3S_F32: return launch_attn_half<float>(mk, mv, q8, prm, s);
+    case H3S_BF16: return launch_attn_half<__nv_bfloat16>(mk, mv, q8, prm, s);
+    default: return launch_attn_half<__half>(mk, mv, q8, prm, s);
+  }
+}

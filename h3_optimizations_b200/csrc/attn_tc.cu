@@ -1,4 +1,5 @@
-// Block-sparse attention on the INT8 Q/K + FP8 V carriers for sm_100a.
+// Block-sparse attention on the INT8 Q/K + FP8 V carriers for sm_100a: the kernel for
+// hosts that keep no BF16 copy of V (attn_half.cu needs one) and for single-term P.
 //
 // One CTA owns one 128-row query tile of one head and walks that tile's list
 // of 64-row KV tiles:
@@ -20,8 +21,7 @@
 // exceeds it by more than 8.75 (P then stays <= 2^8.75 = 431 < 448 = E4M3 max).
 #include <climits>
 
-#include "common.cuh"
-#include "ptx.cuh"
+#include "attn_common.cuh"
 #include "tma.cuh"
 
 namespace h3s {
@@ -46,39 +46,6 @@ constexpr uint32_t kAttnSmemBytes = kOffBar + 1024 + 1024;  // barriers/scalars 
 // for ~2 % more time spent rescaling.
 constexpr float kRescaleThreshold = 8.75f;
 constexpr float kPOffset = 7.0f;
-constexpr float kIntBias = 12582912.0f;  // 1.5 * 2^23: float(kIntBias + s) has bits 0x4b400000 + s
-
-enum AbortCode {
-  kAbortQFull = 1, kAbortKvFull, kAbortKvEmpty, kAbortSFull, kAbortPFull, kAbortPEmpty,
-  kAbortPvDone, kAbortFinal
-};
-
-struct AttnParams {
-  const float *q_scale;
-  const float *k_scale;
-  const float *v_scale;
-  const int32_t *route;  // (heads, q_stop-q_start, route_len) or null
-  void *out;
-  int32_t *status;
-  int64_t out_stride_h, out_stride_s;
-  int route_len, q_start, q_stop;
-  int heads, sequence, q_tiles, kv_tiles;
-  int out_dtype;
-  // head-sharded runs: every output tile is also stored into these buffers
-  // (the same slice of each peer GPU's full output, reached over NVLink with
-  // plain stores), so no separate gather pass is needed
-  void *peer_out[H3S_MAX_PEER_OUTPUTS];
-  int n_peer_out;
-  // Bound of the waits for TMA loads; a wait further down the pipeline (QK^T
-  // result 2x, P 3x, P.V and free stages 4x) gets a multiple, so that when a
-  // stage stalls the wait closest to the cause is the one that runs out first
-  // and names it in the status words.
-  unsigned long long wait_budget_ns;
-  // self-test of the bounded waits (H3S_ATTN_TEST_DROP_KV_LOAD): the producer
-  // never issues the K/V load of this iteration, so the wait for it runs out
-  int drop_kv_load;                   // iteration index, -1 = none
-};
-
 struct AttnShared {
   uint64_t q_full;
   uint64_t kv_full[kStages];
@@ -93,47 +60,6 @@ struct AttnShared {
   float v_scale[H3S_HEAD_DIM];
 };
 static_assert(sizeof(AttnShared) <= 1024, "barrier block too large");
-
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Every lane polls the barrier; the warp then agrees on the outcome so that
-// the .sync.aligned tcgen05 instructions that follow stay convergent even if
-// the abort word was raised between two lanes' polls.
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_word, int code,
-                                          unsigned long long budget_ns) {
-  const bool ok = ptx::mbar_wait(bar, parity, abort_word, code, budget_ns);
-  return __all_sync(0xffffffffu, ok);
-}
-
-// packed fp32x2 arithmetic (one instruction for two lanes of a 64-bit register pair)
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long &>(d))
-      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)),
-        "l"(reinterpret_cast<unsigned long long &>(c)));
-  return d;
-}
-
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("mul.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<unsigned long long &>(d))
-      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
-  return d;
-}
-
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("add.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<unsigned long long &>(d))
-      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
-  return d;
-}
 
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
   uint16_t lo, hi;
@@ -185,30 +111,6 @@ __device__ __forceinline__ float exp_and_pack(const uint32_t (&s)[64], const Exp
     }
   }
   return sum2.x + sum2.y;
-}
-
-template <typename OutT> __device__ __forceinline__ void store_out8(OutT *dst, const float (&v)[8]);
-template <> __device__ __forceinline__ void store_out8<float>(float *dst, const float (&v)[8]) {
-  reinterpret_cast<float4 *>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-  reinterpret_cast<float4 *>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-}
-template <> __device__ __forceinline__ void store_out8<__nv_bfloat16>(__nv_bfloat16 *dst, const float (&v)[8]) {
-  uint4 w;
-  __nv_bfloat162 t;
-  t = __floats2bfloat162_rn(v[0], v[1]); w.x = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2bfloat162_rn(v[2], v[3]); w.y = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2bfloat162_rn(v[4], v[5]); w.z = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2bfloat162_rn(v[6], v[7]); w.w = *reinterpret_cast<uint32_t *>(&t);
-  *reinterpret_cast<uint4 *>(dst) = w;
-}
-template <> __device__ __forceinline__ void store_out8<__half>(__half *dst, const float (&v)[8]) {
-  uint4 w;
-  __half2 t;
-  t = __floats2half2_rn(v[0], v[1]); w.x = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2half2_rn(v[2], v[3]); w.y = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2half2_rn(v[4], v[5]); w.z = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2half2_rn(v[6], v[7]); w.w = *reinterpret_cast<uint32_t *>(&t);
-  *reinterpret_cast<uint4 *>(dst) = w;
 }
 
 template <typename OutT, bool kSplitP>
@@ -488,7 +390,6 @@ sparse_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       ptx::tc_fence_after();
       const float inv_l = 1.0f / l;
       constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
-      constexpr int kChunksPerRow = kRowBytes / 16;
       unsigned char *stage = smem + kOffK;
       static_assert(H3S_Q_TILE * kRowBytes <= kStages * (kKBytes + kVBytes), "output tile must fit the stage ring");
       unsigned char *my_row = stage + row * kRowBytes;
@@ -517,19 +418,7 @@ sparse_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
       ptx::tc_fence_before();
       __syncwarp();
-      const int warp_row0 = warp * 32;
-      unsigned char *base = static_cast<unsigned char *>(prm.out);
-#pragma unroll 4
-      for (int idx = lane; idx < 32 * kChunksPerRow; idx += 32) {
-        const int r = warp_row0 + idx / kChunksPerRow, c = idx % kChunksPerRow;
-        const int grow = tq * H3S_Q_TILE + r;
-        if (grow < prm.sequence) {
-          const uint4 value = *reinterpret_cast<const uint4 *>(stage + r * kRowBytes + ((c ^ (r & 15)) << 4));
-          unsigned char *dst = base + (head * prm.out_stride_h + static_cast<int64_t>(grow) * prm.out_stride_s) *
-                                          static_cast<int64_t>(sizeof(OutT)) + c * 16;
-          *reinterpret_cast<uint4 *>(dst) = value;
-        }
-      }
+      store_rows<OutT>(prm, stage, head, tq, warp * 32, 32, lane);
     }
   }
 
@@ -551,29 +440,8 @@ sparse_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, kTmemCols);
   }
-  // Head-sharded run: the finished tile, still staged in shared memory, goes to
-  // the same slice of every peer GPU's output with plain stores over NVLink.
-  // All six warps share the copy (the producer and MMA warps have nothing left
-  // to do), and each 16-byte chunk is sent to all peers back to back, so the
-  // stores of one CTA are spread over every link at once instead of filling
-  // one destination after the other.
-  if (code == 0 && prm.n_peer_out > 0) {
-    constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
-    constexpr int kChunksPerRow = kRowBytes / 16;
-    const unsigned char *stage = smem + kOffK;
-    const int64_t tile_offset = head * prm.out_stride_h * static_cast<int64_t>(sizeof(OutT));
-    for (int idx = threadIdx.x; idx < H3S_Q_TILE * kChunksPerRow; idx += kAttnThreads) {
-      const int r = idx / kChunksPerRow, c = idx % kChunksPerRow;
-      const int grow = tq * H3S_Q_TILE + r;
-      if (grow < prm.sequence) {
-        const uint4 value = *reinterpret_cast<const uint4 *>(stage + r * kRowBytes + ((c ^ (r & 15)) << 4));
-        const int64_t at = tile_offset + static_cast<int64_t>(grow) * prm.out_stride_s * static_cast<int64_t>(sizeof(OutT)) + c * 16;
-#pragma unroll
-        for (int d = 0; d < H3S_MAX_PEER_OUTPUTS; ++d)
-          if (d < prm.n_peer_out) *reinterpret_cast<uint4 *>(static_cast<unsigned char *>(prm.peer_out[d]) + at) = value;
-      }
-    }
-  }
+  // head-sharded run: the producer and MMA warps have nothing left to do and share the copy
+  if (code == 0 && prm.n_peer_out > 0) scatter_to_peers<OutT>(prm, smem + kOffK, head, tq, kAttnThreads);
 }
 
 template <typename OutT, bool kSplitP>
@@ -615,44 +483,24 @@ int check_attn_args(const int8_t *q8, const int8_t *k8, const uint8_t *v8t, cons
   return H3S_OK;
 }
 
-}  // namespace h3s
-
-namespace h3s {
-static int sparse_attn_fwd_impl(const int8_t *q8, const int8_t *k8, const uint8_t *v8t,
-                                const float *q_scale, const float *k_scale, const float *v_scale,
-                                const int32_t *route, int route_len, int q_start, int q_stop,
-                                void *out, void *const *peer_out, int n_peer_out, int out_dtype,
-                                int64_t out_stride_h, int64_t out_stride_s,
-                                int heads, int sequence, int flags, int32_t *status,
-                                h3s_stream_t stream) {
+int fill_attn_params(AttnParams *params, const int8_t *q8, const int8_t *k8, const void *v, const float *q_scale,
+                     const float *k_scale, const float *v_scale, const int32_t *route, int route_len, int q_start,
+                     int q_stop, void *out, void *const *peer_out, int n_peer_out, int out_dtype, int64_t out_stride_h,
+                     int64_t out_stride_s, int heads, int sequence, int flags, int32_t *status, const char *who) {
   H3S_CHECK_ARG(n_peer_out >= 0 && n_peer_out <= H3S_MAX_PEER_OUTPUTS && (n_peer_out == 0 || peer_out != nullptr),
-                "sparse_attn_fwd: %d peer outputs (at most %d)", n_peer_out, H3S_MAX_PEER_OUTPUTS);
+                "%s: %d peer outputs (at most %d)", who, n_peer_out, H3S_MAX_PEER_OUTPUTS);
   for (int i = 0; i < n_peer_out; ++i)
     H3S_CHECK_ARG(peer_out[i] != nullptr && (reinterpret_cast<uintptr_t>(peer_out[i]) & 15) == 0,
-                  "sparse_attn_fwd: peer output %d is NULL or not 16-byte aligned", i);
+                  "%s: peer output %d is NULL or not 16-byte aligned", who, i);
   {
-    int rc = check_attn_args(q8, k8, v8t, q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out,
-                             out_dtype, out_stride_h, out_stride_s, heads, sequence, "sparse_attn_fwd");
+    int rc = check_attn_args(q8, k8, static_cast<const uint8_t *>(v), q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out,
+                             out_dtype, out_stride_h, out_stride_s, heads, sequence, who);
     if (rc) return rc;
   }
   const int cap = h3s_device_capability();
   if (cap < 0) return cap;
-  if (cap / 10 != 10) return fail(H3S_EARCH, "sparse_attn_fwd: needs an sm_100 device, found sm_%d", cap);
-
-  const uint64_t S = static_cast<uint64_t>(sequence);
-  const uint64_t padded = static_cast<uint64_t>(ceil_div(sequence, 128)) * 128;
-  CUtensorMap mq, mk, mv;
-  int rc = make_tensor_map_u8_3d(&mq, q8, H3S_HEAD_DIM, S, heads, H3S_HEAD_DIM, S * H3S_HEAD_DIM,
-                                 H3S_HEAD_DIM, H3S_Q_TILE, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_fwd Q map");
-  if (rc) return rc;
-  rc = make_tensor_map_u8_3d(&mk, k8, H3S_HEAD_DIM, S, heads, H3S_HEAD_DIM, S * H3S_HEAD_DIM, H3S_HEAD_DIM,
-                             H3S_KV_TILE, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_fwd K map");
-  if (rc) return rc;
-  rc = make_tensor_map_u8_3d(&mv, v8t, padded, H3S_HEAD_DIM, heads, padded, padded * H3S_HEAD_DIM,
-                             H3S_KV_TILE, H3S_HEAD_DIM, CU_TENSOR_MAP_SWIZZLE_64B, "sparse_attn_fwd V map");
-  if (rc) return rc;
-
-  AttnParams prm;
+  if (cap / 10 != 10) return fail(H3S_EARCH, "%s: needs an sm_100 device, found sm_%d", who, cap);
+  AttnParams &prm = *params;
   prm.q_scale = q_scale; prm.k_scale = k_scale; prm.v_scale = v_scale;
   prm.route = route; prm.out = out; prm.status = status;
   prm.out_stride_h = out_stride_h; prm.out_stride_s = out_stride_s;
@@ -664,6 +512,34 @@ static int sparse_attn_fwd_impl(const int8_t *q8, const int8_t *k8, const uint8_
   prm.wait_budget_ns = wait_budget_ns();
   prm.drop_kv_load = (flags & H3S_ATTN_TEST_DROP_KV_LOAD) ? 0 : -1;
   for (int i = 0; i < H3S_MAX_PEER_OUTPUTS; ++i) prm.peer_out[i] = i < n_peer_out ? peer_out[i] : nullptr;
+  return H3S_OK;
+}
+
+static int sparse_attn_fwd_impl(const int8_t *q8, const int8_t *k8, const uint8_t *v8t,
+                                const float *q_scale, const float *k_scale, const float *v_scale,
+                                const int32_t *route, int route_len, int q_start, int q_stop,
+                                void *out, void *const *peer_out, int n_peer_out, int out_dtype,
+                                int64_t out_stride_h, int64_t out_stride_s,
+                                int heads, int sequence, int flags, int32_t *status,
+                                h3s_stream_t stream) {
+  AttnParams prm;
+  int rc = fill_attn_params(&prm, q8, k8, v8t, q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out, peer_out,
+                            n_peer_out, out_dtype, out_stride_h, out_stride_s, heads, sequence, flags, status,
+                            "sparse_attn_fwd");
+  if (rc) return rc;
+  const uint64_t S = static_cast<uint64_t>(sequence);
+  const uint64_t padded = static_cast<uint64_t>(ceil_div(sequence, 128)) * 128;
+  CUtensorMap mq, mk, mv;
+  rc = make_tensor_map_u8_3d(&mq, q8, H3S_HEAD_DIM, S, heads, H3S_HEAD_DIM, S * H3S_HEAD_DIM,
+                                 H3S_HEAD_DIM, H3S_Q_TILE, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_fwd Q map");
+  if (rc) return rc;
+  rc = make_tensor_map_u8_3d(&mk, k8, H3S_HEAD_DIM, S, heads, H3S_HEAD_DIM, S * H3S_HEAD_DIM, H3S_HEAD_DIM,
+                             H3S_KV_TILE, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_fwd K map");
+  if (rc) return rc;
+  rc = make_tensor_map_u8_3d(&mv, v8t, padded, H3S_HEAD_DIM, heads, padded, padded * H3S_HEAD_DIM,
+                             H3S_KV_TILE, H3S_HEAD_DIM, CU_TENSOR_MAP_SWIZZLE_64B, "sparse_attn_fwd V map");
+  if (rc) return rc;
+
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool split_p = (flags & H3S_ATTN_P_SINGLE) == 0;
   switch (out_dtype) {

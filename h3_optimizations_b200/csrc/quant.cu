@@ -239,8 +239,8 @@ __device__ __forceinline__ int v_tile_offset(int d, int s) {
 template <typename T>
 __global__ void __launch_bounds__(kVThreads)
 quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
-                   const float *__restrict__ v_scale, uint8_t *__restrict__ out, int rows,
-                   int row_start, int padded_total, float v_bound) {
+                   const float *__restrict__ v_scale, uint8_t *__restrict__ out, uint16_t *__restrict__ out_half,
+                   int rows, int row_start, int padded_total, float v_bound) {
   __shared__ __align__(16) uint8_t tile[H3S_HEAD_DIM * kVTile];
   const int head = blockIdx.y;
   const int first_row = blockIdx.x * kVTile;
@@ -305,13 +305,20 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
   };
   if (all_exact) fill(std::true_type{}); else fill(std::false_type{});
   __syncthreads();
-  uint8_t *dst = out + static_cast<int64_t>(head) * H3S_HEAD_DIM * padded_total + row_start + first_row;
+  const int64_t base_at = static_cast<int64_t>(head) * H3S_HEAD_DIM * padded_total + row_start + first_row;
 #pragma unroll
   for (int p = 0; p < H3S_HEAD_DIM / (kVThreads / 8); ++p) {
     const int d = p * (kVThreads / 8) + (threadIdx.x >> 3);
     const int chunk = threadIdx.x & 7;
     const uint4 data = *reinterpret_cast<const uint4 *>(&tile[v_tile_offset(d, chunk * 16)]);
-    *reinterpret_cast<uint4 *>(dst + static_cast<int64_t>(d) * padded_total + chunk * 16) = data;
+    const int64_t at = base_at + static_cast<int64_t>(d) * padded_total + chunk * 16;
+    *reinterpret_cast<uint4 *>(out + at) = data;
+    if (out_half != nullptr) {  // the copy the attention kernel multiplies with BF16 probabilities
+      uint4 half[2];
+      e4m3x16_to_bf16(data, half);
+      *reinterpret_cast<uint4 *>(out_half + at) = half[0];
+      *reinterpret_cast<uint4 *>(out_half + at + 8) = half[1];
+    }
   }
 }
 
@@ -432,7 +439,7 @@ static int launch_quant_qk(const void *x, int64_t sh, int64_t ss, const float *m
 
 template <typename T>
 static int launch_quant_v(const void *v, int64_t sh, int64_t ss, const float *v_scale, uint8_t *out,
-                          int heads, int rows, int row_start, int sequence_total, float v_bound,
+                          uint16_t *out_half, int heads, int rows, int row_start, int sequence_total, float v_bound,
                           cudaStream_t stream) {
   const int padded_total = ceil_div(sequence_total, 128) * 128;
   // the final chunk also writes the zero padding up to the carrier's end
@@ -440,7 +447,7 @@ static int launch_quant_v(const void *v, int64_t sh, int64_t ss, const float *v_
   const int covered = last ? padded_total - row_start : rows;
   dim3 grid(ceil_div(covered, kVTile), heads);
   quant_v_fp8_kernel<T><<<grid, kVThreads, 0, stream>>>(static_cast<const T *>(v), sh, ss, v_scale, out,
-                                                        rows, row_start, padded_total, v_bound);
+                                                        out_half, rows, row_start, padded_total, v_bound);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
 }
@@ -577,6 +584,13 @@ int h3s_quant_qk_blocks(const void *x, int dtype, int64_t x_stride_h, int64_t x_
 int h3s_quant_v_fp8(const void *v, int dtype, int64_t v_stride_h, int64_t v_stride_s,
                     const float *v_scale, uint8_t *out, int heads, int rows, int row_start,
                     int sequence_total, float v_bound, h3s_stream_t stream) {
+  return h3s_quant_v_fp8_half(v, dtype, v_stride_h, v_stride_s, v_scale, out, nullptr, heads, rows, row_start,
+                              sequence_total, v_bound, stream);
+}
+
+int h3s_quant_v_fp8_half(const void *v, int dtype, int64_t v_stride_h, int64_t v_stride_s, const float *v_scale,
+                         uint8_t *out, void *out_half, int heads, int rows, int row_start, int sequence_total,
+                         float v_bound, h3s_stream_t stream) {
   using namespace h3s;
   H3S_CHECK_ARG(heads > 0 && rows > 0 && sequence_total > 0, "quant_v_fp8: empty problem");
   H3S_CHECK_ARG(row_start >= 0 && row_start % 128 == 0, "quant_v_fp8: row_start %d must be 128 aligned", row_start);
@@ -584,14 +598,15 @@ int h3s_quant_v_fp8(const void *v, int dtype, int64_t v_stride_h, int64_t v_stri
   H3S_CHECK_ARG(rows % 128 == 0 || row_start + rows == sequence_total,
                 "quant_v_fp8: only the final chunk may contain a partial tile");
   H3S_CHECK_ARG(v != nullptr && v_scale != nullptr && out != nullptr, "quant_v_fp8: NULL pointer");
-  H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(out) & 15) == 0, "quant_v_fp8: out must be 16-byte aligned");
+  H3S_CHECK_ARG(((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_half)) & 15) == 0, "quant_v_fp8: outputs must be 16-byte aligned");
+  uint16_t *half = static_cast<uint16_t *>(out_half);
   H3S_CHECK_ARG(v_bound > 0.f, "quant_v_fp8: v_bound must be positive");
   { int rc = check_view(v, dtype, v_stride_h, v_stride_s, "quant_v_fp8 v"); if (rc) return rc; }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case H3S_F32: return launch_quant_v<float>(v, v_stride_h, v_stride_s, v_scale, out, heads, rows, row_start, sequence_total, v_bound, s);
-    case H3S_BF16: return launch_quant_v<__nv_bfloat16>(v, v_stride_h, v_stride_s, v_scale, out, heads, rows, row_start, sequence_total, v_bound, s);
-    default: return launch_quant_v<__half>(v, v_stride_h, v_stride_s, v_scale, out, heads, rows, row_start, sequence_total, v_bound, s);
+    case H3S_F32: return launch_quant_v<float>(v, v_stride_h, v_stride_s, v_scale, out, half, heads, rows, row_start, sequence_total, v_bound, s);
+    case H3S_BF16: return launch_quant_v<__nv_bfloat16>(v, v_stride_h, v_stride_s, v_scale, out, half, heads, rows, row_start, sequence_total, v_bound, s);
+    default: return launch_quant_v<__half>(v, v_stride_h, v_stride_s, v_scale, out, half, heads, rows, row_start, sequence_total, v_bound, s);
   }
 }
 

@@ -183,7 +183,8 @@ def allocate_v_carrier(sequence, heads, device):
     return torch.empty((1, int(heads), HEAD_DIM, padded), dtype=torch.float8_e4m3fn, device=device)
 
 
-def quant_v_fp8_into(v, v_scale, carrier, *, row_start=0, sequence_total=None, v_bound=FP8_V_BOUND):
+def quant_v_fp8_into(v, v_scale, carrier, *, row_start=0, sequence_total=None, v_bound=FP8_V_BOUND, half=None):
+    """``half``: optional bf16 tensor shaped like ``carrier`` that receives the codes' values."""
     lib = _native.load()
     heads, rows = _hnd(v, "quant_v_fp8 input")
     sequence_total = int(sequence_total if sequence_total is not None else row_start + rows)
@@ -193,9 +194,11 @@ def quant_v_fp8_into(v, v_scale, carrier, *, row_start=0, sequence_total=None, v
         raise _native.NativeError("quant_v_fp8: carrier must be contiguous e4m3 (1,H,128,%d)" % padded)
     if tuple(v_scale.shape) != (1, heads, HEAD_DIM) or v_scale.dtype != torch.float32 or not v_scale.is_contiguous():
         raise _native.NativeError("quant_v_fp8: scale must be contiguous fp32 (1,H,128)")
+    if half is not None and (half.shape != carrier.shape or half.dtype != torch.bfloat16 or not half.is_contiguous()):
+        raise _native.NativeError("quant_v_fp8: half must be a contiguous bf16 tensor shaped like the carrier")
     check(
-        lib.h3s_quant_v_fp8(
-            ptr(v), dtype_code(v.dtype), v.stride(1), v.stride(2), ptr(v_scale), ptr(carrier), heads, rows,
+        lib.h3s_quant_v_fp8_half(
+            ptr(v), dtype_code(v.dtype), v.stride(1), v.stride(2), ptr(v_scale), ptr(carrier), ptr(half), heads, rows,
             int(row_start), sequence_total, float(v_bound), stream_ptr(v.device),
         ),
         "h3s_quant_v_fp8",
@@ -486,6 +489,16 @@ def _attn_args(q8, k8, v_carrier, q_scale, k_scale, v_scale, route, q_start, q_s
     return heads, sequence, route_len
 
 
+def v_half_copy(v_carrier):
+    """The V carrier ``(1,H,128,pad128(S))`` as BF16 (exact), which the attention kernel multiplies with BF16
+    probabilities."""
+    lib = _native.load()
+    out = torch.empty(v_carrier.shape, dtype=torch.bfloat16, device=v_carrier.device)
+    check(lib.h3s_v_half(ptr(v_carrier), ptr(out), v_carrier.shape[1], v_carrier.shape[3], stream_ptr(v_carrier.device)),
+          "h3s_v_half")
+    return out
+
+
 def new_attention_output(heads, sequence, dtype, device):
     """HND view of a token-major ``(S, H*128)`` buffer, so the caller's
     transpose+reshape before ``out_proj`` (attention_forward.py:123-128) is free."""
@@ -495,9 +508,11 @@ def new_attention_output(heads, sequence, dtype, device):
 
 def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *, q_start=0, q_stop=0,
                      out=None, out_dtype=torch.bfloat16, status=None, legacy_mma=False, single_term_p=False,
-                     peer_out_ptrs=None, extra_flags=0):
+                     peer_out_ptrs=None, extra_flags=0, v_half=None):
     """Launch the attention kernel.  Returns ``out`` (HND).  ``single_term_p``
-    carries the probabilities as one E4M3 term instead of hi + lo.
+    carries the probabilities as one E4M3 term instead of in BF16.
+    ``v_half``: the BF16 copy of the V carrier (``v_half_copy``) where the caller
+    keeps one; made here otherwise.
     ``peer_out_ptrs``: device addresses (ints) of up to 7 further buffers,
     addressed like ``out``, that receive every output tile as well (the slices
     of the peer GPUs' full outputs in a head-sharded run)."""
@@ -505,23 +520,23 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
     if out is None:
         out = new_attention_output(q8.shape[1], q8.shape[2], out_dtype, q8.device)
     heads, sequence, route_len = _attn_args(q8, k8, v_carrier, q_scale, k_scale, v_scale, route, q_start, q_stop, out)
-    common = (
-        ptr(q8), ptr(k8), ptr(v_carrier), ptr(q_scale), ptr(k_scale), ptr(v_scale), ptr(route), route_len,
-        int(q_start), int(q_stop), ptr(out), dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence,
-    )
     flags = (ATTN_P_SINGLE if single_term_p else 0) | int(extra_flags)
-    if peer_out_ptrs:
+    table, n_peers = None, len(peer_out_ptrs or ())
+    if n_peers:
         if legacy_mma:
             raise _native.NativeError("sparse_attention: the cross-check kernel does not scatter to peers")
-        table = (ctypes.c_void_p * len(peer_out_ptrs))(*[ctypes.c_void_p(int(p)) for p in peer_out_ptrs])
-        check(
-            lib.h3s_sparse_attn_fwd_scatter(*common[:11], table, len(peer_out_ptrs), *common[11:], flags,
-                                            ptr(status), stream_ptr(q8.device)),
-            "h3s_sparse_attn_fwd_scatter",
-        )
-        return out
+        table = (ctypes.c_void_p * n_peers)(*[ctypes.c_void_p(int(p)) for p in peer_out_ptrs])
+    before = (ptr(q_scale), ptr(k_scale), ptr(v_scale), ptr(route), route_len, int(q_start), int(q_stop), ptr(out))
+    after = (dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence, flags)
+    stream = stream_ptr(q8.device)
     if legacy_mma:
-        check(lib.h3s_sparse_attn_fwd_mma(*common, flags, stream_ptr(q8.device)), "h3s_sparse_attn_fwd_mma")
+        check(lib.h3s_sparse_attn_fwd_mma(ptr(q8), ptr(k8), ptr(v_carrier), *before, *after, stream), "h3s_sparse_attn_fwd_mma")
+    elif single_term_p:
+        check(lib.h3s_sparse_attn_fwd_scatter(ptr(q8), ptr(k8), ptr(v_carrier), *before, table, n_peers, *after,
+                                              ptr(status), stream), "h3s_sparse_attn_fwd_scatter")
     else:
-        check(lib.h3s_sparse_attn_fwd(*common, flags, ptr(status), stream_ptr(q8.device)), "h3s_sparse_attn_fwd")
+        if v_half is None:
+            v_half = v_half_copy(v_carrier)
+        check(lib.h3s_sparse_attn_half_fwd(ptr(q8), ptr(k8), ptr(v_half), *before, table, n_peers, *after,
+                                           ptr(status), stream), "h3s_sparse_attn_half_fwd")
     return out

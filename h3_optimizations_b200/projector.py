@@ -176,6 +176,7 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
         k_mean, v_scale = ops.column_stats_finalize(stats, heads, sequence, want_k_mean=smooth_k,
                                                     dtype=torch.bfloat16, v_bound=V_QUANT_BOUND)
         v_carrier = ops.allocate_v_carrier(sequence, heads, device)
+        v_half = torch.empty(v_carrier.shape, dtype=torch.bfloat16, device=device)
         if smooth_k:
             # the two second-phase quantisers are independent and each leaves part of the
             # memory system idle: V runs on a second stream underneath K
@@ -183,12 +184,12 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
             side.wait_stream(main)
             try:
                 with torch.cuda.stream(side):
-                    ops.quant_v_fp8_into(v_stage, v_scale, v_carrier, v_bound=V_QUANT_BOUND)
+                    ops.quant_v_fp8_into(v_stage, v_scale, v_carrier, v_bound=V_QUANT_BOUND, half=v_half)
                 ops.quant_qk_blocks_into(k_stage, k_int8, k_scale, None, block=KV_TILE, mean=k_mean)
             finally:
                 main.wait_stream(side)  # on every exit path, before the staging can be freed
         else:
-            ops.quant_v_fp8_into(v_stage, v_scale, v_carrier, v_bound=V_QUANT_BOUND)
+            ops.quant_v_fp8_into(v_stage, v_scale, v_carrier, v_bound=V_QUANT_BOUND, half=v_half)
     except _native.NativeError as exc:
         raise FusedQKVError("chunked QKV projection failed: layer=%d: %s" % (layer_index, exc)) from exc
     return validate_prepared_fused_qkv(
@@ -196,6 +197,6 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
             q_int8=q_int8, q_scale=q_scale, k_int8=k_int8, k_scale=k_scale, v=None,
             q_summary=q_summary, k_summary=k_summary, output_dtype=x.dtype, sequence=sequence,
             heads=heads, head_dim=HEAD_DIM, layer_index=int(layer_index), smooth_k=bool(smooth_k),
-            v_carrier=v_carrier, v_scale=v_scale,
+            v_carrier=v_carrier, v_scale=v_scale, v_half=v_half,
         )
     )
