@@ -181,6 +181,82 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {
                : "memory");
 }
 
+// ---- clusters of two CTAs (cta_group::2) -------------------------------------
+// A kernel uses either the cta_group::1 calls or these, never both.
+
+__device__ __forceinline__ int cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return static_cast<int>(r);
+}
+
+// Whole cluster: every thread of both CTAs.
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Address, within the cluster, of CTA `rank`'s copy of a shared-memory object
+__device__ __forceinline__ uint32_t cluster_address(const void *local, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+  return a;
+}
+
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t address) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(address) : "memory");
+}
+
+// Load into this CTA's shared memory, completion counted on a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+
+// One warp of each CTA of the pair, both with the same arguments.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t *slot, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(columns)
+               : "memory");
+}
+
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t base, uint32_t columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
+}
+
+// Arrives once on the barrier at this offset in BOTH CTAs when the MMAs issued so far have completed.
+__device__ __forceinline__ void tc_commit_pair(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_u32(bar)),
+               "h"(static_cast<uint16_t>(3))
+               : "memory");
+}
+
+#define H3S_UMMA_PAIR(name, kind)                                                                        \
+  __device__ __forceinline__ void name(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, \
+                                       uint32_t accumulate) {                                            \
+    asm volatile(                                                                                        \
+        "{\n\t"                                                                                          \
+        ".reg .pred p;\n\t"                                                                              \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                                      \
+        "tcgen05.mma.cta_group::2.kind::" kind " [%0], %1, %2, %3, p;\n\t"                              \
+        "}\n" ::"r"(d_tmem),                                                                             \
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)                                            \
+        : "memory");                                                                                     \
+  }
+// M = 256: rows 0-127 of A and D belong to the first CTA, 128-255 to the second; each
+// CTA's shared memory holds half of B's rows.  Issued by one thread of the first CTA.
+H3S_UMMA_PAIR(umma_i8_pair, "i8")
+H3S_UMMA_PAIR(umma_f8_pair, "f8f6f4")
+H3S_UMMA_PAIR(umma_f16_pair, "f16")
+#undef H3S_UMMA_PAIR
+
 // ---- tcgen05: descriptors ---------------------------------------------------
 
 // Shared-memory matrix descriptor, K-major operand, rows packed at the

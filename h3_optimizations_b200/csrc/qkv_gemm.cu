@@ -6,9 +6,10 @@
 //                        HBM-bound, one warp per 256-channel group.
 //   qkv_gemm_chunk     : persistent warp-specialised tcgen05 GEMM
 //                        acc[rows, n] = x_i8 . w_i8^T (kind::i8, int32 in TMEM),
-//                        128x256 tiles, K step 128 bytes (SWIZZLE_128B), 4-stage
-//                        TMA ring, two TMEM accumulators so the epilogue of one
-//                        tile overlaps the MMAs of the next.  The epilogue
+//                        256x256 tiles on a pair of SMs (cta_group::2), K step 128
+//                        bytes (SWIZZLE_128B), TMA ring, two TMEM accumulators so
+//                        the epilogue of one tile overlaps the MMAs of the next.
+//                        The epilogue
 //                        de-quantises (acc * (x_scale[row] * w_scale[col])), rounds
 //                        to bf16 and scatters into head-major (3*H, rows, 128)
 //                        staging that the carrier kernels consume.
@@ -114,14 +115,27 @@ convrot_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_stride,
 // INT8 GEMM
 // ---------------------------------------------------------------------------
 
-constexpr int kGemmM = 128, kGemmN = 256, kGemmK = 128;  // K in bytes == int8 elements
+// One tile is 256 x 256, computed by a cluster of two CTAs on neighbouring SMs: each CTA
+// holds the accumulators of its own 128 rows x 256 columns, loads its 128 rows of A and
+// HALF of B's 256 rows, and the first CTA issues the MMAs of both (cta_group::2).  A
+// 128x256 tile per SM pulled 48 KB through L2 for every 512 cycles of MMA work, 96 bytes
+// a clock and SM, which is more than L2 delivers to all SMs at once; the pair needs 64,
+// and the smaller stages leave room for one more.  MLP of 33272 x 3072 x 12288: 3.59 ->
+// 3.06 ms (with gelu_tanh below), of 1000 tokens 147 -> 120 us; attention block of 33272
+// tokens 6.09 -> 5.91 ms.  A single row tile wastes half a pair, but what such a call
+// waits for is the weights, which are read once either way.
+constexpr int kGemmM = 128, kGemmN = 256, kGemmK = 128;  // per CTA; K in bytes == int8 elements
+constexpr int kGemmPairM = 2 * kGemmM;
+// Row pairs visited before the next column of tiles: 4096 rows of A (12 to 50 MB) and the
+// weights stay in L2 while every column passes over them.
+constexpr int kGemmGroupM = 16;
 // warps 0-3: epilogue of the tile's first 128 columns, 4: TMA, 5: MMA, 6-7: idle,
 // 8-11: epilogue of the second 128 columns (a warp may only touch the TMEM lanes
 // 32*(warp%4)..: two warps per lane quarter halve the epilogue's time, which
 // exceeds the MMA time of a tile once the norm and the rotation run in it)
 constexpr int kGemmThreads = 384;
 constexpr uint32_t kGemmABytes = kGemmM * kGemmK;  // 16384
-constexpr uint32_t kGemmBBytes = kGemmN * kGemmK;  // 32768
+constexpr uint32_t kGemmBBytes = kGemmN / 2 * kGemmK;  // 16384: this CTA's half
 constexpr uint32_t kGemmTmemCols = 512;
 
 // What the eight 16-thread row slots of one 128-column half of a tile tell each
@@ -136,7 +150,7 @@ constexpr uint32_t kEpilogueTileBytes = kGemmM * H3S_HEAD_DIM * 2;  // one half 
 // Shared-memory layout.  The carrier epilogue stages each half tile as bf16 so
 // that it can be re-read column-wise (quantisation, statistics and every global
 // store then run on contiguous lines); it pays for the two 32 KB staging tiles
-// with one stage of the operand ring.
+// with stages of the operand ring.
 // Epilogue of the GEMM kernel
 enum GemmMode {
   kModeStaging = 0,   // INT8 x INT8 -> bf16 head-major staging (h3s_qkv_gemm_chunk[_norm_rope])
@@ -147,23 +161,24 @@ enum GemmMode {
 template <int kMode>
 struct GemmLayout {
   static constexpr bool kCarriers = kMode != kModeStaging;  // both stage half tiles for coalesced stores
-  static constexpr int kStages = kCarriers ? 3 : 4;
+  static constexpr int kStages = kMode == kModeStaging ? 6 : kMode == kModeDense ? 5 : 4;
   static constexpr uint32_t kOffB = kStages * kGemmABytes;
   static constexpr uint32_t kOffTile = kOffB + kStages * kGemmBBytes;
   static constexpr uint32_t kOffExchange = kOffTile + (kCarriers ? 2 * kEpilogueTileBytes : 0);
-  static constexpr uint32_t kOffBar = kOffExchange + (kCarriers ? 2 * sizeof(EpilogueExchange) : 0);
+  static constexpr uint32_t kOffBar = kOffExchange + (kMode == kModeCarriers ? 2 * sizeof(EpilogueExchange) : 0);
   static constexpr uint32_t kBytes = kOffBar + 256 + 1024;
+  static_assert(sizeof(uint64_t) * (2 * 6 + 8) + 8 <= 256, "barriers");
   static_assert(kBytes <= 227 * 1024, "GEMM shared memory exceeds the per-CTA limit");
 };
-constexpr int kGemmMaxStages = 4;
+constexpr int kGemmMaxStages = 6;
 
 enum GemmAbort { kGemmAbortFull = 21, kGemmAbortEmpty, kGemmAbortAccFull, kGemmAbortAccEmpty, kGemmAbortTile, kGemmAbortExchange };
 
 struct GemmShared {
-  uint64_t full[kGemmMaxStages];
-  uint64_t empty[kGemmMaxStages];
-  uint64_t acc_full[2];
-  uint64_t acc_empty[2];
+  uint64_t full[kGemmMaxStages];   // first CTA's: the stage's four loads, two by each CTA
+  uint64_t empty[kGemmMaxStages];  // both CTAs': the pair's MMAs have read the stage
+  uint64_t acc_full[2];            // both CTAs'
+  uint64_t acc_empty[2];           // first CTA's: sixteen epilogue warps, eight in each CTA
   uint64_t tile_ready[2];      // per tile half: its four warps have staged their rows
   uint64_t exchange_ready[2];  // per tile half: its four warps have written their EpilogueExchange
   uint32_t tmem_base;
@@ -177,7 +192,7 @@ struct GemmParams {
   int64_t out_stride_head;  // elements between consecutive 128-column groups
   int32_t *status;
   int rows, n_out, hidden;
-  int m_tiles, n_tiles;
+  int m_pairs, n_tiles;  // pairs of 128-row tiles, 256-column tiles
   // Column tiles are visited in the order (i * n_step) % n_tiles (n_step coprime with
   // n_tiles, about a third of it): weight rows are ordered [Q | K | V], so consecutive
   // tiles of a CTA alternate between the three kinds and the costlier epilogues of
@@ -211,9 +226,21 @@ struct GemmParams {
 };
 
 __device__ __forceinline__ float gelu_tanh(float x) {
-  // 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3))), the formula of torch's approximate='tanh'
-  const float inner = 0.7978845608028654f * __fmaf_rn(0.044715f * x, x * x, x);
-  return 0.5f * x * (1.0f + tanhf(inner));
+  // 0.5 x (1 + tanh(u)), u = sqrt(2/pi) (x + 0.044715 x^3), the formula of torch's approximate='tanh',
+  // as x / (1 + exp(-2u)): nine instructions, and nothing cancels for negative x, where
+  // 1 + tanh(u) loses all but a few bits
+  const float t = (-2.0f * 0.7978845608028654f * 1.4426950408889634f) * __fmaf_rn(0.044715f * x, x * x, x);
+  float e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+  return __fdividef(x, 1.0f + e);
+}
+
+// Four consecutive floats of a per-column vector; n_out is a multiple of 8, so a group of
+// four lies inside or outside as a whole
+__device__ __forceinline__ float4 column4(const float *base, int col, int n_out, float otherwise) {
+  if (base == nullptr || col >= n_out) return make_float4(otherwise, otherwise, otherwise, otherwise);
+  if ((reinterpret_cast<uintptr_t>(base) & 15) == 0) return __ldg(reinterpret_cast<const float4 *>(base + col));
+  return make_float4(__ldg(base + col), __ldg(base + col + 1), __ldg(base + col + 2), __ldg(base + col + 3));
 }
 
 __device__ __forceinline__ float rope_load(const void *base, int64_t index, int dtype) {
@@ -327,8 +354,19 @@ __device__ __forceinline__ void norm_rope_row(uint32_t (&y)[H3S_HEAD_DIM / 2], c
   }
 }
 
+// Tile `tile` of the persistent order: row pair and column tile
+__device__ __forceinline__ void tile_position(const GemmParams &prm, int tile, int &pair, int &tn) {
+  const int per_group = kGemmGroupM * prm.n_tiles;
+  const int group = tile / per_group, within = tile - group * per_group;
+  const int first = group * kGemmGroupM;
+  const int height = min(kGemmGroupM, prm.m_pairs - first);
+  const int column = within / height;
+  pair = first + within - column * height;
+  tn = column * prm.n_step % prm.n_tiles;
+}
+
 template <int kMode>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const GemmParams prm) {
   extern __shared__ unsigned char smem_dyn[];
@@ -340,7 +378,9 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   volatile int *abort_word = &sh.abort_word;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_steps = prm.hidden / kGemmK;
-  const int total_tiles = prm.m_tiles * prm.n_tiles;
+  const int total_tiles = prm.m_pairs * prm.n_tiles;
+  const int rank = ptx::cluster_rank();  // 0: issues the pair's MMAs
+  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < L::kStages; ++i) {
@@ -349,7 +389,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&sh.acc_full[i], 1);
-      ptx::mbar_init(&sh.acc_empty[i], 8);
+      ptx::mbar_init(&sh.acc_empty[i], 16);
       ptx::mbar_init(&sh.tile_ready[i], 4);
       ptx::mbar_init(&sh.exchange_ready[i], 4);
     }
@@ -357,11 +397,12 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     ptx::fence_mbar_init();
   }
   if (warp == 5) {
-    ptx::tmem_alloc(&sh.tmem_base, kGemmTmemCols);
-    ptx::tmem_relinquish();
+    ptx::tmem_alloc_pair(&sh.tmem_base, kGemmTmemCols);
+    ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before();
   __syncthreads();
+  ptx::cluster_sync();  // both CTAs' barriers are initialised
   ptx::tc_fence_after();
   const uint32_t tmem_base = sh.tmem_base;
 
@@ -371,29 +412,36 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       ptx::prefetch_tensormap(&map_b);
       uint32_t it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-        const int tm = tile % prm.m_tiles, tn = (tile / prm.m_tiles) * prm.n_step % prm.n_tiles;
+      for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step) {
+        int pair, tn;
+        tile_position(prm, tile, pair, tn);
+        const int row0 = pair * kGemmPairM + rank * kGemmM, col0 = tn * kGemmN + rank * (kGemmN / 2);
         for (int ks = 0; ks < k_steps; ++ks, ++it) {
           const int s = it % L::kStages;
           const uint32_t use = it / L::kStages;
           if (!ptx::mbar_wait(&sh.empty[s], (use & 1u) ^ 1u, abort_word, kGemmAbortEmpty, prm.wait_budget_ns)) { ok = false; break; }
-          ptx::mbar_arrive_expect_tx(&sh.full[s], kGemmABytes + kGemmBBytes);
-          ptx::tma_load_2d(smem + s * kGemmABytes, &map_a, &sh.full[s], ks * kGemmK, tm * kGemmM);
-          ptx::tma_load_2d(smem + L::kOffB + s * kGemmBBytes, &map_b, &sh.full[s], ks * kGemmK, tn * kGemmN);
+          // all four loads of the pair count on the first CTA's barrier
+          const uint32_t full = ptx::cluster_address(&sh.full[s], 0);
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&sh.full[s], 2 * (kGemmABytes + kGemmBBytes));
+          ptx::tma_load_2d_pair(smem + s * kGemmABytes, &map_a, full, ks * kGemmK, row0);
+          ptx::tma_load_2d_pair(smem + L::kOffB + s * kGemmBBytes, &map_b, full, ks * kGemmK, col0);
         }
       }
+      // the other CTA's last arrivals on `empty` have landed before this CTA may exit
+      for (uint32_t i = it > L::kStages ? it - L::kStages : 0; ok && i < it; ++i)
+        ok = ptx::mbar_wait(&sh.empty[i % L::kStages], (i / L::kStages) & 1u, abort_word, kGemmAbortEmpty, prm.wait_budget_ns);
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {
       // every kind consumes 32 bytes of K per instruction: four instructions per 128-byte stage
       const int kind = kMode == kModeDense ? prm.operand_kind : H3S_GEMM_I8;
-      const uint32_t idesc = kind == H3S_GEMM_I8     ? ptx::umma_idesc(2, 1, 1, kGemmM, kGemmN)
-                             : kind == H3S_GEMM_E4M3 ? ptx::umma_idesc(1, 0, 0, kGemmM, kGemmN)
-                             : kind == H3S_GEMM_BF16 ? ptx::umma_idesc(1, 1, 1, kGemmM, kGemmN)
-                                                     : ptx::umma_idesc(1, 0, 0, kGemmM, kGemmN);
+      const uint32_t idesc = kind == H3S_GEMM_I8     ? ptx::umma_idesc(2, 1, 1, kGemmPairM, kGemmN)
+                             : kind == H3S_GEMM_E4M3 ? ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN)
+                             : kind == H3S_GEMM_BF16 ? ptx::umma_idesc(1, 1, 1, kGemmPairM, kGemmN)
+                                                     : ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN);
       uint32_t it = 0, local = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++local) {
+      for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step, ++local) {
         const int a = local & 1;
         const uint32_t acc_use = local >> 1;
         if (!ptx::mbar_wait(&sh.acc_empty[a], (acc_use & 1u) ^ 1u, abort_word, kGemmAbortAccEmpty, prm.wait_budget_ns)) { ok = false; break; }
@@ -409,19 +457,19 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           if (kind == H3S_GEMM_I8) {
 #pragma unroll
             for (int k = 0; k < kGemmK / 32; ++k)
-              ptx::umma_i8(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+              ptx::umma_i8_pair(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
           } else if (kind == H3S_GEMM_E4M3) {
 #pragma unroll
             for (int k = 0; k < kGemmK / 32; ++k)
-              ptx::umma_f8(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+              ptx::umma_f8_pair(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
           } else {
 #pragma unroll
             for (int k = 0; k < kGemmK / 32; ++k)
-              ptx::umma_f16(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+              ptx::umma_f16_pair(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
           }
-          ptx::tc_commit(&sh.empty[s]);
+          ptx::tc_commit_pair(&sh.empty[s]);
         }
-        if (ok) ptx::tc_commit(&sh.acc_full[a]);
+        if (ok) ptx::tc_commit_pair(&sh.acc_full[a]);
       }
     }
   } else if (warp < 4 || warp >= 8) {
@@ -430,10 +478,13 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int gi = warp >= 8 ? 1 : 0;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     uint32_t local = 0;
+    const uint32_t acc_empty[2] = {ptx::cluster_address(&sh.acc_empty[0], 0), ptx::cluster_address(&sh.acc_empty[1], 0)};
     uint32_t exchanges = 0;  // uses of this half's exchange buffer and barrier so far
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++local) {
-      const int tm = tile % prm.m_tiles, tn = (tile / prm.m_tiles) * prm.n_step % prm.n_tiles;
+    for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step, ++local) {
+      int pair, tn;
+      tile_position(prm, tile, pair, tn);
+      const int tm = 2 * pair + rank;  // this CTA's 128 rows; may lie past the last row
       const int a = local & 1;
       const uint32_t acc_use = local >> 1;
       {
@@ -447,7 +498,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       {
         const int group_col0 = tn * kGemmN + gi * H3S_HEAD_DIM;
         const int group = group_col0 >> 7;  // 128-column group == (kind, head)
-        const bool group_ok = group_col0 < prm.n_out;
+        const bool group_ok = group_col0 < prm.n_out && tm * kGemmM < prm.rows;
         const bool normed = prm.q_norm != nullptr && group < 2 * prm.heads;
         if (kMode == kModeDense) {
           // ---- dense epilogue: scaled, biased, activated bf16 rows, staged for coalesced stores ----
@@ -460,23 +511,24 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
             uint32_t acc[32];
             H3S_TMEM_LD32(tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM + cc * 32, acc);
-            ptx::tmem_wait_ld();
+            ptx::tmem_wait_ld(acc);
             uint32_t y[16];
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              float v[2];
+            for (int i = 0; i < 32; i += 4) {
+              const int col = group_col0 + cc * 32 + i;
+              const float4 cs4 = column4(prm.col_scale, col, prm.n_out, 1.0f), bias4 = column4(prm.bias, col, prm.n_out, 0.f);
+              const float cs[4] = {cs4.x, cs4.y, cs4.z, cs4.w}, bias[4] = {bias4.x, bias4.y, bias4.z, bias4.w};
+              float v[4];
 #pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int col = group_col0 + cc * 32 + i + e;
-                const bool col_ok = col < prm.n_out;
+              for (int e = 0; e < 4; ++e) {
                 float value = integer ? static_cast<float>(static_cast<int>(acc[i + e])) : __uint_as_float(acc[i + e]);
-                const float cs = (prm.col_scale != nullptr && col_ok) ? __ldg(prm.col_scale + col) : 1.0f;
-                value = __fmul_rn(value, __fmul_rn(rs, cs));
-                if (prm.bias != nullptr && col_ok) value = __fadd_rn(value, __ldg(prm.bias + col));
+                value = __fmul_rn(value, __fmul_rn(rs, cs[e]));
+                if (prm.bias != nullptr) value = __fadd_rn(value, bias[e]);
                 if (prm.activation == H3S_ACT_GELU_TANH) value = gelu_tanh(value);
                 v[e] = value;
               }
               y[i >> 1] = pack_bf16x2(v[0], v[1]);
+              y[(i >> 1) + 1] = pack_bf16x2(v[2], v[3]);
             }
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4)
@@ -485,7 +537,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           // the accumulator has been read: the MMA warp may refill it
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&sh.acc_empty[a]);
+          if (lane == 0) ptx::mbar_arrive_cluster(acc_empty[a]);
           if (!group_ok) continue;  // the same for the four warps of this half
           if (lane == 0) ptx::mbar_arrive(&sh.tile_ready[gi]);
           {
@@ -535,7 +587,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
               uint32_t acc[32];
               H3S_TMEM_LD32(tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM + cc * 32, acc);
-              ptx::tmem_wait_ld();
+              ptx::tmem_wait_ld(acc);
 #pragma unroll
               for (int i = 0; i < 32; i += 2) {
                 const float2 ws = group_ok ? __ldg(reinterpret_cast<const float2 *>(prm.w_scale + group_col0 + cc * 32 + i))
@@ -548,7 +600,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             // the accumulator is in registers: the MMA warp may refill it
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&sh.acc_empty[a]);
+            if (lane == 0) ptx::mbar_arrive_cluster(acc_empty[a]);
             if (!group_ok) continue;  // the same for the four warps of this half
             if (normed && row_ok) {
               const void *rope_row = nullptr;
@@ -731,7 +783,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
             uint32_t acc[32];
             H3S_TMEM_LD32(tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM + cc * 32, acc);
-            ptx::tmem_wait_ld();
+            ptx::tmem_wait_ld(acc);
             const int col0 = group_col0 + cc * 32;
             if (row_ok && group_ok) {
               __nv_bfloat16 *dst = prm.out + group * prm.out_stride_head + static_cast<int64_t>(row) * H3S_HEAD_DIM + cc * 32;
@@ -758,7 +810,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
             uint32_t acc[32];
             H3S_TMEM_LD32(tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM + cc * 32, acc);
-            ptx::tmem_wait_ld();
+            ptx::tmem_wait_ld(acc);
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
               const float2 ws = __ldg(reinterpret_cast<const float2 *>(prm.w_scale + group_col0 + cc * 32 + i));
@@ -786,7 +838,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
       ptx::tc_fence_before();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&sh.acc_empty[a]);
+      if (lane == 0) ptx::mbar_arrive_cluster(acc_empty[a]);
     }
   }
 
@@ -798,9 +850,10 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       if (atomicCAS(prm.status, 0, code) == 0) prm.status[1] = blockIdx.x;
     }
   }
+  ptx::cluster_sync();  // neither CTA leaves while the other may still signal its barriers or its TMEM is written
   if (warp == 5) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem_base, kGemmTmemCols);
+    ptx::tmem_dealloc_pair(tmem_base, kGemmTmemCols);
   }
 }
 
@@ -888,13 +941,13 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
   CUtensorMap ma, mb;
   int rc = make_tensor_map_u8_2d(&ma, x_i8, hidden, rows, hidden, kGemmK, kGemmM, "qkv_gemm_chunk A map");
   if (rc) return rc;
-  rc = make_tensor_map_u8_2d(&mb, w_i8, hidden, n_out, hidden, kGemmK, kGemmN, "qkv_gemm_chunk B map");
+  rc = make_tensor_map_u8_2d(&mb, w_i8, hidden, n_out, hidden, kGemmK, kGemmN / 2, "qkv_gemm_chunk B map");
   if (rc) return rc;
   GemmParams prm;
   prm.x_scale = x_scale; prm.w_scale = w_scale; prm.out = static_cast<__nv_bfloat16 *>(out_bf16);
   prm.out_stride_head = out_stride_head; prm.status = status;
   prm.rows = rows; prm.n_out = n_out; prm.hidden = hidden;
-  prm.m_tiles = ceil_div(rows, kGemmM); prm.n_tiles = ceil_div(n_out, kGemmN);
+  prm.m_pairs = ceil_div(rows, kGemmPairM); prm.n_tiles = ceil_div(n_out, kGemmN);
   prm.n_step = 1;
   if (carriers != nullptr) {
     auto gcd = [](int a, int b) { while (b) { const int t = a % b; a = b; b = t; } return a; };
@@ -926,8 +979,8 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
   int device = 0, sms = 0;
   H3S_CHECK_CUDA(cudaGetDevice(&device));
   H3S_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const int tiles = prm.m_tiles * prm.n_tiles;
-  const int grid = tiles < sms ? tiles : sms;
+  const int tiles = prm.m_pairs * prm.n_tiles;
+  const int grid = 2 * (tiles < sms / 2 ? tiles : sms / 2);
   if (carriers != nullptr) {
     H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeCarriers>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(GemmLayout<kModeCarriers>::kBytes)));
@@ -979,13 +1032,13 @@ int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_
   CUtensorMap ma, mb;
   int rc = make_tensor_map_u8_2d(&ma, a, k_bytes, rows, lda_bytes, kGemmK, kGemmM, "dense_gemm A map");
   if (rc) return rc;
-  rc = make_tensor_map_u8_2d(&mb, b, k_bytes, n_out, ldb_bytes, kGemmK, kGemmN, "dense_gemm B map");
+  rc = make_tensor_map_u8_2d(&mb, b, k_bytes, n_out, ldb_bytes, kGemmK, kGemmN / 2, "dense_gemm B map");
   if (rc) return rc;
   GemmParams prm;
   memset(&prm, 0, sizeof(prm));
   prm.x_scale = row_scale; prm.status = status;
   prm.rows = rows; prm.n_out = n_out; prm.hidden = k_bytes;
-  prm.m_tiles = ceil_div(rows, kGemmM); prm.n_tiles = ceil_div(n_out, kGemmN); prm.n_step = 1;
+  prm.m_pairs = ceil_div(rows, kGemmPairM); prm.n_tiles = ceil_div(n_out, kGemmN); prm.n_step = 1;
   prm.heads = 1; prm.wait_budget_ns = wait_budget_ns();
   prm.operand_kind = operand_kind; prm.row_scale = row_scale; prm.col_scale = col_scale; prm.bias = bias;
   prm.activation = activation; prm.dense_out = static_cast<__nv_bfloat16 *>(out_bf16); prm.ldc = ldc;
@@ -994,8 +1047,8 @@ int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_
   H3S_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeDense>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(GemmLayout<kModeDense>::kBytes)));
-  const int tiles = prm.m_tiles * prm.n_tiles;
-  qkv_gemm_kernel<kModeDense><<<tiles < sms ? tiles : sms, kGemmThreads, GemmLayout<kModeDense>::kBytes,
+  const int tiles = prm.m_pairs * prm.n_tiles;
+  qkv_gemm_kernel<kModeDense><<<2 * (tiles < sms / 2 ? tiles : sms / 2), kGemmThreads, GemmLayout<kModeDense>::kBytes,
                                static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
