@@ -36,6 +36,17 @@ class QKVCarriers(ctypes.Structure):
     ]
 
 
+class LayerCarriers(ctypes.Structure):
+    """``h3s_layer_carriers`` of include/h3sparse.h."""
+
+    _fields_ = [
+        ("q8", c_void_p), ("q_scale", c_void_p), ("q_summary", c_void_p),
+        ("k8", c_void_p), ("k_scale", c_void_p), ("k_summary", c_void_p),
+        ("k_mean", c_void_p), ("v_scale", c_void_p), ("v8", c_void_p), ("v16", c_void_p), ("scratch", c_void_p),
+        ("summary_dtype", c_int),
+    ]
+
+
 class NativeError(RuntimeError):
     """The native library is missing, mismatched, or a call failed."""
 
@@ -89,6 +100,13 @@ PROTOTYPES = {
     "h3s_sparse_attn_half_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                          c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
                                          c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "h3s_stream_order": (c_int, [c_void_p, c_void_p, c_void_p]),
+    "h3s_quant_qkv": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                              c_int, c_float, c_int, c_void_p, c_void_p, c_void_p]),
+    "h3s_project_qkv": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p,
+                                c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_float,
+                                c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "h3s_status_mirror": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p]),
     "h3s_sparse_attn_fwd_mma": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int64,
                                         c_int64, c_int, c_int, c_int, c_void_p]),
@@ -135,7 +153,10 @@ def ptr(tensor):
 
 
 def stream_ptr(device=None):
-    return c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """Raw handle of torch's current stream on ``device`` (without the Stream object of
+    ``torch.cuda.current_stream``, which takes several microseconds to build)."""
+    index = None if device is None else torch.device(device).index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def dtype_code(dtype):

@@ -215,6 +215,104 @@ def quant_v_fp8(v, v_scale=None, v_bound=FP8_V_BOUND):
     return carrier, v_scale
 
 
+class SideStream:
+    """A second stream of ``device`` and the event that orders it and the callers' streams."""
+
+    def __init__(self, device):
+        self.stream = torch.cuda.Stream(device)
+        self.handle = self.stream.cuda_stream
+        self.event = torch.cuda.Event()
+        self.event.record(self.stream)  # the native event exists from the first record on
+        self.event_handle = self.event.cuda_event
+
+    def join(self, stream):
+        """``stream`` (a raw handle) goes on behind everything issued here."""
+        check(_native.load().h3s_stream_order(self.handle, stream, self.event_handle), "h3s_stream_order")
+
+
+class LayerBuffers:
+    """Carriers, scales, tile means and scratch of one layer call (batch 1), as ``h3s_quant_qkv`` and
+    ``h3s_project_qkv`` fill them; all allocated on the current stream."""
+
+    def __init__(self, heads, sequence, device, *, smooth_k, summary_dtype):
+        lib = _native.load()
+        q_blocks, k_blocks = _ceil_div(sequence, Q_TILE), _ceil_div(sequence, KV_TILE)
+        shape, small = (1, heads, sequence, HEAD_DIM), (1, heads, HEAD_DIM)
+        self.q_int8 = torch.empty(shape, dtype=torch.int8, device=device)
+        self.k_int8 = torch.empty(shape, dtype=torch.int8, device=device)
+        self.q_scale = torch.empty((1, heads, q_blocks), dtype=torch.float32, device=device)
+        self.k_scale = torch.empty((1, heads, k_blocks), dtype=torch.float32, device=device)
+        self.q_summary = self.k_summary = self.k_mean = None
+        if summary_dtype is not None:
+            self.q_summary = torch.empty((1, heads, q_blocks, HEAD_DIM), dtype=summary_dtype, device=device)
+            self.k_summary = torch.empty((1, heads, k_blocks, HEAD_DIM), dtype=summary_dtype, device=device)
+        if smooth_k:
+            self.k_mean = torch.empty(small, dtype=torch.float32, device=device)
+        self.v_scale = torch.empty(small, dtype=torch.float32, device=device)
+        self.v_carrier = allocate_v_carrier(sequence, heads, device)
+        self.v_half = torch.empty(self.v_carrier.shape, dtype=torch.bfloat16, device=device)
+        self.scratch = torch.empty(lib.h3s_column_stats_scratch_bytes(heads), dtype=torch.uint8, device=device)
+        self.native = _native.LayerCarriers(
+            self.q_int8.data_ptr(), self.q_scale.data_ptr(), _address(self.q_summary),
+            self.k_int8.data_ptr(), self.k_scale.data_ptr(), _address(self.k_summary),
+            _address(self.k_mean), self.v_scale.data_ptr(), self.v_carrier.data_ptr(), self.v_half.data_ptr(),
+            self.scratch.data_ptr(), 0 if summary_dtype is None else dtype_code(summary_dtype))
+
+
+def _address(tensor):
+    return None if tensor is None else tensor.data_ptr()
+
+
+def quant_qkv(q, k, v, buffers, side, stream, *, smooth_k, v_after_k, v_bound=FP8_V_BOUND):
+    """Carriers of HND ``q``, ``k``, ``v`` into ``buffers``, on ``stream`` (the raw handle of the current
+    stream) and ``side``.  The caller joins ``side`` on every path, before the buffers can be freed."""
+    strides = (ctypes.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
+    check(
+        _native.load().h3s_quant_qkv(
+            buffers.native, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, dtype_code(q.dtype), q.shape[1], q.shape[2],
+            int(smooth_k), v_bound, int(v_after_k), side.event_handle, stream, side.handle),
+        "h3s_quant_qkv",
+    )
+
+
+def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, smooth_k, q_norm=None, k_norm=None,
+                epsilon=0.0, rope=None, status=None, v_bound=FP8_V_BOUND):
+    """The chunked projection of ``x`` (S, hidden) bf16 into ``buffers`` (see ``quant_qkv``).  Returns the
+    scratch tensors, which live until ``side`` has been joined."""
+    if x.stride(1) != 1:
+        raise _native.NativeError("project_qkv: x must have contiguous rows")
+    sequence, hidden = x.shape
+    device, rows = x.device, min(chunk_rows, sequence)
+    x_i8 = torch.empty((rows, hidden), dtype=torch.int8, device=device)
+    x_scale = torch.empty((rows,), dtype=torch.float32, device=device)
+    # bf16 staging of what needs whole-sequence statistics before it can be quantised
+    shape = (1, heads, sequence, HEAD_DIM)
+    v_stage = torch.empty(shape, dtype=torch.bfloat16, device=device)
+    k_stage = torch.empty(shape, dtype=torch.bfloat16, device=device) if smooth_k else None
+    rope_code, strides = 0, None
+    if rope is not None:
+        rope_code = dtype_code(rope.dtype)
+        strides = (ctypes.c_int64 * 4)(rope.stride(1), rope.stride(3), rope.stride(4), rope.stride(5))
+    scratch = (x_i8, x_scale, v_stage, k_stage)
+    check(
+        _native.load().h3s_project_qkv(
+            buffers.native, x.data_ptr(), x.stride(0), sequence, hidden, chunk_rows, x_i8.data_ptr(), x_scale.data_ptr(),
+            w_i8.data_ptr(), w_scale.data_ptr(), heads, int(smooth_k), _address(k_stage), v_stage.data_ptr(),
+            _address(q_norm), _address(k_norm), epsilon, _address(rope), rope_code, strides, v_bound, _address(status),
+            side.event_handle, stream, side.handle),
+        "h3s_project_qkv",
+    )
+    return scratch
+
+
+def status_mirror(word, mirror, event, stream):
+    """Queue the copy of the status words into pinned ``mirror`` and ``event`` behind it."""
+    if not event.cuda_event:
+        event.record()  # brings the native event into being
+    check(_native.load().h3s_status_mirror(word.data_ptr(), mirror.data_ptr(), event.cuda_event, stream),
+          "h3s_status_mirror")
+
+
 def convrot_quant_rows(x, x_i8=None, x_scale=None):
     """ConvRot (Hadamard-256) + per-row INT8 of ``x`` (rows, hidden) bf16.
     Returns ``(codes int8 (rows, hidden), scale fp32 (rows,))``."""

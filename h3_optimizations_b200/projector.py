@@ -52,7 +52,7 @@ _SIDE_STREAMS = {}
 def _side_stream(device):
     key = device.index if device.index is not None else torch.cuda.current_device()
     if key not in _SIDE_STREAMS:
-        _SIDE_STREAMS[key] = torch.cuda.Stream(device)
+        _SIDE_STREAMS[key] = ops.SideStream(device)
     return _SIDE_STREAMS[key]
 
 
@@ -149,54 +149,24 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
         if rope_freqs.dtype not in (torch.float32, torch.bfloat16):
             rope_freqs = rope_freqs.float()
     try:
-        q_blocks = (sequence + Q_TILE - 1) // Q_TILE
-        k_blocks = (sequence + KV_TILE - 1) // KV_TILE
-        shape = (1, heads, sequence, HEAD_DIM)
-        q_int8 = torch.empty(shape, dtype=torch.int8, device=device)
-        k_int8 = torch.empty(shape, dtype=torch.int8, device=device)
-        q_scale = torch.empty((1, heads, q_blocks), dtype=torch.float32, device=device)
-        k_scale = torch.empty((1, heads, k_blocks), dtype=torch.float32, device=device)
-        q_summary = torch.empty((1, heads, q_blocks, HEAD_DIM), dtype=summary_dtype, device=device)
-        k_summary = torch.empty((1, heads, k_blocks, HEAD_DIM), dtype=summary_dtype, device=device)
-        # bf16 staging of what needs whole-sequence statistics before it can be quantised
-        v_stage = torch.empty(shape, dtype=torch.bfloat16, device=device)
-        k_stage = torch.empty(shape, dtype=torch.bfloat16, device=device) if smooth_k else None
-        stats = ops.column_stats_scratch(heads, device)
-        x_i8 = torch.empty((min(chunk_rows, sequence), hidden), dtype=torch.int8, device=device)
-        x_scale = torch.empty((min(chunk_rows, sequence),), dtype=torch.float32, device=device)
-        w_i8 = w_i8.contiguous()
-        for start, end in chunk_ranges(sequence, chunk_rows):
-            rows = end - start
-            ops.convrot_quant_rows(x[start:end], x_i8, x_scale)
-            ops.qkv_gemm_chunk_carriers(
-                x_i8[:rows], x_scale[:rows], w_i8, w_scale, heads=heads, row_start=start,
-                q_int8=q_int8, q_scale=q_scale, q_summary=q_summary, k_summary=k_summary, v_stage=v_stage,
-                stats=stats, k_int8=None if smooth_k else k_int8, k_scale=None if smooth_k else k_scale,
-                k_stage=k_stage, status=status, q_norm=q_norm, k_norm=k_norm, epsilon=epsilon, rope=rope_freqs)
-        k_mean, v_scale = ops.column_stats_finalize(stats, heads, sequence, want_k_mean=smooth_k,
-                                                    dtype=torch.bfloat16, v_bound=V_QUANT_BOUND)
-        v_carrier = ops.allocate_v_carrier(sequence, heads, device)
-        v_half = torch.empty(v_carrier.shape, dtype=torch.bfloat16, device=device)
-        if smooth_k:
-            # the two second-phase quantisers are independent and each leaves part of the
-            # memory system idle: V runs on a second stream underneath K
-            main, side = torch.cuda.current_stream(device), _side_stream(device)
-            side.wait_stream(main)
-            try:
-                with torch.cuda.stream(side):
-                    ops.quant_v_fp8_into(v_stage, v_scale, v_carrier, v_bound=V_QUANT_BOUND, half=v_half)
-                ops.quant_qk_blocks_into(k_stage, k_int8, k_scale, None, block=KV_TILE, mean=k_mean)
-            finally:
-                main.wait_stream(side)  # on every exit path, before the staging can be freed
-        else:
-            ops.quant_v_fp8_into(v_stage, v_scale, v_carrier, v_bound=V_QUANT_BOUND, half=v_half)
+        buffers = ops.LayerBuffers(heads, sequence, device, smooth_k=smooth_k, summary_dtype=summary_dtype)
+        stream, side = _native.stream_ptr(device), _side_stream(device)
+        try:
+            # every launch of the projection from one native call (24 heads x 2304 tokens, with
+            # backend and out_proj: 344 -> 259 us)
+            scratch = ops.project_qkv(x, w_i8.contiguous(), w_scale.contiguous(), buffers, side, stream, heads=heads,
+                                      chunk_rows=chunk_rows, smooth_k=smooth_k, q_norm=q_norm, k_norm=k_norm,
+                                      epsilon=float(epsilon), rope=rope_freqs, status=status, v_bound=V_QUANT_BOUND)
+        finally:
+            side.join(stream)  # on every exit path, before the staging can be freed
+        del scratch
     except _native.NativeError as exc:
         raise FusedQKVError("chunked QKV projection failed: layer=%d: %s" % (layer_index, exc)) from exc
     return validate_prepared_fused_qkv(
         PreparedFusedQKV(
-            q_int8=q_int8, q_scale=q_scale, k_int8=k_int8, k_scale=k_scale, v=None,
-            q_summary=q_summary, k_summary=k_summary, output_dtype=x.dtype, sequence=sequence,
+            q_int8=buffers.q_int8, q_scale=buffers.q_scale, k_int8=buffers.k_int8, k_scale=buffers.k_scale, v=None,
+            q_summary=buffers.q_summary, k_summary=buffers.k_summary, output_dtype=x.dtype, sequence=sequence,
             heads=heads, head_dim=HEAD_DIM, layer_index=int(layer_index), smooth_k=bool(smooth_k),
-            v_carrier=v_carrier, v_scale=v_scale, v_half=v_half,
+            v_carrier=buffers.v_carrier, v_scale=buffers.v_scale, v_half=buffers.v_half,
         )
     )
