@@ -36,6 +36,12 @@
 // Warp roles: warps 0-7 softmax/epilogue (TMEM lanes 32*(w%4).., group w/4), warp 8
 // TMA producer and QK^T issuer, warp 9 P.V issuer and TMEM owner.
 //
+// Dense rows (query tiles that see every key) are cut into parts where one of them is
+// longer than what a CTA slot gets on average, i.e. where a few long rows would outlast
+// all others: see split_dense_rows.  Each part is a CTA with its own reference point; it
+// leaves its sums in memory and the part that comes last adds them up, in the order of
+// the list, so that the result does not depend on which one that was.
+//
 // What bounds it: per tile and SM the ex2 pipe needs 512 cycles, the tensor pipe 453
 // (measured: 144 for QK^T with A in TMEM, 258 with A in shared memory, 309 for P.V),
 // the remaining softmax instructions about 290 issue slots; a tile takes 800.  24
@@ -70,10 +76,11 @@ struct HalfShared {
   uint64_t pv_done[2];         // P.V of tile j has completed: its stage and its slot are free
   uint64_t first_max;          // group 0 has left the first tile's row maxima in `row`
   uint64_t pass_end;           // row sums (or maxima) of a pass are in `row`, `again` is valid; all warps wait
-  uint64_t staged;             // softmax warps only: the output tile is in shared memory
+  uint64_t staged;             // softmax warps only: the output tile is in shared memory (and steps before that)
   uint32_t tmem_base;
   int abort_word;
   int again;                   // some row sum passed the limit
+  int finish;                  // this CTA writes the output tile
   int tile_index[kHStages];    // KV tile held by each stage ...
   float tile_scale[kHStages];  // ... and its k_scale, written by the producer
   float v_scale[H3S_HEAD_DIM];
@@ -136,14 +143,17 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
   const int n_dense = prm.q_tiles - n_sparse;
   int head, tq;
+  int dense_row = 0, part = 0;  // running number of a dense row, part of its list
   bool dense;
   {
     const int w = blockIdx.x;
-    const int dense_items = prm.heads * n_dense;
+    const int dense_items = prm.heads * n_dense * prm.parts;
     if (w < dense_items) {
       dense = true;
-      head = w / n_dense;
-      const int i = w - head * n_dense;
+      dense_row = w / prm.parts;
+      part = w - dense_row * prm.parts;
+      head = dense_row / n_dense;
+      const int i = dense_row - head * n_dense;
       tq = (n_sparse == 0 || i < prm.q_start) ? i : prm.q_stop + (i - prm.q_start);
     } else {
       dense = false;
@@ -152,7 +162,9 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       tq = prm.q_start + (v - head * n_sparse);
     }
   }
-  const int n_iter = dense ? prm.kv_tiles : prm.route_len;
+  const bool split = dense && prm.parts > 1;
+  const int first_tile = part * prm.part_tiles;  // of a dense row's list
+  const int n_iter = dense ? min(prm.part_tiles, prm.kv_tiles - first_tile) : prm.route_len;
   const int32_t *route_row =
       dense ? nullptr
             : prm.route + (static_cast<int64_t>(head) * n_sparse + (tq - prm.q_start)) * prm.route_len;
@@ -172,6 +184,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     ptx::mbar_init(&sh.staged, kHSoftmaxWarps);
     sh.abort_word = 0;
     sh.again = 0;
+    sh.finish = 1;
     ptx::fence_mbar_init();
   }
   if (threadIdx.x < H3S_HEAD_DIM) sh.v_scale[threadIdx.x] = __ldg(prm.v_scale + head * H3S_HEAD_DIM + threadIdx.x);
@@ -219,7 +232,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     float my_scale = 0.f, next_scale = 0.f;
     auto fetch_block = [&](int b) {
       const int mine = min(b * 32 + lane, n_iter - 1);
-      next_tile = dense ? mine : __ldg(route_row + mine);
+      next_tile = dense ? first_tile + mine : __ldg(route_row + mine);
       next_scale = __ldg(k_scale + next_tile);
     };
     auto load = [&](int i) {      // tile i of the list, into the stage of its running number
@@ -385,15 +398,82 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       // 32 rows of one column half; the two warps of a row quarter then each write
       // 16 of the quarter's rows as full contiguous lines.
       ptx::tc_fence_after();
+      uint32_t staged_uses = 0;
+      auto meet = [&]() {  // all softmax warps
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&sh.staged);
+        return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      };
+      // Partial sums of part p: [32 groups of 4 columns][128 rows] float4, so that a warp's rows are
+      // neighbours; then 128 row sums and 128 reference points.
+      constexpr int kPartFloats = H3S_Q_TILE * (H3S_HEAD_DIM + 2);
+      const float *parts_base = prm.partial + static_cast<int64_t>(dense_row) * prm.parts * kPartFloats;
+      float top = 0.f;  // largest reference point of the parts
+      if (split) {
+        float *mine = const_cast<float *>(parts_base) + static_cast<int64_t>(part) * kPartFloats;
+#pragma unroll 1
+        for (int cc = group * 2; cc < group * 2 + 2; ++cc) {
+          uint32_t o[32];
+          H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
+          ptx::tmem_wait_ld(o);
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            __stcg(reinterpret_cast<float4 *>(mine) + (cc * 8 + i / 4) * H3S_Q_TILE + row,
+                   make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]),
+                               __uint_as_float(o[i + 3])));
+        }
+        if (group == 0) {
+          __stcg(mine + H3S_Q_TILE * H3S_HEAD_DIM + row, l);
+          __stcg(mine + H3S_Q_TILE * (H3S_HEAD_DIM + 1) + row, m);
+        }
+        __threadfence();
+        ok = meet();
+        if (ok && warp == 0 && lane == 0) {
+          __threadfence();
+          sh.finish = atomicAdd(prm.arrived + dense_row, 1u) == static_cast<unsigned int>(prm.parts - 1);
+          __threadfence();
+        }
+        ok = ok && meet();
+        if (ok && sh.finish) {
+          l = 0.f;
+          top = -INFINITY;
+          for (int p = 0; p < prm.parts; ++p)
+            top = fmaxf(top, __ldcg(parts_base + p * kPartFloats + H3S_Q_TILE * (H3S_HEAD_DIM + 1) + row));
+          for (int p = 0; p < prm.parts; ++p) {
+            const float *at = parts_base + p * kPartFloats + H3S_Q_TILE * H3S_HEAD_DIM + row;
+            l = fmaf(__ldcg(at), fast_exp2(__ldcg(at + H3S_Q_TILE) - top), l);
+          }
+        }
+      }
+      const bool finish = ok && sh.finish;
       const float inv_l = 1.0f / l;
       constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
       static_assert(H3S_Q_TILE * kRowBytes <= kHOffBar, "output tile must fit the stage ring");
       unsigned char *my_row = smem + row * kRowBytes;
 #pragma unroll 1
-      for (int cc = group * 2; cc < group * 2 + 2; ++cc) {
+      for (int cc = group * 2; finish && cc < group * 2 + 2; ++cc) {
         uint32_t o[32];
-        H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
-        ptx::tmem_wait_ld(o);
+        if (!split) {
+          H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
+          ptx::tmem_wait_ld(o);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
+#pragma unroll 1
+          for (int p = 0; p < prm.parts; ++p) {
+            const float *at = parts_base + p * kPartFloats;
+            // the reference points are integers: the factors are powers of two
+            const float weight = fast_exp2(__ldcg(at + H3S_Q_TILE * (H3S_HEAD_DIM + 1) + row) - top);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 x = __ldcg(reinterpret_cast<const float4 *>(at) + (cc * 8 + i / 4) * H3S_Q_TILE + row);
+              o[i] = __float_as_uint(fmaf(x.x, weight, __uint_as_float(o[i])));
+              o[i + 1] = __float_as_uint(fmaf(x.y, weight, __uint_as_float(o[i + 1])));
+              o[i + 2] = __float_as_uint(fmaf(x.z, weight, __uint_as_float(o[i + 2])));
+              o[i + 3] = __float_as_uint(fmaf(x.w, weight, __uint_as_float(o[i + 3])));
+            }
+          }
+        }
 #pragma unroll
         for (int i = 0; i < 32; i += 8) {
           float v[8];
@@ -413,10 +493,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         }
       }
       ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&sh.staged);
       // both halves of the rows are staged
-      if (warp_wait(&sh.staged, 0, abort_word, kAbortFinal, 4 * prm.wait_budget_ns)) store_rows<OutT>(prm, smem, head, tq, quarter * 32 + group * 16, 16, lane);
+      if (finish && meet()) store_rows<OutT>(prm, smem, head, tq, quarter * 32 + group * 16, 16, lane);
     }
   }
 
@@ -439,7 +517,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     ptx::tmem_dealloc(tmem_o, kHTmemCols);
   }
   // head-sharded run: the producer and MMA warps have nothing left to do and share the copy
-  if (code == 0 && prm.n_peer_out > 0) scatter_to_peers<OutT>(prm, smem, head, tq, kHThreads);
+  if (code == 0 && prm.n_peer_out > 0 && sh.finish) scatter_to_peers<OutT>(prm, smem, head, tq, kHThreads);
 }
 
 // E4M3 codes -> BF16 values: 16 per thread
@@ -452,12 +530,43 @@ __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v
   v16[2 * i + 1] = out[1];
 }
 
+// Whether and how the dense rows' tile lists are cut.  Two CTAs run on each of 148 SMs; a
+// slot gets `share` tiles on average.  A dense row much longer than that ends after
+// everything else has: seven heads of 10384 tokens at 15 % (28 dense rows of 163 tiles
+// beside 546 routed ones of 31, share 73) take 195 us for the whole layer uncut, 176 us in
+// parts.  At the line itself, an eighth longer than the share, both are equal (three heads
+// of 33272 tokens at 30 %: 520 against a share of 441, 523 and 521 us), and below it the
+// order "long rows first" fills the slots, so that parts would only cost their traffic.  A
+// quarter of the share keeps the last parts short; under 24 tiles a part's start and end
+// (about 4 us) would show.
+constexpr int kSlots = 2 * 148, kMinPartTiles = 24, kMaxParts = 16;
+
+static int split_dense_rows(int heads, int q_tiles, int kv_tiles, int n_sparse, int route_len, int *part_tiles) {
+  const int64_t n_dense = q_tiles - n_sparse;
+  const int64_t total = heads * (n_dense * kv_tiles + static_cast<int64_t>(n_sparse) * route_len);
+  *part_tiles = kv_tiles;
+  if (n_dense == 0 || static_cast<int64_t>(kv_tiles) * kSlots * 7 <= total * 8) return 1;
+  int tiles = static_cast<int>(total / (4 * kSlots));
+  if (tiles < kMinPartTiles) tiles = kMinPartTiles;
+  if (tiles < ceil_div(kv_tiles, kMaxParts)) tiles = ceil_div(kv_tiles, kMaxParts);
+  const int parts = ceil_div(kv_tiles, tiles);
+  *part_tiles = ceil_div(kv_tiles, parts);  // even parts; none is empty
+  return ceil_div(kv_tiles, *part_tiles);
+}
+
+static size_t split_bytes(int64_t dense_rows, int parts, size_t *arrived_bytes) {
+  *arrived_bytes = (static_cast<size_t>(dense_rows) * sizeof(unsigned int) + 255) & ~static_cast<size_t>(255);
+  return *arrived_bytes + static_cast<size_t>(dense_rows) * parts * H3S_Q_TILE * (H3S_HEAD_DIM + 2) * sizeof(float);
+}
+
 template <typename OutT>
 static int launch_attn_half(const CUtensorMap &mk, const CUtensorMap &mv, const int8_t *q8, const AttnParams &prm,
                             cudaStream_t stream) {
   H3S_CHECK_CUDA(cudaFuncSetAttribute(sparse_attn_half_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(kHSmemBytes)));
-  sparse_attn_half_kernel<OutT><<<prm.heads * prm.q_tiles, kHThreads, kHSmemBytes, stream>>>(mk, mv, q8, prm);
+  const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
+  const int ctas = prm.heads * ((prm.q_tiles - n_sparse) * prm.parts + n_sparse);
+  sparse_attn_half_kernel<OutT><<<ctas, kHThreads, kHSmemBytes, stream>>>(mk, mv, q8, prm);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
 }
@@ -476,11 +585,23 @@ extern "C" int h3s_v_half(const uint8_t *v8t, void *v16t, int heads, int sequenc
   return H3S_OK;
 }
 
+extern "C" size_t h3s_sparse_attn_half_workspace_bytes(int heads, int sequence, int route_len, int q_start, int q_stop) {
+  using namespace h3s;
+  if (heads <= 0 || sequence <= 0) return 0;
+  const int q_tiles = ceil_div(sequence, H3S_Q_TILE), kv_tiles = ceil_div(sequence, H3S_KV_TILE);
+  const int n_sparse = route_len > 0 ? q_stop - q_start : 0;
+  int part_tiles;
+  const int parts = split_dense_rows(heads, q_tiles, kv_tiles, n_sparse, route_len, &part_tiles);
+  size_t arrived_bytes;
+  return parts > 1 ? split_bytes(static_cast<int64_t>(heads) * (q_tiles - n_sparse), parts, &arrived_bytes) : 0;
+}
+
 extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, const void *v16t, const float *q_scale,
                                         const float *k_scale, const float *v_scale, const int32_t *route,
                                         int route_len, int q_start, int q_stop, void *out, void *const *peer_out,
                                         int n_peer_out, int out_dtype, int64_t out_stride_h, int64_t out_stride_s,
-                                        int heads, int sequence, int flags, int32_t *status, h3s_stream_t stream) {
+                                        int heads, int sequence, int flags, void *workspace, size_t workspace_bytes,
+                                        int32_t *status, h3s_stream_t stream) {
   using namespace h3s;
   AttnParams prm;
   int rc = fill_attn_params(&prm, q8, k8, v16t, q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out,
@@ -497,6 +618,22 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
                              H3S_KV_TILE * 2, H3S_HEAD_DIM, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_half_fwd V map");
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  prm.parts = 1; prm.part_tiles = prm.kv_tiles; prm.partial = nullptr; prm.arrived = nullptr;
+  if (workspace != nullptr) {
+    const int n_sparse = route != nullptr ? q_stop - q_start : 0;
+    int part_tiles;
+    const int parts = split_dense_rows(heads, prm.q_tiles, prm.kv_tiles, n_sparse, n_sparse ? route_len : 0, &part_tiles);
+    size_t arrived_bytes;
+    const size_t need = split_bytes(static_cast<int64_t>(heads) * (prm.q_tiles - n_sparse), parts, &arrived_bytes);
+    if (parts > 1) {
+      H3S_CHECK_ARG(workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
+                    "sparse_attn_half_fwd: the workspace must be 16-byte aligned and hold %zu bytes, got %zu", need, workspace_bytes);
+      prm.parts = parts; prm.part_tiles = part_tiles;
+      prm.arrived = static_cast<unsigned int *>(workspace);
+      prm.partial = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + arrived_bytes);
+      H3S_CHECK_CUDA(cudaMemsetAsync(workspace, 0, arrived_bytes, s));
+    }
+  }
   switch (out_dtype) {
     case H3S_F32: return launch_attn_half<float>(mk, mv, q8, prm, s);
     case H3S_BF16: return launch_attn_half<__nv_bfloat16>(mk, mv, q8, prm, s);

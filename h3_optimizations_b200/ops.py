@@ -635,6 +635,8 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
     else:
         if v_half is None:
             v_half = v_half_copy(v_carrier)
+        size = lib.h3s_sparse_attn_half_workspace_bytes(heads, sequence, route_len, int(q_start), int(q_stop))
+        workspace = torch.empty(size, dtype=torch.uint8, device=q8.device) if size else None
         check(lib.h3s_sparse_attn_half_fwd(ptr(q8), ptr(k8), ptr(v_half), *before, table, n_peers, *after,
-                                           ptr(status), stream), "h3s_sparse_attn_half_fwd")
+                                           ptr(workspace), size, ptr(status), stream), "h3s_sparse_attn_half_fwd")
     return out
