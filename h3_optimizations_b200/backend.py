@@ -436,12 +436,14 @@ class B200SparseBackend:
         if q.ndim != 4 or q.shape != k.shape or q.shape != v.shape:
             raise SparseSageError("forward expects equal rank-4 HND Q/K/V; got %s %s %s"
                                   % (tuple(q.shape), tuple(k.shape), tuple(v.shape)))
+        # a batch is written in place (gathering the elements afterwards moved every output twice)
+        whole = torch.empty(q.shape, dtype=q.dtype, device=q.device) if q.shape[0] > 1 else None
         outputs = []
         for b in range(q.shape[0]):
             prepared = self.prepare(q[b:b + 1], k[b:b + 1], v[b:b + 1], layer_index=layer_index,
                                     transformer_options=transformer_options)
-            outputs.append(self.execute(prepared))
-        return outputs[0] if len(outputs) == 1 else torch.cat(outputs, dim=0)
+            outputs.append(self.execute(prepared, out=None if whole is None else whole[b:b + 1]))
+        return whole if whole is not None else outputs[0] if outputs else torch.cat(outputs, dim=0)
 
     # -- host-resident activations -------------------------------------------
 
