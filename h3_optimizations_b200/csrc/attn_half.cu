@@ -524,10 +524,9 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v8, uint4 *__restrict__ v16, int64_t chunks) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= chunks) return;
-  uint4 out[2];
-  e4m3x16_to_bf16(__ldg(v8 + i), out);
-  v16[2 * i] = out[0];
-  v16[2 * i + 1] = out[1];
+  const uint4 codes = __ldg(v8 + i);
+  v16[2 * i] = e4m3x8_to_bf16(make_uint2(codes.x, codes.y));
+  v16[2 * i + 1] = e4m3x8_to_bf16(make_uint2(codes.z, codes.w));
 }
 
 // Whether and how the dense rows' tile lists are cut.  Two CTAs run on each of 148 SMs; a

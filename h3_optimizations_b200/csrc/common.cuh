@@ -127,19 +127,18 @@ __device__ __forceinline__ float divide(const SharedDivisor &d, float a) {
   return __fmaf_rn(e, d.r, q0);
 }
 
-// 16 E4M3 codes -> the same values as BF16 (exact: four significant bits)
-__device__ __forceinline__ void e4m3x16_to_bf16(const uint4 &codes, uint4 (&out)[2]) {
-  const uint32_t in[4] = {codes.x, codes.y, codes.z, codes.w};
-  uint32_t pair[8];
+// 8 E4M3 codes -> the same values as BF16 (exact: four significant bits)
+__device__ __forceinline__ uint4 e4m3x8_to_bf16(const uint2 &codes) {
+  const uint32_t in[2] = {codes.x, codes.y};
+  uint32_t pair[4];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
+  for (int k = 0; k < 4; ++k) {
     uint32_t half2;
     asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(half2) : "h"(static_cast<uint16_t>(in[k >> 1] >> ((k & 1) * 16))));
     const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&half2));
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(pair[k]) : "f"(f.y), "f"(f.x));
   }
-  out[0] = make_uint4(pair[0], pair[1], pair[2], pair[3]);
-  out[1] = make_uint4(pair[4], pair[5], pair[6], pair[7]);
+  return make_uint4(pair[0], pair[1], pair[2], pair[3]);
 }
 
 __device__ __forceinline__ float warp_max(float v) {

@@ -223,6 +223,9 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
 // FP8-E4M3 V carrier, transposed to (heads, 128, pad128(S)).
 // One CTA = 128 sequence rows of one head, staged through shared memory so
 // that both the row-major reads and the channel-major writes are full lines.
+// All eight rows of a thread are requested before the first is used, and the BF16 copy
+// is written as whole lines of 256 bytes (two 16-byte pieces a thread with a gap between
+// them cost twice the L2 writes): 24 heads x 33272 tokens 133 -> 88 us.
 // ---------------------------------------------------------------------------
 
 constexpr int kVTile = 128;
@@ -260,34 +263,40 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
   }
 
   const T *base = v + head * stride_h + c0;
+  constexpr int kPasses = kVTile / (kVThreads / 16 * 4);
+  typename Elem<T>::Raw raw[kPasses][4];
+#pragma unroll
+  for (int p = 0; p < kPasses; ++p) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = (p * (kVThreads / 16) + slot) * 4 + j;  // four consecutive rows
+      raw[p][j] = r < valid_rows ? Elem<T>::load_raw(base + static_cast<int64_t>(first_row + r) * stride_s)
+                                 : Elem<T>::zero_raw();  // 0 / scale is the padding's code
+    }
+  }
   // the divisors' exactness is tested once, around the whole loop (see divide<>)
   auto fill = [&](auto exact_tag) {
   constexpr bool kExact = decltype(exact_tag)::value;
 #pragma unroll
-  for (int p = 0; p < kVTile / (kVThreads / 16 * 4); ++p) {
-    const int r0 = (p * (kVThreads / 16) + slot) * 4;  // four consecutive rows
+  for (int p = 0; p < kPasses; ++p) {
+    const int r0 = (p * (kVThreads / 16) + slot) * 4;
     // four consecutive rows of 8 channels -> per channel one word of four codes
     // (two 2-wide conversions and one byte permute)
     float q[4][8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (r0 + j < valid_rows) {
-        float raw[8];
-        Elem<T>::load8(base + static_cast<int64_t>(first_row + r0 + j) * stride_s, raw);
+      float x[8];
+      Elem<T>::unpack(raw[p][j], x);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if (kExact) {  // shared-divisor division, see SharedDivisor
-            const float q0 = __fmul_rn(raw[i], rc[i]);
-            q[j][i] = __fmaf_rn(__fmaf_rn(-sc[i], q0, raw[i]), rc[i], q0);
-          } else {
-            q[j][i] = __fdiv_rn(raw[i], sc[i]);
-          }
-          // the conversion saturates at +-448 by itself; a tighter bound is applied here
-          if (clamp) q[j][i] = fminf(fmaxf(q[j][i], -v_bound), v_bound);
+      for (int i = 0; i < 8; ++i) {
+        if (kExact) {  // shared-divisor division, see SharedDivisor
+          const float q0 = __fmul_rn(x[i], rc[i]);
+          q[j][i] = __fmaf_rn(__fmaf_rn(-sc[i], q0, x[i]), rc[i], q0);
+        } else {
+          q[j][i] = __fdiv_rn(x[i], sc[i]);
         }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q[j][i] = 0.f;
+        // the conversion saturates at +-448 by itself; a tighter bound is applied here
+        if (clamp) q[j][i] = fminf(fmaxf(q[j][i], -v_bound), v_bound);
       }
     }
     uint32_t word[8];
@@ -313,19 +322,79 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
     const uint4 data = *reinterpret_cast<const uint4 *>(&tile[v_tile_offset(d, chunk * 16)]);
     const int64_t at = base_at + static_cast<int64_t>(d) * padded_total + chunk * 16;
     *reinterpret_cast<uint4 *>(out + at) = data;
-    if (out_half != nullptr) {  // the copy the attention kernel multiplies with BF16 probabilities
-      uint4 half[2];
-      e4m3x16_to_bf16(data, half);
-      *reinterpret_cast<uint4 *>(out_half + at) = half[0];
-      *reinterpret_cast<uint4 *>(out_half + at + 8) = half[1];
+  }
+  if (out_half != nullptr) {  // the copy the attention kernel multiplies with BF16 probabilities
+#pragma unroll
+    for (int p = 0; p < H3S_HEAD_DIM / (kVThreads / 16); ++p) {
+      const int d = p * (kVThreads / 16) + slot, s = (threadIdx.x & 15) * 8;
+      const uint2 data = *reinterpret_cast<const uint2 *>(&tile[v_tile_offset(d, s)]);
+      *reinterpret_cast<uint4 *>(out_half + base_at + static_cast<int64_t>(d) * padded_total + s) = e4m3x8_to_bf16(data);
     }
   }
 }
 
 // ---------------------------------------------------------------------------
 // Per-row FP8-E4M3 quantisation of a bf16 matrix (activations of the FP8 MLP).
-// One CTA = one row, kept in registers between the amax reduction and the store.
+// Kept in registers between the amax reduction and the store.  Rows of up to 4096
+// channels: one warp each, no barrier, all loads of the row in flight (4096 x 3072: 23 -> 13 us);
+// longer rows: one CTA each.
 // ---------------------------------------------------------------------------
+
+// E4M3 codes of 8 consecutive channels
+template <bool kExact>
+__device__ __forceinline__ uint2 row_codes8(const SharedDivisor &by_scale, const float (&v)[8]) {
+  uint32_t word[2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    uint16_t lo, hi;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(lo)
+        : "f"(divide<kExact>(by_scale, v[4 * w + 1])), "f"(divide<kExact>(by_scale, v[4 * w])));
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(hi)
+        : "f"(divide<kExact>(by_scale, v[4 * w + 3])), "f"(divide<kExact>(by_scale, v[4 * w + 2])));
+    word[w] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+  }
+  return make_uint2(word[0], word[1]);
+}
+
+constexpr int kRowWarps = 4;  // rows (warps) per CTA
+
+template <int kChunks>  // 16-byte loads per lane
+__global__ void __launch_bounds__(kRowWarps * 32)
+quant_rows_fp8_warp_kernel(const __nv_bfloat16 *__restrict__ x, int64_t stride_row, int rows, int channels,
+                           uint8_t *__restrict__ out, float *__restrict__ row_scale) {
+  const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const __nv_bfloat16 *src = x + row * stride_row;
+  Elem<__nv_bfloat16>::Raw raw[kChunks];
+#pragma unroll
+  for (int i = 0; i < kChunks; ++i) {
+    const int c0 = (i * 32 + lane) * 8;
+    raw[i] = c0 < channels ? Elem<__nv_bfloat16>::load_raw(src + c0) : Elem<__nv_bfloat16>::zero_raw();
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < kChunks; ++i) {
+    float v[8];
+    Elem<__nv_bfloat16>::unpack(raw[i], v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
+  }
+  amax = warp_max(amax);
+  const float scale = fmaxf(__fdiv_rn(amax, 448.0f), 1.0e-20f);
+  if (lane == 0) row_scale[row] = scale;
+  const SharedDivisor by_scale = make_divisor(scale);
+  uint8_t *dst = out + static_cast<int64_t>(row) * channels;
+  auto emit = [&](auto exact_tag) {
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+      const int c0 = (i * 32 + lane) * 8;
+      float v[8];
+      Elem<__nv_bfloat16>::unpack(raw[i], v);
+      if (c0 < channels) *reinterpret_cast<uint2 *>(dst + c0) = row_codes8<decltype(exact_tag)::value>(by_scale, v);
+    }
+  };
+  if (by_scale.exact) emit(std::true_type{}); else emit(std::false_type{});
+}
 
 constexpr int kRowQuantThreads = 256;
 constexpr int kRowQuantMaxChunks = 8;  // 16-byte loads per thread: rows of up to 16384 channels
@@ -365,17 +434,7 @@ quant_rows_fp8_kernel(const __nv_bfloat16 *__restrict__ x, int64_t stride_row, i
         if (c0 < channels) {
           float v[8];
           Elem<__nv_bfloat16>::unpack(raw[i], v);
-          uint32_t word[2];
-#pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            uint16_t lo, hi;
-            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(lo)
-                : "f"(divide<kExact>(by_scale, v[4 * w + 1])), "f"(divide<kExact>(by_scale, v[4 * w])));
-            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(hi)
-                : "f"(divide<kExact>(by_scale, v[4 * w + 3])), "f"(divide<kExact>(by_scale, v[4 * w + 2])));
-            word[w] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
-          }
-          *reinterpret_cast<uint2 *>(out + static_cast<int64_t>(row) * channels + c0) = make_uint2(word[0], word[1]);
+          *reinterpret_cast<uint2 *>(out + static_cast<int64_t>(row) * channels + c0) = row_codes8<kExact>(by_scale, v);
         }
       }
     };
@@ -527,6 +586,17 @@ int h3s_quant_rows_fp8(const void *x_bf16, int64_t x_stride_row, int rows, int c
   H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(x_bf16) & 15) == 0 && x_stride_row % 8 == 0 && x_stride_row >= channels,
                 "quant_rows_fp8: input must be 16-byte aligned with a row stride that is a multiple of 8");
   H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(out) & 7) == 0, "quant_rows_fp8: output must be 8-byte aligned");
+  const __nv_bfloat16 *bf16 = static_cast<const __nv_bfloat16 *>(x_bf16);
+#define H3S_LAUNCH_ROWS(CHUNKS)                                                                                  \
+  quant_rows_fp8_warp_kernel<CHUNKS><<<ceil_div(rows, kRowWarps), kRowWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>( \
+      bf16, x_stride_row, rows, channels, out, row_scale)
+  if (channels <= 4096) {
+    if (channels <= 1024) H3S_LAUNCH_ROWS(4); else if (channels <= 2048) H3S_LAUNCH_ROWS(8);
+    else if (channels <= 3072) H3S_LAUNCH_ROWS(12); else H3S_LAUNCH_ROWS(16);
+    H3S_CHECK_CUDA(cudaGetLastError());
+    return H3S_OK;
+  }
+#undef H3S_LAUNCH_ROWS
   const int grid = rows < 148 * 8 ? rows : 148 * 8;
   quant_rows_fp8_kernel<<<grid, kRowQuantThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16 *>(x_bf16), x_stride_row, rows, channels, out, row_scale);
