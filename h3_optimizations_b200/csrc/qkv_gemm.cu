@@ -2,8 +2,8 @@
 //
 //   convrot_quant_rows : x (rows, hidden) bf16 -> Hadamard-256 on every
 //                        256-channel group (fast Walsh-Hadamard in registers
-//                        and warp shuffles), per-row INT8 (scale = amax/127).
-//                        HBM-bound, one warp per 256-channel group.
+//                        across one pass through shared memory), per-row INT8
+//                        (scale = amax/127).  HBM-bound, one warp per row.
 //   qkv_gemm_chunk     : persistent warp-specialised tcgen05 GEMM
 //                        acc[rows, n] = x_i8 . w_i8^T (kind::i8, int32 in TMEM),
 //                        256x256 tiles on a pair of SMs (cta_group::2), K step 128
@@ -50,66 +50,93 @@ __device__ __forceinline__ void fwht8(float (&v)[8]) {
   }
 }
 
-__global__ void __launch_bounds__(384)
+// One warp per row.  The three low index bits are transformed as loaded (8 channels a lane);
+// the row then crosses shared memory once, so that a lane holds the 32 values that share
+// their low bits and the five remaining stages are additions of its own registers.  With
+// those stages as warp shuffles (40 per 8 channels) and a row spread over all warps of a CTA
+// (two barriers a row), 4096 rows of 3072 channels took
+// 24.5 us, 21.4 us now.
+// Shared memory of a warp: [32 upper indices][8 * groups + 4 floats]; the padding puts
+// the 16-byte stores of eight lanes into different banks.
+constexpr int kRotWarps = 4;    // rows (warps) per CTA
+constexpr int kRotAhead = 6;    // 16-byte loads of a lane in flight
+
+__host__ __device__ constexpr int rot_stride(int groups) { return 8 * groups + 4; }
+
+__global__ void __launch_bounds__(kRotWarps * 32)
 convrot_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_stride, int rows, int hidden,
                           int8_t *__restrict__ out, float *__restrict__ scale_out) {
-  extern __shared__ float warp_amax[];  // one per warp
+  extern __shared__ __align__(16) float rot_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int groups = hidden / kRotGroup;  // == warps per CTA
-  // the next row's 16 bytes are requested before this row is transformed, so every
-  // thread keeps two loads in flight across the row's two barriers
-  const __nv_bfloat16 *column = x + warp * kRotGroup + lane * 8;
-  Elem<__nv_bfloat16>::Raw ahead = blockIdx.x < rows ? Elem<__nv_bfloat16>::load_raw(column + blockIdx.x * x_stride)
-                                                     : Elem<__nv_bfloat16>::zero_raw();
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    float v[8];
-    Elem<__nv_bfloat16>::unpack(ahead, v);
-    const int next = row + gridDim.x;
-    if (next < rows) ahead = Elem<__nv_bfloat16>::load_raw(column + static_cast<int64_t>(next) * x_stride);
-    fwht8(v);
+  const int groups = hidden / kRotGroup, stride = rot_stride(groups);
+  float *mine = rot_smem + warp * 32 * stride;
+  const int row = blockIdx.x * kRotWarps + warp;
+  if (row >= rows) return;  // warps of a CTA do not meet
+  const __nv_bfloat16 *src = x + row * x_stride + lane * 8;
+  for (int g0 = 0; g0 < groups; g0 += kRotAhead) {
+    Elem<__nv_bfloat16>::Raw raw[kRotAhead];
 #pragma unroll
-    for (int bit = 0; bit < 5; ++bit) {
-      const bool upper = (lane >> bit) & 1;
+    for (int i = 0; i < kRotAhead; ++i)
+      raw[i] = g0 + i < groups ? Elem<__nv_bfloat16>::load_raw(src + (g0 + i) * kRotGroup) : Elem<__nv_bfloat16>::zero_raw();
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float other = __shfl_xor_sync(0xffffffffu, v[i], 1 << bit);
-        v[i] = upper ? __fsub_rn(other, v[i]) : __fadd_rn(v[i], other);
+    for (int i = 0; i < kRotAhead; ++i) {
+      if (g0 + i < groups) {
+        float v[8];
+        Elem<__nv_bfloat16>::unpack(raw[i], v);
+        fwht8(v);
+        float4 *dst = reinterpret_cast<float4 *>(mine + lane * stride + (g0 + i) * 8);
+        dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+        dst[1] = make_float4(v[4], v[5], v[6], v[7]);
       }
     }
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[i] *= 0.0625f;  // 1/sqrt(256), exact
-      amax = fmaxf(amax, fabsf(v[i]));
-    }
-    amax = warp_max(amax);
-    __syncthreads();  // previous row's readers are done
-    if (lane == 0) warp_amax[warp] = amax;
-    __syncthreads();
-    amax = warp_amax[0];
-    for (int w = 1; w < groups; ++w) amax = fmaxf(amax, warp_amax[w]);
-    const float scale = amax > 0.f ? __fdiv_rn(amax, 127.0f) : 1.0f;
-    const SharedDivisor by_scale = make_divisor(scale);  // exact v/scale without a divide per element
-    uint32_t packed[2] = {0u, 0u};
-    if (by_scale.exact) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        int code = __float2int_rn(divide<true>(by_scale, v[i]));
-        code = max(-127, min(127, code));
-        packed[i >> 2] |= (static_cast<uint32_t>(code) & 0xffu) << ((i & 3) * 8);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        int code = __float2int_rn(divide<false>(by_scale, v[i]));
-        code = max(-127, min(127, code));
-        packed[i >> 2] |= (static_cast<uint32_t>(code) & 0xffu) << ((i & 3) * 8);
-      }
-    }
-    *reinterpret_cast<uint2 *>(out + static_cast<int64_t>(row) * hidden + warp * kRotGroup + lane * 8) =
-        make_uint2(packed[0], packed[1]);
-    if (threadIdx.x == 0) scale_out[row] = scale;
   }
+  __syncwarp();
+  float amax = 0.f;
+  for (int c = lane; c < 8 * groups; c += 32) {  // (group, low bits)
+    float v[32];
+#pragma unroll
+    for (int l = 0; l < 32; ++l) v[l] = mine[l * stride + c];
+#pragma unroll
+    for (int step = 1; step < 32; step <<= 1) {
+#pragma unroll
+      for (int l = 0; l < 32; ++l) {
+        if ((l & step) == 0) {
+          const float a = v[l], b = v[l + step];
+          v[l] = __fadd_rn(a, b);
+          v[l + step] = __fsub_rn(a, b);
+        }
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < 32; ++l) {
+      v[l] *= 0.0625f;  // 1/sqrt(256), exact
+      amax = fmaxf(amax, fabsf(v[l]));
+      mine[l * stride + c] = v[l];
+    }
+  }
+  amax = warp_max(amax);
+  __syncwarp();
+  const float scale = amax > 0.f ? __fdiv_rn(amax, 127.0f) : 1.0f;
+  if (lane == 0) scale_out[row] = scale;
+  const SharedDivisor by_scale = make_divisor(scale);  // exact v/scale without a divide per element
+  int8_t *dst = out + static_cast<int64_t>(row) * hidden + lane * 8;
+  auto emit = [&](auto exact_tag) {
+#pragma unroll 2
+    for (int g = 0; g < groups; ++g) {
+      const float4 *at = reinterpret_cast<const float4 *>(mine + lane * stride + g * 8);
+      const float4 lo = at[0], hi = at[1];
+      const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      uint32_t packed[2] = {0u, 0u};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        int code = __float2int_rn(divide<decltype(exact_tag)::value>(by_scale, v[i]));
+        code = max(-127, min(127, code));
+        packed[i >> 2] |= (static_cast<uint32_t>(code) & 0xffu) << ((i & 3) * 8);
+      }
+      *reinterpret_cast<uint2 *>(dst + g * kRotGroup) = make_uint2(packed[0], packed[1]);
+    }
+  };
+  if (by_scale.exact) emit(std::true_type{}); else emit(std::false_type{});
 }
 
 // ---------------------------------------------------------------------------
@@ -194,11 +221,11 @@ struct GemmParams {
   int32_t *status;
   int rows, n_out, hidden;
   int m_pairs, n_tiles;  // pairs of 128-row tiles, 256-column tiles
-  // Column tiles are visited in the order (i * n_step) % n_tiles (n_step coprime with
-  // n_tiles, about a third of it): weight rows are ordered [Q | K | V], so consecutive
-  // tiles of a CTA alternate between the three kinds and the costlier epilogues of
-  // one kind spread out instead of arriving in a row.
-  int n_step;
+  // Column tiles are visited in the order of the weight rows, [Q | K | V]: the tiles that are
+  // dearer in the epilogue (norm, rotation, quantisation) are dealt out first, the cheap
+  // V tiles even out what is left.  Alternating between the kinds, as suits a kernel that is
+  // bound by its MMAs, left some pairs of SMs with seven dear tiles and others with four
+  // (4096 rows with norm and rotation, together with the spills below: 174 -> 159 us).
   // optional per-head RMS norm (+ split-half rotation) of the Q and K groups
   const float *q_norm;    // (128) or null: no norm, no rotation
   const float *k_norm;    // (128)
@@ -329,7 +356,7 @@ __device__ __forceinline__ void quantise8(const uint4 &raw, const SharedDivisor 
 // form is decided once per row, so that the loads of a batch are all in flight together
 // and the first batch travels while the norm is computed.  With the decision inside the
 // element loop, and one chain of dependent FP64 additions, a 4096-row chunk of the QKV
-// projection with norm and rotation took 197 us, 184 us now.
+// projection with norm and rotation took 197 us, 159 us now.
 enum RopeForm { kRopeNone, kRopeBf16, kRopeF32, kRopeStrided };
 
 __device__ __forceinline__ void rotate_pair(uint32_t &first, uint32_t &second, const float (&f)[2][4]) {
@@ -400,6 +427,25 @@ __device__ __forceinline__ void norm_rope_packed(uint32_t (&y)[H3S_HEAD_DIM / 2]
   }
 }
 
+// Tables of any strides.  A call of its own with the row in local memory: unrolled in place,
+// its addresses took registers from the common forms, which then spilled 336 bytes a thread.
+__device__ __noinline__ void rotate_strided(uint32_t *row, const void *rope_row, int rope_dtype, int64_t stride_dim,
+                                            int64_t stride_rot, int64_t stride_pair) {
+#pragma unroll 1
+  for (int i = 0; i < 24; ++i) {
+    float f[2][4];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int64_t at = (2 * i + e) * stride_dim;
+      f[e][0] = rope_load(rope_row, at, rope_dtype);
+      f[e][1] = rope_load(rope_row, at + stride_pair, rope_dtype);
+      f[e][2] = rope_load(rope_row, at + stride_rot, rope_dtype);
+      f[e][3] = rope_load(rope_row, at + stride_rot + stride_pair, rope_dtype);
+    }
+    rotate_pair(row[i], row[i + 24], f);
+  }
+}
+
 __device__ __forceinline__ void norm_rope_row(uint32_t (&y)[H3S_HEAD_DIM / 2], const float *__restrict__ norm_weight,
                                               float epsilon, const void *rope_row, int rope_dtype,
                                               int64_t stride_dim, int64_t stride_rot, int64_t stride_pair) {
@@ -412,19 +458,12 @@ __device__ __forceinline__ void norm_rope_row(uint32_t (&y)[H3S_HEAD_DIM / 2], c
   if (form == kRopeF32) return norm_rope_packed<kRopeF32>(y, norm_weight, epsilon, static_cast<const uint4 *>(rope_row));
   norm_row(y, norm_weight, epsilon);
   if (form == kRopeNone) return;
+  uint32_t row[H3S_HEAD_DIM / 2];
 #pragma unroll
-  for (int i = 0; i < 24; ++i) {
-    float f[2][4];
+  for (int i = 0; i < H3S_HEAD_DIM / 2; ++i) row[i] = y[i];
+  rotate_strided(row, rope_row, rope_dtype, stride_dim, stride_rot, stride_pair);
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int64_t at = (2 * i + e) * stride_dim;
-      f[e][0] = rope_load(rope_row, at, rope_dtype);
-      f[e][1] = rope_load(rope_row, at + stride_pair, rope_dtype);
-      f[e][2] = rope_load(rope_row, at + stride_rot, rope_dtype);
-      f[e][3] = rope_load(rope_row, at + stride_rot + stride_pair, rope_dtype);
-    }
-    rotate_pair(y[i], y[i + 24], f);
-  }
+  for (int i = 0; i < H3S_HEAD_DIM / 2; ++i) y[i] = row[i];
 }
 
 // Tile `tile` of the persistent order: row pair and column tile
@@ -435,7 +474,7 @@ __device__ __forceinline__ void tile_position(const GemmParams &prm, int tile, i
   const int height = min(kGemmGroupM, prm.m_pairs - first);
   const int column = within / height;
   pair = first + within - column * height;
-  tn = column * prm.n_step % prm.n_tiles;
+  tn = column;
 }
 
 template <int kMode>
@@ -985,9 +1024,10 @@ int h3s_convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hi
   H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && x_stride_row % 8 == 0 && x_stride_row >= hidden,
                 "convrot_quant_rows: input must be 16-byte aligned with a row stride that is a multiple of 8");
   H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(x_i8) & 7) == 0, "convrot_quant_rows: output must be 8-byte aligned");
-  const int groups = hidden / kRotGroup;
-  const int grid = rows < 148 * 8 ? rows : 148 * 8;
-  convrot_quant_rows_kernel<<<grid, groups * 32, groups * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
+  const int smem = kRotWarps * 32 * rot_stride(hidden / kRotGroup) * static_cast<int>(sizeof(float));
+  constexpr int kMostSmem = kRotWarps * 32 * rot_stride(32) * static_cast<int>(sizeof(float));  // 133 KB; one value for all callers
+  H3S_CHECK_CUDA(cudaFuncSetAttribute(convrot_quant_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
+  convrot_quant_rows_kernel<<<ceil_div(rows, kRotWarps), kRotWarps * 32, smem, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16 *>(x), x_stride_row, rows, hidden, x_i8, x_scale);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
@@ -1047,13 +1087,6 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
   prm.out_stride_head = out_stride_head; prm.status = status;
   prm.rows = rows; prm.n_out = n_out; prm.hidden = hidden;
   prm.m_pairs = ceil_div(rows, kGemmPairM); prm.n_tiles = ceil_div(n_out, kGemmN);
-  prm.n_step = 1;
-  if (carriers != nullptr) {
-    auto gcd = [](int a, int b) { while (b) { const int t = a % b; a = b; b = t; } return a; };
-    int step = prm.n_tiles / 3 + 1;
-    while (step > 1 && gcd(step, prm.n_tiles) != 1) --step;
-    prm.n_step = step;
-  }
   prm.q_norm = q_norm; prm.k_norm = k_norm; prm.rope = rope; prm.rope_dtype = rope_dtype;
   prm.rope_stride_seq = rope ? rope_strides[0] : 0; prm.rope_stride_dim = rope ? rope_strides[1] : 0;
   prm.rope_stride_rot = rope ? rope_strides[2] : 0; prm.rope_stride_pair = rope ? rope_strides[3] : 0;
@@ -1137,7 +1170,7 @@ int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_
   memset(&prm, 0, sizeof(prm));
   prm.x_scale = row_scale; prm.status = status;
   prm.rows = rows; prm.n_out = n_out; prm.hidden = k_bytes;
-  prm.m_pairs = ceil_div(rows, kGemmPairM); prm.n_tiles = ceil_div(n_out, kGemmN); prm.n_step = 1;
+  prm.m_pairs = ceil_div(rows, kGemmPairM); prm.n_tiles = ceil_div(n_out, kGemmN);
   prm.heads = 1; prm.wait_budget_ns = wait_budget_ns();
   prm.operand_kind = operand_kind; prm.row_scale = row_scale; prm.col_scale = col_scale; prm.bias = bias;
   prm.vector_columns = ((reinterpret_cast<uintptr_t>(col_scale) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0;
