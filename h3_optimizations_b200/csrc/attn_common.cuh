@@ -70,24 +70,6 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volati
   return __all_sync(0xffffffffu, ok);
 }
 
-// packed fp32x2 arithmetic (one instruction for two lanes of a 64-bit register pair)
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(reinterpret_cast<unsigned long long &>(d))
-      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)),
-        "l"(reinterpret_cast<unsigned long long &>(c)));
-  return d;
-}
-
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("add.f32x2 %0, %1, %2;"
-      : "=l"(reinterpret_cast<unsigned long long &>(d))
-      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
-  return d;
-}
-
 template <typename OutT> __device__ __forceinline__ void store_out8(OutT *dst, const float (&v)[8]);
 template <> __device__ __forceinline__ void store_out8<float>(float *dst, const float (&v)[8]) {
   reinterpret_cast<float4 *>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);

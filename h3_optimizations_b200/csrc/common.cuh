@@ -98,6 +98,39 @@ struct Elem<__half> {
   }
 };
 
+// Packed fp32x2 arithmetic: one instruction for the two halves of a 64-bit register pair, each
+// rounded as by itself.  The quantisers are bound by the instructions they issue (K of 24
+// heads x 33272 tokens 75 -> 70 us); the GEMM epilogues, bound by latency, gain 1 to 3 %.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long &>(d))
+      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)),
+        "l"(reinterpret_cast<unsigned long long &>(c)));
+  return d;
+}
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long &>(d))
+      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
+  return d;
+}
+
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long &>(d))
+      : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
+  return d;
+}
+
+// the two bf16 of a word
+__device__ __forceinline__ float2 bf16_pair(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
 // Correctly rounded a/b for many a and one b: with r = RN(1/b),
 //   q0 = RN(a*r), e = a - b*q0 (exact in an FMA), q = RN(q0 + e*r)
 // equals RN(a/b) (Markstein) unless b's significand is all ones, where RN(1/b)
@@ -125,6 +158,23 @@ __device__ __forceinline__ float divide(const SharedDivisor &d, float a) {
   const float q0 = __fmul_rn(a, d.r);
   const float e = __fmaf_rn(-d.b, q0, a);
   return __fmaf_rn(e, d.r, q0);
+}
+
+template <bool kExact>
+__device__ __forceinline__ float2 divide2(const SharedDivisor &d, float2 a) {
+  if (!kExact) return make_float2(__fdiv_rn(a.x, d.b), __fdiv_rn(a.y, d.b));
+  const float2 r = make_float2(d.r, d.r), minus_b = make_float2(-d.b, -d.b);
+  const float2 q0 = mul2(a, r);
+  return fma2(fma2(minus_b, q0, a), r, q0);
+}
+
+// trunc(q +- 0.5), the half with q's sign
+__device__ __forceinline__ void round_codes(float2 q, uint32_t &first, uint32_t &second) {
+  const float2 half = make_float2(__uint_as_float((__float_as_uint(q.x) & 0x80000000u) | 0x3f000000u),
+                                  __uint_as_float((__float_as_uint(q.y) & 0x80000000u) | 0x3f000000u));
+  q = add2(q, half);
+  first = static_cast<uint32_t>(static_cast<int>(q.x));
+  second = static_cast<uint32_t>(static_cast<int>(q.y));
 }
 
 // 8 E4M3 codes -> the same values as BF16 (exact: four significant bits)

@@ -285,11 +285,12 @@ __device__ __forceinline__ void dense_row32(const uint32_t (&acc)[32], float row
     const float c[4] = {cs.x, cs.y, cs.z, cs.w}, b[4] = {shift.x, shift.y, shift.z, shift.w};
     float v[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float value = __fmul_rn(__uint_as_float(acc[i + e]), __fmul_rn(row_scale, c[e]));
-      if (kBias) value = __fadd_rn(value, b[e]);
-      if (kGelu) value = gelu_tanh(value);
-      v[e] = value;
+    for (int e = 0; e < 4; e += 2) {
+      float2 value = mul2(make_float2(__uint_as_float(acc[i + e]), __uint_as_float(acc[i + e + 1])),
+                          mul2(make_float2(row_scale, row_scale), make_float2(c[e], c[e + 1])));
+      if (kBias) value = add2(value, make_float2(b[e], b[e + 1]));
+      v[e] = kGelu ? gelu_tanh(value.x) : value.x;
+      v[e + 1] = kGelu ? gelu_tanh(value.y) : value.y;
     }
     y[i >> 1] = pack_bf16x2(v[0], v[1]);
     y[(i >> 1) + 1] = pack_bf16x2(v[2], v[3]);
@@ -330,12 +331,7 @@ __device__ __forceinline__ void quantise8(const uint4 &raw, const SharedDivisor 
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
   uint32_t code[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float q = divide<kExact>(by_scale, (i & 1) ? bf16_hi(w[i >> 1]) : bf16_lo(w[i >> 1]));
-    const float half_ulp = __uint_as_float((__float_as_uint(q) & 0x80000000u) | 0x3f000000u);  // +-0.5
-    q = __fadd_rn(q, half_ulp);
-    code[i] = static_cast<uint32_t>(static_cast<int>(q));  // truncation toward zero
-  }
+  for (int i = 0; i < 4; ++i) round_codes(divide2<kExact>(by_scale, bf16_pair(w[i])), code[2 * i], code[2 * i + 1]);
   uint32_t packed[2];
 #pragma unroll
   for (int k = 0; k < 2; ++k)
@@ -356,19 +352,15 @@ __device__ __forceinline__ void quantise8(const uint4 &raw, const SharedDivisor 
 // form is decided once per row, so that the loads of a batch are all in flight together
 // and the first batch travels while the norm is computed.  With the decision inside the
 // element loop, and one chain of dependent FP64 additions, a 4096-row chunk of the QKV
-// projection with norm and rotation took 197 us, 159 us now.
+// projection with norm and rotation took 197 us, 158 us now.
 enum RopeForm { kRopeNone, kRopeBf16, kRopeF32, kRopeStrided };
 
 __device__ __forceinline__ void rotate_pair(uint32_t &first, uint32_t &second, const float (&f)[2][4]) {
-  const float a[2] = {bf16_lo(first), bf16_hi(first)}, b[2] = {bf16_lo(second), bf16_hi(second)};
-  float out_first[2], out_second[2];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    out_first[e] = __fadd_rn(__fmul_rn(f[e][0], a[e]), __fmul_rn(f[e][1], b[e]));
-    out_second[e] = __fadd_rn(__fmul_rn(f[e][2], a[e]), __fmul_rn(f[e][3], b[e]));
-  }
-  first = pack_bf16x2(out_first[0], out_first[1]);
-  second = pack_bf16x2(out_second[0], out_second[1]);
+  const float2 a = bf16_pair(first), b = bf16_pair(second);
+  const float2 out_first = add2(mul2(make_float2(f[0][0], f[1][0]), a), mul2(make_float2(f[0][1], f[1][1]), b));
+  const float2 out_second = add2(mul2(make_float2(f[0][2], f[1][2]), a), mul2(make_float2(f[0][3], f[1][3]), b));
+  first = pack_bf16x2(out_first.x, out_first.y);
+  second = pack_bf16x2(out_second.x, out_second.y);
 }
 
 __device__ __forceinline__ void norm_row(uint32_t (&y)[H3S_HEAD_DIM / 2], const float *__restrict__ norm_weight,
@@ -386,8 +378,8 @@ __device__ __forceinline__ void norm_row(uint32_t (&y)[H3S_HEAD_DIM / 2], const 
 #pragma unroll
   for (int i = 0; i < H3S_HEAD_DIM / 2; ++i) {
     const float2 w = __ldg(reinterpret_cast<const float2 *>(norm_weight) + i);
-    y[i] = pack_bf16x2(__fmul_rn(__fmul_rn(bf16_lo(y[i]), inverse_rms), w.x),
-                       __fmul_rn(__fmul_rn(bf16_hi(y[i]), inverse_rms), w.y));
+    const float2 normed = mul2(mul2(bf16_pair(y[i]), make_float2(inverse_rms, inverse_rms)), w);
+    y[i] = pack_bf16x2(normed.x, normed.y);
   }
 }
 
@@ -721,6 +713,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           const int local_row = quarter * 32 + lane;
           {
             uint32_t y[H3S_HEAD_DIM / 2];
+            const float2 xs2 = make_float2(xs, xs);
             const float *w_scale = prm.w_scale + (group_ok ? group_col0 : 0);  // without a group nothing is stored
 #pragma unroll
             for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
@@ -730,9 +723,9 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
               for (int i = 0; i < 32; i += 2) {
                 const float2 ws = __ldg(reinterpret_cast<const float2 *>(w_scale + cc * 32 + i));
-                y[cc * 16 + (i >> 1)] =
-                    pack_bf16x2(__fmul_rn(static_cast<float>(static_cast<int>(acc[i])), __fmul_rn(xs, ws.x)),
-                                __fmul_rn(static_cast<float>(static_cast<int>(acc[i + 1])), __fmul_rn(xs, ws.y)));
+                const float2 value = mul2(make_float2(static_cast<float>(static_cast<int>(acc[i])),
+                                                      static_cast<float>(static_cast<int>(acc[i + 1]))), mul2(xs2, ws));
+                y[cc * 16 + (i >> 1)] = pack_bf16x2(value.x, value.y);
               }
             }
             // the accumulator is in registers: the MMA warp may refill it
@@ -795,8 +788,9 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     part[h][2 * i] = fmaxf(part[h][2 * i], fabsf(bf16_lo(w[i])));
                     part[h][2 * i + 1] = fmaxf(part[h][2 * i + 1], fabsf(bf16_hi(w[i])));
                   } else {
-                    part[h][2 * i] = __fadd_rn(part[h][2 * i], bf16_lo(w[i]));
-                    part[h][2 * i + 1] = __fadd_rn(part[h][2 * i + 1], bf16_hi(w[i]));
+                    const float2 sum = add2(make_float2(part[h][2 * i], part[h][2 * i + 1]), bf16_pair(w[i]));
+                    part[h][2 * i] = sum.x;
+                    part[h][2 * i + 1] = sum.y;
                     if (quantise_here) {  // magnitudes two at a time: clear both sign bits, packed bf16 maximum
                       const uint32_t magnitude = w[i] & 0x7fff7fffu;
                       top[h] = __hmax2(top[h], *reinterpret_cast<const __nv_bfloat162 *>(&magnitude));

@@ -132,18 +132,21 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
   const int first_row = local_block * BLOCK;  // within this chunk
   const int valid_rows = min(BLOCK, rows - first_row);
 
-  float mu[8];
+  float2 minus_mu[4];  // x - mu == x + (-mu)
 #pragma unroll
-  for (int i = 0; i < 8; ++i) mu[i] = 0.f;
+  for (int i = 0; i < 4; ++i) minus_mu[i] = make_float2(0.f, 0.f);
   if (kHasMean) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) mu[i] = __ldg(mean + head * H3S_HEAD_DIM + c0 + i);
+    for (int i = 0; i < 4; ++i) {
+      const float *mu = mean + head * H3S_HEAD_DIM + c0 + 2 * i;
+      minus_mu[i] = make_float2(-__ldg(mu), -__ldg(mu + 1));
+    }
   }
 
   typename Elem<T>::Raw raw[kPasses];
-  float col[8];  // this thread's rows (at most 8) summed in fp32, widened once
+  float2 col[4];  // this thread's rows (at most 8) summed in fp32, widened once
 #pragma unroll
-  for (int i = 0; i < 8; ++i) col[i] = 0.f;
+  for (int i = 0; i < 4; ++i) col[i] = make_float2(0.f, 0.f);
   float amax = 0.f;
   const T *base = x + head * stride_h + c0;
 #pragma unroll
@@ -159,9 +162,11 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
       float v[8];
       Elem<T>::unpack(raw[p], v);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        col[i] = __fadd_rn(col[i], v[i]);
-        amax = fmaxf(amax, fabsf(kHasMean ? __fsub_rn(v[i], mu[i]) : v[i]));
+      for (int i = 0; i < 4; ++i) {
+        const float2 pair = make_float2(v[2 * i], v[2 * i + 1]);
+        col[i] = add2(col[i], pair);
+        const float2 x = kHasMean ? add2(pair, minus_mu[i]) : pair;
+        amax = fmaxf(amax, fmaxf(fabsf(x.x), fabsf(x.y)));
       }
     }
   }
@@ -169,7 +174,10 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
   if ((threadIdx.x & 31) == 0) warp_amax[threadIdx.x >> 5] = amax;
   if (summary != nullptr) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) red[slot][c0 + i] = static_cast<double>(col[i]);
+    for (int i = 0; i < 4; ++i) {
+      red[slot][c0 + 2 * i] = static_cast<double>(col[i].x);
+      red[slot][c0 + 2 * i + 1] = static_cast<double>(col[i].y);
+    }
   }
   __syncthreads();
   amax = warp_amax[0];
@@ -196,11 +204,9 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
         Elem<T>::unpack(raw[p], v);
         uint32_t code[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float q = divide<kExact>(by_scale, kHasMean ? __fsub_rn(v[i], mu[i]) : v[i]);
-          const float half = __uint_as_float((__float_as_uint(q) & 0x80000000u) | 0x3f000000u);
-          q = __fadd_rn(q, half);
-          code[i] = static_cast<uint32_t>(static_cast<int>(q));  // truncation toward zero
+        for (int i = 0; i < 4; ++i) {
+          const float2 pair = make_float2(v[2 * i], v[2 * i + 1]);
+          round_codes(divide2<kExact>(by_scale, kHasMean ? add2(pair, minus_mu[i]) : pair), code[2 * i], code[2 * i + 1]);
         }
         uint32_t packed[2];
 #pragma unroll
@@ -266,15 +272,17 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
   const int slot = threadIdx.x >> 4;
   const int c0 = (threadIdx.x & 15) * 8;
 
-  float sc[8], rc[8];
+  float2 sc[4], rc[4], minus_sc[4];
   bool all_exact = true;
   const bool clamp = v_bound < 448.0f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    sc[i] = fmaxf(__ldg(v_scale + head * H3S_HEAD_DIM + c0 + i), 1.0e-20f);
-    const SharedDivisor d = make_divisor(sc[i]);
-    rc[i] = d.r;
-    all_exact = all_exact && d.exact;
+  for (int i = 0; i < 4; ++i) {
+    const float *scale = v_scale + head * H3S_HEAD_DIM + c0 + 2 * i;
+    const SharedDivisor a = make_divisor(fmaxf(__ldg(scale), 1.0e-20f)), b = make_divisor(fmaxf(__ldg(scale + 1), 1.0e-20f));
+    sc[i] = make_float2(a.b, b.b);
+    minus_sc[i] = make_float2(-a.b, -b.b);
+    rc[i] = make_float2(a.r, b.r);
+    all_exact = all_exact && a.exact && b.exact;
   }
 
   const T *base = v + head * stride_h + c0;
@@ -303,15 +311,19 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
       float x[8];
       Elem<T>::unpack(raw[p][j], x);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < 4; ++i) {
+        const float2 pair = make_float2(x[2 * i], x[2 * i + 1]);
+        float2 y;
         if (kExact) {  // shared-divisor division, see SharedDivisor
-          const float q0 = __fmul_rn(x[i], rc[i]);
-          q[j][i] = __fmaf_rn(__fmaf_rn(-sc[i], q0, x[i]), rc[i], q0);
+          const float2 q0 = mul2(pair, rc[i]);
+          y = fma2(fma2(minus_sc[i], q0, pair), rc[i], q0);
         } else {
-          q[j][i] = __fdiv_rn(x[i], sc[i]);
+          y = make_float2(__fdiv_rn(pair.x, sc[i].x), __fdiv_rn(pair.y, sc[i].y));
         }
         // the conversion saturates at +-448 by itself; a tighter bound is applied here
-        if (clamp) q[j][i] = fminf(fmaxf(q[j][i], -v_bound), v_bound);
+        if (clamp) y = make_float2(fminf(fmaxf(y.x, -v_bound), v_bound), fminf(fmaxf(y.y, -v_bound), v_bound));
+        q[j][2 * i] = y.x;
+        q[j][2 * i + 1] = y.y;
       }
     }
     uint32_t word[8];
@@ -362,10 +374,10 @@ __device__ __forceinline__ uint2 row_codes8(const SharedDivisor &by_scale, const
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
     uint16_t lo, hi;
-    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(lo)
-        : "f"(divide<kExact>(by_scale, v[4 * w + 1])), "f"(divide<kExact>(by_scale, v[4 * w])));
-    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(hi)
-        : "f"(divide<kExact>(by_scale, v[4 * w + 3])), "f"(divide<kExact>(by_scale, v[4 * w + 2])));
+    const float2 a = divide2<kExact>(by_scale, make_float2(v[4 * w], v[4 * w + 1]));
+    const float2 b = divide2<kExact>(by_scale, make_float2(v[4 * w + 2], v[4 * w + 3]));
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(lo) : "f"(a.y), "f"(a.x));
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(hi) : "f"(b.y), "f"(b.x));
     word[w] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
   }
   return make_uint2(word[0], word[1]);
