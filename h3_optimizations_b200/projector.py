@@ -158,7 +158,10 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
                                       chunk_rows=chunk_rows, smooth_k=smooth_k, q_norm=q_norm, k_norm=k_norm,
                                       epsilon=float(epsilon), rope=rope_freqs, status=status, v_bound=V_QUANT_BOUND)
         finally:
-            side.join(stream)  # on every exit path, before the staging can be freed
+            # on every exit path, before the staging can be freed; without smoothing the second
+            # stream has not been forked, and a capture must not wait for a stream outside it
+            if smooth_k:
+                side.join(stream)
         del scratch
     except _native.NativeError as exc:
         raise FusedQKVError("chunked QKV projection failed: layer=%d: %s" % (layer_index, exc)) from exc
