@@ -75,7 +75,8 @@ struct HalfShared {
   uint64_t p_full[2];          // P(j) is in TMEM
   uint64_t pv_done[2];         // P.V of tile j has completed: its stage and its slot are free
   uint64_t first_max;          // group 0 has left the first tile's row maxima in `row`
-  uint64_t pass_end;           // row sums (or maxima) of a pass are in `row`, `again` is valid; all warps wait
+  uint64_t pass_end;           // row sums (or maxima) of a pass are in `row`, `again` is valid; all warps wait,
+                               // and the P.V warp arrives too: see there
   uint64_t staged;             // softmax warps only: the output tile is in shared memory (and steps before that)
   uint32_t tmem_base;
   int abort_word;
@@ -180,7 +181,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       ptx::mbar_init(&sh.pv_done[g], 1);
     }
     ptx::mbar_init(&sh.first_max, 4);
-    ptx::mbar_init(&sh.pass_end, kHSoftmaxWarps);
+    ptx::mbar_init(&sh.pass_end, kHSoftmaxWarps + 1);
     ptx::mbar_init(&sh.staged, kHSoftmaxWarps);
     sh.abort_word = 0;
     sh.again = 0;
@@ -301,6 +302,10 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         __syncwarp();
       }
       done += n_iter;
+      // Lists of one or two tiles: nothing in the next pass up to its own pass_end waits for this
+      // warp, so that without its arrival here two passes could end before it looks, and the
+      // parity it waits for would be that of a third.
+      if (ok && lane == 0) ptx::mbar_arrive(&sh.pass_end);
       ok = ok && warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
       if (pass == 2 || (pass == 0 && sh.again == 0)) break;
     }
