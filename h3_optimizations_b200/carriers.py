@@ -34,7 +34,7 @@ class PreparedFusedQKV:
     smooth_k: bool = False
     v_carrier: torch.Tensor | None = None
     v_scale: torch.Tensor | None = None
-    v_half: torch.Tensor | None = None  # BF16 copy of v_carrier (optional: the attention call makes it otherwise)
+    v_half: torch.Tensor | None = None  # FP16 copy of v_carrier (optional: the attention call makes it otherwise)
 
 
 def _carrier_spec(prepared):
@@ -117,7 +117,7 @@ class PreparedSparse:
     sequence: int
     heads: int
     metadata: dict = field(default_factory=dict)
-    v_half: torch.Tensor | None = None  # BF16 copy of v_carrier
+    v_half: torch.Tensor | None = None  # FP16 copy of v_carrier
 
 
 @dataclass

@@ -48,7 +48,7 @@ struct AttnParams {
 };
 
 // Checks the arguments of an attention launch and fills `params` (attn_tc.cu).  `v` is the V
-// carrier the kernel reads, E4M3 or FP16.
+// carrier the kernel reads, E4M3 or its FP16 copy.
 int fill_attn_params(AttnParams *params, const int8_t *q8, const int8_t *k8, const void *v, const float *q_scale,
                      const float *k_scale, const float *v_scale, const int32_t *route, int route_len, int q_start,
                      int q_stop, void *out, void *const *peer_out, int n_peer_out, int out_dtype, int64_t out_stride_h,

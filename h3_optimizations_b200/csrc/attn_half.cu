@@ -1,4 +1,4 @@
-// Block-sparse attention on INT8 Q/K and a BF16 copy of the FP8 V carrier, for
+// Block-sparse attention on INT8 Q/K and an FP16 copy of the FP8 V carrier, for
 // sm_100a.
 //
 // One CTA owns one 128-row query tile of one head and walks that tile's list
@@ -6,26 +6,40 @@
 //   S = Q8 . K8^T      tcgen05.mma kind::i8, 128x64x128, Q8 in TMEM, int32 in TMEM
 //   P = exp2(c*S - m)  FP32 in registers, one thread per query row, m an integer
 //   O += P16 . V16     tcgen05.mma kind::f16, 128x128x64, P in TMEM, fp32 in TMEM
-// V16 holds the E4M3 codes as BF16 (exact), so the product is that of the FP8
-// carrier; P is rounded once to BF16 (relative error up to 2^-9, the two E4M3
-// terms of attn_tc.cu have 2^-8).
+// V16 holds the E4M3 codes as FP16 (exact), so the product is that of the FP8
+// carrier; P is rounded once to FP16 (relative error up to 2^-11).
 //
-// Why BF16 P instead of two E4M3 terms: the tensor pipe takes the same time for
-// one 16-bit product as for two 8-bit products, but a softmax thread needs one
+// Why FP16 P.  The tensor pipe takes the same time for one 16-bit product as for two
+// 8-bit products (the two E4M3 terms of attn_tc.cu), but a softmax thread needs one
 // packed conversion per pair of scores instead of a mask, a residual and two
-// conversions per score, and BF16's exponent range makes the running maximum
-// unnecessary: m is the row maximum of the first tile and stays.  P may then
-// grow to 2^100 (70 nats above the first tile) before anything is lost; the row
-// sums tell, and a query tile where it happens is done again with the true row
-// maximum (one more pass over the scores to find it).
+// conversions per score.  BF16 would do as well for speed and never overflow, but its
+// eight bits lose precision: against 64-bit arithmetic on the same carriers the
+// outputs of 11 layers (1960 to 33272 tokens, 10 to 100 %) were off by 1.64e-3 to 1.67e-3
+// (relative 2-norm) with BF16, 1.19e-3 to 1.31e-3 with two E4M3 terms, 2.1e-4 to 2.3e-4
+// with FP16.
+//
+// FP16 ends at 2^16 and 2^-24, and there is no running maximum: it would put two serial
+// phases (maximum, O rescale) into every tile.  Instead m is fixed by the first two
+// tiles: their row maximum becomes 2^-5, which leaves the rows 21 bits of room above
+// and puts the last unit 19 bits below (two E4M3 terms: 16 to 19 bits below the largest
+// score).  A row whose sum over a tile passes 65504 leaves that tile out (P = 0), and
+// the tile is noted; when the list is through, O and the row sums are brought to a new m
+// and the noted tiles, and only those, are walked again.  The walk begins in the middle of
+// the list: a routed list has the context in front, and the tiles that were selected for
+// their scores are the better measure.  Of 16 layers with scores of 4 bits standard
+// deviation, held over groups of 64 tokens, 2 to 14 % of the query tiles (27 % in a dense one of
+// 24792 tokens) came round again, with 0.03 to 0.5 % of all tiles; with the first tile of
+// the list and 2^-7 it was 17 to 61 % and 1.5 to 9 %.  What it costs at 24 heads x 33272
+// tokens, 30 %: 3.09 to 3.26 ms on the inputs above; 3.29 to 3.48 with one row of every query
+// tile 48 bits ahead in every 40th tile; 3.78 to 3.94 with a third of the rows ahead in every tenth;
+// two E4M3 terms take 4.2 to 4.3 ms of each.  All but the first two tiles of a list
+// ahead is the worst: two walks, three where a sum overflows (120 bits).
 //
 // Without a running maximum the tiles of a row are independent but for the sum:
 // the eight softmax warps form two groups, group g takes tiles g, g+2, ..., and
 // with two CTAs per SM four warps share a scheduler, each in its own phase of
-// wait / load / exponentials / store.  That is what keeps the ex2 pipe (512 cycles
-// per tile and SM) and the tensor pipe (384) busy; with one group, or with two
-// threads per row, the CTAs fall into step and both pipes idle a third of the
-// time.
+// wait / load / exponentials / store.  With one group, or with two threads per row,
+// the CTAs fall into step and both pipes idle a third of the time.
 //
 // TMEM (256 columns per CTA, two CTAs per SM): O 128, Q8 32 (A operand of QK^T:
 // Q is read once instead of with every K tile, which takes a third off the
@@ -43,13 +57,12 @@
 // the list, so that the result does not depend on which one that was.
 //
 // What bounds it: per tile and SM the ex2 pipe needs 512 cycles, the tensor pipe 453
-// (measured: 144 for QK^T with A in TMEM, 258 with A in shared memory, 309 for P.V),
-// the remaining softmax instructions about 290 issue slots; a tile takes 800.  24
-// heads x 33272 tokens at 30 %: 3.81 ms with two E4M3 terms -> 2.88 ms, and 4.20 ->
-// 3.33 ms once the board has reached its power cap (1 kW, 1.7 GHz), which it does
-// after half a second.  Tried and slower: a polynomial for a share of the
-// exponentials, two threads per row, one group per CTA, scores of the next tile
-// fetched between the halves of this one.
+// (measured: 144 for QK^T with A in TMEM, 258 with A in shared memory, 309 for P.V; at
+// the nominal rates 384 in all), the remaining softmax instructions about 290 issue
+// slots; a tile takes about 800.  24 heads x 33272 tokens at 30 %, launches in a row: 4.20 to
+// 4.33 ms with two E4M3 terms, 3.09 to 3.26 ms here.  Tried and slower: a polynomial for a
+// share of the exponentials, two threads per row, one group per CTA, scores of the next
+// tile fetched between the halves of this one.
 #include "attn_common.cuh"
 #include "tma.cuh"
 
@@ -65,7 +78,13 @@ constexpr uint32_t kHOffK = 0;
 constexpr uint32_t kHOffV = kHOffK + kHStages * kHKBytes;
 constexpr uint32_t kHOffBar = kHOffV + kHStages * kHVBytes;
 constexpr uint32_t kHSmemBytes = kHOffBar + 4096 + 1024;  // barriers/scalars + alignment slack
-constexpr float kHSumLimit = 1.2676506e30f;  // 2^100: row sums above this send the query tile round again
+constexpr float kHSumLimit = 65504.f;  // of a row over one tile: no P above it can have overflowed FP16
+constexpr float kHFirstBits = 5.f;     // the reference tiles' row maximum becomes 2^-5 ...
+constexpr float kHMostBits = 15.f;     // ... P may grow to 2^15 ...
+constexpr float kHAgainBits = 8.f;     // ... and the largest sum of a row that did not fit becomes 2^8 at most
+constexpr int kHNoted = 2048;          // bits of the note of tiles left out, each for 2^n neighbours of a longer list
+
+enum { kAgainNoted = 1, kAgainFar = 2 };
 
 struct HalfShared {
   uint64_t q_ready;            // four softmax warps have put the Q rows into TMEM
@@ -74,34 +93,36 @@ struct HalfShared {
   uint64_t s_taken[2];         // S(j) is in registers
   uint64_t p_full[2];          // P(j) is in TMEM
   uint64_t pv_done[2];         // P.V of tile j has completed: its stage and its slot are free
-  uint64_t first_max;          // group 0 has left the first tile's row maxima in `row`
-  uint64_t pass_end;           // row sums (or maxima) of a pass are in `row`, `again` is valid; all warps wait,
+  uint64_t first_max;          // both groups have left their first tile's row maxima in `first`
+  uint64_t pass_end;           // the rows' values of a pass are in `row`, `noted` is complete; all warps wait,
                                // and the P.V warp arrives too: see there
   uint64_t staged;             // softmax warps only: the output tile is in shared memory (and steps before that)
   uint32_t tmem_base;
   int abort_word;
-  int again;                   // some row sum passed the limit
+  int again;                   // kAgainNoted: some row has left out a tile; kAgainFar: its sum there is no number
   int finish;                  // this CTA writes the output tile
   int tile_index[kHStages];    // KV tile held by each stage ...
   float tile_scale[kHStages];  // ... and its k_scale, written by the producer
   float v_scale[H3S_HEAD_DIM];
-  float first[H3S_Q_TILE];
+  uint32_t noted[kHNoted / 32];  // tiles of the list that some row has left out
+  float first[2][H3S_Q_TILE];
   float row[2][2][H3S_Q_TILE];  // values the two threads of a row give each other, in turn
 };
 static_assert(sizeof(HalfShared) <= 4096, "barrier block too large");
 
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
   uint32_t d;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
 
-// Row sum and BF16 P of 64 scores.  The int32 scores become fp32 without a
+// Row sum and, with kPack, FP16 P of 64 scores.  The int32 scores become fp32 without a
 // conversion instruction: for |s| < 2^22, bits(12582912.0f) + s are the bits of
 // the float 12582912 + s exactly, and the offset is folded into the constants of
 // the FMA that follows: P = exp2(c*f + bias) = exp2(c*s - m).
-__device__ __forceinline__ float exp_pack(const uint32_t (&s)[H3S_KV_TILE], float c, float bias,
-                                          uint32_t (&packed)[H3S_KV_TILE / 2]) {
+template <bool kPack>
+__device__ __forceinline__ float exp_sum(const uint32_t (&s)[H3S_KV_TILE], float c, float bias,
+                                         uint32_t (&packed)[H3S_KV_TILE / 2]) {
   const float2 c2 = make_float2(c, c), bias2 = make_float2(bias, bias);
   float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
 #pragma unroll
@@ -110,7 +131,7 @@ __device__ __forceinline__ float exp_pack(const uint32_t (&s)[H3S_KV_TILE], floa
     const float2 x = fma2(c2, f, bias2);
     const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
     if (i & 1) sum_b = add2(sum_b, p); else sum_a = add2(sum_a, p);
-    packed[i] = pack_bf16x2(p.x, p.y);
+    if (kPack) packed[i] = pack_half2(p.x, p.y);
   }
   sum_a = add2(sum_a, sum_b);
   return sum_a.x + sum_a.y;
@@ -124,6 +145,16 @@ __device__ __forceinline__ int max_score(const uint32_t (&s)[H3S_KV_TILE]) {
     b = __vimax3_s32(b, s[i + 2], s[i + 3]);
   }
   return max(__vimax3_s32(a, s[H3S_KV_TILE - 2], s[H3S_KV_TILE - 1]), b);
+}
+
+// Number of tiles the noted bits stand for (whole warp)
+__device__ __forceinline__ int noted_tiles(const uint32_t *noted, int n_iter, int coarse, int lane) {
+  const uint32_t last = static_cast<uint32_t>(n_iter - 1) >> coarse;
+  int bits = 0;
+  for (int w = lane; w < kHNoted / 32; w += 32) bits += __popc(noted[w]);
+  bits = __reduce_add_sync(0xffffffffu, bits) << coarse;
+  const bool ends = (noted[last >> 5] >> (last & 31)) & 1u;  // the last bit may stand for fewer
+  return bits - (ends ? static_cast<int>((last + 1) << coarse) - n_iter : 0);
 }
 
 template <typename OutT>
@@ -180,7 +211,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       ptx::mbar_init(&sh.p_full[g], 4);
       ptx::mbar_init(&sh.pv_done[g], 1);
     }
-    ptx::mbar_init(&sh.first_max, 4);
+    ptx::mbar_init(&sh.first_max, kHSoftmaxWarps);
     ptx::mbar_init(&sh.pass_end, kHSoftmaxWarps + 1);
     ptx::mbar_init(&sh.staged, kHSoftmaxWarps);
     sh.abort_word = 0;
@@ -188,6 +219,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     sh.finish = 1;
     ptx::fence_mbar_init();
   }
+  if (threadIdx.x < kHNoted / 32) sh.noted[threadIdx.x] = 0u;
   if (threadIdx.x < H3S_HEAD_DIM) sh.v_scale[threadIdx.x] = __ldg(prm.v_scale + head * H3S_HEAD_DIM + threadIdx.x);
   if (warp == kHSoftmaxWarps + 1) {
     ptx::tmem_alloc(&sh.tmem_base, kHTmemCols);
@@ -200,12 +232,18 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const uint32_t tmem_q = tmem_o + 128;         // 32 columns, four int8 codes each
   const uint32_t tmem_s = tmem_o + 160;         // slots A B C, 32 columns each
 
-  // Passes over the tile list: one, or three when a row sum passed the limit (the
-  // second only finds the row maxima).  Every warp waits for `pass_end`, so all
-  // agree on `again`.  `done` counts the tiles of earlier passes: stages and
-  // parities run on.
+  // Passes: one over the list; where tiles were left out another one over those, with a
+  // pass for the rows' true maxima in between where a sum has overflowed.  Every warp waits
+  // for `pass_end`, so all agree on the tiles.  `done` counts the tiles of earlier passes:
+  // stages and parities run on.
   bool ok = true;
-  int done = 0;
+  int done = 0, count = n_iter;
+  const int coarse = 32 - __clz((n_iter - 1) / kHNoted);  // a bit of the note stands for 2^coarse tiles
+  auto last_pass = [&]() {
+    const int again = *static_cast<volatile int *>(&sh.again);
+    return again == 0 ? 0 : again & kAgainFar ? 2 : 1;
+  };
+  auto list_position = [&](int i) { return i + n_iter / 2 < n_iter ? i + n_iter / 2 : i + n_iter / 2 - n_iter; };
 
   // wait for tile j's use of one of a pair of barriers (tile j uses number j & 1)
   auto wait_tile = [&](uint64_t (&bar)[2], int j, int code, int factor) {
@@ -232,19 +270,34 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     int my_tile = 0, next_tile = 0, block = -1;  // tile list entries 32*block .. +31, one per lane, and the 32 after
     float my_scale = 0.f, next_scale = 0.f;
     auto fetch_block = [&](int b) {
-      const int mine = min(b * 32 + lane, n_iter - 1);
+      const int mine = list_position(min(b * 32 + lane, n_iter - 1));
       next_tile = dense ? first_tile + mine : __ldg(route_row + mine);
       next_scale = __ldg(k_scale + next_tile);
     };
-    auto load = [&](int i) {      // tile i of the list, into the stage of its running number
-      if (i >= n_iter) return;
-      if ((i >> 5) != block) {
-        block = i >> 5;
-        my_tile = next_tile; my_scale = next_scale;
-        fetch_block(block + 1);
+    int cursor = 0;               // where a later pass goes on in the note
+    auto load = [&](int pass, int i) {  // tile i of the pass, into the stage of its running number
+      if (i >= count) return;
+      int t;
+      float ks;
+      if (pass == 0) {
+        if ((i >> 5) != block) {
+          block = i >> 5;
+          my_tile = next_tile; my_scale = next_scale;
+          fetch_block(block + 1);
+        }
+        t = __shfl_sync(0xffffffffu, my_tile, i & 31);
+        ks = __shfl_sync(0xffffffffu, my_scale, i & 31);
+      } else {
+        for (;;) {  // the next noted tile; there is one, i < count
+          const int bit = cursor >> coarse;
+          const uint32_t w = sh.noted[bit >> 5] >> (bit & 31);
+          if (w & 1u) break;
+          cursor = (w != 0u ? bit + __ffs(w) - 1 : ((bit >> 5) + 1) << 5) << coarse;
+        }
+        const int at = list_position(cursor++);
+        t = dense ? first_tile + at : __ldg(route_row + at);
+        ks = __ldg(k_scale + t);
       }
-      const int t = __shfl_sync(0xffffffffu, my_tile, i & 31);
-      const float ks = __shfl_sync(0xffffffffu, my_scale, i & 31);
       if (lane == 0 && done + i != prm.drop_kv_load) {
         const int s = (done + i) % kHStages;
         sh.tile_index[s] = t;
@@ -256,11 +309,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       __syncwarp();
     };
     for (int pass = 0; ok; ++pass) {
-      block = -1;
-      fetch_block(0);
-      for (int i = 0; i < kHStages; ++i) load(i);
+      cursor = 0;
+      if (pass == 0) fetch_block(0);
+      for (int i = 0; i < kHStages; ++i) load(pass, i);
       if (pass == 0) ok = warp_wait(&sh.q_ready, 0, abort_word, kAbortQFull, prm.wait_budget_ns);
-      for (int i = 0; ok && i < n_iter; ++i) {
+      for (int i = 0; ok && i < count; ++i) {
         const int j = done + i;
         ok = wait_stage(j) && (i < 1 || wait_tile(sh.s_taken, j - 1, kAbortPEmpty, 3)) &&
              (i < 2 || wait_tile(sh.pv_done, j - 2, kAbortPvDone, 4));
@@ -274,40 +327,42 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
           ptx::tc_commit(&sh.s_full[j & 1]);
         }
         __syncwarp();
-        if (i >= 2) load(i + 2);
+        if (i >= 2) load(pass, i + 2);
       }
       // (what the loop has not waited for, so that every barrier is one use behind at most)
-      const int last = done + n_iter - 1;
-      ok = ok && wait_tile(sh.s_taken, last, kAbortPEmpty, 3) && (n_iter < 2 || wait_tile(sh.pv_done, last - 1, kAbortFinal, 4)) &&
+      const int last = done + count - 1;
+      ok = ok && wait_tile(sh.s_taken, last, kAbortPEmpty, 3) && (count < 2 || wait_tile(sh.pv_done, last - 1, kAbortFinal, 4)) &&
            wait_tile(sh.pv_done, last, kAbortFinal, 4);
-      done += n_iter;
+      done += count;
       ok = ok && warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
-      if (pass == 2 || (pass == 0 && sh.again == 0)) break;
+      if (pass == last_pass()) break;
+      if (pass == 0) count = noted_tiles(sh.noted, n_iter, coarse, lane);
     }
   } else if (warp == kHSoftmaxWarps + 1) {
     // =================== P.V issuer ===================
-    constexpr uint32_t idesc_pv = ptx::umma_idesc(1, 1, 1, H3S_Q_TILE, H3S_HEAD_DIM);
+    constexpr uint32_t idesc_pv = ptx::umma_idesc(1, 0, 0, H3S_Q_TILE, H3S_HEAD_DIM);
     const uint64_t v_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + kHOffV), 1024, ptx::kSwizzle128);
     for (int pass = 0; ok; ++pass) {
-      for (int j = done; j < done + n_iter; ++j) {
+      for (int j = done; j < done + count; ++j) {
         if (!wait_tile(sh.p_full, j, kAbortPFull, 3) || !wait_stage(j)) { ok = false; break; }
         ptx::tc_fence_after();
         if (ptx::elect_one()) {
           const uint64_t v_desc = v_desc0 + static_cast<uint64_t>((j % kHStages) * (kHVBytes >> 4));
 #pragma unroll
           for (int k = 0; k < H3S_KV_TILE / 16; ++k)
-            ptx::umma_f16_ts(tmem_o, tmem_s + (j & 1) * 64 + k * 8, v_desc + 2 * k, idesc_pv, (j > done || k > 0) ? 1u : 0u);
+            ptx::umma_f16_ts(tmem_o, tmem_s + (j & 1) * 64 + k * 8, v_desc + 2 * k, idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
           ptx::tc_commit(&sh.pv_done[j & 1]);
         }
         __syncwarp();
       }
-      done += n_iter;
+      done += count;
       // Lists of one or two tiles: nothing in the next pass up to its own pass_end waits for this
       // warp, so that without its arrival here two passes could end before it looks, and the
       // parity it waits for would be that of a third.
       if (ok && lane == 0) ptx::mbar_arrive(&sh.pass_end);
       ok = ok && warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
-      if (pass == 2 || (pass == 0 && sh.again == 0)) break;
+      if (pass == last_pass()) break;
+      if (pass == 0) count = noted_tiles(sh.noted, n_iter, coarse, lane);
     }
   } else {
     // =================== softmax + epilogue (warps 0-7) ===================
@@ -333,69 +388,163 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const float q_scale = __ldg(prm.q_scale + head * prm.q_tiles + tq) * (0.08838834764831845f * 1.4426950408889634f);
     float m = 0.f, l = 0.f;
 
-    for (int pass = 0; ok; ++pass) {
-      const int last = done + n_iter - 1;
-      float top = -INFINITY;
-      l = 0.f;
-      for (int j = (done & 1) == group ? done : done + 1; j <= last; j += 2) {
-        if (!wait_tile(sh.s_full, j, kAbortSFull, 2)) { ok = false; break; }
-        ptx::tc_fence_after();
-        uint32_t s[H3S_KV_TILE];
-        H3S_TMEM_LD64(tmem_s + lane_addr + group * 32, s);
-        // index and K scale of this tile, left in shared memory by the producer
-        // before the stage was handed to the tensor pipe (free only after P.V(j))
-        const int n_valid = prm.sequence - sh.tile_index[j % kHStages] * H3S_KV_TILE;
-        const float c = q_scale * sh.tile_scale[j % kHStages];
-        ptx::tmem_wait_ld(s);
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&sh.s_taken[group]);
-
-        // Keys beyond the sequence (ragged last tile only): the integer whose biased
-        // bits are those of -inf, so that P becomes 0; it is also below every score.
-        if (n_valid < H3S_KV_TILE) {
+    // scores of tile j -> registers, and the factor that belongs to them
+    auto take = [&](int j, uint32_t (&s)[H3S_KV_TILE], float &c) {
+      if (!wait_tile(sh.s_full, j, kAbortSFull, 2)) return false;
+      ptx::tc_fence_after();
+      H3S_TMEM_LD64(tmem_s + lane_addr + group * 32, s);
+      // index and K scale of this tile, left in shared memory by the producer
+      // before the stage was handed to the tensor pipe (free only after P.V(j))
+      const int n_valid = prm.sequence - sh.tile_index[j % kHStages] * H3S_KV_TILE;
+      c = q_scale * sh.tile_scale[j % kHStages];
+      ptx::tmem_wait_ld(s);
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.s_taken[group]);
+      // Keys beyond the sequence (ragged last tile only): the integer whose biased
+      // bits are those of -inf, so that P becomes 0; it is also below every score.
+      if (n_valid < H3S_KV_TILE) {
 #pragma unroll
-          for (int i = 0; i < H3S_KV_TILE; ++i)
-            if (i >= n_valid) s[i] = 0xff800000u - kIntBiasBits;
-        }
-        if (j == 0) {
-          m = ceilf(c * static_cast<float>(max_score(s)));  // c > 0
-          sh.first[row] = m;
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&sh.first_max);
-        } else if (j == 1 && pass == 0) {
-          if (!warp_wait(&sh.first_max, 0, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
-          m = sh.first[row];
-        }
-        if (pass == 1) {
-          top = fmaxf(top, c * static_cast<float>(max_score(s)));
-        } else {
-          uint32_t packed[H3S_KV_TILE / 2];
-          l += exp_pack(s, c, -fmaf(c, kIntBias, m), packed);
-          // slot A or C: part of S(j), which is in registers
-          H3S_TMEM_ST32(tmem_s + lane_addr + group * 64, packed);
-          ptx::tmem_wait_st();
-          ptx::tc_fence_before();
-        }
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&sh.p_full[group]);
+        for (int i = 0; i < H3S_KV_TILE; ++i)
+          if (i >= n_valid) s[i] = 0xff800000u - kIntBiasBits;
       }
-      if (!ok) break;
-      done += n_iter;
-      // the row's two threads add up their sums (or agree on the maximum); two buffers,
-      // each written again only after every warp has passed the barrier in between
-      if (pass == 0 && __any_sync(0xffffffffu, !(l <= kHSumLimit)) && lane == 0) sh.again = 1;
-      float (&buffer)[2][H3S_Q_TILE] = sh.row[pass & 1];
-      buffer[group][row] = pass == 1 ? top : l;
+      return true;
+    };
+    // P -> slot A or C: part of S(j), which is in registers
+    auto put = [&](const uint32_t (&packed)[H3S_KV_TILE / 2]) { H3S_TMEM_ST32(tmem_s + lane_addr + group * 64, packed); };
+    auto hand_over = [&]() {
+      ptx::tmem_wait_st();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.p_full[group]);
+    };
+    auto own_first = [&](int from) { return (from & 1) == group ? from : from + 1; };  // of this group's tiles
+    // both threads of a row leave a value, then wait for everything else of the pass
+    auto end_pass = [&](int pass, float value) {
+      sh.row[pass & 1][group][row] = value;
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
-      ok = warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
-      if (pass == 1) m = ceilf(fmaxf(buffer[0][row], buffer[1][row])); else l = buffer[0][row] + buffer[1][row];
-      if (pass == 2 || (pass == 0 && *static_cast<volatile int *>(&sh.again) == 0)) break;
+      return warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+    };
+    auto leave_first = [&](float value) {
+      sh.first[group][row] = value;
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.first_max);
+    };
+    auto first_reference = [&]() { return ceilf(fmaxf(sh.first[0][row], sh.first[1][row])) + kHFirstBits; };
+    uint32_t staged_uses = 0;
+    auto meet = [&]() {  // all softmax warps
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.staged);
+      return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+    };
+
+    float largest = 0.f;  // sum over a tile that this thread has left out
+    if (group == 1 && n_iter == 1) leave_first(-INFINITY);
+    for (int j = group; j < n_iter; j += 2) {
+      uint32_t s[H3S_KV_TILE];
+      float c;
+      if (!take(j, s, c)) { ok = false; break; }
+      if (j < 2) {
+        leave_first(c * static_cast<float>(max_score(s)));  // c > 0
+        if (!warp_wait(&sh.first_max, 0, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
+        m = first_reference();
+      }
+      uint32_t packed[H3S_KV_TILE / 2];
+      float sum = exp_sum<true>(s, c, -fmaf(c, kIntBias, m), packed);
+      put(packed);
+      const bool out = !(sum <= kHSumLimit);
+      if (__any_sync(0xffffffffu, out)) {  // these rows leave the tile out
+        const bool far = __any_sync(0xffffffffu, sum == INFINITY);
+        ptx::tmem_wait_st();
+        if (out) {
+          largest = fmaxf(largest, sum);
+          sum = 0.f;
+#pragma unroll
+          for (int i = 0; i < H3S_KV_TILE / 2; ++i) packed[i] = 0u;
+        }
+        put(packed);
+        if (lane == 0) {
+          atomicOr(&sh.noted[(j >> coarse) >> 5], 1u << ((j >> coarse) & 31));
+          atomicOr(&sh.again, far ? kAgainNoted | kAgainFar : kAgainNoted);
+        }
+      }
+      l += sum;
+      hand_over();
     }
+    done = n_iter;
+    sh.row[1][group][row] = largest;
+    ok = ok && end_pass(0, l);
+    const int final_pass = ok ? last_pass() : 0;
+    if (final_pass > 0) {
+      count = noted_tiles(sh.noted, n_iter, coarse, lane);
+      m = first_reference();  // (a group without a tile has none yet)
+      float m_again = m;
+      if (final_pass == 1) {
+        const uint32_t bits = __float_as_uint(fmaxf(sh.row[1][0][row], sh.row[1][1][row]));
+        if (bits != 0u) m_again = m + (static_cast<float>(static_cast<int>(bits >> 23) - 126) - kHAgainBits);
+      } else {
+        float top = -INFINITY;
+        for (int j = own_first(done); j < done + count; j += 2) {
+          uint32_t s[H3S_KV_TILE];
+          float c;
+          if (!take(j, s, c)) { ok = false; break; }
+          top = fmaxf(top, c * static_cast<float>(max_score(s)));
+          uint32_t none[H3S_KV_TILE / 2];  // O stays as it is
+#pragma unroll
+          for (int i = 0; i < H3S_KV_TILE / 2; ++i) none[i] = 0u;
+          put(none);
+          hand_over();
+        }
+        done += count;
+        ok = ok && end_pass(1, top);
+        top = fmaxf(sh.row[1][0][row], sh.row[1][1][row]);
+        if (top > m + kHMostBits) m_again = ceilf(top) - kHAgainBits;
+      }
+      // every P.V so far (one barrier per group): O may be touched
+      ok = ok && (done < 2 || wait_tile(sh.pv_done, done - 2, kAbortFinal, 4)) && wait_tile(sh.pv_done, done - 1, kAbortFinal, 4);
+      const float factor = fast_exp2(m - m_again);  // a power of two
+      l *= factor;
+      if (ok && __any_sync(0xffffffffu, m_again != m)) {
+        ptx::tc_fence_after();
+#pragma unroll 1
+        for (int cc = group * 2; cc < group * 2 + 2; ++cc) {
+          uint32_t o[32];
+          H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
+          ptx::tmem_wait_ld(o);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+          H3S_TMEM_ST32(tmem_o + lane_addr + cc * 32, o);
+        }
+        ptx::tmem_wait_st();
+        ptx::tc_fence_before();
+      }
+      ok = ok && meet();  // the first P.V of the next pass waits for one group only
+      for (int j = own_first(done); ok && j < done + count; j += 2) {
+        uint32_t s[H3S_KV_TILE];
+        float c;
+        if (!take(j, s, c)) { ok = false; break; }
+        uint32_t packed[H3S_KV_TILE / 2];
+        // the same sum as in the first pass, so the same tiles
+        const bool out = !(exp_sum<false>(s, c, -fmaf(c, kIntBias, m), packed) <= kHSumLimit);
+        const float sum = exp_sum<true>(s, c, -fmaf(c, kIntBias, m_again), packed);
+        if (out) {
+          l += sum;
+        } else {
+#pragma unroll
+          for (int i = 0; i < H3S_KV_TILE / 2; ++i) packed[i] = 0u;
+        }
+        put(packed);
+        hand_over();
+      }
+      done += count;
+      m = m_again;
+      ok = ok && end_pass(final_pass, l);
+    }
+    if (ok) l = sh.row[final_pass & 1][0][row] + sh.row[final_pass & 1][1][row];
 
     // every P.V of the last pass (one barrier per group)
-    if (ok && n_iter > 1) ok = wait_tile(sh.pv_done, done - 2, kAbortFinal, 4);
+    if (ok && done > 1) ok = wait_tile(sh.pv_done, done - 2, kAbortFinal, 4);
     if (ok) ok = wait_tile(sh.pv_done, done - 1, kAbortFinal, 4);
     if (ok) {
       // Epilogue: O * v_scale / l -> OutT, staged through shared memory (the
@@ -403,12 +552,6 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       // 32 rows of one column half; the two warps of a row quarter then each write
       // 16 of the quarter's rows as full contiguous lines.
       ptx::tc_fence_after();
-      uint32_t staged_uses = 0;
-      auto meet = [&]() {  // all softmax warps
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&sh.staged);
-        return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
-      };
       // Partial sums of part p: [32 groups of 4 columns][128 rows] float4, so that a warp's rows are
       // neighbours; then 128 row sums and 128 reference points.
       constexpr int kPartFloats = H3S_Q_TILE * (H3S_HEAD_DIM + 2);
@@ -525,13 +668,13 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   if (code == 0 && prm.n_peer_out > 0 && sh.finish) scatter_to_peers<OutT>(prm, smem, head, tq, kHThreads);
 }
 
-// E4M3 codes -> BF16 values: 16 per thread
+// E4M3 codes -> FP16 values: 16 per thread
 __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v8, uint4 *__restrict__ v16, int64_t chunks) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= chunks) return;
   const uint4 codes = __ldg(v8 + i);
-  v16[2 * i] = e4m3x8_to_bf16(make_uint2(codes.x, codes.y));
-  v16[2 * i + 1] = e4m3x8_to_bf16(make_uint2(codes.z, codes.w));
+  v16[2 * i] = e4m3x8_to_half(make_uint2(codes.x, codes.y));
+  v16[2 * i + 1] = e4m3x8_to_half(make_uint2(codes.z, codes.w));
 }
 
 // Whether and how the dense rows' tile lists are cut.  Two CTAs run on each of 148 SMs; a

@@ -1,5 +1,5 @@
 // Block-sparse attention on the INT8 Q/K + FP8 V carriers for sm_100a: the kernel for
-// hosts that keep no BF16 copy of V (attn_half.cu needs one) and for single-term P.
+// hosts that keep no FP16 copy of V (attn_half.cu needs one) and for single-term P.
 //
 // One CTA owns one 128-row query tile of one head and walks that tile's list
 // of 64-row KV tiles:

@@ -177,17 +177,13 @@ __device__ __forceinline__ void round_codes(float2 q, uint32_t &first, uint32_t 
   second = static_cast<uint32_t>(static_cast<int>(q.y));
 }
 
-// 8 E4M3 codes -> the same values as BF16 (exact: four significant bits)
-__device__ __forceinline__ uint4 e4m3x8_to_bf16(const uint2 &codes) {
+// 8 E4M3 codes -> the same values as FP16 (exact: four significant bits, 2^-9 to 448)
+__device__ __forceinline__ uint4 e4m3x8_to_half(const uint2 &codes) {
   const uint32_t in[2] = {codes.x, codes.y};
   uint32_t pair[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    uint32_t half2;
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(half2) : "h"(static_cast<uint16_t>(in[k >> 1] >> ((k & 1) * 16))));
-    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&half2));
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(pair[k]) : "f"(f.y), "f"(f.x));
-  }
+  for (int k = 0; k < 4; ++k)
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(pair[k]) : "h"(static_cast<uint16_t>(in[k >> 1] >> ((k & 1) * 16))));
   return make_uint4(pair[0], pair[1], pair[2], pair[3]);
 }
 

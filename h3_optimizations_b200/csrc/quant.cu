@@ -244,7 +244,7 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
 // FP8-E4M3 V carrier, transposed to (heads, 128, pad128(S)).
 // One CTA = 128 sequence rows of one head, staged through shared memory so
 // that both the row-major reads and the channel-major writes are full lines.
-// All eight rows of a thread are requested before the first is used, and the BF16 copy
+// All eight rows of a thread are requested before the first is used, and the FP16 copy
 // is written as whole lines of 256 bytes (two 16-byte pieces a thread with a gap between
 // them cost twice the L2 writes): 24 heads x 33272 tokens 133 -> 88 us.
 // ---------------------------------------------------------------------------
@@ -350,12 +350,12 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
     const int64_t at = base_at + static_cast<int64_t>(d) * padded_total + chunk * 16;
     *reinterpret_cast<uint4 *>(out + at) = data;
   }
-  if (out_half != nullptr) {  // the copy the attention kernel multiplies with BF16 probabilities
+  if (out_half != nullptr) {  // the copy the attention kernel multiplies with FP16 probabilities
 #pragma unroll
     for (int p = 0; p < H3S_HEAD_DIM / (kVThreads / 16); ++p) {
       const int d = p * (kVThreads / 16) + slot, s = (threadIdx.x & 15) * 8;
       const uint2 data = *reinterpret_cast<const uint2 *>(&tile[v_tile_offset(d, s)]);
-      *reinterpret_cast<uint4 *>(out_half + base_at + static_cast<int64_t>(d) * padded_total + s) = e4m3x8_to_bf16(data);
+      *reinterpret_cast<uint4 *>(out_half + base_at + static_cast<int64_t>(d) * padded_total + s) = e4m3x8_to_half(data);
     }
   }
 }

@@ -184,7 +184,7 @@ def allocate_v_carrier(sequence, heads, device):
 
 
 def quant_v_fp8_into(v, v_scale, carrier, *, row_start=0, sequence_total=None, v_bound=FP8_V_BOUND, half=None):
-    """``half``: optional bf16 tensor shaped like ``carrier`` that receives the codes' values."""
+    """``half``: optional fp16 tensor shaped like ``carrier`` that receives the codes' values."""
     lib = _native.load()
     heads, rows = _hnd(v, "quant_v_fp8 input")
     sequence_total = int(sequence_total if sequence_total is not None else row_start + rows)
@@ -194,8 +194,8 @@ def quant_v_fp8_into(v, v_scale, carrier, *, row_start=0, sequence_total=None, v
         raise _native.NativeError("quant_v_fp8: carrier must be contiguous e4m3 (1,H,128,%d)" % padded)
     if tuple(v_scale.shape) != (1, heads, HEAD_DIM) or v_scale.dtype != torch.float32 or not v_scale.is_contiguous():
         raise _native.NativeError("quant_v_fp8: scale must be contiguous fp32 (1,H,128)")
-    if half is not None and (half.shape != carrier.shape or half.dtype != torch.bfloat16 or not half.is_contiguous()):
-        raise _native.NativeError("quant_v_fp8: half must be a contiguous bf16 tensor shaped like the carrier")
+    if half is not None and (half.shape != carrier.shape or half.dtype != torch.float16 or not half.is_contiguous()):
+        raise _native.NativeError("quant_v_fp8: half must be a contiguous fp16 tensor shaped like the carrier")
     check(
         lib.h3s_quant_v_fp8_half(
             ptr(v), dtype_code(v.dtype), v.stride(1), v.stride(2), ptr(v_scale), ptr(carrier), ptr(half), heads, rows,
@@ -250,7 +250,7 @@ class LayerBuffers:
             self.k_mean = torch.empty(small, dtype=torch.float32, device=device)
         self.v_scale = torch.empty(small, dtype=torch.float32, device=device)
         self.v_carrier = allocate_v_carrier(sequence, heads, device)
-        self.v_half = torch.empty(self.v_carrier.shape, dtype=torch.bfloat16, device=device)
+        self.v_half = torch.empty(self.v_carrier.shape, dtype=torch.float16, device=device)
         self.scratch = torch.empty(lib.h3s_column_stats_scratch_bytes(heads), dtype=torch.uint8, device=device)
         self.native = _native.LayerCarriers(
             self.q_int8.data_ptr(), self.q_scale.data_ptr(), _address(self.q_summary),
@@ -588,10 +588,10 @@ def _attn_args(q8, k8, v_carrier, q_scale, k_scale, v_scale, route, q_start, q_s
 
 
 def v_half_copy(v_carrier):
-    """The V carrier ``(1,H,128,pad128(S))`` as BF16 (exact), which the attention kernel multiplies with BF16
+    """The V carrier ``(1,H,128,pad128(S))`` as FP16 (exact), which the attention kernel multiplies with FP16
     probabilities."""
     lib = _native.load()
-    out = torch.empty(v_carrier.shape, dtype=torch.bfloat16, device=v_carrier.device)
+    out = torch.empty(v_carrier.shape, dtype=torch.float16, device=v_carrier.device)
     check(lib.h3s_v_half(ptr(v_carrier), ptr(out), v_carrier.shape[1], v_carrier.shape[3], stream_ptr(v_carrier.device)),
           "h3s_v_half")
     return out
@@ -608,8 +608,8 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
                      out=None, out_dtype=torch.bfloat16, status=None, legacy_mma=False, single_term_p=False,
                      peer_out_ptrs=None, extra_flags=0, v_half=None):
     """Launch the attention kernel.  Returns ``out`` (HND).  ``single_term_p``
-    carries the probabilities as one E4M3 term instead of in BF16.
-    ``v_half``: the BF16 copy of the V carrier (``v_half_copy``) where the caller
+    carries the probabilities as one E4M3 term instead of in FP16.
+    ``v_half``: the FP16 copy of the V carrier (``v_half_copy``) where the caller
     keeps one; made here otherwise.
     ``peer_out_ptrs``: device addresses (ints) of up to 7 further buffers,
     addressed like ``out``, that receive every output tile as well (the slices

@@ -62,12 +62,13 @@ def test_scores_that_outgrow_the_first_tile(native_lib, tiles):
     _check(native_lib, q, k, v, oracle.geometry(sequence, 0), None)
 
 
-def test_many_repeated_lists_of_two_tiles(native_lib):
-    """The shortest lists that are done again: in their passes the P.V warp is behind all others."""
-    sequence, heads = 123, 900                                                    # three waves of two CTAs on every SM
+def test_many_short_lists_that_are_walked_again(native_lib):
+    """The first of the tiles, walked last, is far above the others: nothing but the P.V warp's own arrival holds
+    back the pass behind it."""
+    sequence, heads = 187, 900                                                    # six waves of two CTAs on every SM
     spec = workloads.small_spec("edge", heads, 0, sequence)
     q, k, v = workloads.gaussian_qkv(spec, seed=12, widen=True)
-    sign = torch.ones(sequence)
-    sign[:64] = -1.0
+    sign = -torch.ones(sequence)
+    sign[:64] = 1.0
     q, k = q + 3.0, k + 3.0 * sign[:, None]
     _check(native_lib, q, k, v, oracle.geometry(sequence, 0), None)
