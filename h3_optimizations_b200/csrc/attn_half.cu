@@ -547,7 +547,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     if (ok && done > 1) ok = wait_tile(sh.pv_done, done - 2, kAbortFinal, 4);
     if (ok) ok = wait_tile(sh.pv_done, done - 1, kAbortFinal, 4);
     if (ok) {
-      // Epilogue: O * v_scale / l -> OutT, staged through shared memory (the
+      // Epilogue: O / l * v_scale -> OutT, staged through shared memory (the
       // stage ring is free: every TMA load has been consumed).  A warp converts its
       // 32 rows of one column half; the two warps of a row quarter then each write
       // 16 of the quarter's rows as full contiguous lines.
@@ -627,7 +627,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
           float v[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            v[e] = __uint_as_float(o[i + e]) * sh.v_scale[cc * 32 + i + e] * inv_l;
+            v[e] = __uint_as_float(o[i + e]) * inv_l * sh.v_scale[cc * 32 + i + e];  // |o / l| <= 448: nothing overflows
           // 8 values = one (bf16/fp16) or two (fp32) 16-byte chunks; the chunk index is
           // XORed with the row so that the 32 rows of a warp do not collide on banks
           constexpr int kChunks8 = 8 * static_cast<int>(sizeof(OutT)) / 16;
