@@ -58,6 +58,10 @@ def _carrier_spec(prepared):
         rows.append(("v_carrier", prepared.v_carrier, (1, heads, head_dim, padded), None,
                      "prepacked H3 FP8 V carrier shape is invalid"))
         rows.append(("v_carrier", prepared.v_carrier, None, torch.float8_e4m3fn, "prepacked H3 V carrier must be E4M3 FP8"))
+        v_half = getattr(prepared, "v_half", None)
+        if v_half is not None:
+            rows.append(("v_half", v_half, (1, heads, head_dim, padded), torch.float16,
+                         "FP16 copy of the prepacked H3 FP8 V is invalid"))
         if prepared.v_scale is None:
             raise FusedQKVError("prepacked H3 FP8 V requires V scale")
         rows.append(("v_scale", prepared.v_scale, (1, heads, head_dim), None, "prepacked H3 V scale shape is invalid"))

@@ -590,11 +590,21 @@ def _attn_args(q8, k8, v_carrier, q_scale, k_scale, v_scale, route, q_start, q_s
 def v_half_copy(v_carrier):
     """The V carrier ``(1,H,128,pad128(S))`` as FP16 (exact), which the attention kernel multiplies with FP16
     probabilities."""
+    if (v_carrier.ndim != 4 or v_carrier.shape[0] != 1 or v_carrier.shape[2] != HEAD_DIM or v_carrier.shape[3] % 128
+            or v_carrier.dtype != torch.float8_e4m3fn or not v_carrier.is_contiguous() or not v_carrier.is_cuda):
+        raise _native.NativeError("v_half_copy: carrier must be contiguous CUDA e4m3 (1,H,128,pad128(S))")
     lib = _native.load()
     out = torch.empty(v_carrier.shape, dtype=torch.float16, device=v_carrier.device)
     check(lib.h3s_v_half(ptr(v_carrier), ptr(out), v_carrier.shape[1], v_carrier.shape[3], stream_ptr(v_carrier.device)),
           "h3s_v_half")
     return out
+
+
+def check_v_half(v_half, v_carrier):
+    """The kernel reads the copy by the carrier's shape alone."""
+    if (v_half.dtype != torch.float16 or v_half.shape != v_carrier.shape or not v_half.is_contiguous()
+            or v_half.device != v_carrier.device):
+        raise _native.NativeError("sparse_attention: v_half must be a contiguous fp16 tensor of the V carrier's shape on its device")
 
 
 def new_attention_output(heads, sequence, dtype, device):
@@ -635,6 +645,8 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
     else:
         if v_half is None:
             v_half = v_half_copy(v_carrier)
+        else:
+            check_v_half(v_half, v_carrier)
         size = lib.h3s_sparse_attn_half_workspace_bytes(heads, sequence, route_len, int(q_start), int(q_stop))
         workspace = torch.empty(size, dtype=torch.uint8, device=q8.device) if size else None
         check(lib.h3s_sparse_attn_half_fwd(ptr(q8), ptr(k8), ptr(v_half), *before, table, n_peers, *after,
