@@ -28,7 +28,7 @@ from __future__ import annotations
 import torch
 
 from . import _native, ops
-from .carriers import PreparedFusedQKV, PreparedHybrid, PreparedSparse, validate_prepared_fused_qkv
+from .carriers import PreparedFusedQKV, PreparedHybrid, PreparedSparse, VCarrier, validate_prepared_fused_qkv
 from .config import MODE_SAGE128_FUSED_QKV, HybridSparseConfig, resolve_video_budget
 from .errors import FusedQKVError, SparseRouterError, SparseSageError
 from .router import KV_TILE, Q_TILE, SparseTileRouter
@@ -341,9 +341,9 @@ class B200SparseBackend:
                 projected.q_summary, projected.k_summary, snapshot.layout, video_budget,
                 **self._sink(transformer_options, layer_index),
             )
-            if projected.v_carrier is not None:
-                v_carrier, v_scale = projected.v_carrier, projected.v_scale
-            else:
+            v_carrier, v_scale = VCarrier.of(projected), projected.v_scale
+            prepacked = v_carrier.codes is not None
+            if not prepacked:
                 v_carrier, v_scale = ops.quant_v_fp8(projected.v, None, V_QUANT_BOUND)
         except SparseRouterError as exc:
             raise SparseSageError("sparse routing failed: %s" % exc) from exc
@@ -354,7 +354,7 @@ class B200SparseBackend:
             {
                 "qkv_projection": "fused_int8",
                 "smooth_k": bool(projected.smooth_k),
-                "prepacked_fp8_v": projected.v_carrier is not None,
+                "prepacked_fp8_v": prepacked,
             }
         )
         sparse = PreparedSparse(
@@ -362,7 +362,6 @@ class B200SparseBackend:
             q_scale=projected.q_scale, k_scale=projected.k_scale, v_scale=v_scale, route=route,
             output_dtype=projected.output_dtype, output_shape=(1, heads, sequence, projected.head_dim),
             layer_index=int(projected.layer_index), sequence=sequence, heads=heads, metadata=metadata,
-            v_half=projected.v_half if projected.v_carrier is not None else None,
         )
         return PreparedHybrid(sparse=sparse)
 
@@ -377,13 +376,14 @@ class B200SparseBackend:
         geometry = route.geometry
         device = sparse.q_int8.device
         word, mirror, copied = self._status_slot(device)
+        v = VCarrier.of(sparse)
         try:
             out_dtype = sparse.output_dtype
             result = ops.sparse_attention(
-                sparse.q_int8, sparse.k_int8, sparse.v_carrier, sparse.q_scale, sparse.k_scale,
+                sparse.q_int8, sparse.k_int8, v.codes, sparse.q_scale, sparse.k_scale,
                 sparse.v_scale, route.indices,
                 q_start=geometry.pure_video_q_start, q_stop=geometry.pure_video_q_stop,
-                out=out, out_dtype=out_dtype, status=word, peer_out_ptrs=peer_out_ptrs, v_half=sparse.v_half,
+                out=out, out_dtype=out_dtype, status=word, peer_out_ptrs=peer_out_ptrs, v_half=v.half,
             )
             if not torch.cuda.is_current_stream_capturing():
                 # (an event recorded inside a capture could not be queried afterwards: replays are

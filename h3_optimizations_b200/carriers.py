@@ -3,7 +3,7 @@ attention/sparse/sparse_sage.py:401-417)."""
 
 from __future__ import annotations
 
-from dataclasses import dataclass, field
+from dataclasses import InitVar, dataclass, field
 
 import torch
 
@@ -13,11 +13,43 @@ from .router import KV_TILE, Q_TILE
 HEAD_DIM = 128
 
 
+class VCarrier:
+    """The E4M3 codes of V and, while nobody else holds them, the FP16 copy that was written with
+    them.  Whoever is handed the codes may write to them, so the copy is dropped then and the
+    attention call makes its own (about 50 us at 24 heads x 33272 tokens)."""
+
+    __slots__ = ("codes", "half")
+
+    def __init__(self, codes, half=None):
+        self.codes = codes
+        self.half = half
+
+    @classmethod
+    def of(cls, prepared):
+        """The pair that ``prepared`` holds; its codes alone where it is no class of this module."""
+        pair = getattr(prepared, "_v", None)
+        return pair if isinstance(pair, cls) else cls(prepared.v_carrier)
+
+    @classmethod
+    def field(cls):
+        """``v_carrier`` of a class that keeps its codes in a pair (``_v``)."""
+
+        def get(prepared):
+            prepared._v.half = None
+            return prepared._v.codes
+
+        def put(prepared, codes):
+            prepared._v = codes if isinstance(codes, cls) else cls(codes)
+
+        return property(get, put)
+
+
 @dataclass
 class PreparedFusedQKV:
     """Output of a QKV projector: INT8 Q/K carriers with per-block scales and
     tile means, plus V either floating HND (``v``) or already packed
-    (``v_carrier`` e4m3 ``(1,H,128,pad128(S))`` + ``v_scale`` ``(1,H,128)``)."""
+    (``v_carrier`` e4m3 ``(1,H,128,pad128(S))`` + ``v_scale`` ``(1,H,128)``;
+    ``v_half``: its FP16 copy, see ``VCarrier``, which may also be given as ``v_carrier``)."""
 
     q_int8: torch.Tensor
     q_scale: torch.Tensor
@@ -34,7 +66,14 @@ class PreparedFusedQKV:
     smooth_k: bool = False
     v_carrier: torch.Tensor | None = None
     v_scale: torch.Tensor | None = None
-    v_half: torch.Tensor | None = None  # FP16 copy of v_carrier (optional: the attention call makes it otherwise)
+    v_half: InitVar[torch.Tensor | None] = None
+
+    def __post_init__(self, v_half):
+        if v_half is not None:
+            self._v.half = v_half
+
+
+PreparedFusedQKV.v_carrier = VCarrier.field()
 
 
 def _carrier_spec(prepared):
@@ -49,18 +88,18 @@ def _carrier_spec(prepared):
         ("q_int8", prepared.q_int8, None, torch.int8, "fused H3 Q/K carriers must be INT8"),
         ("k_int8", prepared.k_int8, None, torch.int8, "fused H3 Q/K carriers must be INT8"),
     ]
-    if prepared.v_carrier is None:
+    v = VCarrier.of(prepared)
+    if v.codes is None:
         if prepared.v is None:
             raise FusedQKVError("fused H3 V is missing")
         rows.append(("v", prepared.v, full, prepared.output_dtype, "fused H3 V carrier is invalid"))
     else:
         padded = -(-sequence // 128) * 128
-        rows.append(("v_carrier", prepared.v_carrier, (1, heads, head_dim, padded), None,
+        rows.append(("v_carrier", v.codes, (1, heads, head_dim, padded), None,
                      "prepacked H3 FP8 V carrier shape is invalid"))
-        rows.append(("v_carrier", prepared.v_carrier, None, torch.float8_e4m3fn, "prepacked H3 V carrier must be E4M3 FP8"))
-        v_half = getattr(prepared, "v_half", None)
-        if v_half is not None:
-            rows.append(("v_half", v_half, (1, heads, head_dim, padded), torch.float16,
+        rows.append(("v_carrier", v.codes, None, torch.float8_e4m3fn, "prepacked H3 V carrier must be E4M3 FP8"))
+        if v.half is not None:
+            rows.append(("v_half", v.half, (1, heads, head_dim, padded), torch.float16,
                          "FP16 copy of the prepacked H3 FP8 V is invalid"))
         if prepared.v_scale is None:
             raise FusedQKVError("prepacked H3 FP8 V requires V scale")
@@ -121,7 +160,14 @@ class PreparedSparse:
     sequence: int
     heads: int
     metadata: dict = field(default_factory=dict)
-    v_half: torch.Tensor | None = None  # FP16 copy of v_carrier
+    v_half: InitVar[torch.Tensor | None] = None  # FP16 copy of v_carrier, see VCarrier
+
+    def __post_init__(self, v_half):
+        if v_half is not None:
+            self._v.half = v_half
+
+
+PreparedSparse.v_carrier = VCarrier.field()
 
 
 @dataclass
