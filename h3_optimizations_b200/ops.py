@@ -639,7 +639,7 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
     stream = stream_ptr(q8.device)
     if legacy_mma:
         check(lib.h3s_sparse_attn_fwd_mma(ptr(q8), ptr(k8), ptr(v_carrier), *before, *after, stream), "h3s_sparse_attn_fwd_mma")
-    elif single_term_p:
+    elif flags & ATTN_P_SINGLE:
         check(lib.h3s_sparse_attn_fwd_scatter(ptr(q8), ptr(k8), ptr(v_carrier), *before, table, n_peers, *after,
                                               ptr(status), stream), "h3s_sparse_attn_fwd_scatter")
     else:
