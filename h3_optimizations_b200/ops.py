@@ -616,9 +616,10 @@ def new_attention_output(heads, sequence, dtype, device):
 
 def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *, q_start=0, q_stop=0,
                      out=None, out_dtype=torch.bfloat16, status=None, legacy_mma=False, single_term_p=False,
-                     peer_out_ptrs=None, extra_flags=0, v_half=None):
+                     peer_out_ptrs=None, extra_flags=0, v_half=None, two_term_p=False):
     """Launch the attention kernel.  Returns ``out`` (HND).  ``single_term_p``
-    carries the probabilities as one E4M3 term instead of in FP16.
+    carries the probabilities as one E4M3 term instead of in FP16, ``two_term_p``
+    as two; both work on the carrier itself and make no copy of it.
     ``v_half``: the FP16 copy of the V carrier (``v_half_copy``) where the caller
     keeps one; made here otherwise.
     ``peer_out_ptrs``: device addresses (ints) of up to 7 further buffers,
@@ -639,9 +640,13 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
     stream = stream_ptr(q8.device)
     if legacy_mma:
         check(lib.h3s_sparse_attn_fwd_mma(ptr(q8), ptr(k8), ptr(v_carrier), *before, *after, stream), "h3s_sparse_attn_fwd_mma")
-    elif flags & ATTN_P_SINGLE:
-        check(lib.h3s_sparse_attn_fwd_scatter(ptr(q8), ptr(k8), ptr(v_carrier), *before, table, n_peers, *after,
-                                              ptr(status), stream), "h3s_sparse_attn_fwd_scatter")
+    elif two_term_p or flags & ATTN_P_SINGLE:
+        if n_peers:
+            check(lib.h3s_sparse_attn_fwd_scatter(ptr(q8), ptr(k8), ptr(v_carrier), *before, table, n_peers, *after,
+                                                  ptr(status), stream), "h3s_sparse_attn_fwd_scatter")
+        else:
+            check(lib.h3s_sparse_attn_fwd(ptr(q8), ptr(k8), ptr(v_carrier), *before, *after, ptr(status), stream),
+                  "h3s_sparse_attn_fwd")
     else:
         if v_half is None:
             v_half = v_half_copy(v_carrier)
