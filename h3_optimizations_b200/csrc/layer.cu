@@ -95,17 +95,20 @@ int h3s_project_qkv(const h3s_layer_carriers *c, const void *x_bf16, int64_t x_s
                                  c->v_scale, s);
   if (rc) return rc;
   const int64_t head = static_cast<int64_t>(sequence) * H3S_HEAD_DIM;
+  // the two second-phase quantisers are independent and each leaves part of the memory
+  // system idle: V runs on the second stream underneath K
   if (smooth_k) {
-    // the two second-phase quantisers are independent and each leaves part of the memory
-    // system idle: V runs on the second stream underneath K
     rc = order_after(s, side, event);
     if (rc) return rc;
     rc = h3s_quant_qk_blocks(k_stage, H3S_BF16, head, H3S_HEAD_DIM, c->k_mean, c->k8, c->k_scale, nullptr, H3S_F32,
                              heads, sequence, 0, sequence, H3S_KV_TILE, s);
-    if (rc) return rc;
   }
-  return h3s_quant_v_fp8_half(v_stage, H3S_BF16, head, H3S_HEAD_DIM, c->v_scale, c->v8, c->v16, heads, sequence, 0,
-                              sequence, v_bound, smooth_k ? side : s);
+  if (!rc) rc = h3s_quant_v_fp8_half(v_stage, H3S_BF16, head, H3S_HEAD_DIM, c->v_scale, c->v8, c->v16, heads, sequence, 0,
+                                     sequence, v_bound, smooth_k ? side : s);
+  if (!smooth_k) return rc;
+  // joined wherever it was forked, and only there: a capture must not wait for a stream outside it
+  const int joined = order_after(side, s, event);
+  return rc ? rc : joined;
 }
 
 int h3s_status_mirror(const int32_t *status, int32_t *host_mirror, void *event, h3s_stream_t stream) {

@@ -277,8 +277,8 @@ def quant_qkv(q, k, v, buffers, side, stream, *, smooth_k, v_after_k, v_bound=FP
 
 def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, smooth_k, q_norm=None, k_norm=None,
                 epsilon=0.0, rope=None, status=None, v_bound=FP8_V_BOUND):
-    """The chunked projection of ``x`` (S, hidden) bf16 into ``buffers`` (see ``quant_qkv``).  Returns the
-    scratch tensors, which live until ``side`` has been joined."""
+    """The chunked projection of ``x`` (S, hidden) bf16 into ``buffers``; ``stream`` and ``side`` as in
+    ``quant_qkv``, but ``stream`` is behind ``side`` again when the call returns or raises."""
     if x.stride(1) != 1:
         raise _native.NativeError("project_qkv: x must have contiguous rows")
     sequence, hidden = x.shape
@@ -293,7 +293,6 @@ def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, s
     if rope is not None:
         rope_code = dtype_code(rope.dtype)
         strides = (ctypes.c_int64 * 4)(rope.stride(1), rope.stride(3), rope.stride(4), rope.stride(5))
-    scratch = (x_i8, x_scale, v_stage, k_stage)
     check(
         _native.load().h3s_project_qkv(
             buffers.native, x.data_ptr(), x.stride(0), sequence, hidden, chunk_rows, x_i8.data_ptr(), x_scale.data_ptr(),
@@ -302,7 +301,6 @@ def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, s
             side.event_handle, stream, side.handle),
         "h3s_project_qkv",
     )
-    return scratch
 
 
 def status_mirror(word, mirror, event, stream):

@@ -150,19 +150,11 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
             rope_freqs = rope_freqs.float()
     try:
         buffers = ops.LayerBuffers(heads, sequence, device, smooth_k=smooth_k, summary_dtype=summary_dtype)
-        stream, side = _native.stream_ptr(device), _side_stream(device)
-        try:
-            # every launch of the projection from one native call (24 heads x 2304 tokens, with
-            # backend and out_proj: 344 -> 259 us)
-            scratch = ops.project_qkv(x, w_i8.contiguous(), w_scale.contiguous(), buffers, side, stream, heads=heads,
-                                      chunk_rows=chunk_rows, smooth_k=smooth_k, q_norm=q_norm, k_norm=k_norm,
-                                      epsilon=float(epsilon), rope=rope_freqs, status=status, v_bound=V_QUANT_BOUND)
-        finally:
-            # on every exit path, before the staging can be freed; without smoothing the second
-            # stream has not been forked, and a capture must not wait for a stream outside it
-            if smooth_k:
-                side.join(stream)
-        del scratch
+        # every launch of the projection from one native call (24 heads x 2304 tokens, with
+        # backend and out_proj: 344 -> 259 us)
+        ops.project_qkv(x, w_i8.contiguous(), w_scale.contiguous(), buffers, _side_stream(device), _native.stream_ptr(device),
+                        heads=heads, chunk_rows=chunk_rows, smooth_k=smooth_k, q_norm=q_norm, k_norm=k_norm,
+                        epsilon=float(epsilon), rope=rope_freqs, status=status, v_bound=V_QUANT_BOUND)
     except _native.NativeError as exc:
         raise FusedQKVError("chunked QKV projection failed: layer=%d: %s" % (layer_index, exc)) from exc
     return validate_prepared_fused_qkv(
