@@ -148,6 +148,8 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
             raise FusedQKVError("rope_freqs must be (1, %d, 1, 48, 2, 2) on the projection's device" % sequence)
         if rope_freqs.dtype not in (torch.float32, torch.bfloat16):
             rope_freqs = rope_freqs.float()
+    if summary_dtype is None:  # as torch.empty takes it
+        summary_dtype = torch.get_default_dtype()
     try:
         buffers = ops.LayerBuffers(heads, sequence, device, smooth_k=smooth_k, summary_dtype=summary_dtype)
         # every launch of the projection from one native call (24 heads x 2304 tokens, with

@@ -3,6 +3,8 @@
 import pytest
 import torch
 
+from h3_optimizations_b200 import workloads
+
 pytestmark = pytest.mark.gpu
 
 
@@ -29,3 +31,12 @@ def test_a_refused_projection_leaves_a_capture_usable(native_lib):
     torch.cuda.synchronize()
     assert bool((doubled == 6.0).all())
 
+
+def test_summary_type_none_is_the_default_type(native_lib):
+    from h3_optimizations_b200.projector import run_chunked_sparse_qkv
+
+    x, w, w_scale = (t.cuda() for t in workloads.projection_inputs(300, hidden=256, heads=1, seed=4))
+    default = run_chunked_sparse_qkv(x, w, w_scale, heads=1)
+    none = run_chunked_sparse_qkv(x, w, w_scale, heads=1, summary_dtype=None)
+    assert none.q_summary.dtype == torch.float32
+    assert torch.equal(none.q_summary, default.q_summary) and torch.equal(none.k_summary, default.k_summary)
