@@ -309,8 +309,6 @@ __device__ __forceinline__ float rope_load(const void *base, int64_t index, int 
                           : __bfloat162float(__ldg(static_cast<const __nv_bfloat16 *>(base) + index));
 }
 
-__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 

@@ -66,10 +66,6 @@ def _validate_chunk_rows(chunk_rows, q_tile=Q_TILE, kv_tile=KV_TILE):
     return chunk_rows
 
 
-def chunk_ranges(sequence, chunk_rows):
-    return [(start, min(start + chunk_rows, sequence)) for start in range(0, sequence, chunk_rows)]
-
-
 class ChunkedSparseQKVProjector:
     name = "chunked_b200_sparse_qkv"
     qk_format = "sparge_block_int8"
