@@ -365,11 +365,15 @@ def workload_name(spec, budget):
                " + ".join("%d %s" % (b - a, kind) for a, b, kind in spec.segments), budget * 100))
 
 
-# DRAM traffic of one sparse_attn_tc_kernel launch per head of the 33272-token,
+# DRAM traffic of one sparse_attn_half_kernel launch per head of the 33272-token,
 # 30 % workload: dram__bytes_read.sum + dram__bytes_write.sum of the ncu capture
-# summarised in profiles/sparse_attn_tc_kernel_config1_4heads.md (4 heads), divided
+# summarised in profiles/sparse_attn_half_kernel_4heads.md (4 heads), divided
 # by 4; the traffic grows in proportion to the heads of a launch.
-ATTN_DRAM_BYTES_PER_HEAD = (51.9e6 + 6.9e6) / 4
+ATTN_DRAM_BYTES_PER_HEAD = (72.0e6 + 13.1e6) / 4
+# Bytes an element of Q, K and V leaves in the carriers: INT8 Q and K, E4M3 V and its FP16 copy.
+CARRIER_BYTES = 1 + 1 + 1 + 2
+# Operations at the 8-bit rate (QK^T, twice the 16-bit one) and at the 16-bit rate (P.V), half each.
+ATTN_RATE = 4.0 / 3.0
 
 
 def init_ranks(args):
@@ -410,19 +414,21 @@ def int8_gemm_peak(device, size=8192, repeats=10):
         return {"tops": None, "how": "unavailable: %s" % str(exc).splitlines()[0][:80]}
 
 
-def tensor_roofline(kernel, achieved_tops, peaks, peak_source, region_seconds, traffic):
-    burst = 2.0 * float(peaks["bf16_tflops"])
-    sustained = 2.0 * float(peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"]))
+def tensor_roofline(kernel, achieved_tops, peaks, peak_source, region_seconds, traffic, rate=2.0):
+    """``rate``: of the kernel's operations, in units of the BF16 rate."""
+    burst = rate * float(peaks["bf16_tflops"])
+    sustained = rate * float(peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"]))
     long_region = region_seconds >= 1.0
     peak = sustained if long_region else burst
     return {
         "bound": "tensor", "kernel": kernel, "achieved": achieved_tops, "peak": peak, "unit": "TOP/s",
         "frac": achieved_tops / peak,
-        "peak_source": "2 x %s of MEASURED_PEAKS.json (%s): INT8/FP8 tensor rate is twice BF16; the timed region "
-                       "lasts %.2f s" % ("bf16_tflops_sustained" if long_region else "bf16_tflops (burst)", peak_source,
-                                         region_seconds),
+        "peak_source": "%.3g x %s of MEASURED_PEAKS.json (%s): INT8/FP8 tensor rate is twice the 16-bit rate%s; the timed "
+                       "region lasts %.2f s" % (rate, "bf16_tflops_sustained" if long_region else "bf16_tflops (burst)", peak_source,
+                                                ", which half of the operations (P.V) run at" if rate < 2.0 else "",
+                                                region_seconds),
         "frac_of_burst": achieved_tops / burst, "frac_of_sustained": achieved_tops / sustained,
-        "frac_of_nominal_4500": achieved_tops / NOMINAL_INT8_TOPS, "traffic": traffic,
+        "frac_of_nominal": achieved_tops / (NOMINAL_INT8_TOPS * rate / 2.0), "traffic": traffic,
     }
 
 
@@ -474,7 +480,7 @@ def projection_summary(spec, device, steps=3):
                         "GEMM epilogue" % (spec.sequence, hidden, 3 * spec.heads * HEAD_DIM, hidden),
             "projection_ms": project_ms, "qkv_gemm_all_chunks_ms": gemm_ms, "qkv_gemm_ops": gemm_ops,
             "qkv_gemm_tops": tops, "frac_of_burst": tops / (2.0 * float(peaks["bf16_tflops"])),
-            "frac_of_nominal_4500": tops / NOMINAL_INT8_TOPS, "gpu_launches_per_projection": len(chunks) * 2 + 4}
+            "frac_of_nominal_4500": tops / NOMINAL_INT8_TOPS, "gpu_launches_per_projection": len(chunks) * 2 + 3}
 
 
 def run_attention(args, spec, stdout):
@@ -672,14 +678,15 @@ def run_attention(args, spec, stdout):
     if rank == 0:
         peaks, peak_source = measured_peaks()
         heads_local = h1 - h0
-        carrier_bytes = heads_local * spec.sequence * HEAD_DIM * (3 * 2 + 3 * 1) + heads_local * spec.sequence * HEAD_DIM * 2 * 2
+        # inputs read once, K and V once more for the statistics, carriers written
+        carrier_bytes = heads_local * spec.sequence * HEAD_DIM * (3 * 2 + 2 * 2 + CARRIER_BYTES)
         traffic = ATTN_DRAM_BYTES_PER_HEAD * heads_local if (spec.sequence == 33272 and abs(args.budget - 0.3) < 1e-9
                                                               and not args.schedule) else None
         step_ms = graph_ms if graph_ms is not None else device_ms
         line = {
             "metric": METRIC, "value": total_ops / (step_ms * 1e-3) / 1e12, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True,
-            "scaling": "strong", "vs_baseline": None, "dtype": "int8 QK^T / fp8-e4m3 PV, fp32 softmax",
+            "scaling": "strong", "vs_baseline": None, "dtype": "int8 QK^T / fp16 P x fp8-e4m3 V, fp32 softmax",
             "data": "synthetic",
             "launch": launch, "eager_ms_per_step": device_ms,
             "config": {
@@ -688,9 +695,9 @@ def run_attention(args, spec, stdout):
                 "l2_policy": "no flush: a step streams %.0f MB of bf16 Q/K/V, %.0f MB of carriers (written, then read) and "
                              "the %.0f MB gathered output through this GPU's 126 MB L2"
                              % (heads_local * spec.sequence * HEAD_DIM * 2 * 3 / 1e6,
-                                heads_local * spec.sequence * HEAD_DIM * 3 / 1e6,
+                                heads_local * spec.sequence * HEAD_DIM * CARRIER_BYTES / 1e6,
                                 spec.heads * spec.sequence * HEAD_DIM * 2 / 1e6),
-                "p_terms": 2, "algorithmic_ops": total_ops, "route_len": sparse.route.route_len,
+                "p_format": "fp16", "algorithmic_ops": total_ops, "route_len": sparse.route.route_len,
                 "layer_calls_per_step": len(positions),
             },
             "stages_ms": {"prepare (stats+quant+route)": prep_ms, "attention": attn_ms, "exchange tail": exch_ms},
@@ -698,7 +705,8 @@ def run_attention(args, spec, stdout):
             "stages_ms_per_rank": per_rank,
             "prepare_hbm": {"bytes": carrier_bytes, "gbs": carrier_bytes / (prep_ms * 1e-3) / 1e9,
                             "frac_of_measured_copy": carrier_bytes / (prep_ms * 1e-3) / 1e9 / float(peaks["hbm_gbs"])},
-            "roofline": tensor_roofline("sparse_attn_tc_kernel", attn_ops_rate, peaks, peak_source, region_seconds, traffic),
+            "roofline": tensor_roofline("sparse_attn_half_kernel", attn_ops_rate, peaks, peak_source, region_seconds, traffic,
+                                        rate=ATTN_RATE),
             "int8_peak_measured": int8_gemm_peak(device),
             "clocks": clocks,
             "gpu_launches": calls * 7,
@@ -858,7 +866,7 @@ def run_config2(args, spec, stdout):
         line = {
             "metric": METRIC, "value": (attn_ops + gemm_ops) / (step_ms * 1e-3) / 1e12, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True,
-            "scaling": "strong", "vs_baseline": None, "dtype": "int8 GEMM + int8 QK^T / fp8-e4m3 PV", "data": "synthetic",
+            "scaling": "strong", "vs_baseline": None, "dtype": "int8 GEMM + int8 QK^T / fp16 P x fp8-e4m3 V", "data": "synthetic",
             "config": {"workload": "config2: x (%d,%d) bf16 -> ConvRot INT8 QKV projection (W %dx%d int8, 4096-token chunks, "
                                    "carriers from the GEMM epilogue) -> %s"
                                    % (spec.sequence, hidden, 3 * spec.heads * HEAD_DIM, hidden, workload_name(spec, args.budget)),
@@ -873,7 +881,7 @@ def run_config2(args, spec, stdout):
             "int8_peak_measured": int8_gemm_peak(device),
             "convrot_hbm": {"bytes": rot_bytes, "gbs": rot_bytes / (rot_ms * 1e-3) / 1e9,
                             "frac_of_measured_copy": rot_bytes / (rot_ms * 1e-3) / 1e9 / float(peaks["hbm_gbs"])},
-            "clocks": clocks, "gpu_launches": args.steps * (len(chunks) * 2 + 7),
+            "clocks": clocks, "gpu_launches": args.steps * (len(chunks) * 2 + 5),
         }
         stdout.emit(line)
     if world > 1:
@@ -975,7 +983,7 @@ def run_config4(args, spec, stdout):
             "metric": METRIC, "value": (attn_ops + proj_ops + mlp_ops) / (step_ms * 1e-3) / 1e12, "unit": UNIT,
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_ms,
             "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-            "dtype": "int8 QK^T / fp8-e4m3 PV; bf16 out_proj; fp8-e4m3 MLP", "data": "synthetic",
+            "dtype": "int8 QK^T / fp16 P x fp8-e4m3 V; bf16 out_proj; fp8-e4m3 MLP", "data": "synthetic",
             "config": {"workload": "config4: B2 H%d D128, %d tokens per batch element (%s), video x video tiles sparse at %.0f%%, "
                                    "then out_proj %d->%d (bf16) and FP8-E4M3 MLP %d->%d (GELU-tanh)->%d in 4096-token chunks"
                                    % (spec.heads, spec.sequence, " + ".join("%d %s" % (b - a, kind) for a, b, kind in spec.segments),

@@ -1,5 +1,5 @@
-// What the two tcgen05 attention kernels share: launch parameters, status codes,
-// packed FP32 arithmetic and the 8-channel output store.
+// What the two tcgen05 attention kernels share: launch parameters, status codes, bounded waits
+// and the output stores.
 #pragma once
 
 #include "common.cuh"

@@ -149,9 +149,10 @@ convrot_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_stride,
 // 128x256 tile per SM pulled 48 KB through L2 for every 512 cycles of MMA work, 96 bytes
 // a clock and SM, which is more than L2 delivers to all SMs at once; the pair needs 64,
 // and the smaller stages leave room for one more.  MLP of 33272 x 3072 x 12288: 3.59 ->
-// 3.06 ms (with gelu_tanh below), of 1000 tokens 147 -> 120 us; attention block of 33272
-// tokens 6.09 -> 5.91 ms.  A single row tile wastes half a pair, but what such a call
-// waits for is the weights, which are read once either way.
+// 3.02 ms (with gelu_tanh below), of 1000 tokens 147 -> 119 us; attention block of 33272
+// tokens 6.09 -> 5.90 ms; 2.74 ms, 108 us and 5.5 ms with the epilogues and quantisers as they
+// are now.  A single row tile wastes half a pair, but what such a call waits for is the
+// weights, which are read once either way.
 constexpr int kGemmM = 128, kGemmN = 256, kGemmK = 128;  // per CTA; K in bytes == int8 elements
 constexpr int kGemmPairM = 2 * kGemmM;
 // Row pairs visited before the next column of tiles: 4096 rows of A (12 to 50 MB) and the
