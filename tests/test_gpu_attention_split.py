@@ -39,7 +39,7 @@ def test_long_rows_beside_routed_ones(native_lib):
 
 @pytest.mark.parametrize("low", [slice(0, 900), slice(900, 1601), slice(0, 64)])
 def test_parts_whose_scores_lie_hundreds_of_bits_apart(native_lib, low):
-    """One part's sums vanish beside another's, or a part has to be done again with its true maximum."""
+    """One part's sums vanish beside another's, or a part has to come back to tiles that it left out."""
     sequence = 1601
     assert _workspace(2, sequence) > 0
     spec = workloads.small_spec("split", 2, 0, sequence)

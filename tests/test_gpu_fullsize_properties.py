@@ -101,18 +101,16 @@ def test_attention_normalisation_and_determinism(prepared):
     dequant = carrier[..., :1].float().transpose(-1, -2) * v_scale[..., None, :]  # what the kernel sees as V
     ratio = out / dequant
     assert bool(torch.isfinite(out).all())
-    # FP8 probabilities span 2^-9 .. 2^8.75 around a reference point 7 bits below
-    # the row maximum: keys more than ~17 bits below the maximum are counted in
-    # the row sum l (exact FP32) but reach the numerator as zero.  On strongly
-    # peaked rows of a 33k/76k-key softmax that tail holds up to 2-3 % of the
-    # mass, so the ratio may fall short of 1 by that much and never exceeds it;
-    # the typical row is within 2^-9.
+    # Keys more than 17 bits below the row maximum with FP8 probabilities, 19 or more with
+    # FP16's, are counted in the row sum l (exact FP32) but reach the numerator as zero.
+    # On strongly peaked rows of a 33k/76k-key softmax that tail holds up to 2-3 % of
+    # the mass with FP8, which these bounds have room for.
     shortfall = float((1.0 - ratio).max())
     excess = float((ratio - 1.0).max())
     mean_deviation = float((ratio - 1.0).abs().mean())
     assert shortfall < 3.5e-2 and excess < 4.0e-3 and mean_deviation < 2.0e-3, (shortfall, excess, mean_deviation)
 
-    # The rows that lose the most FP8 tail mass are where the kernel differs most from
+    # The rows that lose the most tail mass are where the kernel differs most from
     # arithmetic with FP32 probabilities: the three (head, query tile) pairs with the
     # largest shortfall go through the CPU oracle with the real V, and the gate must
     # hold on them as on any other tile.

@@ -6,10 +6,10 @@ attention: the Triton kernels of attention/sparse/triton_sparse_kernels.py
 206-246).  They import nothing but torch and Triton, so the unmodified file -
 staged under oracle/_ref by oracle/build_ref.py - runs on the same GPU, on the
 same seeded inputs, the same INT8 Q/K codes and the same route as
-`sparse_attn_tc_kernel`.  The two differ only where the formats differ: the
+`sparse_attn_half_kernel`.  The two differ only where the formats differ: the
 reference carries V as per-(64-key block, channel) INT8 with unsigned 8-bit
 probabilities (triton_sparse_kernels.py:34-42), this library carries V as
-per-channel FP8-E4M3 with two E4M3 probability terms.
+per-channel FP8-E4M3 with FP16 probabilities.
 
 Both outputs are also compared with the reference's FP32 attention on the same
 block mask (benchmarks/bench_sparse_backends.py:302-326), run from the staged
