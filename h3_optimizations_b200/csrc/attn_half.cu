@@ -33,7 +33,8 @@
 // tokens, 30 %: 3.09 to 3.26 ms on the inputs above; 3.29 to 3.48 with one row of every query
 // tile 48 bits ahead in every 40th tile; 3.78 to 3.94 with a third of the rows ahead in every tenth;
 // two E4M3 terms take 4.2 to 4.3 ms of each.  All but the first two tiles of a list
-// ahead is the worst: two walks, three where a sum overflows (120 bits).
+// ahead is the worst: two walks, three where a sum overflows (120 bits): 24 heads x 9872,
+// dense, 0.83 ms, then 2.1 to 2.2 and 2.9, where two E4M3 terms take 1.13.
 //
 // Without a running maximum the tiles of a row are independent but for the sum:
 // the eight softmax warps form two groups, group g takes tiles g, g+2, ..., and
@@ -100,7 +101,7 @@ struct HalfShared {
   uint64_t staged;             // softmax warps only: the output tile is in shared memory (and steps before that)
   uint32_t tmem_base;
   int abort_word;
-  int again;                   // kAgainNoted: some row has left out a tile; kAgainFar: its sum there is no number
+  int again;                   // kAgainNoted: some row has left out a tile; kAgainFar: its sum there does not tell the maximum
   int finish;                  // this CTA writes the output tile
   int tile_index[kHStages];    // KV tile held by each stage ...
   float tile_scale[kHStages];  // ... and its k_scale, written by the producer
@@ -120,15 +121,18 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 // Row sum and, with kPack, FP16 P of 64 scores.  The int32 scores become fp32 without a
 // conversion instruction: for |s| < 2^22, bits(12582912.0f) + s are the bits of
 // the float 12582912 + s exactly, and the offset is folded into the constants of
-// the FMA that follows: P = exp2(c*f + bias) = exp2(c*s - m).
-template <bool kPack>
+// the FMA that follows: P = exp2(c*f + bias) = exp2(c*s - m).  The folded constant is
+// rounded, by 2^-24 of c*12582912: nothing for attention scores, but a factor of two from c = 1 on
+// (scores of 2^20 bits).  With kExact the offset is taken off first and `bias` is -m.
+template <bool kPack, bool kExact>
 __device__ __forceinline__ float exp_sum(const uint32_t (&s)[H3S_KV_TILE], float c, float bias,
                                          uint32_t (&packed)[H3S_KV_TILE / 2]) {
   const float2 c2 = make_float2(c, c), bias2 = make_float2(bias, bias);
   float2 sum_a = make_float2(0.f, 0.f), sum_b = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < H3S_KV_TILE / 2; ++i) {
-    const float2 f = make_float2(__uint_as_float(s[2 * i] + kIntBiasBits), __uint_as_float(s[2 * i + 1] + kIntBiasBits));
+    float2 f = make_float2(__uint_as_float(s[2 * i] + kIntBiasBits), __uint_as_float(s[2 * i + 1] + kIntBiasBits));
+    if (kExact) f = add2(f, make_float2(-kIntBias, -kIntBias));
     const float2 x = fma2(c2, f, bias2);
     const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
     if (i & 1) sum_b = add2(sum_b, p); else sum_a = add2(sum_a, p);
@@ -456,7 +460,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         if (j == 1 && !warp_wait(&sh.first_exp, 0, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
       }
       uint32_t packed[H3S_KV_TILE / 2];
-      float sum = exp_sum<true>(s, c, -fmaf(c, kIntBias, m), packed);
+      float sum = exp_sum<true, false>(s, c, -fmaf(c, kIntBias, m), packed);
       if (j == 0) {
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&sh.first_exp);
@@ -464,7 +468,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       put(packed);
       const bool out = !(sum <= kHSumLimit);
       if (__any_sync(0xffffffffu, out)) {  // these rows leave the tile out
-        const bool far = __any_sync(0xffffffffu, sum == INFINITY);
+        const bool far = __any_sync(0xffffffffu, sum == INFINITY || c > 1.f);  // no measure of the maximum
         ptx::tmem_wait_st();
         if (out) {
           largest = fmaxf(largest, sum);
@@ -535,8 +539,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         if (!take(j, s, c)) { ok = false; break; }
         uint32_t packed[H3S_KV_TILE / 2];
         // the same sum as in the first pass, so the same tiles
-        const bool out = !(exp_sum<false>(s, c, -fmaf(c, kIntBias, m), packed) <= kHSumLimit);
-        const float sum = exp_sum<true>(s, c, -fmaf(c, kIntBias, m_again), packed);
+        const bool out = !(exp_sum<false, false>(s, c, -fmaf(c, kIntBias, m), packed) <= kHSumLimit);
+        const float sum = exp_sum<true, true>(s, c, -m_again, packed);
         if (out) {
           l += sum;
         } else {

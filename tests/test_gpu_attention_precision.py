@@ -79,3 +79,25 @@ def test_tiles_left_out_of_a_list_longer_than_the_note(native_lib):
     sequence = 64 * 2187 + 9
     q, k, v = _spikes(sequence, 1, [2, 700, 701, 1500, 2186, 2187], seed=1)
     _compare(q, k, v, oracle.geometry(sequence, 0), None, tiles=[0, 500, 1093])
+
+
+@pytest.mark.parametrize("scale", [1e2, 1e4, 1e5])
+def test_scores_of_a_hundred_to_a_million_bits(native_lib, scale):
+    """Finite, and no further off than at ordinary scales: what has the weight there is left out at first and walked
+    again with the exponent's offset taken off exactly.  Against 64-bit arithmetic on the carriers."""
+    from h3_optimizations_b200 import ops
+
+    sequence, heads = 1000, 2
+    q, k, v = workloads.gaussian_qkv(workloads.small_spec("scale", heads, 0, sequence), seed=6, widen=True)
+    q8, qs = oracle.quantize_blocks(q * scale ** 0.5, 128)
+    k8, ks = oracle.quantize_blocks(k * scale ** 0.5, 64)
+    vc, vs = oracle.v_fp8_carrier(v)
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    out = ops.sparse_attention(*(t.cuda() for t in (q8, k8, vc, qs, ks, vs)), status=status, out_dtype=torch.float32).cpu()
+    assert status.tolist() == [0, 0, 0, 0] and bool(torch.isfinite(out).all())
+    z = q8[0].double() @ k8[0].double().transpose(1, 2) * 128 ** -0.5
+    z *= qs[0].double().repeat_interleave(128, 1)[:, :sequence, None] * ks[0].double().repeat_interleave(64, 1)[:, None, :sequence]
+    want = torch.softmax(z, -1) @ (vc[0, :, :, :sequence].double() * vs[0].double()[:, :, None]).transpose(1, 2)
+    # 2^-11 of each probability; 2^-24 * c * 12582912 bits of a tile that was not left out, where c is about 1e-4 * scale
+    # and such tiles have weight at the smaller scales only
+    assert float((out[0].double() - want).norm() / want.norm()) <= 1e-3
