@@ -1,8 +1,8 @@
 // Block-sparse attention on INT8 Q/K and an FP16 copy of the FP8 V carrier, for
 // sm_100a.
 //
-// One CTA owns one 128-row query tile of one head and walks that tile's list
-// of 64-row KV tiles:
+// An item is a 128-row query tile of one head and that tile's list of 64-row KV tiles (or a part of
+// it).  One CTA per SM walks item after item:
 //   S = Q8 . K8^T      tcgen05.mma kind::i8, 128x64x128, Q8 in TMEM, int32 in TMEM
 //   P = exp2(c*S - m)  FP32 in registers, one thread per query row, m an integer
 //   O += P16 . V16     tcgen05.mma kind::f16, 128x128x64, P in TMEM, fp32 in TMEM
@@ -36,49 +36,57 @@
 // ahead is the worst: two walks, three where a sum overflows (120 bits): 24 heads x 9872,
 // dense, 0.83 ms, then 2.1 to 2.2 and 2.9, where two E4M3 terms take 1.13.
 //
-// Without a running maximum the tiles of a row are independent but for the sum:
-// the eight softmax warps form two groups, group g takes tiles g, g+2, ..., and
-// with two CTAs per SM four warps share a scheduler, each in its own phase of
-// wait / load / exponentials / store.  With one group, or with two threads per row,
-// the CTAs fall into step and both pipes idle a third of the time.
+// Without a running maximum the tiles of a row are independent but for the sum: the sixteen
+// softmax warps form four groups, group g takes every fourth tile, and each scheduler has one
+// warp of every group, in its own phase of wait / load / exponentials / store.
 //
-// TMEM (256 columns per CTA, two CTAs per SM): O 128, Q8 32 (A operand of QK^T:
-// Q is read once instead of with every K tile, which takes a third off the
-// shared-memory traffic), and three 32-column slots A B C.  S(j) is 64 columns:
-// A+B for even j, B+C for odd j; P(j) is 32 columns: A for even, C for odd.
-// QK^T(j) needs S(j-1) in registers (slot B) and P.V(j-2) complete.
+// TMEM (all 512 columns): O 128, Q8 2 x 32 (A operand of QK^T, copied from shared memory by the tensor
+// pipe; the next item's rows arrive while this one's are used), P 4 x 32 (one per group), S 3 x 64.  QK^T runs up
+// to three tiles ahead of the groups, P.V behind them in the order of the list, and no tile waits for
+// another one's P.V.  Two CTAs of 256 columns an SM, as before, have room for S or P of two tiles each:
+// QK^T(j+2) had to wait for P.V(j), and a group's softmax, its P.V and its next QK^T were one chain.
+// One query tile an SM also ends twice as soon, which evens out what the last CTAs do.
 //
-// Warp roles: warps 0-7 softmax/epilogue (TMEM lanes 32*(w%4).., group w/4), warp 8
-// TMA producer and QK^T issuer, warp 9 P.V issuer and TMEM owner.
+// Warp roles: warps 0-15 softmax/epilogue (TMEM lanes 32*(w%4).., group w/4), 16 K loader, 17 QK^T
+// issuer, 18 P.V issuer and TMEM owner, 19 V loader.  The last four are one thread each but for
+// fetching the list: what such a thread does for a tile is a chain of dependent instructions, and with
+// votes of the whole warp, or K and V from one thread, that chain was as long as a tile takes (600 cycles).
+//
+// A CTA that is through with an item takes over one that has not started (clusterlaunchcontrol), the long
+// ones first; the next item's Q, scales and first tile indices are fetched under the last tiles of this one.
 //
 // Dense rows (query tiles that see every key) are cut into parts where one of them is
-// longer than what a CTA slot gets on average, i.e. where a few long rows would outlast
-// all others: see split_dense_rows.  Each part is a CTA with its own reference point; it
+// longer than half of what an SM gets on average, i.e. where a few long rows would outlast
+// all others: see split_dense_rows.  Each part is an item with its own reference point; it
 // leaves its sums in memory and the part that comes last adds them up, in the order of
 // the list, so that the result does not depend on which one that was.
 //
-// What bounds it: per tile and SM the ex2 pipe needs 512 cycles, the tensor pipe 453
-// (measured: 144 for QK^T with A in TMEM, 258 with A in shared memory, 309 for P.V; at
-// the nominal rates 384 in all), the remaining softmax instructions about 290 issue
-// slots; a tile takes about 800.  24 heads x 33272 tokens at 30 %, launches in a row: 4.20 to
-// 4.33 ms with two E4M3 terms, 3.09 to 3.26 ms here.  Tried and slower: a polynomial for a
-// share of the exponentials, two threads per row, one group per CTA, scores of the next
-// tile fetched between the halves of this one.
+// What bounds it: per tile and SM the ex2 pipe needs 512 cycles, the tensor pipe 453 (measured: 144 for QK^T with A
+// in TMEM, 258 with A in shared memory, 309 for P.V; at the nominal rates 384 in all), the softmax
+// instructions of four warps a scheduler together 535; a tile takes about 780.  Beside that an item has
+// about 7000 cycles of its own (last P.V, epilogue, first tiles), and the power cap holds the clock at 1.65 to
+// 1.75 GHz.  Attention alone, two CTAs of two groups an SM before and this now: 24 heads x 33272 tokens at 30 %, 3.08 ms
+// and 2.84 (3.38 and 3.26 in a loop); 24 x 9872 dense 866 us and 786; 3 x 33272 412 and 384; 7 x 10384 at 15 % 96.5 and
+// 88; 4 x 2304 28.7 and 22.9; 24 x 2304 43.6 and 43.1.  Tried and slower on the earlier form: a polynomial
+// for a share of the exponentials, two threads per row, one group per CTA.
 #include "attn_common.cuh"
 #include "tma.cuh"
 
 namespace h3s {
 
-constexpr int kHStages = 4;  // tile i+2 is loaded when tile i-2 is done
-constexpr int kHSoftmaxWarps = 8;
-constexpr int kHThreads = (kHSoftmaxWarps + 2) * 32;
-constexpr int kHTmemCols = 256;
+constexpr int kHGroups = 4;  // of softmax warps; a group takes every fourth tile
+constexpr int kHSoftmaxWarps = 4 * kHGroups;
+constexpr int kHKeyLoader = kHSoftmaxWarps, kHScoreIssuer = kHSoftmaxWarps + 1, kHValueIssuer = kHSoftmaxWarps + 2,
+              kHValueLoader = kHSoftmaxWarps + 3;
+constexpr int kHWarps = kHSoftmaxWarps + 4, kHThreads = kHWarps * 32;
+constexpr int kHScoreSlots = 3;
+constexpr int kHMaxKStages = 5, kHMaxVStages = 8;
+constexpr int kHTmemCols = 512, kHTmemQ = 128, kHTmemP = 192, kHTmemS = 320;  // O from 0
 constexpr uint32_t kHKBytes = H3S_KV_TILE * H3S_HEAD_DIM;      // 8192
 constexpr uint32_t kHVBytes = H3S_HEAD_DIM * H3S_KV_TILE * 2;  // 16384
-constexpr uint32_t kHOffK = 0;
-constexpr uint32_t kHOffV = kHOffK + kHStages * kHKBytes;
-constexpr uint32_t kHOffBar = kHOffV + kHStages * kHVBytes;
-constexpr uint32_t kHSmemBytes = kHOffBar + 4096 + 1024;  // barriers/scalars + alignment slack
+constexpr uint32_t kHQBytes = H3S_Q_TILE * H3S_HEAD_DIM;       // 16384
+constexpr int kHBlock = 16;  // tiles of a list that are fetched at a time
+constexpr int kHMeta = 32;   // tiles whose scale is kept: a block and those before it that are loaded but not taken yet
 constexpr float kHSumLimit = 65504.f;  // of a row over one tile: no P above it can have overflowed FP16
 constexpr float kHFirstBits = 5.f;     // the reference tiles' row maximum becomes 2^-5 ...
 constexpr float kHMostBits = 15.f;     // ... P may grow to 2^15 ...
@@ -87,30 +95,54 @@ constexpr int kHNoted = 2048;          // bits of the note of tiles left out, ea
 
 enum { kAgainNoted = 1, kAgainFar = 2 };
 
-struct HalfShared {
-  uint64_t q_ready;            // four softmax warps have put the Q rows into TMEM
-  uint64_t kv_full[kHStages];
-  uint64_t s_full[2];          // QK^T of tile j has completed (one per group)
-  uint64_t s_taken[2];         // S(j) is in registers
-  uint64_t p_full[2];          // P(j) is in TMEM
-  uint64_t pv_done[2];         // P.V of tile j has completed: its stage and its slot are free
-  uint64_t first_max;          // both groups have left their first tile's row maxima in `first`
-  uint64_t first_exp;          // group 0 is through its first tile's exponentials
-  uint64_t pass_end;           // the rows' values of a pass are in `row`, `noted` is complete; all warps wait,
-                               // and the P.V warp arrives too: see there
+// What the warps need to know of an item before its first tile
+struct HalfItem {
+  int number;  // of the launch, -1: no more
+  float q_scale;
+  float v_scale[H3S_HEAD_DIM];
+};
+
+struct alignas(16) HalfShared {
+  uint4 next_reply;            // of the request for another item
+  uint64_t next_ready;         // ... has arrived
+  uint64_t q_full, q_free;     // the next item's Q rows are in shared memory, have been copied to TMEM
+  uint64_t k_full[kHMaxKStages], k_empty[kHMaxKStages];
+  uint64_t v_full[kHMaxVStages], v_empty[kHMaxVStages];
+  uint64_t s_full[kHGroups];       // QK^T of a tile has completed; by group and not by slot, whose last user is another
+                                   // group: a wait must never be two uses ahead
+  uint64_t s_taken[kHScoreSlots];  // S of a tile is in registers
+  uint64_t p_full[kHGroups];       // P of a tile is in TMEM
+  uint64_t pv_done[kHGroups];      // P.V of a tile has completed: P may be written again
+  uint64_t o_full, o_free;     // every P.V of a pass has completed; the softmax warps have read or scaled O
+  uint64_t first_max;          // the reference tiles' row maxima are in `first`
+  uint64_t pass_end;           // the rows' values of a pass are in `row`, `noted` is complete; all warps arrive and wait
   uint64_t staged;             // softmax warps only: the output tile is in shared memory (and steps before that)
   uint32_t tmem_base;
   int abort_word;
-  int again;                   // kAgainNoted: some row has left out a tile; kAgainFar: its sum there does not tell the maximum
-  int finish;                  // this CTA writes the output tile
-  int tile_index[kHStages];    // KV tile held by each stage ...
-  float tile_scale[kHStages];  // ... and its k_scale, written by the producer
-  float v_scale[H3S_HEAD_DIM];
-  uint32_t noted[kHNoted / 32];  // tiles of the list that some row has left out
+  int finish;                  // of an item that is a part: this CTA writes the output tile
+  int again[4];                // per item in turn.  kAgainNoted: some row has left out a tile; kAgainFar: its sum
+                               // there does not tell the maximum
+  HalfItem item[3];            // in turn: an epilogue may still read the last one when the one after next is known
+  struct { int n_valid; float scale; } tile[kHMeta];  // keys of a tile inside the sequence, and its k_scale
+  int block[2][kHBlock];            // the next tiles of the list, for the threads that load K and V
+  uint32_t noted[2][kHNoted / 32];  // tiles of the list that some row has left out, per item in turn
   float first[2][H3S_Q_TILE];
-  float row[2][2][H3S_Q_TILE];  // values the two threads of a row give each other, in turn
+  float over[kHGroups][H3S_Q_TILE];    // largest sum that a row has left out
+  float row[2][kHGroups][H3S_Q_TILE];  // values the threads of a row give each other at a pass's end, in turn
 };
-static_assert(sizeof(HalfShared) <= 4096, "barrier block too large");
+
+// The output tile has room of its own, so that the next item's tiles can arrive under it
+template <typename OutT>
+struct HalfLayout {
+  static constexpr int kKStages = sizeof(OutT) == 4 ? 3 : 5, kVStages = sizeof(OutT) == 4 ? 6 : 8;
+  static constexpr uint32_t kOffK = 0;
+  static constexpr uint32_t kOffV = kOffK + kKStages * kHKBytes;
+  static constexpr uint32_t kOffQ = kOffV + kVStages * kHVBytes;
+  static constexpr uint32_t kOffOut = kOffQ + kHQBytes;
+  static constexpr uint32_t kOffShared = kOffOut + H3S_Q_TILE * H3S_HEAD_DIM * sizeof(OutT);
+  static constexpr uint32_t kBytes = kOffShared + sizeof(HalfShared) + 1024;  // alignment slack
+  static_assert(kKStages + kHScoreSlots < kHBlock && kKStages <= kHMaxKStages && kVStages <= kHMaxVStages && kBytes <= 227 * 1024, "attention shared memory exceeds the per-CTA limit");
+};
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
   uint32_t d;
@@ -162,251 +194,372 @@ __device__ __forceinline__ int noted_tiles(const uint32_t *noted, int n_iter, in
   return bits - (ends ? static_cast<int>((last + 1) << coarse) - n_iter : 0);
 }
 
+// Item `w` of a launch: dense (long) rows first, then the routed rows
+struct HalfWork {
+  int head, tq;
+  int dense_row, part;  // running number of a dense row, part of its list
+  bool dense;
+  int first_tile, n_iter;
+  const int32_t *route_row;
+};
+
+__device__ __forceinline__ HalfWork work_item(const AttnParams &prm, int w) {
+  HalfWork it;
+  const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
+  const int n_dense = prm.q_tiles - n_sparse;
+  const int dense_items = prm.heads * n_dense * prm.parts;
+  it.dense = w < dense_items;
+  it.dense_row = it.part = it.first_tile = 0;
+  it.route_row = nullptr;
+  if (it.dense) {
+    it.dense_row = w / prm.parts;
+    it.part = w - it.dense_row * prm.parts;
+    it.head = it.dense_row / n_dense;
+    const int i = it.dense_row - it.head * n_dense;
+    it.tq = (n_sparse == 0 || i < prm.q_start) ? i : prm.q_stop + (i - prm.q_start);
+    it.first_tile = it.part * prm.part_tiles;
+    it.n_iter = min(prm.part_tiles, prm.kv_tiles - it.first_tile);
+  } else {
+    const int v = w - dense_items;
+    it.head = v / n_sparse;
+    const int i = v - it.head * n_sparse;
+    it.tq = prm.q_start + i;
+    it.n_iter = prm.route_len;
+    it.route_row = prm.route + (static_cast<int64_t>(it.head) * n_sparse + i) * prm.route_len;
+  }
+  return it;
+}
+
+// The i-th tile that is walked
+__device__ __forceinline__ int list_position(int i, int n_iter) {
+  return i + n_iter / 2 < n_iter ? i + n_iter / 2 : i + n_iter / 2 - n_iter;
+}
+
+// A bit of the note stands for 2^n tiles
+__device__ __forceinline__ int note_scale(int n_iter) { return 32 - __clz((n_iter - 1) / kHNoted); }
+
 template <typename OutT>
-__global__ void __launch_bounds__(kHThreads, 2)
-sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                        const int8_t *__restrict__ q8, const AttnParams prm) {
+__global__ void __launch_bounds__(kHThreads, 1)
+sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                        const __grid_constant__ CUtensorMap map_v, const AttnParams prm) {
+  using L = HalfLayout<OutT>;
   extern __shared__ unsigned char smem_dyn[];
   // SWIZZLE_128B tiles need 1024-byte alignment
   // (offset arithmetic, so that the compiler still sees shared memory)
   unsigned char *smem = smem_dyn + ((1024u - (ptx::smem_u32(smem_dyn) & 1023u)) & 1023u);
-  HalfShared &sh = *reinterpret_cast<HalfShared *>(smem + kHOffBar);
+  HalfShared &sh = *reinterpret_cast<HalfShared *>(smem + L::kOffShared);
   volatile int *abort_word = &sh.abort_word;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  // ---- work item: dense (long) rows first, then the routed rows ----
-  const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
-  const int n_dense = prm.q_tiles - n_sparse;
-  int head, tq;
-  int dense_row = 0, part = 0;  // running number of a dense row, part of its list
-  bool dense;
-  {
-    const int w = blockIdx.x;
-    const int dense_items = prm.heads * n_dense * prm.parts;
-    if (w < dense_items) {
-      dense = true;
-      dense_row = w / prm.parts;
-      part = w - dense_row * prm.parts;
-      head = dense_row / n_dense;
-      const int i = dense_row - head * n_dense;
-      tq = (n_sparse == 0 || i < prm.q_start) ? i : prm.q_stop + (i - prm.q_start);
-    } else {
-      dense = false;
-      const int v = w - dense_items;
-      head = v / n_sparse;
-      tq = prm.q_start + (v - head * n_sparse);
-    }
-  }
-  const bool split = dense && prm.parts > 1;
-  const int first_tile = part * prm.part_tiles;  // of a dense row's list
-  const int n_iter = dense ? min(prm.part_tiles, prm.kv_tiles - first_tile) : prm.route_len;
-  const int32_t *route_row =
-      dense ? nullptr
-            : prm.route + (static_cast<int64_t>(head) * n_sparse + (tq - prm.q_start)) * prm.route_len;
+  int item = blockIdx.x;  // the first; more are asked for
+  HalfWork work = work_item(prm, item);
 
   // ---- setup ----
   if (threadIdx.x == 0) {
-    ptx::mbar_init(&sh.q_ready, 4);
-    for (int i = 0; i < kHStages; ++i) ptx::mbar_init(&sh.kv_full[i], 1);
-    for (int g = 0; g < 2; ++g) {
+    ptx::mbar_init(&sh.next_ready, 1);
+    ptx::mbar_init(&sh.q_full, 1);
+    ptx::mbar_init(&sh.q_free, 1);
+    for (int i = 0; i < L::kKStages; ++i) {
+      ptx::mbar_init(&sh.k_full[i], 1);
+      ptx::mbar_init(&sh.k_empty[i], 1);
+    }
+    for (int i = 0; i < L::kVStages; ++i) {
+      ptx::mbar_init(&sh.v_full[i], 1);
+      ptx::mbar_init(&sh.v_empty[i], 1);
+    }
+    for (int i = 0; i < kHScoreSlots; ++i) ptx::mbar_init(&sh.s_taken[i], 4);
+    for (int g = 0; g < kHGroups; ++g) {
       ptx::mbar_init(&sh.s_full[g], 1);
-      ptx::mbar_init(&sh.s_taken[g], 4);
       ptx::mbar_init(&sh.p_full[g], 4);
       ptx::mbar_init(&sh.pv_done[g], 1);
     }
-    ptx::mbar_init(&sh.first_max, kHSoftmaxWarps);
-    ptx::mbar_init(&sh.first_exp, 4);
-    ptx::mbar_init(&sh.pass_end, kHSoftmaxWarps + 1);
+    ptx::mbar_init(&sh.o_full, 1);
+    ptx::mbar_init(&sh.o_free, kHSoftmaxWarps);
+    ptx::mbar_init(&sh.first_max, 8);
+    ptx::mbar_init(&sh.pass_end, kHWarps);
     ptx::mbar_init(&sh.staged, kHSoftmaxWarps);
     sh.abort_word = 0;
-    sh.again = 0;
-    sh.finish = 1;
+    sh.finish = 0;
+    for (int i = 0; i < 4; ++i) sh.again[i] = 0;
+    sh.item[0].q_scale = __ldg(prm.q_scale + work.head * prm.q_tiles + work.tq);
     ptx::fence_mbar_init();
   }
-  if (threadIdx.x < kHNoted / 32) sh.noted[threadIdx.x] = 0u;
-  if (threadIdx.x < H3S_HEAD_DIM) sh.v_scale[threadIdx.x] = __ldg(prm.v_scale + head * H3S_HEAD_DIM + threadIdx.x);
-  if (warp == kHSoftmaxWarps + 1) {
+  if (threadIdx.x < 2 * kHNoted / 32) (&sh.noted[0][0])[threadIdx.x] = 0u;
+  if (threadIdx.x < H3S_HEAD_DIM) sh.item[0].v_scale[threadIdx.x] = __ldg(prm.v_scale + work.head * H3S_HEAD_DIM + threadIdx.x);
+  if (warp == kHValueIssuer) {
     ptx::tmem_alloc(&sh.tmem_base, kHTmemCols);
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_o = sh.tmem_base;         // 128 columns, fp32
-  const uint32_t tmem_q = tmem_o + 128;         // 32 columns, four int8 codes each
-  const uint32_t tmem_s = tmem_o + 160;         // slots A B C, 32 columns each
+  const uint32_t tmem_o = sh.tmem_base;
 
-  // Passes: one over the list; where tiles were left out another one over those, with a
-  // pass for the rows' true maxima in between where a sum has overflowed.  Every warp waits
-  // for `pass_end`, so all agree on the tiles.  `done` counts the tiles of earlier passes:
-  // stages and parities run on.
+  // Passes of an item: one over the list; where tiles were left out another one over those,
+  // with a pass for the rows' true maxima in between where a sum has overflowed.  Every warp
+  // arrives at `pass_end` and waits for it, so all agree on the tiles and the next item.
+  // `done` counts the tiles of earlier items and passes, `passes` the passes, `items` the items:
+  // slots and parities run on.
   bool ok = true;
-  int done = 0, count = n_iter;
-  const int coarse = 32 - __clz((n_iter - 1) / kHNoted);  // a bit of the note stands for 2^coarse tiles
+  int done = 0, passes = 0;
+  uint32_t items = 0;
   auto last_pass = [&]() {
-    const int again = *static_cast<volatile int *>(&sh.again);
+    const int again = *static_cast<volatile int *>(&sh.again[items & 3]);
     return again == 0 ? 0 : again & kAgainFar ? 2 : 1;
   };
-  auto list_position = [&](int i) { return i + n_iter / 2 < n_iter ? i + n_iter / 2 : i + n_iter / 2 - n_iter; };
-
-  // wait for tile j's use of one of a pair of barriers (tile j uses number j & 1)
-  auto wait_tile = [&](uint64_t (&bar)[2], int j, int code, int factor) {
-    return warp_wait(&bar[j & 1], static_cast<uint32_t>(j >> 1) & 1u, abort_word, code, factor * prm.wait_budget_ns);
+  auto arrive_pass = [&]() {
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
   };
-  auto wait_stage = [&](int j) {
-    return warp_wait(&sh.kv_full[j % kHStages], static_cast<uint32_t>(j / kHStages) & 1u, abort_word, kAbortKvFull,
-                     prm.wait_budget_ns);
+  auto wait_pass = [&]() {
+    return warp_wait(&sh.pass_end, passes & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+  };
+  auto end_pass = [&]() {
+    arrive_pass();
+    return wait_pass();
+  };
+  auto count_noted = [&]() { return noted_tiles(sh.noted[items & 1], work.n_iter, note_scale(work.n_iter), lane); };
+  // after an item's last pass: the next one, if there is one
+  auto next_item = [&]() {
+    ++items;
+    const int next = *static_cast<volatile int *>(&sh.item[items % 3u].number);
+    if (next < 0) return false;
+    item = next;
+    work = work_item(prm, item);
+    return true;
   };
 
-  if (warp == kHSoftmaxWarps) {
-    // =================== TMA producer and QK^T issuer ===================
-    // QK^T(j) waits for P.V(j-2), which also frees that tile's stage: tile j+2's
-    // loads go out behind it.  The whole warp fetches the tile indices and K scales
-    // of 32 tiles at a time, one block ahead of their use; lane 0 leaves each stage's
-    // index and scale in shared memory for the softmax warps.
-    constexpr uint32_t idesc_qk = ptx::umma_idesc(2, 1, 1, H3S_Q_TILE, H3S_KV_TILE);
-    const uint64_t k_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + kHOffK), 1024, ptx::kSwizzle128);
-    const float *k_scale = prm.k_scale + static_cast<int64_t>(head) * prm.kv_tiles;
+  if (warp == kHKeyLoader || warp == kHValueLoader) {
+    // =================== K and V loaders ===================
+    // Both walk the list: the whole warp fetches a block of tile indices, one block ahead of
+    // their use, and one thread then loads those tiles.  The K loader also leaves the tiles'
+    // scales in shared memory for the softmax warps, asks for the next item and, while this one's
+    // last tiles are worked on, fetches that one's Q rows and scales.
+    const bool keys = warp == kHKeyLoader;
+    const CUtensorMap *map = keys ? &map_k : &map_v;
     if (lane == 0) {
-      ptx::prefetch_tensormap(&map_k);
-      ptx::prefetch_tensormap(&map_v);
+      ptx::prefetch_tensormap(map);
+      if (keys) ptx::prefetch_tensormap(&map_q);
     }
-    int my_tile = 0, next_tile = 0, block = -1;  // tile list entries 32*block .. +31, one per lane, and the 32 after
-    float my_scale = 0.f, next_scale = 0.f;
-    auto fetch_block = [&](int b) {
-      const int mine = list_position(min(b * 32 + lane, n_iter - 1));
-      next_tile = dense ? first_tile + mine : __ldg(route_row + mine);
-      next_scale = __ldg(k_scale + next_tile);
+    int next_tile = 0;  // of the block of the list that comes next, one per lane
+    float next_scale = 0.f;
+    auto fetch = [&](const HalfWork &it, int position) {
+      next_tile = it.dense ? it.first_tile + position : __ldg(it.route_row + position);
+      if (keys) next_scale = __ldg(prm.k_scale + static_cast<int64_t>(it.head) * prm.kv_tiles + next_tile);
     };
-    int cursor = 0;               // where a later pass goes on in the note
-    auto load = [&](int pass, int i) {  // tile i of the pass, into the stage of its running number
-      if (i >= count) return;
-      int t;
-      float ks;
-      if (pass == 0) {
-        if ((i >> 5) != block) {
-          block = i >> 5;
-          my_tile = next_tile; my_scale = next_scale;
-          fetch_block(block + 1);
-        }
-        t = __shfl_sync(0xffffffffu, my_tile, i & 31);
-        ks = __shfl_sync(0xffffffffu, my_scale, i & 31);
-      } else {
-        for (;;) {  // the next noted tile; there is one, i < count
-          const int bit = cursor >> coarse;
-          const uint32_t w = sh.noted[bit >> 5] >> (bit & 31);
-          if (w & 1u) break;
-          cursor = (w != 0u ? bit + __ffs(w) - 1 : ((bit >> 5) + 1) << 5) << coarse;
-        }
-        const int at = list_position(cursor++);
-        t = dense ? first_tile + at : __ldg(route_row + at);
-        ks = __ldg(k_scale + t);
-      }
-      if (lane == 0 && done + i != prm.drop_kv_load) {
-        const int s = (done + i) % kHStages;
-        sh.tile_index[s] = t;
-        sh.tile_scale[s] = ks;
-        ptx::mbar_arrive_expect_tx(&sh.kv_full[s], kHKBytes + kHVBytes);
-        ptx::tma_load_3d(smem + kHOffK + s * kHKBytes, &map_k, &sh.kv_full[s], 0, t * H3S_KV_TILE, head);
-        ptx::tma_load_3d(smem + kHOffV + s * kHVBytes, &map_v, &sh.kv_full[s], t * H3S_KV_TILE * 2, 0, head);
+    auto fetch_block = [&](const HalfWork &it, int i) {  // from the i-th tile on
+      fetch(it, list_position(min(i + lane % kHBlock, it.n_iter - 1), it.n_iter));
+    };
+    auto load_q = [&](const HalfWork &it) {
+      if (lane == 0) {
+        ptx::mbar_arrive_expect_tx(&sh.q_full, kHQBytes);
+        ptx::tma_load_3d(smem + L::kOffQ, &map_q, &sh.q_full, 0, it.tq * H3S_Q_TILE, it.head);
       }
       __syncwarp();
     };
-    for (int pass = 0; ok; ++pass) {
-      cursor = 0;
-      if (pass == 0) fetch_block(0);
-      for (int i = 0; i < kHStages; ++i) load(pass, i);
-      if (pass == 0) ok = warp_wait(&sh.q_ready, 0, abort_word, kAbortQFull, prm.wait_budget_ns);
-      for (int i = 0; ok && i < count; ++i) {
-        const int j = done + i;
-        ok = wait_stage(j) && (i < 1 || wait_tile(sh.s_taken, j - 1, kAbortPEmpty, 3)) &&
-             (i < 2 || wait_tile(sh.pv_done, j - 2, kAbortPvDone, 4));
-        if (!ok) break;
-        ptx::tc_fence_after();
-        if (ptx::elect_one()) {
-          const uint64_t k_desc = k_desc0 + static_cast<uint64_t>((j % kHStages) * (kHKBytes >> 4));
+    int *block = sh.block[keys ? 0 : 1];
+    uint64_t *full = keys ? sh.k_full : sh.v_full, *empty = keys ? sh.k_empty : sh.v_empty;
+    unsigned char *ring = smem + (keys ? L::kOffK : L::kOffV);
+    const int stages = keys ? L::kKStages : L::kVStages;
+    const uint32_t bytes = keys ? kHKBytes : kHVBytes;
+    uint32_t seq = 0;    // tiles so far
+    int stage = 0;       // state of the loading thread ...
+    uint32_t round = 1;  // ... parity of the ring's previous use
+    bool drop = prm.drop_kv_load == 0;
+    // the fetched block's first `tiles` tiles into the next stages; `meanwhile` may fetch again
+    auto load_block = [&](int tiles, auto meanwhile) {
+      if (lane < tiles) block[lane] = next_tile;
+      if (keys && lane < tiles) {
+        auto &tile = sh.tile[(seq + lane) % kHMeta];
+        tile.n_valid = prm.sequence - next_tile * H3S_KV_TILE;
+        tile.scale = next_scale;
+      }
+      seq += tiles;
+      __syncwarp();
+      meanwhile();
+      bool fine = true;
+      if (ptx::elect_one()) {
+        const int head = work.head;
+        for (int i = 0; i < tiles; ++i) {
+          const int t = block[i];
+          fine = ptx::mbar_wait(&empty[stage], round, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
+          if (!fine) break;
+          if (!drop) {
+            ptx::mbar_arrive_expect_tx(&full[stage], bytes);
+            ptx::tma_load_3d(ring + stage * bytes, map, &full[stage], keys ? 0 : t * H3S_KV_TILE * 2, keys ? t * H3S_KV_TILE : 0, head);
+          }
+          drop = false;
+          if (++stage == stages) { stage = 0; round ^= 1u; }
+        }
+      }
+      __syncwarp();
+      return __all_sync(0xffffffffu, fine) != 0;
+    };
+    if (keys) load_q(work);
+    fetch_block(work, 0);
+    while (ok) {
+      if (keys && lane == 0) {
+        ptx::fence_proxy_async_smem();  // the last reply has been read
+        ptx::mbar_arrive_expect_tx(&sh.next_ready, sizeof(sh.next_reply));
+        ptx::request_block(&sh.next_reply, &sh.next_ready);
+      }
+      __syncwarp();
+      for (int i = 0; ok && i < work.n_iter; i += kHBlock)
+        ok = load_block(min(kHBlock, work.n_iter - i), [&]() { if (i + kHBlock < work.n_iter) fetch_block(work, i + kHBlock); });
+      ok = ok && warp_wait(&sh.next_ready, items & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      if (!ok) break;
+      const int next = ptx::granted_block(&sh.next_reply);
+      if (next >= 0) {
+        const HalfWork it = work_item(prm, next);
+        fetch_block(it, 0);
+        if (keys) {
+          HalfItem &to = sh.item[(items + 1) % 3u];
+          if (lane == 0) to.q_scale = __ldg(prm.q_scale + it.head * prm.q_tiles + it.tq);
 #pragma unroll
-          for (int k = 0; k < H3S_HEAD_DIM / 32; ++k)
-            ptx::umma_i8_ts(tmem_s + (j & 1) * 32, tmem_q + k * 8, k_desc + 2 * k, idesc_qk, k > 0);
-          ptx::tc_commit(&sh.s_full[j & 1]);
+          for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + it.head * H3S_HEAD_DIM + i * 32 + lane);
+          ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
+          if (!ok) break;
+          load_q(it);
+        }
+      }
+      if (keys && lane == 0) sh.item[(items + 1) % 3u].number = next;
+      ok = end_pass();
+      ++passes;
+      if (!ok) break;
+      const int final_pass = last_pass();
+      if (final_pass > 0) {
+        const int first_tile = next_tile;  // of the next item, put aside
+        const float first_scale = next_scale;
+        const int count = count_noted(), coarse = note_scale(work.n_iter);
+        const uint32_t *noted = sh.noted[items & 1];
+        for (int pass = 1; ok && pass <= final_pass; ++pass) {
+          int cursor = 0;
+          for (int i = 0; ok && i < count; ++i) {
+            for (;;) {  // the next noted tile; there is one, i < count
+              const int bit = cursor >> coarse;
+              const uint32_t w = noted[bit >> 5] >> (bit & 31);
+              if (w & 1u) break;
+              cursor = (w != 0u ? bit + __ffs(w) - 1 : ((bit >> 5) + 1) << 5) << coarse;
+            }
+            fetch(work, list_position(cursor++, work.n_iter));
+            ok = load_block(1, []() {});
+          }
+          ok = ok && end_pass();
+          ++passes;
+        }
+        next_tile = first_tile;
+        next_scale = first_scale;
+      }
+      if (!ok || !next_item()) break;
+    }
+  } else if (warp == kHScoreIssuer) {
+    // =================== QK^T issuer ===================
+    constexpr uint32_t idesc_qk = ptx::umma_idesc(2, 1, 1, H3S_Q_TILE, H3S_KV_TILE);
+    const uint64_t k_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + L::kOffK), 1024, ptx::kSwizzle128);
+    const uint64_t q_desc = ptx::umma_desc_kmajor(ptx::smem_u32(smem + L::kOffQ), 1024, ptx::kSwizzle128);
+    int stage = 0, slot = 0;  // state of the issuing thread
+    uint32_t round = 0, slot_round = 0;
+    while (ok) {
+      const uint32_t tmem_q = tmem_o + kHTmemQ + (items & 1) * 32;
+      ok = warp_wait(&sh.q_full, items & 1u, abort_word, kAbortQFull, prm.wait_budget_ns);
+      if (!ok) break;
+      if (ptx::elect_one()) {
+#pragma unroll
+        for (int k = 0; k < H3S_HEAD_DIM / 32; ++k) ptx::tmem_copy_256b(tmem_q + k * 8, q_desc + 2 * k);
+        ptx::tc_commit(&sh.q_free);
+      }
+      __syncwarp();
+      int count = work.n_iter;
+      for (int pass = 0;; ++pass) {
+        arrive_pass();  // nothing of the pass's end depends on this warp
+        if (ptx::elect_one()) {
+          for (int i = 0; i < count; ++i) {
+            ok = ptx::mbar_wait(&sh.k_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
+                 ptx::mbar_wait(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortPEmpty, 3 * prm.wait_budget_ns);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(stage * (kHKBytes >> 4));
+#pragma unroll
+            for (int k = 0; k < H3S_HEAD_DIM / 32; ++k)
+              ptx::umma_i8_ts(tmem_o + kHTmemS + slot * 64, tmem_q + k * 8, k_desc + 2 * k, idesc_qk, k > 0);
+            ptx::tc_commit(&sh.s_full[(done + i) % kHGroups]);
+            ptx::tc_commit(&sh.k_empty[stage]);
+            if (++stage == L::kKStages) { stage = 0; round ^= 1u; }
+            if (++slot == kHScoreSlots) { slot = 0; slot_round ^= 1u; }
+          }
         }
         __syncwarp();
-        if (i >= 2) load(pass, i + 2);
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        done += count;
+        ok = ok && wait_pass();
+        ++passes;
+        if (!ok || pass == last_pass()) break;
+        if (pass == 0) count = count_noted();
       }
-      // (what the loop has not waited for, so that every barrier is one use behind at most)
-      const int last = done + count - 1;
-      ok = ok && wait_tile(sh.s_taken, last, kAbortPEmpty, 3) && (count < 2 || wait_tile(sh.pv_done, last - 1, kAbortFinal, 4)) &&
-           wait_tile(sh.pv_done, last, kAbortFinal, 4);
-      done += count;
-      ok = ok && warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
-      if (pass == last_pass()) break;
-      if (pass == 0) count = noted_tiles(sh.noted, n_iter, coarse, lane);
+      if (!ok || !next_item()) break;
     }
-  } else if (warp == kHSoftmaxWarps + 1) {
+  } else if (warp == kHValueIssuer) {
     // =================== P.V issuer ===================
     constexpr uint32_t idesc_pv = ptx::umma_idesc(1, 0, 0, H3S_Q_TILE, H3S_HEAD_DIM);
-    const uint64_t v_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + kHOffV), 1024, ptx::kSwizzle128);
-    for (int pass = 0; ok; ++pass) {
-      for (int j = done; j < done + count; ++j) {
-        if (!wait_tile(sh.p_full, j, kAbortPFull, 3) || !wait_stage(j)) { ok = false; break; }
-        ptx::tc_fence_after();
-        if (ptx::elect_one()) {
-          const uint64_t v_desc = v_desc0 + static_cast<uint64_t>((j % kHStages) * (kHVBytes >> 4));
+    const uint64_t v_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + L::kOffV), 1024, ptx::kSwizzle128);
+    int stage = 0;
+    uint32_t round = 0;
+    while (ok) {
+      int count = work.n_iter;
+      for (int pass = 0;; ++pass) {
+        arrive_pass();  // nothing of the pass's end depends on this warp
+        ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+        if (ok && ptx::elect_one()) {
+          for (int i = 0; i < count; ++i) {
+            const int j = done + i, g = j % kHGroups;
+            ok = ptx::mbar_wait(&sh.v_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
+                 ptx::mbar_wait(&sh.p_full[g], (j / kHGroups) & 1u, abort_word, kAbortPFull, 3 * prm.wait_budget_ns);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            const uint64_t v_desc = v_desc0 + static_cast<uint64_t>(stage * (kHVBytes >> 4));
 #pragma unroll
-          for (int k = 0; k < H3S_KV_TILE / 16; ++k)
-            ptx::umma_f16_ts(tmem_o, tmem_s + (j & 1) * 64 + k * 8, v_desc + 2 * k, idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
-          ptx::tc_commit(&sh.pv_done[j & 1]);
+            for (int k = 0; k < H3S_KV_TILE / 16; ++k)
+              ptx::umma_f16_ts(tmem_o, tmem_o + kHTmemP + g * 32 + k * 8, v_desc + 2 * k, idesc_pv,
+                               (pass > 0 || i > 0 || k > 0) ? 1u : 0u);
+            ptx::tc_commit(&sh.pv_done[g]);
+            ptx::tc_commit(&sh.v_empty[stage]);
+            if (i == count - 1) ptx::tc_commit(&sh.o_full);
+            if (++stage == L::kVStages) { stage = 0; round ^= 1u; }
+          }
         }
         __syncwarp();
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        done += count;
+        ok = ok && wait_pass();
+        ++passes;
+        if (!ok || pass == last_pass()) break;
+        if (pass == 0) count = count_noted();
       }
-      done += count;
-      // Lists of one or two tiles: nothing in the next pass up to its own pass_end waits for this
-      // warp, so that without its arrival here two passes could end before it looks, and the
-      // parity it waits for would be that of a third.
-      if (ok && lane == 0) ptx::mbar_arrive(&sh.pass_end);
-      ok = ok && warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
-      if (pass == last_pass()) break;
-      if (pass == 0) count = noted_tiles(sh.noted, n_iter, coarse, lane);
+      if (!ok || !next_item()) break;
     }
   } else {
-    // =================== softmax + epilogue (warps 0-7) ===================
+    // =================== softmax + epilogue (warps 0-15) ===================
     const int quarter = warp & 3, group = warp >> 2;
     const int row = quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    if (group == 0) {
-      // this thread's Q row -> its TMEM lane
-      uint32_t q[32];
-      const int grow = tq * H3S_Q_TILE + row;
-      const uint4 *src = reinterpret_cast<const uint4 *>(q8 + (static_cast<int64_t>(head) * prm.sequence + grow) * H3S_HEAD_DIM);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint4 w = grow < prm.sequence ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
-        q[4 * i] = w.x; q[4 * i + 1] = w.y; q[4 * i + 2] = w.z; q[4 * i + 3] = w.w;
-      }
-      H3S_TMEM_ST32(tmem_q + lane_addr, q);
-      ptx::tmem_wait_st();
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&sh.q_ready);
-    }
-    const float q_scale = __ldg(prm.q_scale + head * prm.q_tiles + tq) * (0.08838834764831845f * 1.4426950408889634f);
-    float m = 0.f, l = 0.f;
+    const uint32_t tmem_p = tmem_o + kHTmemP + group * 32 + lane_addr;
 
     // scores of tile j -> registers, and the factor that belongs to them
-    auto take = [&](int j, uint32_t (&s)[H3S_KV_TILE], float &c) {
-      if (!wait_tile(sh.s_full, j, kAbortSFull, 2)) return false;
+    auto take = [&](uint32_t j, float q_scale, uint32_t (&s)[H3S_KV_TILE], float &c) {
+      if (!warp_wait(&sh.s_full[group], (j / kHGroups) & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) return false;
+      const uint32_t slot = j % kHScoreSlots;
       ptx::tc_fence_after();
-      H3S_TMEM_LD64(tmem_s + lane_addr + group * 32, s);
-      // index and K scale of this tile, left in shared memory by the producer
-      // before the stage was handed to the tensor pipe (free only after P.V(j))
-      const int n_valid = prm.sequence - sh.tile_index[j % kHStages] * H3S_KV_TILE;
-      c = q_scale * sh.tile_scale[j % kHStages];
+      H3S_TMEM_LD64(tmem_o + kHTmemS + slot * 64 + lane_addr, s);
+      // left in shared memory by the K loader before the stage was handed to the tensor
+      // pipe; the entry is written again when P.V of this tile is long complete
+      const int n_valid = sh.tile[j % kHMeta].n_valid;
+      c = q_scale * sh.tile[j % kHMeta].scale;
       ptx::tmem_wait_ld(s);
       ptx::tc_fence_before();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&sh.s_taken[group]);
+      if (lane == 0) ptx::mbar_arrive(&sh.s_taken[slot]);
       // Keys beyond the sequence (ragged last tile only): the integer whose biased
       // bits are those of -inf, so that P becomes 0; it is also below every score.
       if (n_valid < H3S_KV_TILE) {
@@ -416,24 +569,20 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       }
       return true;
     };
-    // P -> slot A or C: part of S(j), which is in registers
-    auto put = [&](const uint32_t (&packed)[H3S_KV_TILE / 2]) { H3S_TMEM_ST32(tmem_s + lane_addr + group * 64, packed); };
+    // whether the group's P columns are free, asked while there is other work; then certainly
+    auto room_already = [&](uint32_t j) { return ptx::mbar_test_wait(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u); };
+    auto room = [&](uint32_t j) {
+      return warp_wait(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
+    };
+    auto put = [&](const uint32_t (&packed)[H3S_KV_TILE / 2]) { H3S_TMEM_ST32(tmem_p, packed); };
     auto hand_over = [&]() {
       ptx::tmem_wait_st();
       ptx::tc_fence_before();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&sh.p_full[group]);
     };
-    auto own_first = [&](int from) { return (from & 1) == group ? from : from + 1; };  // of this group's tiles
-    // both threads of a row leave a value, then wait for everything else of the pass
-    auto end_pass = [&](int pass, float value) {
-      sh.row[pass & 1][group][row] = value;
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
-      return warp_wait(&sh.pass_end, pass & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
-    };
-    auto leave_first = [&](float value) {
-      sh.first[group][row] = value;
+    auto leave_first = [&](int which, float value) {
+      sh.first[which][row] = value;
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&sh.first_max);
     };
@@ -444,207 +593,226 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       if (lane == 0) ptx::mbar_arrive(&sh.staged);
       return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
     };
+    // every P.V of the pass that has ended
+    auto all_products = [&]() {
+      return warp_wait(&sh.o_full, (passes - 1) & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+    };
+    auto release_o = [&]() {
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&sh.o_free);
+    };
 
-    float largest = 0.f;  // sum over a tile that this thread has left out
-    if (group == 1 && n_iter == 1) leave_first(-INFINITY);
-    for (int j = group; j < n_iter; j += 2) {
-      uint32_t s[H3S_KV_TILE];
-      float c;
-      if (!take(j, s, c)) { ok = false; break; }
-      if (j < 2) {
-        leave_first(c * static_cast<float>(max_score(s)));  // c > 0
-        if (!warp_wait(&sh.first_max, 0, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
-        m = first_reference();
-        // the maxima bring the groups together; the second one waits, so that they are out of
-        // step again (24 heads x 2304 tokens 45.1 -> 43.3 us, 7 x 10384 84.5 -> 83.6, long lists alike)
-        if (j == 1 && !warp_wait(&sh.first_exp, 0, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
-      }
-      uint32_t packed[H3S_KV_TILE / 2];
-      float sum = exp_sum<true, false>(s, c, -fmaf(c, kIntBias, m), packed);
-      if (j == 0) {
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&sh.first_exp);
-      }
-      put(packed);
-      const bool out = !(sum <= kHSumLimit);
-      if (__any_sync(0xffffffffu, out)) {  // these rows leave the tile out
-        const bool far = __any_sync(0xffffffffu, sum == INFINITY || c > 1.f);  // no measure of the maximum
-        ptx::tmem_wait_st();
-        if (out) {
-          largest = fmaxf(largest, sum);
-          sum = 0.f;
-#pragma unroll
-          for (int i = 0; i < H3S_KV_TILE / 2; ++i) packed[i] = 0u;
+    while (ok) {
+      const int n_iter = work.n_iter;
+      // Which of the four groups has the first tile depends on what the CTA has done before; sums are
+      // added up in the order of the tiles all the same, so that a result does not depend on that.
+      const int rank = (group - done) & (kHGroups - 1);
+      const float q_scale = sh.item[items % 3u].q_scale * (0.08838834764831845f * 1.4426950408889634f);
+      const int coarse = note_scale(n_iter);
+      float m = 0.f, l = 0.f;
+      sh.over[group][row] = 0.f;
+      if (rank == 1 && n_iter == 1) leave_first(1, -INFINITY);
+      for (int i = rank; i < n_iter; i += kHGroups) {
+        uint32_t s[H3S_KV_TILE];
+        float c;
+        if (!take(done + i, q_scale, s, c)) { ok = false; break; }
+        if (i < kHGroups) {
+          if (i < 2) leave_first(i, c * static_cast<float>(max_score(s)));  // c > 0
+          if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
+          m = first_reference();
         }
+        const bool free_already = room_already(done + i);
+        uint32_t packed[H3S_KV_TILE / 2];
+        float sum = exp_sum<true, false>(s, c, -fmaf(c, kIntBias, m), packed);
+        if (!__all_sync(0xffffffffu, free_already) && !room(done + i)) { ok = false; break; }
         put(packed);
-        if (lane == 0) {
-          atomicOr(&sh.noted[(j >> coarse) >> 5], 1u << ((j >> coarse) & 31));
-          atomicOr(&sh.again, far ? kAgainNoted | kAgainFar : kAgainNoted);
+        const bool out = !(sum <= kHSumLimit);
+        if (__any_sync(0xffffffffu, out)) {  // these rows leave the tile out
+          const bool far = __any_sync(0xffffffffu, sum == INFINITY || c > 1.f);  // no measure of the maximum
+          ptx::tmem_wait_st();
+          if (out) {
+            sh.over[group][row] = fmaxf(sh.over[group][row], sum);
+            sum = 0.f;
+#pragma unroll
+            for (int e = 0; e < H3S_KV_TILE / 2; ++e) packed[e] = 0u;
+          }
+          put(packed);
+          if (lane == 0) {
+            atomicOr(&sh.noted[items & 1][(i >> coarse) >> 5], 1u << ((i >> coarse) & 31));
+            atomicOr(&sh.again[items & 3], far ? kAgainNoted | kAgainFar : kAgainNoted);
+          }
         }
+        l += sum;
+        hand_over();
       }
-      l += sum;
-      hand_over();
-    }
-    done = n_iter;
-    sh.row[1][group][row] = largest;
-    ok = ok && end_pass(0, l);
-    const int final_pass = ok ? last_pass() : 0;
-    if (final_pass > 0) {
-      count = noted_tiles(sh.noted, n_iter, coarse, lane);
-      m = first_reference();  // (a group without a tile has none yet)
-      float m_again = m;
-      if (final_pass == 1) {
-        const uint32_t bits = __float_as_uint(fmaxf(sh.row[1][0][row], sh.row[1][1][row]));
-        if (bits != 0u) m_again = m + (static_cast<float>(static_cast<int>(bits >> 23) - 126) - kHAgainBits);
-      } else {
-        float top = -INFINITY;
-        for (int j = own_first(done); j < done + count; j += 2) {
+      if (!ok) break;
+      done += n_iter;
+      sh.row[passes & 1][rank][row] = l;
+      // the word of the item after next: its last readers (two items ago) have all been at a pass's end since
+      if (threadIdx.x == 0) sh.again[(items + 2) & 3] = 0;
+      ok = end_pass();
+      ++passes;
+      if (!ok) break;
+      if (rank >= n_iter) m = first_reference();  // a group without a tile has none yet
+      const int final_pass = last_pass();
+      if (final_pass > 0) {
+        const int count = count_noted();
+        ok = all_products();
+        float m_again = m;
+        if (final_pass == 1) {
+          const float most = fmaxf(fmaxf(sh.over[0][row], sh.over[1][row]), fmaxf(sh.over[2][row], sh.over[3][row]));
+          const uint32_t bits = __float_as_uint(most);
+          if (bits != 0u) m_again = m + (static_cast<float>(static_cast<int>(bits >> 23) - 126) - kHAgainBits);
+        } else {
+          release_o();
+          float top = -INFINITY;
+          for (int i = (group - done) & (kHGroups - 1); ok && i < count; i += kHGroups) {
+            uint32_t s[H3S_KV_TILE];
+            float c;
+            ok = take(done + i, q_scale, s, c) && room(done + i);
+            if (!ok) break;
+            top = fmaxf(top, c * static_cast<float>(max_score(s)));
+            uint32_t none[H3S_KV_TILE / 2];  // O stays as it is
+#pragma unroll
+            for (int e = 0; e < H3S_KV_TILE / 2; ++e) none[e] = 0u;
+            put(none);
+            hand_over();
+          }
+          done += count;
+          sh.row[passes & 1][rank][row] = top;
+          ok = ok && end_pass();
+          const float *tops = &sh.row[passes & 1][0][row];
+          ++passes;
+          top = fmaxf(fmaxf(tops[0], tops[H3S_Q_TILE]), fmaxf(tops[2 * H3S_Q_TILE], tops[3 * H3S_Q_TILE]));
+          if (top > m + kHMostBits) m_again = ceilf(top) - kHAgainBits;
+          ok = ok && all_products();
+        }
+        const float factor = fast_exp2(m - m_again);  // a power of two
+        l *= factor;
+        if (ok && __any_sync(0xffffffffu, m_again != m)) {
+          ptx::tc_fence_after();
+          uint32_t o[32];
+          H3S_TMEM_LD32(tmem_o + lane_addr + group * 32, o);
+          ptx::tmem_wait_ld(o);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * factor);
+          H3S_TMEM_ST32(tmem_o + lane_addr + group * 32, o);
+          ptx::tmem_wait_st();
+        }
+        release_o();
+        for (int i = (group - done) & (kHGroups - 1); ok && i < count; i += kHGroups) {
           uint32_t s[H3S_KV_TILE];
           float c;
-          if (!take(j, s, c)) { ok = false; break; }
-          top = fmaxf(top, c * static_cast<float>(max_score(s)));
-          uint32_t none[H3S_KV_TILE / 2];  // O stays as it is
+          ok = take(done + i, q_scale, s, c) && room(done + i);
+          if (!ok) break;
+          uint32_t packed[H3S_KV_TILE / 2];
+          // the same sum as in the first pass, so the same tiles
+          const bool out = !(exp_sum<false, false>(s, c, -fmaf(c, kIntBias, m), packed) <= kHSumLimit);
+          const float sum = exp_sum<true, true>(s, c, -m_again, packed);
+          if (out) {
+            l += sum;
+          } else {
 #pragma unroll
-          for (int i = 0; i < H3S_KV_TILE / 2; ++i) none[i] = 0u;
-          put(none);
+            for (int e = 0; e < H3S_KV_TILE / 2; ++e) packed[e] = 0u;
+          }
+          put(packed);
           hand_over();
         }
         done += count;
-        ok = ok && end_pass(1, top);
-        top = fmaxf(sh.row[1][0][row], sh.row[1][1][row]);
-        if (top > m + kHMostBits) m_again = ceilf(top) - kHAgainBits;
+        m = m_again;
+        sh.row[passes & 1][rank][row] = l;
+        ok = ok && end_pass();
+        ++passes;
+        if (!ok) break;
+        // (this note's next item is the one after next, and its last reader has been at the pass's end)
+        if (threadIdx.x < kHNoted / 32) sh.noted[items & 1][threadIdx.x] = 0u;
       }
-      // every P.V so far (one barrier per group): O may be touched
-      ok = ok && (done < 2 || wait_tile(sh.pv_done, done - 2, kAbortFinal, 4)) && wait_tile(sh.pv_done, done - 1, kAbortFinal, 4);
-      const float factor = fast_exp2(m - m_again);  // a power of two
-      l *= factor;
-      if (ok && __any_sync(0xffffffffu, m_again != m)) {
-        ptx::tc_fence_after();
-#pragma unroll 1
-        for (int cc = group * 2; cc < group * 2 + 2; ++cc) {
-          uint32_t o[32];
-          H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
-          ptx::tmem_wait_ld(o);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-          H3S_TMEM_ST32(tmem_o + lane_addr + cc * 32, o);
-        }
-        ptx::tmem_wait_st();
-        ptx::tc_fence_before();
+      {
+        const float *sums = &sh.row[(passes - 1) & 1][0][row];
+        l = (sums[0] + sums[H3S_Q_TILE]) + (sums[2 * H3S_Q_TILE] + sums[3 * H3S_Q_TILE]);
       }
-      ok = ok && meet();  // the first P.V of the next pass waits for one group only
-      for (int j = own_first(done); ok && j < done + count; j += 2) {
-        uint32_t s[H3S_KV_TILE];
-        float c;
-        if (!take(j, s, c)) { ok = false; break; }
-        uint32_t packed[H3S_KV_TILE / 2];
-        // the same sum as in the first pass, so the same tiles
-        const bool out = !(exp_sum<false, false>(s, c, -fmaf(c, kIntBias, m), packed) <= kHSumLimit);
-        const float sum = exp_sum<true, true>(s, c, -m_again, packed);
-        if (out) {
-          l += sum;
-        } else {
-#pragma unroll
-          for (int i = 0; i < H3S_KV_TILE / 2; ++i) packed[i] = 0u;
-        }
-        put(packed);
-        hand_over();
-      }
-      done += count;
-      m = m_again;
-      ok = ok && end_pass(final_pass, l);
-    }
-    if (ok) l = sh.row[final_pass & 1][0][row] + sh.row[final_pass & 1][1][row];
+      ok = all_products();
+      if (!ok) break;
 
-    // every P.V of the last pass (one barrier per group)
-    if (ok && done > 1) ok = wait_tile(sh.pv_done, done - 2, kAbortFinal, 4);
-    if (ok) ok = wait_tile(sh.pv_done, done - 1, kAbortFinal, 4);
-    if (ok) {
-      // Epilogue: O / l * v_scale -> OutT, staged through shared memory (the
-      // stage ring is free: every TMA load has been consumed).  A warp converts its
-      // 32 rows of one column half; the two warps of a row quarter then each write
-      // 16 of the quarter's rows as full contiguous lines.
+      // Epilogue: O / l * v_scale -> OutT, staged through shared memory.  A warp converts
+      // its 32 rows of 32 columns; the four warps of a row quarter then each write eight of the
+      // quarter's rows as full contiguous lines.
       ptx::tc_fence_after();
-      // Partial sums of part p: [32 groups of 4 columns][128 rows] float4, so that a warp's rows are
-      // neighbours; then 128 row sums and 128 reference points.
-      constexpr int kPartFloats = H3S_Q_TILE * (H3S_HEAD_DIM + 2);
-      const float *parts_base = prm.partial + static_cast<int64_t>(dense_row) * prm.parts * kPartFloats;
-      float top = 0.f;  // largest reference point of the parts
+      const bool split = work.dense && prm.parts > 1;
+      uint32_t o[32];
+      H3S_TMEM_LD32(tmem_o + lane_addr + group * 32, o);
+      ptx::tmem_wait_ld(o);
+      release_o();
+      bool finish = true;
       if (split) {
-        float *mine = const_cast<float *>(parts_base) + static_cast<int64_t>(part) * kPartFloats;
-#pragma unroll 1
-        for (int cc = group * 2; cc < group * 2 + 2; ++cc) {
-          uint32_t o[32];
-          H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
-          ptx::tmem_wait_ld(o);
+        // Partial sums of part p: [32 groups of 4 columns][128 rows] float4, so that a warp's rows are
+        // neighbours; then 128 row sums and 128 reference points.
+        constexpr int kPartFloats = H3S_Q_TILE * (H3S_HEAD_DIM + 2);
+        const float *parts_base = prm.partial + static_cast<int64_t>(work.dense_row) * prm.parts * kPartFloats;
+        float *mine = const_cast<float *>(parts_base) + static_cast<int64_t>(work.part) * kPartFloats;
 #pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            __stcg(reinterpret_cast<float4 *>(mine) + (cc * 8 + i / 4) * H3S_Q_TILE + row,
-                   make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]), __uint_as_float(o[i + 2]),
-                               __uint_as_float(o[i + 3])));
-        }
+        for (int e = 0; e < 32; e += 4)
+          __stcg(reinterpret_cast<float4 *>(mine) + (group * 8 + e / 4) * H3S_Q_TILE + row,
+                 make_float4(__uint_as_float(o[e]), __uint_as_float(o[e + 1]), __uint_as_float(o[e + 2]),
+                             __uint_as_float(o[e + 3])));
         if (group == 0) {
           __stcg(mine + H3S_Q_TILE * H3S_HEAD_DIM + row, l);
           __stcg(mine + H3S_Q_TILE * (H3S_HEAD_DIM + 1) + row, m);
         }
         __threadfence();
         ok = meet();
-        if (ok && warp == 0 && lane == 0) {
+        if (ok && threadIdx.x == 0) {
           __threadfence();
-          sh.finish = atomicAdd(prm.arrived + dense_row, 1u) == static_cast<unsigned int>(prm.parts - 1);
+          sh.finish = atomicAdd(prm.arrived + work.dense_row, 1u) == static_cast<unsigned int>(prm.parts - 1);
           __threadfence();
         }
         ok = ok && meet();
-        if (ok && sh.finish) {
+        if (!ok) break;
+        finish = *static_cast<volatile int *>(&sh.finish) != 0;
+        if (finish) {
           l = 0.f;
-          top = -INFINITY;
+          float top = -INFINITY;  // largest reference point of the parts
           for (int p = 0; p < prm.parts; ++p)
             top = fmaxf(top, __ldcg(parts_base + p * kPartFloats + H3S_Q_TILE * (H3S_HEAD_DIM + 1) + row));
           for (int p = 0; p < prm.parts; ++p) {
             const float *at = parts_base + p * kPartFloats + H3S_Q_TILE * H3S_HEAD_DIM + row;
             l = fmaf(__ldcg(at), fast_exp2(__ldcg(at + H3S_Q_TILE) - top), l);
           }
-        }
-      }
-      const bool finish = ok && sh.finish;
-      const float inv_l = 1.0f / l;
-      constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
-      static_assert(H3S_Q_TILE * kRowBytes <= kHOffBar, "output tile must fit the stage ring");
-      unsigned char *my_row = smem + row * kRowBytes;
-#pragma unroll 1
-      for (int cc = group * 2; finish && cc < group * 2 + 2; ++cc) {
-        uint32_t o[32];
-        if (!split) {
-          H3S_TMEM_LD32(tmem_o + lane_addr + cc * 32, o);
-          ptx::tmem_wait_ld(o);
-        } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0u;
+          for (int e = 0; e < 32; ++e) o[e] = 0u;
 #pragma unroll 1
           for (int p = 0; p < prm.parts; ++p) {
             const float *at = parts_base + p * kPartFloats;
             // the reference points are integers: the factors are powers of two
             const float weight = fast_exp2(__ldcg(at + H3S_Q_TILE * (H3S_HEAD_DIM + 1) + row) - top);
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 x = __ldcg(reinterpret_cast<const float4 *>(at) + (cc * 8 + i / 4) * H3S_Q_TILE + row);
-              o[i] = __float_as_uint(fmaf(x.x, weight, __uint_as_float(o[i])));
-              o[i + 1] = __float_as_uint(fmaf(x.y, weight, __uint_as_float(o[i + 1])));
-              o[i + 2] = __float_as_uint(fmaf(x.z, weight, __uint_as_float(o[i + 2])));
-              o[i + 3] = __float_as_uint(fmaf(x.w, weight, __uint_as_float(o[i + 3])));
+            for (int e = 0; e < 32; e += 4) {
+              const float4 x = __ldcg(reinterpret_cast<const float4 *>(at) + (group * 8 + e / 4) * H3S_Q_TILE + row);
+              o[e] = __float_as_uint(fmaf(x.x, weight, __uint_as_float(o[e])));
+              o[e + 1] = __float_as_uint(fmaf(x.y, weight, __uint_as_float(o[e + 1])));
+              o[e + 2] = __float_as_uint(fmaf(x.z, weight, __uint_as_float(o[e + 2])));
+              o[e + 3] = __float_as_uint(fmaf(x.w, weight, __uint_as_float(o[e + 3])));
             }
           }
         }
+      }
+      if (finish) {
+        const float inv_l = 1.0f / l;
+        constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
+        unsigned char *out_tile = smem + L::kOffOut;
+        unsigned char *my_row = out_tile + row * kRowBytes;
+        const float *v_scale = sh.item[items % 3u].v_scale + group * 32;
 #pragma unroll
-        for (int i = 0; i < 32; i += 8) {
+        for (int e0 = 0; e0 < 32; e0 += 8) {
           float v[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            v[e] = __uint_as_float(o[i + e]) * inv_l * sh.v_scale[cc * 32 + i + e];  // |o / l| <= 448: nothing overflows
+            v[e] = __uint_as_float(o[e0 + e]) * inv_l * v_scale[e0 + e];  // |o / l| <= 448: nothing overflows
           // 8 values = one (bf16/fp16) or two (fp32) 16-byte chunks; the chunk index is
           // XORed with the row so that the 32 rows of a warp do not collide on banks
           constexpr int kChunks8 = 8 * static_cast<int>(sizeof(OutT)) / 16;
-          const int chunk0 = (cc * 32 + i) * static_cast<int>(sizeof(OutT)) / 16;
+          const int chunk0 = (group * 32 + e0) * static_cast<int>(sizeof(OutT)) / 16;
           __align__(16) OutT tmp[8];
           store_out8<OutT>(tmp, v);
 #pragma unroll
@@ -652,10 +820,12 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             *reinterpret_cast<uint4 *>(my_row + (((chunk0 + k) ^ (row & 15)) << 4)) =
                 reinterpret_cast<const uint4 *>(tmp)[k];
         }
+        ok = meet();
+        if (!ok) break;
+        store_rows<OutT>(prm, out_tile, work.head, work.tq, quarter * 32 + group * 8, 8, lane);
+        if (prm.n_peer_out > 0) scatter_to_peers<OutT>(prm, out_tile, work.head, work.tq, kHSoftmaxWarps * 32);
       }
-      ptx::tc_fence_before();
-      // both halves of the rows are staged
-      if (finish && meet()) store_rows<OutT>(prm, smem, head, tq, quarter * 32 + group * 16, 16, lane);
+      if (!next_item()) break;
     }
   }
 
@@ -667,18 +837,16 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     __nanosleep(200000);
     if (threadIdx.x == 0 && prm.status != nullptr) {
       if (atomicCAS(prm.status, 0, code) == 0) {
-        prm.status[1] = blockIdx.x;
-        prm.status[2] = head;
-        prm.status[3] = tq;
+        prm.status[1] = item;
+        prm.status[2] = work.head;
+        prm.status[3] = work.tq;
       }
     }
   }
-  if (warp == kHSoftmaxWarps + 1) {
+  if (warp == kHValueIssuer) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_o, kHTmemCols);
   }
-  // head-sharded run: the producer and MMA warps have nothing left to do and share the copy
-  if (code == 0 && prm.n_peer_out > 0 && sh.finish) scatter_to_peers<OutT>(prm, smem, head, tq, kHThreads);
 }
 
 // E4M3 codes -> FP16 values: 16 per thread
@@ -690,22 +858,18 @@ __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v
   v16[2 * i + 1] = e4m3x8_to_half(make_uint2(codes.z, codes.w));
 }
 
-// Whether and how the dense rows' tile lists are cut.  Two CTAs run on each of 148 SMs; a
-// slot gets `share` tiles on average.  A dense row much longer than that ends after
-// everything else has: seven heads of 10384 tokens at 15 % (28 dense rows of 163 tiles
-// beside 546 routed ones of 31, share 73) take 195 us for the whole layer uncut, 176 us in
-// parts.  At the line itself, an eighth longer than the share, both are equal (three heads
-// of 33272 tokens at 30 %: 520 against a share of 441, 523 and 521 us), and below it the
-// order "long rows first" fills the slots, so that parts would only cost their traffic.  A
-// quarter of the share keeps the last parts short; under 24 tiles a part's start and end
-// (about 4 us) would show.
-constexpr int kSlots = 2 * 148, kMinPartTiles = 24, kMaxParts = 16;
+// Whether and how the dense rows' tile lists are cut.  An SM gets `share` tiles on average.  A dense row
+// that is longer ends after everything else has; parts of a quarter of the share even that out.  The line
+// is at half a share: there the parts cost nothing measurable (three heads of 33272 tokens at 30 %, 520
+// tiles of a share of 883: 384 us) and the order "long rows first" fills the SMs by itself further down.  Under 24
+// tiles a part's start and end would show.
+constexpr int kSlots = 148, kMinPartTiles = 24, kMaxParts = 16;
 
 static int split_dense_rows(int heads, int q_tiles, int kv_tiles, int n_sparse, int route_len, int *part_tiles) {
   const int64_t n_dense = q_tiles - n_sparse;
   const int64_t total = heads * (n_dense * kv_tiles + static_cast<int64_t>(n_sparse) * route_len);
   *part_tiles = kv_tiles;
-  if (n_dense == 0 || static_cast<int64_t>(kv_tiles) * kSlots * 7 <= total * 8) return 1;
+  if (n_dense == 0 || static_cast<int64_t>(kv_tiles) * kSlots * 2 <= total) return 1;
   int tiles = static_cast<int>(total / (4 * kSlots));
   if (tiles < kMinPartTiles) tiles = kMinPartTiles;
   if (tiles < ceil_div(kv_tiles, kMaxParts)) tiles = ceil_div(kv_tiles, kMaxParts);
@@ -720,13 +884,13 @@ static size_t split_bytes(int64_t dense_rows, int parts, size_t *arrived_bytes) 
 }
 
 template <typename OutT>
-static int launch_attn_half(const CUtensorMap &mk, const CUtensorMap &mv, const int8_t *q8, const AttnParams &prm,
+static int launch_attn_half(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const AttnParams &prm,
                             cudaStream_t stream) {
-  H3S_CHECK_CUDA(cudaFuncSetAttribute(sparse_attn_half_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kHSmemBytes)));
+  constexpr int kBytes = static_cast<int>(HalfLayout<OutT>::kBytes);
+  H3S_CHECK_CUDA(cudaFuncSetAttribute(sparse_attn_half_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
   const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
-  const int ctas = prm.heads * ((prm.q_tiles - n_sparse) * prm.parts + n_sparse);
-  sparse_attn_half_kernel<OutT><<<ctas, kHThreads, kHSmemBytes, stream>>>(mk, mv, q8, prm);
+  const int items = prm.heads * ((prm.q_tiles - n_sparse) * prm.parts + n_sparse);
+  sparse_attn_half_kernel<OutT><<<items, kHThreads, kBytes, stream>>>(mq, mk, mv, prm);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
 }
@@ -770,7 +934,10 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
   if (rc) return rc;
   const uint64_t S = static_cast<uint64_t>(sequence);
   const uint64_t row_bytes = static_cast<uint64_t>(ceil_div(sequence, 128)) * 128 * 2;
-  CUtensorMap mk, mv;
+  CUtensorMap mq, mk, mv;
+  rc = make_tensor_map_u8_3d(&mq, q8, H3S_HEAD_DIM, S, heads, H3S_HEAD_DIM, S * H3S_HEAD_DIM, H3S_HEAD_DIM,
+                             H3S_Q_TILE, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_half_fwd Q map");
+  if (rc) return rc;
   rc = make_tensor_map_u8_3d(&mk, k8, H3S_HEAD_DIM, S, heads, H3S_HEAD_DIM, S * H3S_HEAD_DIM, H3S_HEAD_DIM,
                              H3S_KV_TILE, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_half_fwd K map");
   if (rc) return rc;
@@ -795,8 +962,8 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
     }
   }
   switch (out_dtype) {
-    case H3S_F32: return launch_attn_half<float>(mk, mv, q8, prm, s);
-    case H3S_BF16: return launch_attn_half<__nv_bfloat16>(mk, mv, q8, prm, s);
-    default: return launch_attn_half<__half>(mk, mv, q8, prm, s);
+    case H3S_F32: return launch_attn_half<float>(mq, mk, mv, prm, s);
+    case H3S_BF16: return launch_attn_half<__nv_bfloat16>(mq, mk, mv, prm, s);
+    default: return launch_attn_half<__half>(mq, mk, mv, prm, s);
   }
 }

@@ -102,6 +102,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   // a phase that is already complete costs one test_wait (a try_wait with a
   // suspend hint takes about twice as long even when it succeeds at once)
   if (mbar_test_wait(bar, parity)) return true;
+  if (mbar_try_wait(bar, parity)) return true;
   const unsigned long long start = global_timer_ns();
   uint32_t spins = 0;
   while (true) {
@@ -170,6 +171,41 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    smem_u32(bar))
                : "memory");
+}
+
+// 128 rows of 32 bytes of shared memory -> 128 lanes of 8 columns; ordered before the MMAs
+// that the same thread issues afterwards
+__device__ __forceinline__ void tmem_copy_256b(uint32_t d_tmem, uint64_t s_desc) {
+  asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(d_tmem), "l"(s_desc) : "memory");
+}
+
+// ---- work of blocks that have not started ------------------------------------
+
+// Asks for one; the 16-byte reply arrives like a copy, counted on `bar`.  Not to be asked
+// again after a refusal.
+__device__ __forceinline__ void request_block(void *reply, uint64_t *bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(reply)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+
+// blockIdx.x of the block whose work is now this one's, or -1
+__device__ __forceinline__ int granted_block(const void *reply) {
+  int block;
+  asm volatile(
+      "{\n\t"
+      ".reg .b128 r;\n\t"
+      ".reg .pred p;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t"
+      "}\n"
+      : "=r"(block)
+      : "r"(smem_u32(reply))
+      : "memory");
+  return block;
 }
 
 // ---- clusters of two CTAs (cta_group::2) -------------------------------------
