@@ -510,24 +510,28 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const uint32_t tmem_base = sh.tmem_base;
 
   if (warp == 4) {
-    if (lane == 0) {
+    // One thread, its state kept from step to step: at 128 bytes of K a step the MMAs take 512 cycles, and
+    // what this thread and the issuing one do for a step is a chain of dependent instructions.
+    if (ptx::elect_one()) {
       ptx::prefetch_tensormap(&map_a);
       ptx::prefetch_tensormap(&map_b);
-      uint32_t it = 0;
+      // all four loads of the pair count on the first CTA's barrier
+      const uint32_t full0 = ptx::cluster_address(&sh.full[0], 0);
+      int stage = 0;
+      uint32_t it = 0, previous = 1;  // steps so far, parity of the ring's previous use
       bool ok = true;
       for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step) {
         int pair, tn;
         tile_position(prm, tile, pair, tn);
         const int row0 = pair * kGemmPairM + rank * kGemmM, col0 = tn * kGemmN + rank * (kGemmN / 2);
-        for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % L::kStages;
-          const uint32_t use = it / L::kStages;
-          if (!ptx::mbar_wait(&sh.empty[s], (use & 1u) ^ 1u, abort_word, kGemmAbortEmpty, prm.wait_budget_ns)) { ok = false; break; }
-          // all four loads of the pair count on the first CTA's barrier
-          const uint32_t full = ptx::cluster_address(&sh.full[s], 0);
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&sh.full[s], 2 * (kGemmABytes + kGemmBBytes));
-          ptx::tma_load_2d_pair(smem + s * kGemmABytes, &map_a, full, ks * kGemmK, row0);
-          ptx::tma_load_2d_pair(smem + L::kOffB + s * kGemmBBytes, &map_b, full, ks * kGemmK, col0);
+        for (int k = 0; k < prm.hidden; k += kGemmK) {
+          if (!ptx::mbar_wait(&sh.empty[stage], previous, abort_word, kGemmAbortEmpty, prm.wait_budget_ns)) { ok = false; break; }
+          const uint32_t full = full0 + stage * sizeof(uint64_t);
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&sh.full[stage], 2 * (kGemmABytes + kGemmBBytes));
+          ptx::tma_load_2d_pair(smem + stage * kGemmABytes, &map_a, full, k, row0);
+          ptx::tma_load_2d_pair(smem + L::kOffB + stage * kGemmBBytes, &map_b, full, k, col0);
+          ++it;
+          if (++stage == L::kStages) { stage = 0; previous ^= 1u; }
         }
       }
       // the other CTA's last arrivals on `empty` have landed before this CTA may exit
@@ -535,45 +539,39 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         ok = ptx::mbar_wait(&sh.empty[i % L::kStages], (i / L::kStages) & 1u, abort_word, kGemmAbortEmpty, prm.wait_budget_ns);
     }
   } else if (warp == 5) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && ptx::elect_one()) {
       // every kind consumes 32 bytes of K per instruction: four instructions per 128-byte stage
       const int kind = kMode == kModeDense ? prm.operand_kind : H3S_GEMM_I8;
-      const uint32_t idesc = kind == H3S_GEMM_I8     ? ptx::umma_idesc(2, 1, 1, kGemmPairM, kGemmN)
-                             : kind == H3S_GEMM_E4M3 ? ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN)
-                             : kind == H3S_GEMM_BF16 ? ptx::umma_idesc(1, 1, 1, kGemmPairM, kGemmN)
-                                                     : ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN);
-      uint32_t it = 0, local = 0;
-      bool ok = true;
-      for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step, ++local) {
-        const int a = local & 1;
-        const uint32_t acc_use = local >> 1;
-        if (!ptx::mbar_wait(&sh.acc_empty[a], (acc_use & 1u) ^ 1u, abort_word, kGemmAbortAccEmpty, prm.wait_budget_ns)) { ok = false; break; }
-        ptx::tc_fence_after();
-        for (int ks = 0; ks < k_steps; ++ks, ++it) {
-          const int s = it % L::kStages;
-          const uint32_t use = it / L::kStages;
-          if (!ptx::mbar_wait(&sh.full[s], use & 1u, abort_word, kGemmAbortFull, prm.wait_budget_ns)) { ok = false; break; }
+      const uint64_t a_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem), 1024, ptx::kSwizzle128);
+      const uint64_t b_desc0 = ptx::umma_desc_kmajor(ptx::smem_u32(smem + L::kOffB), 1024, ptx::kSwizzle128);
+      auto issue = [&](uint32_t idesc, auto mma) {
+        int stage = 0;
+        uint32_t round = 0, local = 0;
+        for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++local) {
+          const int a = local & 1;
+          const uint32_t acc_use = local >> 1, acc = tmem_base + a * kGemmN;
+          if (!ptx::mbar_wait(&sh.acc_empty[a], (acc_use & 1u) ^ 1u, abort_word, kGemmAbortAccEmpty, prm.wait_budget_ns)) return;
           ptx::tc_fence_after();
-          const uint64_t a_desc = ptx::umma_desc_kmajor(ptx::smem_u32(smem + s * kGemmABytes), 1024, ptx::kSwizzle128);
-          const uint64_t b_desc =
-              ptx::umma_desc_kmajor(ptx::smem_u32(smem + L::kOffB + s * kGemmBBytes), 1024, ptx::kSwizzle128);
-          if (kind == H3S_GEMM_I8) {
+          for (int ks = 0; ks < k_steps; ++ks) {
+            if (!ptx::mbar_wait(&sh.full[stage], round, abort_word, kGemmAbortFull, prm.wait_budget_ns)) return;
+            ptx::tc_fence_after();
+            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(stage * (kGemmABytes >> 4));
+            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>(stage * (kGemmBBytes >> 4));
 #pragma unroll
-            for (int k = 0; k < kGemmK / 32; ++k)
-              ptx::umma_i8_pair(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
-          } else if (kind == H3S_GEMM_E4M3) {
-#pragma unroll
-            for (int k = 0; k < kGemmK / 32; ++k)
-              ptx::umma_f8_pair(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
-          } else {
-#pragma unroll
-            for (int k = 0; k < kGemmK / 32; ++k)
-              ptx::umma_f16_pair(tmem_base + a * kGemmN, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < kGemmK / 32; ++k) mma(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+            ptx::tc_commit_pair(&sh.empty[stage]);
+            if (++stage == L::kStages) { stage = 0; round ^= 1u; }
           }
-          ptx::tc_commit_pair(&sh.empty[s]);
+          ptx::tc_commit_pair(&sh.acc_full[a]);
         }
-        if (ok) ptx::tc_commit_pair(&sh.acc_full[a]);
-      }
+      };
+      auto i8 = [](uint32_t d, uint64_t x, uint64_t y, uint32_t i, uint32_t accumulate) { ptx::umma_i8_pair(d, x, y, i, accumulate); };
+      auto f8 = [](uint32_t d, uint64_t x, uint64_t y, uint32_t i, uint32_t accumulate) { ptx::umma_f8_pair(d, x, y, i, accumulate); };
+      auto f16 = [](uint32_t d, uint64_t x, uint64_t y, uint32_t i, uint32_t accumulate) { ptx::umma_f16_pair(d, x, y, i, accumulate); };
+      if (kind == H3S_GEMM_I8) issue(ptx::umma_idesc(2, 1, 1, kGemmPairM, kGemmN), i8);
+      else if (kind == H3S_GEMM_E4M3) issue(ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN), f8);
+      else if (kind == H3S_GEMM_BF16) issue(ptx::umma_idesc(1, 1, 1, kGemmPairM, kGemmN), f16);
+      else issue(ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN), f16);
     }
   } else if (warp < 4 || warp >= 8) {
     // epilogue: thread <-> accumulator row, warp group <-> 128-column half of the tile
