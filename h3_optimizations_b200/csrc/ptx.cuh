@@ -371,6 +371,18 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
 
 // ---- tcgen05: TMEM <-> registers (whole warp; lane i <-> TMEM lane base+i) ----
 
+#define H3S_TMEM_LD8(taddr, r) \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" \
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) \
+      : "r"(taddr) \
+      : "memory")
+
+#define H3S_TMEM_LD16(taddr, r) \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) \
+      : "r"(taddr) \
+      : "memory")
+
 #define H3S_TMEM_LD32(taddr, r)                                                                      \
   asm volatile(                                                                                      \
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "                                                      \

@@ -158,21 +158,30 @@ constexpr int kGemmPairM = 2 * kGemmM;
 // Row pairs visited before the next column of tiles: 4096 rows of A (12 to 50 MB) and the
 // weights stay in L2 while every column passes over them.
 constexpr int kGemmGroupM = 16;
-// warps 0-3: epilogue of the tile's first 128 columns, 4: TMA, 5: MMA, 6-7: idle,
-// 8-11: epilogue of the second 128 columns (a warp may only touch the TMEM lanes
-// 32*(warp%4)..: two warps per lane quarter halve the epilogue's time, which
-// exceeds the MMA time of a tile once the norm and the rotation run in it)
-constexpr int kGemmThreads = 384;
+// A warp may only touch the TMEM lanes 32*(warp%4)...  Staging and dense: warps 0-3 epilogue of
+// the tile's first 128 columns, 4 TMA, 5 MMA, 6-7 idle, 8-11 epilogue of the second 128.
+// Carriers: warps 0-15 epilogue (four per lane quarter, two per 128 columns, each thread half a row), 16 TMA,
+// 17 MMA: with eight warps, one row a thread, 168 registers and half the warps to hide latencies behind,
+// the projection of 33272 rows with norm and rotation took 1.63 ms, 1.52 with sixteen.
+template <int kMode>
+struct GemmWarps {
+  static constexpr bool kMany = kMode == 1;  // kModeCarriers
+  static constexpr int kEpilogue = kMany ? 16 : 8;
+  static constexpr int kLoad = kMany ? 16 : 4, kIssue = kLoad + 1;
+  static constexpr int kThreads = kMany ? 18 * 32 : 384;
+  static __device__ __forceinline__ bool epilogue(int warp) { return kMany ? warp < 16 : warp < 4 || warp >= 8; }
+};
 constexpr uint32_t kGemmABytes = kGemmM * kGemmK;  // 16384
 constexpr uint32_t kGemmBBytes = kGemmN / 2 * kGemmK;  // 16384: this CTA's half
 constexpr uint32_t kGemmTmemCols = 512;
 
-// What the eight 16-thread row slots of one 128-column half of a tile tell each
-// other in the carrier epilogue: per-warp largest magnitudes and per-slot
-// per-channel partial sums (maxima for V) of the rows 0-63 and 64-127 of the tile.
+// What the eight warps of one 128-column half of a tile tell each other in the carrier
+// epilogue: the sums of squares of a row's two shares of channels, then per-warp largest
+// magnitudes and per-channel partial sums (maxima for V) of the rows 0-63 and 64-127 of the tile.
 struct EpilogueExchange {
-  float amax[2][4];                 // [row half][warp]
-  float column[2][8][H3S_HEAD_DIM];  // [row half][slot][channel]
+  double squares[2][kGemmM];         // [channel share][row]
+  float amax[2][8];                  // [row half][warp]
+  float column[2][8][H3S_HEAD_DIM];  // [row half][warp][channel]
 };
 constexpr uint32_t kEpilogueTileBytes = kGemmM * H3S_HEAD_DIM * 2;  // one half tile as bf16: 32 KB
 
@@ -187,6 +196,8 @@ enum GemmMode {
   kModeDense = 2,     // any operand kind -> scaled, biased, activated bf16 row-major matrix (h3s_dense_gemm)
 };
 
+static_assert(kModeCarriers == 1, "GemmWarps");
+
 template <int kMode>
 struct GemmLayout {
   static constexpr bool kCarriers = kMode != kModeStaging;  // both stage half tiles for coalesced stores
@@ -196,20 +207,21 @@ struct GemmLayout {
   static constexpr uint32_t kOffExchange = kOffTile + (kCarriers ? 2 * kEpilogueTileBytes : 0);
   static constexpr uint32_t kOffBar = kOffExchange + (kMode == kModeCarriers ? 2 * sizeof(EpilogueExchange) : 0);
   static constexpr uint32_t kBytes = kOffBar + 256 + 1024;
-  static_assert(sizeof(uint64_t) * (2 * 6 + 8) + 8 <= 256, "barriers");
+  static_assert(sizeof(uint64_t) * (2 * 6 + 16) + 8 <= 256, "barriers");
   static_assert(kBytes <= 227 * 1024, "GEMM shared memory exceeds the per-CTA limit");
 };
 constexpr int kGemmMaxStages = 6;
 
-enum GemmAbort { kGemmAbortFull = 21, kGemmAbortEmpty, kGemmAbortAccFull, kGemmAbortAccEmpty, kGemmAbortTile, kGemmAbortExchange };
+enum GemmAbort { kGemmAbortFull = 21, kGemmAbortEmpty, kGemmAbortAccFull, kGemmAbortAccEmpty, kGemmAbortTile, kGemmAbortExchange, kGemmAbortSquares };
 
 struct GemmShared {
   uint64_t full[kGemmMaxStages];   // first CTA's: the stage's four loads, two by each CTA
   uint64_t empty[kGemmMaxStages];  // both CTAs': the pair's MMAs have read the stage
   uint64_t acc_full[2];            // both CTAs'
-  uint64_t acc_empty[2];           // first CTA's: sixteen epilogue warps, eight in each CTA
-  uint64_t tile_ready[2];      // per tile half: its four warps have staged their rows
-  uint64_t exchange_ready[2];  // per tile half: its four warps have written their EpilogueExchange
+  uint64_t acc_empty[2];           // first CTA's: the epilogue warps of both
+  uint64_t tile_ready[2];      // per tile half: its warps have staged their rows
+  uint64_t exchange_ready[2];  // per tile half: its warps have written their EpilogueExchange
+  uint64_t squares_ready[2][4];  // per tile half and lane quarter: its two warps have written their sums of squares
   uint32_t tmem_base;
   int abort_word;
 };
@@ -420,20 +432,22 @@ __device__ __forceinline__ void norm_rope_packed(uint32_t (&y)[H3S_HEAD_DIM / 2]
 
 // Tables of any strides.  A call of its own with the row in local memory: unrolled in place,
 // its addresses took registers from the common forms, which then spilled 336 bytes a thread.
-__device__ __noinline__ void rotate_strided(uint32_t *row, const void *rope_row, int rope_dtype, int64_t stride_dim,
+// kPairs channel pairs from `pair0` on, and as many behind them that they are rotated against.
+template <int kPairs>
+__device__ __noinline__ void rotate_strided(uint32_t *row, int pair0, const void *rope_row, int rope_dtype, int64_t stride_dim,
                                             int64_t stride_rot, int64_t stride_pair) {
 #pragma unroll 1
-  for (int i = 0; i < 24; ++i) {
+  for (int i = 0; i < kPairs; ++i) {
     float f[2][4];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int64_t at = (2 * i + e) * stride_dim;
+      const int64_t at = (2 * (pair0 + i) + e) * stride_dim;
       f[e][0] = rope_load(rope_row, at, rope_dtype);
       f[e][1] = rope_load(rope_row, at + stride_pair, rope_dtype);
       f[e][2] = rope_load(rope_row, at + stride_rot, rope_dtype);
       f[e][3] = rope_load(rope_row, at + stride_rot + stride_pair, rope_dtype);
     }
-    rotate_pair(row[i], row[i + 24], f);
+    rotate_pair(row[i], row[i + kPairs], f);
   }
 }
 
@@ -452,9 +466,62 @@ __device__ __forceinline__ void norm_rope_row(uint32_t (&y)[H3S_HEAD_DIM / 2], c
   uint32_t row[H3S_HEAD_DIM / 2];
 #pragma unroll
   for (int i = 0; i < H3S_HEAD_DIM / 2; ++i) row[i] = y[i];
-  rotate_strided(row, rope_row, rope_dtype, stride_dim, stride_rot, stride_pair);
+  rotate_strided<24>(row, 0, rope_row, rope_dtype, stride_dim, stride_rot, stride_pair);
 #pragma unroll
   for (int i = 0; i < H3S_HEAD_DIM / 2; ++i) y[i] = row[i];
+}
+
+// Half of such a row, as the carrier epilogue deals it to a thread: the channels
+// 24*share + [0, 24) and 48 + 24*share + [0, 24), which are rotated against each other, and
+// 96 + 16*share + [0, 16).
+struct HalfRow {
+  uint32_t first[12], second[12], rest[8];
+};
+
+__device__ __forceinline__ void square_sum(const uint32_t w, double (&part)[4], int i) {
+  const double lo = static_cast<double>(bf16_lo(w)), hi = static_cast<double>(bf16_hi(w));
+  part[(2 * i) & 3] = fma(lo, lo, part[(2 * i) & 3]);
+  part[(2 * i + 1) & 3] = fma(hi, hi, part[(2 * i + 1) & 3]);
+}
+
+__device__ __forceinline__ double half_row_squares(const HalfRow &y) {
+  double part[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < 12; ++i) square_sum(y.first[i], part, i);
+#pragma unroll
+  for (int i = 0; i < 12; ++i) square_sum(y.second[i], part, i);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) square_sum(y.rest[i], part, i);
+  return (part[0] + part[1]) + (part[2] + part[3]);
+}
+
+__device__ __forceinline__ uint32_t norm_pair(uint32_t y, float2 inverse_rms, const float *__restrict__ weight) {
+  const float2 normed = mul2(mul2(bf16_pair(y), inverse_rms), __ldg(reinterpret_cast<const float2 *>(weight)));
+  return pack_bf16x2(normed.x, normed.y);
+}
+
+__device__ __forceinline__ void norm_half_row(HalfRow &y, double squares, const float *__restrict__ norm_weight,
+                                              float epsilon, int share) {
+  const float mean = __fadd_rn(__fmul_rn(static_cast<float>(squares), 1.0f / H3S_HEAD_DIM), epsilon);
+  const float inverse_rms = __frsqrt_rn(mean);
+  const float2 inverse = make_float2(inverse_rms, inverse_rms);
+#pragma unroll
+  for (int i = 0; i < 12; ++i) y.first[i] = norm_pair(y.first[i], inverse, norm_weight + 24 * share + 2 * i);
+#pragma unroll
+  for (int i = 0; i < 12; ++i) y.second[i] = norm_pair(y.second[i], inverse, norm_weight + 48 + 24 * share + 2 * i);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) y.rest[i] = norm_pair(y.rest[i], inverse, norm_weight + 96 + 16 * share + 2 * i);
+}
+
+// The factors of one channel pair: 16 (bf16) or 32 bytes
+__device__ __forceinline__ void rotate_bf16(uint32_t &first, uint32_t &second, const uint4 &w) {
+  const float f[2][4] = {{bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y)},
+                         {bf16_lo(w.z), bf16_hi(w.z), bf16_lo(w.w), bf16_hi(w.w)}};
+  rotate_pair(first, second, f);
+}
+__device__ __forceinline__ void rotate_f32(uint32_t &first, uint32_t &second, const float4 &u, const float4 &w) {
+  const float f[2][4] = {{u.x, u.y, u.z, u.w}, {w.x, w.y, w.z, w.w}};
+  rotate_pair(first, second, f);
 }
 
 // Tile `tile` of the persistent order: row pair and column tile
@@ -469,13 +536,14 @@ __device__ __forceinline__ void tile_position(const GemmParams &prm, int tile, i
 }
 
 template <int kMode>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmWarps<kMode>::kThreads, 1)
 qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const GemmParams prm) {
   extern __shared__ unsigned char smem_dyn[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~static_cast<uintptr_t>(1023));
   using L = GemmLayout<kMode>;
+  using W = GemmWarps<kMode>;
   constexpr bool kCarriers = kMode == kModeCarriers;
   GemmShared &sh = *reinterpret_cast<GemmShared *>(smem + L::kOffBar);
   volatile int *abort_word = &sh.abort_word;
@@ -492,14 +560,15 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&sh.acc_full[i], 1);
-      ptx::mbar_init(&sh.acc_empty[i], 16);
-      ptx::mbar_init(&sh.tile_ready[i], 4);
-      ptx::mbar_init(&sh.exchange_ready[i], 4);
+      ptx::mbar_init(&sh.acc_empty[i], 2 * W::kEpilogue);
+      ptx::mbar_init(&sh.tile_ready[i], W::kEpilogue / 2);
+      ptx::mbar_init(&sh.exchange_ready[i], W::kEpilogue / 2);
+      for (int quarter = 0; quarter < 4; ++quarter) ptx::mbar_init(&sh.squares_ready[i][quarter], 2);
     }
     sh.abort_word = 0;
     ptx::fence_mbar_init();
   }
-  if (warp == 5) {
+  if (warp == W::kIssue) {
     ptx::tmem_alloc_pair(&sh.tmem_base, kGemmTmemCols);
     ptx::tmem_relinquish_pair();
   }
@@ -509,7 +578,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   ptx::tc_fence_after();
   const uint32_t tmem_base = sh.tmem_base;
 
-  if (warp == 4) {
+  if (warp == W::kLoad) {
     // One thread, its state kept from step to step: at 128 bytes of K a step the MMAs take 512 cycles, and
     // what this thread and the issuing one do for a step is a chain of dependent instructions.
     if (ptx::elect_one()) {
@@ -538,7 +607,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       for (uint32_t i = it > L::kStages ? it - L::kStages : 0; ok && i < it; ++i)
         ok = ptx::mbar_wait(&sh.empty[i % L::kStages], (i / L::kStages) & 1u, abort_word, kGemmAbortEmpty, prm.wait_budget_ns);
     }
-  } else if (warp == 5) {
+  } else if (warp == W::kIssue) {
     if (rank == 0 && ptx::elect_one()) {
       // every kind consumes 32 bytes of K per instruction: four instructions per 128-byte stage
       const int kind = kMode == kModeDense ? prm.operand_kind : H3S_GEMM_I8;
@@ -573,14 +642,16 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       else if (kind == H3S_GEMM_BF16) issue(ptx::umma_idesc(1, 1, 1, kGemmPairM, kGemmN), f16);
       else issue(ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN), f16);
     }
-  } else if (warp < 4 || warp >= 8) {
-    // epilogue: thread <-> accumulator row, warp group <-> 128-column half of the tile
+  } else if (W::epilogue(warp)) {
+    // epilogue: warp group <-> 128-column half of the tile, thread <-> accumulator row (carriers: half a row)
     const int quarter = warp & 3;
-    const int gi = warp >= 8 ? 1 : 0;
+    const int gi = W::kMany ? (warp >> 2) & 1 : warp >= 8 ? 1 : 0;
+    const int share = warp >> 3;  // carriers: which half of the channels
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     uint32_t local = 0;
     const uint32_t acc_empty[2] = {ptx::cluster_address(&sh.acc_empty[0], 0), ptx::cluster_address(&sh.acc_empty[1], 0)};
     uint32_t exchanges = 0;  // uses of this half's exchange buffer and barrier so far
+    uint32_t squared = 0;    // ... and of the sums of squares
     bool ok = true;
     for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step, ++local) {
       int pair, tn;
@@ -702,50 +773,118 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
         if (kCarriers) {
           // ---- carriers straight from the accumulators ----
-          // Phase A, one thread per row: de-quantise the row of this head to bf16
+          // Phase A, two threads per row: de-quantise the row of this head to bf16
           // (+ norm and rotation) and stage it in shared memory, 16-byte chunk c of
           // row r at chunk position c ^ (r & 15) so that neither these row-wise
           // writes nor the column-wise reads of phase B collide on banks.
           unsigned char *tile = smem + L::kOffTile + gi * kEpilogueTileBytes;
+          EpilogueExchange &ex = reinterpret_cast<EpilogueExchange *>(smem + L::kOffExchange)[gi];
           const int local_row = quarter * 32 + lane;
           {
-            uint32_t y[H3S_HEAD_DIM / 2];
+            HalfRow y;
             const float2 xs2 = make_float2(xs, xs);
             const float *w_scale = prm.w_scale + (group_ok ? group_col0 : 0);  // without a group nothing is stored
+            const uint32_t columns = tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM;
+            auto dequantise = [&](uint32_t lo, uint32_t hi, int channel) {
+              const float2 ws = __ldg(reinterpret_cast<const float2 *>(w_scale + channel));
+              const float2 value = mul2(make_float2(static_cast<float>(static_cast<int>(lo)),
+                                                    static_cast<float>(static_cast<int>(hi))), mul2(xs2, ws));
+              return pack_bf16x2(value.x, value.y);
+            };
+            auto read24 = [&](uint32_t (&to)[12], int channel) {
+              uint32_t acc[16], more[8];
+              H3S_TMEM_LD16(columns + channel, acc);
+              H3S_TMEM_LD8(columns + channel + 16, more);
+              ptx::tmem_wait_ld(acc);
+              ptx::tmem_wait_ld(more);
 #pragma unroll
-            for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
-              uint32_t acc[32];
-              H3S_TMEM_LD32(tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM + cc * 32, acc);
+              for (int i = 0; i < 8; ++i) to[i] = dequantise(acc[2 * i], acc[2 * i + 1], channel + 2 * i);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) to[8 + i] = dequantise(more[2 * i], more[2 * i + 1], channel + 16 + 2 * i);
+            };
+            read24(y.first, 24 * share);
+            read24(y.second, 48 + 24 * share);
+            {
+              uint32_t acc[16];
+              H3S_TMEM_LD16(columns + 96 + 16 * share, acc);
               ptx::tmem_wait_ld(acc);
 #pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                const float2 ws = __ldg(reinterpret_cast<const float2 *>(w_scale + cc * 32 + i));
-                const float2 value = mul2(make_float2(static_cast<float>(static_cast<int>(acc[i])),
-                                                      static_cast<float>(static_cast<int>(acc[i + 1]))), mul2(xs2, ws));
-                y[cc * 16 + (i >> 1)] = pack_bf16x2(value.x, value.y);
-              }
+              for (int i = 0; i < 8; ++i) y.rest[i] = dequantise(acc[2 * i], acc[2 * i + 1], 96 + 16 * share + 2 * i);
             }
             // the accumulator is in registers: the MMA warp may refill it
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive_cluster(acc_empty[a]);
-            if (!group_ok) continue;  // the same for the four warps of this half
-            if (normed && row_ok) {
+            if (!group_ok) continue;  // the same for the eight warps of this half
+            if (normed) {
+              const double mine = half_row_squares(y);
+              ex.squares[share][local_row] = mine;
+              __syncwarp();
+              if (lane == 0) ptx::mbar_arrive(&sh.squares_ready[gi][quarter]);
               const void *rope_row = nullptr;
-              if (prm.rope != nullptr) {
+              if (prm.rope != nullptr && row_ok) {
                 const int64_t offset = static_cast<int64_t>(row) * prm.rope_stride_seq;
                 rope_row = prm.rope_dtype == H3S_F32
                                ? static_cast<const void *>(static_cast<const float *>(prm.rope) + offset)
                                : static_cast<const void *>(static_cast<const __nv_bfloat16 *>(prm.rope) + offset);
               }
-              norm_rope_row(y, group < prm.heads ? prm.q_norm : prm.k_norm, prm.epsilon, rope_row, prm.rope_dtype,
-                            prm.rope_stride_dim, prm.rope_stride_rot, prm.rope_stride_pair);
+              const bool packed = prm.rope_stride_pair == 1 && prm.rope_stride_rot == 2 && prm.rope_stride_dim == 4 &&
+                                  (reinterpret_cast<uintptr_t>(rope_row) & 15) == 0;
+              const RopeForm form = rope_row == nullptr ? kRopeNone
+                                    : !packed           ? kRopeStrided
+                                    : prm.rope_dtype == H3S_BF16 ? kRopeBf16 : kRopeF32;
+              // the first factors travel while the norm is computed
+              constexpr int kBatch = 4;
+              uint4 ahead[kBatch];
+              if (form == kRopeBf16) {
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) ahead[k] = __ldg(static_cast<const uint4 *>(rope_row) + 12 * share + k);
+              }
+              const bool got = ptx::mbar_wait(&sh.squares_ready[gi][quarter], squared & 1u, abort_word, kGemmAbortSquares,
+                                              prm.wait_budget_ns);
+              if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+              ++squared;
+              norm_half_row(y, mine + ex.squares[1 - share][local_row], group < prm.heads ? prm.q_norm : prm.k_norm,
+                            prm.epsilon, share);
+              if (form == kRopeBf16) {
+                const uint4 *table = static_cast<const uint4 *>(rope_row) + 12 * share;
+#pragma unroll
+                for (int k = 0; k < 12; ++k) {
+                  const uint4 now = ahead[k % kBatch];
+                  if (k + kBatch < 12) ahead[k % kBatch] = __ldg(table + k + kBatch);
+                  rotate_bf16(y.first[k], y.second[k], now);
+                }
+              } else if (form == kRopeF32) {
+                const float4 *table = static_cast<const float4 *>(rope_row) + 24 * share;
+#pragma unroll
+                for (int b = 0; b < 12; b += 4) {
+                  float4 now[8];
+#pragma unroll
+                  for (int k = 0; k < 8; ++k) now[k] = __ldg(table + 2 * b + k);
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) rotate_f32(y.first[b + k], y.second[b + k], now[2 * k], now[2 * k + 1]);
+                }
+              } else if (form == kRopeStrided) {
+                uint32_t pairs[24];
+#pragma unroll
+                for (int k = 0; k < 12; ++k) { pairs[k] = y.first[k]; pairs[12 + k] = y.second[k]; }
+                rotate_strided<12>(pairs, 12 * share, rope_row, prm.rope_dtype, prm.rope_stride_dim, prm.rope_stride_rot,
+                                   prm.rope_stride_pair);
+#pragma unroll
+                for (int k = 0; k < 12; ++k) { y.first[k] = pairs[k]; y.second[k] = pairs[12 + k]; }
+              }
             }
             uint4 *my_row = reinterpret_cast<uint4 *>(tile + local_row * (H3S_HEAD_DIM * 2));
+            auto stage = [&](int chunk, const uint32_t *w) {  // rows past the chunk count as zeros
+              my_row[chunk ^ (local_row & 15)] = row_ok ? make_uint4(w[0], w[1], w[2], w[3]) : make_uint4(0u, 0u, 0u, 0u);
+            };
 #pragma unroll
-            for (int c = 0; c < 16; ++c)
-              my_row[c ^ (local_row & 15)] = row_ok ? make_uint4(y[4 * c], y[4 * c + 1], y[4 * c + 2], y[4 * c + 3])
-                                                    : make_uint4(0u, 0u, 0u, 0u);  // rows past the chunk count as zeros
+            for (int c = 0; c < 3; ++c) {
+              stage(3 * share + c, y.first + 4 * c);
+              stage(6 + 3 * share + c, y.second + 4 * c);
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) stage(12 + 2 * share + c, y.rest + 4 * c);
           }
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&sh.tile_ready[gi]);
@@ -755,20 +894,20 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
           }
           // Phase B, 16 threads per row, 8 channels each: thread (slot, c) holds rows
-          // slot, slot+8, ... slot+120 of channels 8c..8c+7, as in quant_qk_blocks_kernel.
+          // slot, slot+16, ... slot+112 of channels 8c..8c+7.
           const int kind = group / prm.heads, head = group - kind * prm.heads;
-          const int g = quarter * 32 + lane;  // thread within this half's 128
-          const int slot = g >> 4, c = g & 15;
+          const int t = share * 128 + quarter * 32 + lane;  // thread within this half's 256
+          const int slot = t >> 4, c = t & 15;
+          const int half_warp = share * 4 + quarter;
           const bool quantise_here = kind == 0 || (kind == 1 && prm.k8 != nullptr);
-          EpilogueExchange &ex = reinterpret_cast<EpilogueExchange *>(smem + L::kOffExchange)[gi];
-          uint4 raw[16];
+          uint4 raw[8];
 #pragma unroll
-          for (int p = 0; p < 16; ++p) {
-            const int r = p * 8 + slot;
+          for (int p = 0; p < 8; ++p) {
+            const int r = p * 16 + slot;
             raw[p] = *reinterpret_cast<const uint4 *>(tile + r * (H3S_HEAD_DIM * 2) + ((c ^ (r & 15)) << 4));
           }
           {
-            // partial statistics of rows 0-63 (passes 0-7) and 64-127 (passes 8-15)
+            // partial statistics of rows 0-63 (passes 0-3) and 64-127 (passes 4-7)
             float part[2][8];
             __nv_bfloat162 top[2];
 #pragma unroll
@@ -777,7 +916,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
               for (int i = 0; i < 8; ++i) part[h][i] = 0.f;
 #pragma unroll
-              for (int p = 8 * h; p < 8 * h + 8; ++p) {
+              for (int p = 4 * h; p < 4 * h + 4; ++p) {
                 const uint32_t w[4] = {raw[p].x, raw[p].y, raw[p].z, raw[p].w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -795,13 +934,19 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                   }
                 }
               }
-#pragma unroll
-              for (int i = 0; i < 8; ++i) ex.column[h][slot][c * 8 + i] = part[h][i];
               if (quantise_here) {
                 const uint32_t bits = *reinterpret_cast<const uint32_t *>(&top[h]);
                 const float amax = warp_max(fmaxf(bf16_lo(bits), bf16_hi(bits)));
-                if (lane == 0) ex.amax[h][quarter] = amax;
+                if (lane == 0) ex.amax[h][half_warp] = amax;
               }
+            }
+            // the warp's two slots together: one of them leaves the first half's values, one the second's
+            float *column = ex.column[lane >> 4][half_warp] + c * 8;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float mine = lane < 16 ? part[0][i] : part[1][i];
+              const float other = __shfl_xor_sync(0xffffffffu, lane < 16 ? part[1][i] : part[0][i], 16);
+              column[i] = kind == 2 ? fmaxf(mine, other) : mine + other;
             }
           }
           __syncwarp();
@@ -820,88 +965,80 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           float amax_half[2] = {0.f, 0.f};
           if (quantise_here) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-              amax_half[h] = fmaxf(fmaxf(ex.amax[h][0], ex.amax[h][1]), fmaxf(ex.amax[h][2], ex.amax[h][3]));
-          }
-          // channel g of this head: totals over the eight row slots
-          double total[2] = {0.0, 0.0};
-          float peak = 0.f;
+            for (int h = 0; h < 2; ++h) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-#pragma unroll
-            for (int sl = 0; sl < 8; ++sl) {
-              if (kind == 2) peak = fmaxf(peak, ex.column[h][sl][g]);
-              else total[h] += static_cast<double>(ex.column[h][sl][g]);
+              for (int w = 0; w < 8; ++w) amax_half[h] = fmaxf(amax_half[h], ex.amax[h][w]);
             }
           }
+          // channel g of this head, row half `share`: totals over the eight warps
+          const int g = t & (H3S_HEAD_DIM - 1);
+          auto total = [&](int h) {
+            double sum = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) sum += static_cast<double>(ex.column[h][w][g]);
+            return sum;
+          };
           if (kind == 0) {
             const int blocks_total = (prm.sequence_total + H3S_Q_TILE - 1) / H3S_Q_TILE;
             const int block = tile_row0 / H3S_Q_TILE;
             const float scale = __fadd_rn(__fdiv_rn(fmaxf(amax_half[0], amax_half[1]), 127.0f), 1.0e-7f);
-            if (g == 0) prm.q_scale[head * blocks_total + block] = scale;
-            store_summary(prm.q_summary, prm.summary_dtype,
-                          (static_cast<int64_t>(head) * blocks_total + block) * H3S_HEAD_DIM + g, (total[0] + total[1]) / valid);
+            if (t == 0) prm.q_scale[head * blocks_total + block] = scale;
+            if (share == 0)
+              store_summary(prm.q_summary, prm.summary_dtype,
+                            (static_cast<int64_t>(head) * blocks_total + block) * H3S_HEAD_DIM + g, (total(0) + total(1)) / valid);
             int8_t *dst = prm.q8 + (static_cast<int64_t>(head) * prm.sequence_total + tile_row0) * H3S_HEAD_DIM + c * 8;
             const SharedDivisor by_scale = make_divisor(scale);
-            if (by_scale.exact) {
+            auto emit = [&](auto exact) {
 #pragma unroll
-              for (int p = 0; p < 16; ++p) {
-                const int r = p * 8 + slot;
-                if (r < valid) quantise8<true>(raw[p], by_scale, dst + static_cast<int64_t>(r) * H3S_HEAD_DIM);
+              for (int p = 0; p < 8; ++p) {
+                const int r = p * 16 + slot;
+                if (r < valid) quantise8<decltype(exact)::value>(raw[p], by_scale, dst + static_cast<int64_t>(r) * H3S_HEAD_DIM);
               }
-            } else {
-#pragma unroll
-              for (int p = 0; p < 16; ++p) {
-                const int r = p * 8 + slot;
-                if (r < valid) quantise8<false>(raw[p], by_scale, dst + static_cast<int64_t>(r) * H3S_HEAD_DIM);
-              }
-            }
+            };
+            if (by_scale.exact) emit(std::true_type{}); else emit(std::false_type{});
           } else if (kind == 1) {
             const int blocks_total = (prm.sequence_total + H3S_KV_TILE - 1) / H3S_KV_TILE;
             const int block0 = tile_row0 / H3S_KV_TILE;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              if (valid_half[h] > 0)
-                store_summary(prm.k_summary, prm.summary_dtype,
-                              (static_cast<int64_t>(head) * blocks_total + block0 + h) * H3S_HEAD_DIM + g, total[h] / valid_half[h]);
+            const double sum = total(share);
+            if (valid_half[share] > 0) {
+              store_summary(prm.k_summary, prm.summary_dtype,
+                            (static_cast<int64_t>(head) * blocks_total + block0 + share) * H3S_HEAD_DIM + g, sum / valid_half[share]);
+              if (prm.k_sum != nullptr) atomicAdd(prm.k_sum + head * H3S_HEAD_DIM + g, sum);
             }
-            if (prm.k_sum != nullptr) atomicAdd(prm.k_sum + head * H3S_HEAD_DIM + g, total[0] + total[1]);
             if (prm.k8 != nullptr) {
               int8_t *dst = prm.k8 + (static_cast<int64_t>(head) * prm.sequence_total + tile_row0) * H3S_HEAD_DIM + c * 8;
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 const float scale = __fadd_rn(__fdiv_rn(amax_half[h], 127.0f), 1.0e-7f);
-                if (g == 0 && valid_half[h] > 0) prm.k_scale[head * blocks_total + block0 + h] = scale;
+                if (t == 0 && valid_half[h] > 0) prm.k_scale[head * blocks_total + block0 + h] = scale;
                 const SharedDivisor by_scale = make_divisor(scale);
-                if (by_scale.exact) {
+                auto emit = [&](auto exact) {
 #pragma unroll
-                  for (int p = 8 * h; p < 8 * h + 8; ++p) {
-                    const int r = p * 8 + slot;
-                    if (r < valid) quantise8<true>(raw[p], by_scale, dst + static_cast<int64_t>(r) * H3S_HEAD_DIM);
+                  for (int p = 4 * h; p < 4 * h + 4; ++p) {
+                    const int r = p * 16 + slot;
+                    if (r < valid) quantise8<decltype(exact)::value>(raw[p], by_scale, dst + static_cast<int64_t>(r) * H3S_HEAD_DIM);
                   }
-                } else {
-#pragma unroll
-                  for (int p = 8 * h; p < 8 * h + 8; ++p) {
-                    const int r = p * 8 + slot;
-                    if (r < valid) quantise8<false>(raw[p], by_scale, dst + static_cast<int64_t>(r) * H3S_HEAD_DIM);
-                  }
-                }
+                };
+                if (by_scale.exact) emit(std::true_type{}); else emit(std::false_type{});
               }
             } else {
               __nv_bfloat16 *dst = prm.k_stage + (static_cast<int64_t>(head) * prm.sequence_total + tile_row0) * H3S_HEAD_DIM + c * 8;
 #pragma unroll
-              for (int p = 0; p < 16; ++p) {
-                const int r = p * 8 + slot;
+              for (int p = 0; p < 8; ++p) {
+                const int r = p * 16 + slot;
                 if (r < valid) *reinterpret_cast<uint4 *>(dst + static_cast<int64_t>(r) * H3S_HEAD_DIM) = raw[p];
               }
             }
           } else {
+            float peak = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) peak = fmaxf(peak, ex.column[share][w][g]);
             // non-negative floats order like their bit patterns
             atomicMax(prm.v_amax_bits + head * H3S_HEAD_DIM + g, __float_as_uint(peak));
             __nv_bfloat16 *dst = prm.v_stage + (static_cast<int64_t>(head) * prm.sequence_total + tile_row0) * H3S_HEAD_DIM + c * 8;
 #pragma unroll
-            for (int p = 0; p < 16; ++p) {
-              const int r = p * 8 + slot;
+            for (int p = 0; p < 8; ++p) {
+              const int r = p * 16 + slot;
               if (r < valid) *reinterpret_cast<uint4 *>(dst + static_cast<int64_t>(r) * H3S_HEAD_DIM) = raw[p];
             }
           }
@@ -980,7 +1117,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   }
   ptx::cluster_sync();  // neither CTA leaves while the other may still signal its barriers or its TMEM is written
-  if (warp == 5) {
+  if (warp == W::kIssue) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc_pair(tmem_base, kGemmTmemCols);
   }
@@ -1107,11 +1244,11 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
   if (carriers != nullptr) {
     H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeCarriers>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(GemmLayout<kModeCarriers>::kBytes)));
-    qkv_gemm_kernel<kModeCarriers><<<grid, kGemmThreads, GemmLayout<kModeCarriers>::kBytes, static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
+    qkv_gemm_kernel<kModeCarriers><<<grid, GemmWarps<kModeCarriers>::kThreads, GemmLayout<kModeCarriers>::kBytes, static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
   } else {
     H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeStaging>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(GemmLayout<kModeStaging>::kBytes)));
-    qkv_gemm_kernel<kModeStaging><<<grid, kGemmThreads, GemmLayout<kModeStaging>::kBytes, static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
+    qkv_gemm_kernel<kModeStaging><<<grid, GemmWarps<kModeStaging>::kThreads, GemmLayout<kModeStaging>::kBytes, static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
   }
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
@@ -1172,7 +1309,7 @@ int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_
   H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeDense>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(GemmLayout<kModeDense>::kBytes)));
   const int tiles = prm.m_pairs * prm.n_tiles;
-  qkv_gemm_kernel<kModeDense><<<2 * (tiles < sms / 2 ? tiles : sms / 2), kGemmThreads, GemmLayout<kModeDense>::kBytes,
+  qkv_gemm_kernel<kModeDense><<<2 * (tiles < sms / 2 ? tiles : sms / 2), GemmWarps<kModeDense>::kThreads, GemmLayout<kModeDense>::kBytes,
                                static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
