@@ -179,7 +179,7 @@ constexpr uint32_t kGemmTmemCols = 512;
 // epilogue: the sums of squares of a row's two shares of channels, then per-warp largest
 // magnitudes and per-channel partial sums (maxima for V) of the rows 0-63 and 64-127 of the tile.
 struct EpilogueExchange {
-  double squares[2][kGemmM];         // [channel share][row]
+  float2 squares[2][kGemmM];         // [channel share][row], PairSum
   float amax[2][8];                  // [row half][warp]
   float column[2][8][H3S_HEAD_DIM];  // [row half][warp][channel]
 };
@@ -478,21 +478,75 @@ struct HalfRow {
   uint32_t first[12], second[12], rest[8];
 };
 
-__device__ __forceinline__ void square_sum(const uint32_t w, double (&part)[4], int i) {
-  const double lo = static_cast<double>(bf16_lo(w)), hi = static_cast<double>(bf16_hi(w));
-  part[(2 * i) & 3] = fma(lo, lo, part[(2 * i) & 3]);
-  part[(2 * i + 1) & 3] = fma(hi, hi, part[(2 * i + 1) & 3]);
+// A sum as an unevaluated pair of floats, good to about 46 bits
+struct PairSum {
+  float hi, lo;
+};
+
+// a + b exactly (Knuth's two-sum), the small parts added up
+__device__ __forceinline__ PairSum add_pairs(const PairSum &a, const PairSum &b) {
+  const float s = __fadd_rn(a.hi, b.hi), back = __fsub_rn(s, a.hi);
+  const float error = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, back)), __fsub_rn(b.hi, back));
+  return {s, __fadd_rn(error, __fadd_rn(a.lo, b.lo))};
 }
 
-__device__ __forceinline__ double half_row_squares(const HalfRow &y) {
-  double part[4] = {0.0, 0.0, 0.0, 0.0};
+// Rows whose squares leave the range in which every step below is exact
+__device__ __noinline__ PairSum square_sum_wide(const uint32_t *row) {
+  double sum = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < 32; ++i) {
+    const double lo = static_cast<double>(bf16_lo(row[i])), hi = static_cast<double>(bf16_hi(row[i]));
+    sum = fma(lo, lo, sum);
+    sum = fma(hi, hi, sum);
+  }
+  const float hi = static_cast<float>(sum);
+  return {hi, hi < INFINITY ? static_cast<float>(sum - static_cast<double>(hi)) : 0.f};
+}
+
+// The sum of squares of half a row, as good as in 64 bits and without its unit, which took 2000 to 6000 cycles a tile
+// here and 30000 for a CTA's first.  The square of a bf16 value is exact in fp32.  The accumulator begins at a power
+// of two that no square exceeds, so that acc + p - acc loses exactly what rounding took from p (Dekker's
+// fast two-sum, which wants the larger operand first); the losses are added up beside it.
+__device__ __forceinline__ PairSum half_row_squares(const HalfRow &y) {
+  __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
+  auto magnitude = [&](uint32_t w) {
+    w &= 0x7fff7fffu;
+    top = __hmax2_nan(top, *reinterpret_cast<const __nv_bfloat162 *>(&w));
+  };
 #pragma unroll
-  for (int i = 0; i < 12; ++i) square_sum(y.first[i], part, i);
+  for (int i = 0; i < 12; ++i) { magnitude(y.first[i]); magnitude(y.second[i]); }
 #pragma unroll
-  for (int i = 0; i < 12; ++i) square_sum(y.second[i], part, i);
+  for (int i = 0; i < 8; ++i) magnitude(y.rest[i]);
+  const uint32_t bits = *reinterpret_cast<const uint32_t *>(&top);
+  const float lo_top = bf16_lo(bits), hi_top = bf16_hi(bits);
+  const float most = fmaxf(lo_top, hi_top);
+  if (!(lo_top < 1e17f && hi_top < 1e17f) || (most < 1e-12f && most > 0.f)) {
+    uint32_t row[32];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) square_sum(y.rest[i], part, i);
-  return (part[0] + part[1]) + (part[2] + part[3]);
+    for (int i = 0; i < 12; ++i) { row[i] = y.first[i]; row[12 + i] = y.second[i]; }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) row[24 + i] = y.rest[i];
+    return square_sum_wide(row);
+  }
+  // the next power of two above the largest square
+  const float base = __uint_as_float((__float_as_uint(__fmul_rn(most, most)) & 0x7f800000u) + 0x00800000u);
+  const float2 minus = make_float2(-1.f, -1.f);
+  float2 acc[2] = {make_float2(base, base), make_float2(base, base)};
+  float2 lost[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  auto square = [&](uint32_t w, int i) {
+    const float2 v = bf16_pair(w);
+    const float2 p = mul2(v, v), next = add2(acc[i & 1], p);
+    const float2 taken = fma2(acc[i & 1], minus, next);   // next - acc
+    lost[i & 1] = add2(lost[i & 1], fma2(taken, minus, p));  // p - taken
+    acc[i & 1] = next;
+  };
+#pragma unroll
+  for (int i = 0; i < 12; ++i) { square(y.first[i], i); square(y.second[i], i + 1); }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) square(y.rest[i], i);
+  const PairSum a = add_pairs({__fsub_rn(acc[0].x, base), lost[0].x}, {__fsub_rn(acc[0].y, base), lost[0].y});
+  const PairSum b = add_pairs({__fsub_rn(acc[1].x, base), lost[1].x}, {__fsub_rn(acc[1].y, base), lost[1].y});
+  return add_pairs(a, b);
 }
 
 __device__ __forceinline__ uint32_t norm_pair(uint32_t y, float2 inverse_rms, const float *__restrict__ weight) {
@@ -500,9 +554,9 @@ __device__ __forceinline__ uint32_t norm_pair(uint32_t y, float2 inverse_rms, co
   return pack_bf16x2(normed.x, normed.y);
 }
 
-__device__ __forceinline__ void norm_half_row(HalfRow &y, double squares, const float *__restrict__ norm_weight,
+__device__ __forceinline__ void norm_half_row(HalfRow &y, float squares, const float *__restrict__ norm_weight,
                                               float epsilon, int share) {
-  const float mean = __fadd_rn(__fmul_rn(static_cast<float>(squares), 1.0f / H3S_HEAD_DIM), epsilon);
+  const float mean = __fadd_rn(__fmul_rn(squares, 1.0f / H3S_HEAD_DIM), epsilon);
   const float inverse_rms = __frsqrt_rn(mean);
   const float2 inverse = make_float2(inverse_rms, inverse_rms);
 #pragma unroll
@@ -817,8 +871,8 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             if (lane == 0) ptx::mbar_arrive_cluster(acc_empty[a]);
             if (!group_ok) continue;  // the same for the eight warps of this half
             if (normed) {
-              const double mine = half_row_squares(y);
-              ex.squares[share][local_row] = mine;
+              const PairSum mine = half_row_squares(y);
+              ex.squares[share][local_row] = make_float2(mine.hi, mine.lo);
               __syncwarp();
               if (lane == 0) ptx::mbar_arrive(&sh.squares_ready[gi][quarter]);
               const void *rope_row = nullptr;
@@ -844,7 +898,9 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                               prm.wait_budget_ns);
               if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
               ++squared;
-              norm_half_row(y, mine + ex.squares[1 - share][local_row], group < prm.heads ? prm.q_norm : prm.k_norm,
+              const float2 theirs = ex.squares[1 - share][local_row];
+              const PairSum squares = add_pairs(mine, {theirs.x, theirs.y});
+              norm_half_row(y, __fadd_rn(squares.hi, squares.lo), group < prm.heads ? prm.q_norm : prm.k_norm,
                             prm.epsilon, share);
               if (form == kRopeBf16) {
                 const uint4 *table = static_cast<const uint4 *>(rope_row) + 12 * share;
