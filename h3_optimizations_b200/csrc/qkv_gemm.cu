@@ -490,6 +490,10 @@ __device__ __forceinline__ PairSum add_pairs(const PairSum &a, const PairSum &b)
   return {s, __fadd_rn(error, __fadd_rn(a.lo, b.lo))};
 }
 
+__device__ __forceinline__ double wide(const PairSum &a) {
+  return isfinite(a.hi) ? static_cast<double>(a.hi) + static_cast<double>(a.lo) : static_cast<double>(a.hi);
+}
+
 // Rows whose squares leave the range in which every step below is exact
 __device__ __noinline__ PairSum square_sum_wide(const uint32_t *row) {
   double sum = 0.0;
@@ -573,8 +577,21 @@ __device__ __forceinline__ void rotate_bf16(uint32_t &first, uint32_t &second, c
                          {bf16_lo(w.z), bf16_hi(w.z), bf16_lo(w.w), bf16_hi(w.w)}};
   rotate_pair(first, second, f);
 }
-__device__ __forceinline__ void rotate_f32(uint32_t &first, uint32_t &second, const float4 &u, const float4 &w) {
-  const float f[2][4] = {{u.x, u.y, u.z, u.w}, {w.x, w.y, w.z, w.w}};
+// 32 bytes of a row's table: whole sectors where it is aligned to them, as 16-byte loads of 32 different
+// rows visit each one twice
+__device__ __forceinline__ void load_sector(uint4 (&to)[2], const uint4 *from, bool sectors) {
+  if (!sectors) {
+    to[0] = __ldg(from);
+    to[1] = __ldg(from + 1);
+    return;
+  }
+  asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(to[0].x), "=r"(to[0].y), "=r"(to[0].z), "=r"(to[0].w), "=r"(to[1].x), "=r"(to[1].y), "=r"(to[1].z), "=r"(to[1].w)
+               : "l"(from));
+}
+__device__ __forceinline__ void rotate_f32(uint32_t &first, uint32_t &second, const uint4 &u, const uint4 &w) {
+  const float f[2][4] = {{__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w)},
+                         {__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w)}};
   rotate_pair(first, second, f);
 }
 
@@ -884,15 +901,15 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               }
               const bool packed = prm.rope_stride_pair == 1 && prm.rope_stride_rot == 2 && prm.rope_stride_dim == 4 &&
                                   (reinterpret_cast<uintptr_t>(rope_row) & 15) == 0;
+              const bool sectors = (reinterpret_cast<uintptr_t>(rope_row) & 31) == 0;
               const RopeForm form = rope_row == nullptr ? kRopeNone
                                     : !packed           ? kRopeStrided
                                     : prm.rope_dtype == H3S_BF16 ? kRopeBf16 : kRopeF32;
               // the first factors travel while the norm is computed
-              constexpr int kBatch = 4;
-              uint4 ahead[kBatch];
+              uint4 ahead[2][2];
               if (form == kRopeBf16) {
 #pragma unroll
-                for (int k = 0; k < kBatch; ++k) ahead[k] = __ldg(static_cast<const uint4 *>(rope_row) + 12 * share + k);
+                for (int k = 0; k < 2; ++k) load_sector(ahead[k], static_cast<const uint4 *>(rope_row) + 12 * share + 2 * k, sectors);
               }
               const bool got = ptx::mbar_wait(&sh.squares_ready[gi][quarter], squared & 1u, abort_word, kGemmAbortSquares,
                                               prm.wait_budget_ns);
@@ -905,20 +922,21 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               if (form == kRopeBf16) {
                 const uint4 *table = static_cast<const uint4 *>(rope_row) + 12 * share;
 #pragma unroll
-                for (int k = 0; k < 12; ++k) {
-                  const uint4 now = ahead[k % kBatch];
-                  if (k + kBatch < 12) ahead[k % kBatch] = __ldg(table + k + kBatch);
-                  rotate_bf16(y.first[k], y.second[k], now);
+                for (int k = 0; k < 6; ++k) {
+                  const uint4 now[2] = {ahead[k & 1][0], ahead[k & 1][1]};
+                  if (k + 2 < 6) load_sector(ahead[k & 1], table + 2 * (k + 2), sectors);
+                  rotate_bf16(y.first[2 * k], y.second[2 * k], now[0]);
+                  rotate_bf16(y.first[2 * k + 1], y.second[2 * k + 1], now[1]);
                 }
               } else if (form == kRopeF32) {
-                const float4 *table = static_cast<const float4 *>(rope_row) + 24 * share;
+                const uint4 *table = static_cast<const uint4 *>(rope_row) + 24 * share;
 #pragma unroll
                 for (int b = 0; b < 12; b += 4) {
-                  float4 now[8];
+                  uint4 now[4][2];
 #pragma unroll
-                  for (int k = 0; k < 8; ++k) now[k] = __ldg(table + 2 * b + k);
+                  for (int k = 0; k < 4; ++k) load_sector(now[k], table + 2 * (b + k), sectors);
 #pragma unroll
-                  for (int k = 0; k < 4; ++k) rotate_f32(y.first[b + k], y.second[b + k], now[2 * k], now[2 * k + 1]);
+                  for (int k = 0; k < 4; ++k) rotate_f32(y.first[b + k], y.second[b + k], now[k][0], now[k][1]);
                 }
               } else if (form == kRopeStrided) {
                 uint32_t pairs[24];
@@ -1029,10 +1047,19 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           // channel g of this head, row half `share`: totals over the eight warps
           const int g = t & (H3S_HEAD_DIM - 1);
           auto total = [&](int h) {
-            double sum = 0.0;
+            PairSum sum = {ex.column[h][0][g], 0.f};
 #pragma unroll
-            for (int w = 0; w < 8; ++w) sum += static_cast<double>(ex.column[h][w][g]);
+            for (int w = 1; w < 8; ++w) sum = add_pairs(sum, {ex.column[h][w][g], 0.f});
             return sum;
+          };
+          // the mean over `rows` rows; a power of two divides both floats exactly, and their sum is rounded once
+          auto store_mean = [&](void *base, int64_t at, const PairSum &sum, int rows, int whole) {
+            if (rows == whole && prm.summary_dtype == H3S_F32 && fabsf(sum.hi) < 1e30f) {
+              const float part = 1.0f / static_cast<float>(whole);
+              static_cast<float *>(base)[at] = __fadd_rn(__fmul_rn(sum.hi, part), __fmul_rn(sum.lo, part));
+            } else {
+              store_summary(base, prm.summary_dtype, at, wide(sum) / rows);
+            }
           };
           if (kind == 0) {
             const int blocks_total = (prm.sequence_total + H3S_Q_TILE - 1) / H3S_Q_TILE;
@@ -1040,8 +1067,8 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             const float scale = __fadd_rn(__fdiv_rn(fmaxf(amax_half[0], amax_half[1]), 127.0f), 1.0e-7f);
             if (t == 0) prm.q_scale[head * blocks_total + block] = scale;
             if (share == 0)
-              store_summary(prm.q_summary, prm.summary_dtype,
-                            (static_cast<int64_t>(head) * blocks_total + block) * H3S_HEAD_DIM + g, (total(0) + total(1)) / valid);
+              store_mean(prm.q_summary, (static_cast<int64_t>(head) * blocks_total + block) * H3S_HEAD_DIM + g,
+                         add_pairs(total(0), total(1)), valid, H3S_Q_TILE);
             int8_t *dst = prm.q8 + (static_cast<int64_t>(head) * prm.sequence_total + tile_row0) * H3S_HEAD_DIM + c * 8;
             const SharedDivisor by_scale = make_divisor(scale);
             auto emit = [&](auto exact) {
@@ -1055,11 +1082,11 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           } else if (kind == 1) {
             const int blocks_total = (prm.sequence_total + H3S_KV_TILE - 1) / H3S_KV_TILE;
             const int block0 = tile_row0 / H3S_KV_TILE;
-            const double sum = total(share);
+            const PairSum sum = total(share);
             if (valid_half[share] > 0) {
-              store_summary(prm.k_summary, prm.summary_dtype,
-                            (static_cast<int64_t>(head) * blocks_total + block0 + share) * H3S_HEAD_DIM + g, sum / valid_half[share]);
-              if (prm.k_sum != nullptr) atomicAdd(prm.k_sum + head * H3S_HEAD_DIM + g, sum);
+              store_mean(prm.k_summary, (static_cast<int64_t>(head) * blocks_total + block0 + share) * H3S_HEAD_DIM + g, sum,
+                         valid_half[share], H3S_KV_TILE);
+              if (prm.k_sum != nullptr) atomicAdd(prm.k_sum + head * H3S_HEAD_DIM + g, wide(sum));
             }
             if (prm.k8 != nullptr) {
               int8_t *dst = prm.k8 + (static_cast<int64_t>(head) * prm.sequence_total + tile_row0) * H3S_HEAD_DIM + c * 8;
