@@ -1,25 +1,23 @@
 // Block router: exact FP64 tile-mean scores, per-row radix top-k, ordered
 // emission of the packed KV-tile index list.
 //
-// One CTA scores 8 pure-video query tiles of one head against every
+// One CTA scores 16 (or 8) pure-video query tiles of one head against every
 // pure-video KV tile with FP64 tensor-core MMAs (scores kept in shared
 // memory).  The K tile means are brought in 64 tiles at a time by the whole
-// CTA with coalesced loads (every thread has 32 independent loads in flight)
+// CTA with coalesced loads, one block ahead of the MMAs,
 // and widened to FP64 in shared memory; the MMA operands are then read from
 // there.  Each warp then owns one row: an 8-pass MSB-first radix select on
 // order-preserving 64-bit keys finds the retained-th largest score exactly,
 // and a ballot-ordered sweep writes the surviving tile indices in ascending
 // order, so no sort is needed.
-// It is latency bound (2.6 waves of 106 KB CTAs at 24 x 256 rows of 512 scores, one at 3
-// heads): four MMA chains and leaving the selection after the last digit that decides took
-// these from 156 to 139 and from 53 to 48 us.
+// It is bound by those reads, which go through L2, where there are many CTAs, and by latency where there are
+// few: 24 x 256 rows of 512 scores 85 us, 24 x 591 of 1181 370 us (98 and 685 with eight rows a CTA and no
+// block ahead; the latter then have one CTA of eight warps an SM), 3 x 256 of 512 29 us.
 #include "common.cuh"
 
 namespace h3s {
 
-constexpr int kRouteRows = 8;         // query tiles per CTA == warps per CTA
-constexpr int kRouteThreads = kRouteRows * 32;
-constexpr int kRouteKBlock = 64;       // KV tiles staged per round: one 8-tile MMA block per warp
+constexpr int kRouteKBlock = 64;       // KV tiles staged per round: one 8-tile MMA block for each of eight warps
 // Row stride of the staged block in doubles: 128 channels + 4 of padding, so the
 // 16 lanes of a half warp (4 tiles x 4 channels) read 16 different 8-byte banks.
 constexpr int kRouteKStride = H3S_HEAD_DIM + 4;
@@ -36,53 +34,62 @@ __device__ __forceinline__ unsigned long long score_key(double s) {
   return (bits >> 63) ? ~bits : (bits | 0x8000000000000000ull);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kRouteThreads)
+// kRows query tiles per CTA, as many warps
+template <typename T, int kRows>
+__global__ void __launch_bounds__(kRows * 32)
 route_topk_kernel(const T *__restrict__ q_summary, const T *__restrict__ k_summary, int q_tiles,
                   int kv_tiles, int q_start, int q_stop, int kv_start, int kv_stop, int retained,
                   int route_len, int32_t *__restrict__ route) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int pure_q = q_stop - q_start;
   const int pure_kv = kv_stop - kv_start;
-  double *scores = reinterpret_cast<double *>(smem_raw);                                     // [kRouteRows][pure_kv]
-  double *k_block = scores + static_cast<size_t>(kRouteRows) * pure_kv;                     // [kRouteKBlock][kRouteKStride]
-  int *hist = reinterpret_cast<int *>(k_block + kRouteKBlock * kRouteKStride);              // [rows][256]
+  double *scores = reinterpret_cast<double *>(smem_raw);              // [kRows][pure_kv]
+  double *k_block = scores + static_cast<size_t>(kRows) * pure_kv;    // [kRouteKBlock][kRouteKStride]
+  int *hist = reinterpret_cast<int *>(k_block);                       // [kRows][256], when the scores are complete
+  static_assert(kRows * 256 * sizeof(int) <= kRouteKBlock * kRouteKStride * sizeof(double), "histograms");
 
   const int head = blockIdx.y;
-  const int row0 = blockIdx.x * kRouteRows;
+  const int row0 = blockIdx.x * kRows;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
   // ---- scores[r][p] = <q[r], k[p]> in FP64 on the tensor cores ----
-  // mma.m8n8k4.f64: A is the CTA's 8 query tiles x 4 channels, B 4 channels x 8
+  // mma.m8n8k4.f64: A is 8 query tiles x 4 channels, B 4 channels x 8
   // KV tiles; lane l holds A[l/4][l%4], B[l%4][l/4] and C[l/4][2*(l%4) + {0,1}].
   // The 32 A fragments of a lane (all 128 channels) stay in registers.
   {
     const int frag_row = lane >> 2, frag_k = lane & 3;
-    const int a_row = min(row0 + frag_row, pure_q - 1);
+    const int rows8 = warp >> 3, tiles8 = warp & 7;  // this warp's eight query tiles, and eight KV tiles of a block
+    const int a_row = min(row0 + 8 * rows8 + frag_row, pure_q - 1);
     const T *qp = q_summary + (static_cast<int64_t>(head) * q_tiles + q_start + a_row) * H3S_HEAD_DIM + frag_k;
     double a[H3S_HEAD_DIM / 4];
 #pragma unroll
     for (int kk = 0; kk < H3S_HEAD_DIM / 4; ++kk) a[kk] = to_double(qp[4 * kk]);
     const T *k_head = k_summary + (static_cast<int64_t>(head) * kv_tiles + kv_start) * H3S_HEAD_DIM;
-    for (int base = 0; base < pure_kv; base += kRouteKBlock) {
-      // stage tiles [base, base + 64): element e of the block is channel e % 128 of tile e / 128
-      constexpr int kPerThread = kRouteKBlock * H3S_HEAD_DIM / kRouteThreads;  // 32
-      T staged[kPerThread];
+    // element e of a block is channel e % 128 of its tile e / 128
+    constexpr int kPerThread = kRouteKBlock * H3S_HEAD_DIM / (kRows * 32);
+    T ahead[kPerThread];
+    auto fetch = [&](int base) {
 #pragma unroll
       for (int i = 0; i < kPerThread; ++i) {
-        const int e = i * kRouteThreads + threadIdx.x;
+        const int e = i * kRows * 32 + threadIdx.x;
         const int tile = min(base + (e >> 7), pure_kv - 1);  // rows past the end repeat the last tile
-        staged[i] = k_head[static_cast<int64_t>(tile) * H3S_HEAD_DIM + (e & 127)];
+        ahead[i] = k_head[static_cast<int64_t>(tile) * H3S_HEAD_DIM + (e & 127)];
       }
+    };
+    constexpr bool kAhead = kRows == 16;  // eight rows: two CTAs an SM instead, which leaves no registers for it
+    if (kAhead) fetch(0);
+    for (int base = 0; base < pure_kv; base += kRouteKBlock) {
+      if (!kAhead) fetch(base);
       __syncthreads();  // the previous round's readers are done with k_block
 #pragma unroll
       for (int i = 0; i < kPerThread; ++i) {
-        const int e = i * kRouteThreads + threadIdx.x;
-        k_block[(e >> 7) * kRouteKStride + (e & 127)] = to_double(staged[i]);
+        const int e = i * kRows * 32 + threadIdx.x;
+        k_block[(e >> 7) * kRouteKStride + (e & 127)] = to_double(ahead[i]);
       }
       __syncthreads();
-      const double *kp = k_block + (8 * warp + frag_row) * kRouteKStride + frag_k;
+      if (kAhead && base + kRouteKBlock < pure_kv) fetch(base + kRouteKBlock);
+      const double *kp = k_block + (8 * tiles8 + frag_row) * kRouteKStride + frag_k;
       // four chains of eight instead of one of 32: an FP64 MMA waits for its accumulator
       double c[4][2];
 #pragma unroll
@@ -95,9 +102,10 @@ route_topk_kernel(const T *__restrict__ q_summary, const T *__restrict__ k_summa
                      : "d"(a[kk]), "d"(b));
       }
       const double c0 = (c[0][0] + c[1][0]) + (c[2][0] + c[3][0]), c1 = (c[0][1] + c[1][1]) + (c[2][1] + c[3][1]);
-      const int col = base + 8 * warp + 2 * frag_k;
-      if (col < pure_kv) scores[static_cast<size_t>(frag_row) * pure_kv + col] = c0;
-      if (col + 1 < pure_kv) scores[static_cast<size_t>(frag_row) * pure_kv + col + 1] = c1;
+      const int col = base + 8 * tiles8 + 2 * frag_k;
+      double *to = scores + static_cast<size_t>(8 * rows8 + frag_row) * pure_kv;
+      if (col < pure_kv) to[col] = c0;
+      if (col + 1 < pure_kv) to[col + 1] = c1;
     }
   }
   __syncthreads();
@@ -191,21 +199,40 @@ __global__ void route_to_delta_lut_kernel(const int32_t *__restrict__ route, int
   if (threadIdx.x == 0) valid[head * q_tiles + tq] = sparse ? route_len : kv_tiles;
 }
 
-template <typename T>
-static int launch_route(const void *q_summary, const void *k_summary, int heads, int q_tiles, int kv_tiles,
-                        int q_start, int q_stop, int kv_start, int kv_stop, int retained, int route_len,
-                        int32_t *route, cudaStream_t stream) {
-  const int pure_q = q_stop - q_start, pure_kv = kv_stop - kv_start;
-  const size_t smem = sizeof(double) * (static_cast<size_t>(kRouteRows) * pure_kv + kRouteKBlock * kRouteKStride) +
-                      sizeof(int) * kRouteRows * 256;
-  H3S_CHECK_ARG(smem <= 220 * 1024, "route_topk: %d pure-video KV tiles need %zu bytes of shared memory", pure_kv, smem);
-  H3S_CHECK_CUDA(cudaFuncSetAttribute(route_topk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  dim3 grid(ceil_div(pure_q, kRouteRows), heads);
-  route_topk_kernel<T><<<grid, kRouteThreads, smem, stream>>>(
+constexpr size_t route_smem(int rows, int pure_kv) {
+  return sizeof(double) * (static_cast<size_t>(rows) * pure_kv + kRouteKBlock * kRouteKStride);
+}
+
+template <typename T, int kRows>
+static int launch_route_rows(const void *q_summary, const void *k_summary, int heads, int q_tiles, int kv_tiles,
+                             int q_start, int q_stop, int kv_start, int kv_stop, int retained, int route_len,
+                             int32_t *route, cudaStream_t stream) {
+  const size_t smem = route_smem(kRows, kv_stop - kv_start);
+  H3S_CHECK_CUDA(cudaFuncSetAttribute(route_topk_kernel<T, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  dim3 grid(ceil_div(q_stop - q_start, kRows), heads);
+  route_topk_kernel<T, kRows><<<grid, kRows * 32, smem, stream>>>(
       static_cast<const T *>(q_summary), static_cast<const T *>(k_summary), q_tiles, kv_tiles, q_start,
       q_stop, kv_start, kv_stop, retained, route_len, route);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
+}
+
+// Sixteen rows where eight make more CTAs than run at once, two on each of 148 SMs: every CTA reads all K tile
+// means of its head (393 MB in all at 24 x 256 rows of 512 scores, 98 us; 85 with half of that).  Fewer
+// CTAs wait for their own chain, which is shorter with eight rows (3 x 256 rows 28.8 us, 30.4 with sixteen).  From 1233
+// pure-video KV tiles on, sixteen rows of scores do not fit beside a block.
+template <typename T>
+static int launch_route(const void *q_summary, const void *k_summary, int heads, int q_tiles, int kv_tiles,
+                        int q_start, int q_stop, int kv_start, int kv_stop, int retained, int route_len,
+                        int32_t *route, cudaStream_t stream) {
+  const int pure_kv = kv_stop - kv_start;
+  constexpr size_t kMost = 220 * 1024;
+  const size_t least = route_smem(8, pure_kv) + sizeof(int) * 8 * 256;
+  H3S_CHECK_ARG(least <= kMost, "route_topk: %d pure-video KV tiles need %zu bytes of shared memory", pure_kv, least);
+  const int64_t ctas = static_cast<int64_t>(heads) * ceil_div(q_stop - q_start, 8);
+  if (ctas > 2 * 148 && route_smem(16, pure_kv) <= kMost)
+    return launch_route_rows<T, 16>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
+  return launch_route_rows<T, 8>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
 }
 
 }  // namespace h3s
