@@ -369,7 +369,7 @@ def workload_name(spec, budget):
 # 30 % workload: dram__bytes_read.sum + dram__bytes_write.sum of the ncu capture
 # summarised in profiles/sparse_attn_half_kernel_4heads.md (4 heads), divided
 # by 4; the traffic grows in proportion to the heads of a launch.
-ATTN_DRAM_BYTES_PER_HEAD = (72.0e6 + 13.1e6) / 4
+ATTN_DRAM_BYTES_PER_HEAD = (78.3e6 + 15.5e6) / 4
 # Bytes an element of Q, K and V leaves in the carriers: INT8 Q and K, E4M3 V and its FP16 copy.
 CARRIER_BYTES = 1 + 1 + 1 + 2
 # Operations at the 8-bit rate (QK^T, twice the 16-bit one) and at the 16-bit rate (P.V), half each.
