@@ -384,7 +384,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int head = work.head;
         for (int i = 0; i < tiles; ++i) {
           const int t = block[i];
-          fine = ptx::mbar_wait(&empty[stage], round, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
+          fine = ptx::mbar_wait(&empty[stage], round, abort_word, kAbortKvEmpty, 4 * prm.wait_budget_ns);
           if (!fine) break;
           if (!drop) {
             ptx::mbar_arrive_expect_tx(&full[stage], bytes);
