@@ -917,7 +917,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               ++squared;
               const float2 theirs = ex.squares[1 - share][local_row];
               const PairSum squares = add_pairs(mine, {theirs.x, theirs.y});
-              norm_half_row(y, __fadd_rn(squares.hi, squares.lo), group < prm.heads ? prm.q_norm : prm.k_norm,
+              norm_half_row(y, squares.hi < INFINITY ? __fadd_rn(squares.hi, squares.lo) : squares.hi, group < prm.heads ? prm.q_norm : prm.k_norm,
                             prm.epsilon, share);
               if (form == kRopeBf16) {
                 const uint4 *table = static_cast<const uint4 *>(rope_row) + 12 * share;
@@ -1054,7 +1054,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           };
           // the mean over `rows` rows; a power of two divides both floats exactly, and their sum is rounded once
           auto store_mean = [&](void *base, int64_t at, const PairSum &sum, int rows, int whole) {
-            if (rows == whole && prm.summary_dtype == H3S_F32 && fabsf(sum.hi) < 1e30f) {
+            if (rows == whole && prm.summary_dtype == H3S_F32 && fabsf(sum.hi) < 1e30f && (fabsf(sum.hi) > 1e-30f || sum.hi == 0.f)) {
               const float part = 1.0f / static_cast<float>(whole);
               static_cast<float *>(base)[at] = __fadd_rn(__fmul_rn(sum.hi, part), __fmul_rn(sum.lo, part));
             } else {

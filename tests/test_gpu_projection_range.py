@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 def test_codes_of_heads_of_all_sizes(native_lib, epsilon):
     from h3_optimizations_b200 import ChunkedSparseQKVProjector
 
-    sizes = (1.0, 0.0, 1e-13, 1e-11, 1e16, 1e18)
+    sizes = (1.0, 0.0, 1e-13, 1e-11, 1e16, 1e18, 1e20)  # the last one's sum is infinite
     heads, hidden, rows = len(sizes), 512, 300
     x, w, w_scale = workloads.projection_inputs(rows, hidden=hidden, heads=heads, seed=11)
     w_scale = w_scale * torch.tensor(sizes).repeat_interleave(128).repeat(3)
