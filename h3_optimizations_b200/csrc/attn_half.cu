@@ -574,7 +574,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     auto room = [&](uint32_t j) {
       return warp_wait(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
     };
-    auto put = [&](const uint32_t (&packed)[H3S_KV_TILE / 2]) { H3S_TMEM_ST32(tmem_p, packed); };
+    // behind `room`: the fence orders the store after P.V's reads of the same columns
+    auto put = [&](const uint32_t (&packed)[H3S_KV_TILE / 2]) {
+      ptx::tc_fence_after();
+      H3S_TMEM_ST32(tmem_p, packed);
+    };
     auto hand_over = [&]() {
       ptx::tmem_wait_st();
       ptx::tc_fence_before();
