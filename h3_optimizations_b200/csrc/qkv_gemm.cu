@@ -175,11 +175,19 @@ constexpr uint32_t kGemmABytes = kGemmM * kGemmK;  // 16384
 constexpr uint32_t kGemmBBytes = kGemmN / 2 * kGemmK;  // 16384: this CTA's half
 constexpr uint32_t kGemmTmemCols = 512;
 
+// A sum as an unevaluated triple of floats: `sum`, what rounding has taken from it, and what rounding has taken from
+// that.  Of n floats it is off by about n^2 * 2^-72 of the largest intermediate sum, where a 64-bit sum is off by
+// n * 2^-53; sums beyond the range of a float become infinite or NaN.  Against totals kept as pairs of floats (46 bits) the
+// projection of 33272 x 3072 with norm and table takes 1.07 ms for 1.06; in 64 bits it was 1.14 for 1.03 without them.
+struct TripleSum {
+  float sum, lost, rest;
+};
+
 // What the eight warps of one 128-column half of a tile tell each other in the carrier
 // epilogue: the sums of squares of a row's two shares of channels, then per-warp largest
 // magnitudes and per-channel partial sums (maxima for V) of the rows 0-63 and 64-127 of the tile.
 struct EpilogueExchange {
-  float2 squares[2][kGemmM];         // [channel share][row], PairSum
+  TripleSum squares[2][kGemmM];      // [channel share][row]
   float amax[2][8];                  // [row half][warp]
   float column[2][8][H3S_HEAD_DIM];  // [row half][warp][channel]
 };
@@ -478,26 +486,6 @@ struct HalfRow {
   uint32_t first[12], second[12], rest[8];
 };
 
-// A sum as an unevaluated pair of floats, good to about 46 bits
-struct PairSum {
-  float hi, lo;
-};
-
-// a + b exactly (Knuth's two-sum), the small parts added up
-__device__ __forceinline__ PairSum add_pairs(const PairSum &a, const PairSum &b) {
-  const float s = __fadd_rn(a.hi, b.hi), back = __fsub_rn(s, a.hi);
-  const float error = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, back)), __fsub_rn(b.hi, back));
-  return {s, __fadd_rn(error, __fadd_rn(a.lo, b.lo))};
-}
-
-// A sum as an unevaluated triple of floats: `sum`, what rounding has taken from it, and what rounding has taken from
-// that.  Of n floats it is off by about n^2 * 2^-72 of the largest intermediate sum, where a 64-bit sum is off by
-// n * 2^-53; sums beyond the range of a float become infinite or NaN.  Against totals kept as pairs of floats (46 bits) the
-// projection of 33272 x 3072 with norm and table takes 1.07 ms for 1.06; in 64 bits it was 1.14 for 1.03 without them.
-struct TripleSum {
-  float sum, lost, rest;
-};
-
 // sum + x = the result + error, exactly (Knuth's two-sum)
 __device__ __forceinline__ float two_sum(float a, float b, float &error) {
   const float s = __fadd_rn(a, b), back = __fsub_rn(s, a);
@@ -510,6 +498,13 @@ __device__ __forceinline__ void add_to(TripleSum &a, float x) {
   a.sum = two_sum(a.sum, x, e);
   a.lost = two_sum(a.lost, e, f);
   a.rest = __fadd_rn(a.rest, f);
+}
+
+__device__ __forceinline__ TripleSum add_sums(const TripleSum &a, const TripleSum &b) {  // the same in either order
+  float e, f, g;
+  const float sum = two_sum(a.sum, b.sum, e);
+  const float lost = two_sum(two_sum(a.lost, b.lost, f), e, g);
+  return {sum, lost, __fadd_rn(__fadd_rn(a.rest, b.rest), __fadd_rn(f, g))};
 }
 
 // The nearest float: sum + lost = t + r exactly, and r + rest is rounded to odd, which keeps the last
@@ -535,8 +530,18 @@ __device__ __noinline__ double wide_total(const float *partial, int parts, int s
   return sum;
 }
 
-// Rows whose squares leave the range in which every step below is exact
-__device__ __noinline__ PairSum square_sum_wide(const uint32_t *row) {
+__device__ __forceinline__ TripleSum split_wide(double sum) {
+  const float hi = static_cast<float>(sum);
+  if (!(hi < INFINITY)) return {hi, 0.f, 0.f};
+  const float lo = static_cast<float>(sum - static_cast<double>(hi));
+  return {hi, lo, static_cast<float>(sum - static_cast<double>(hi) - static_cast<double>(lo))};
+}
+
+// Half rows whose squares leave the range in which every step below is exact.  Sums that are too small for that
+// are handed on times -2^160.
+constexpr double kTinySquares = 0x1p160;
+
+__device__ __noinline__ TripleSum square_sum_wide(const uint32_t *row, bool tiny) {
   double sum = 0.0;
 #pragma unroll 1
   for (int i = 0; i < 32; ++i) {
@@ -544,15 +549,23 @@ __device__ __noinline__ PairSum square_sum_wide(const uint32_t *row) {
     sum = fma(lo, lo, sum);
     sum = fma(hi, hi, sum);
   }
-  const float hi = static_cast<float>(sum);
-  return {hi, hi < INFINITY ? static_cast<float>(sum - static_cast<double>(hi)) : 0.f};
+  const TripleSum split = split_wide(tiny ? sum * kTinySquares : sum);
+  return tiny ? TripleSum{-split.sum, -split.lost, -split.rest} : split;
 }
 
-// The sum of squares of half a row, as good as in 64 bits and without its unit, which took 2000 to 6000 cycles a tile
-// here and 30000 for a CTA's first.  The square of a bf16 value is exact in fp32.  The accumulator begins at a power
-// of two that no square exceeds, so that acc + p - acc loses exactly what rounding took from p (Dekker's
-// fast two-sum, which wants the larger operand first); the losses are added up beside it.
-__device__ __forceinline__ PairSum half_row_squares(const HalfRow &y) {
+__device__ __noinline__ float add_tiny_squares(const TripleSum &a, const TripleSum &b) {
+  const double x = a.sum < 0.f ? wide(a) / -kTinySquares : wide(a), y = b.sum < 0.f ? wide(b) / -kTinySquares : wide(b);
+  return static_cast<float>(x + y);
+}
+
+// The sum of squares of half a row, as good as in 64 bits (it keeps at least 56) and without its unit, which took 2000 to
+// 6000 cycles a tile here and 30000 for a CTA's first.  The square of a bf16 value is exact in fp32.  The accumulator begins at a
+// power of two that no square exceeds, so that acc + p - acc loses exactly what rounding took from p (Dekker's
+// fast two-sum, which wants the larger operand first).  With base = 2^b the accumulator stays below 2^(b+5) and a loss
+// below 2^(b-20); the losses have an accumulator of their own that begins at 2^(b-14), and what that one loses, at most
+// 2^(b-38) at a time, is added up beside it.  With plain sums of the losses a row with one outlier kept 42 bits; the
+// projection of 33272 x 3072 with norm and table took 1.06 ms then, 1.10 now, 1.52 in 64 bits.
+__device__ __forceinline__ TripleSum half_row_squares(const HalfRow &y) {
   __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
   auto magnitude = [&](uint32_t w) {
     w &= 0x7fff7fffu;
@@ -565,33 +578,39 @@ __device__ __forceinline__ PairSum half_row_squares(const HalfRow &y) {
   const uint32_t bits = *reinterpret_cast<const uint32_t *>(&top);
   const float lo_top = bf16_lo(bits), hi_top = bf16_hi(bits);
   const float most = fmaxf(lo_top, hi_top);
-  if (!(lo_top < 1e17f && hi_top < 1e17f) || (most < 1e-12f && most > 0.f)) {
+  const bool tiny = most < 1e-12f && most > 0.f && lo_top < 1e-12f && hi_top < 1e-12f;  // (a NaN is not)
+  if (!(lo_top < 1e17f && hi_top < 1e17f) || tiny) {
     uint32_t row[32];
 #pragma unroll
     for (int i = 0; i < 12; ++i) { row[i] = y.first[i]; row[12 + i] = y.second[i]; }
 #pragma unroll
     for (int i = 0; i < 8; ++i) row[24 + i] = y.rest[i];
-    return square_sum_wide(row);
+    return square_sum_wide(row, tiny);
   }
   // the next power of two above the largest square
   const float base = __uint_as_float((__float_as_uint(__fmul_rn(most, most)) & 0x7f800000u) + 0x00800000u);
+  const float lost_base = __fmul_rn(base, 0x1p-14f);
   const float2 minus = make_float2(-1.f, -1.f);
   float2 acc[2] = {make_float2(base, base), make_float2(base, base)};
-  float2 lost[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  float2 lost[2] = {make_float2(lost_base, lost_base), make_float2(lost_base, lost_base)};
+  float2 rest[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
   auto square = [&](uint32_t w, int i) {
+    float2 &a = acc[i & 1], &l = lost[i & 1], &r = rest[i & 1];
     const float2 v = bf16_pair(w);
-    const float2 p = mul2(v, v), next = add2(acc[i & 1], p);
-    const float2 taken = fma2(acc[i & 1], minus, next);   // next - acc
-    lost[i & 1] = add2(lost[i & 1], fma2(taken, minus, p));  // p - taken
-    acc[i & 1] = next;
+    const float2 next = fma2(v, v, a);
+    const float2 loss = fma2(v, v, fma2(next, minus, a));  // v * v - (next - a)
+    const float2 after = add2(l, loss);
+    r = add2(r, add2(loss, fma2(after, minus, l)));  // loss - (after - l)
+    a = next;
+    l = after;
   };
 #pragma unroll
   for (int i = 0; i < 12; ++i) { square(y.first[i], i); square(y.second[i], i + 1); }
 #pragma unroll
   for (int i = 0; i < 8; ++i) square(y.rest[i], i);
-  const PairSum a = add_pairs({__fsub_rn(acc[0].x, base), lost[0].x}, {__fsub_rn(acc[0].y, base), lost[0].y});
-  const PairSum b = add_pairs({__fsub_rn(acc[1].x, base), lost[1].x}, {__fsub_rn(acc[1].y, base), lost[1].y});
-  return add_pairs(a, b);
+  auto sum = [&](float a, float l, float r) { return TripleSum{__fsub_rn(a, base), __fsub_rn(l, lost_base), r}; };  // exact
+  return add_sums(add_sums(sum(acc[0].x, lost[0].x, rest[0].x), sum(acc[0].y, lost[0].y, rest[0].y)),
+                  add_sums(sum(acc[1].x, lost[1].x, rest[1].x), sum(acc[1].y, lost[1].y, rest[1].y)));
 }
 
 __device__ __forceinline__ uint32_t norm_pair(uint32_t y, float2 inverse_rms, const float *__restrict__ weight) {
@@ -929,8 +948,8 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             if (lane == 0) ptx::mbar_arrive_cluster(acc_empty[a]);
             if (!group_ok) continue;  // the same for the eight warps of this half
             if (normed) {
-              const PairSum mine = half_row_squares(y);
-              ex.squares[share][local_row] = make_float2(mine.hi, mine.lo);
+              const TripleSum mine = half_row_squares(y);
+              ex.squares[share][local_row] = mine;
               __syncwarp();
               if (lane == 0) ptx::mbar_arrive(&sh.squares_ready[gi][quarter]);
               const void *rope_row = nullptr;
@@ -956,10 +975,15 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                               prm.wait_budget_ns);
               if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
               ++squared;
-              const float2 theirs = ex.squares[1 - share][local_row];
-              const PairSum squares = add_pairs(mine, {theirs.x, theirs.y});
-              norm_half_row(y, squares.hi < INFINITY ? __fadd_rn(squares.hi, squares.lo) : squares.hi, group < prm.heads ? prm.q_norm : prm.k_norm,
-                            prm.epsilon, share);
+              const TripleSum theirs = ex.squares[1 - share][local_row];
+              float squares;
+              if (mine.sum < 0.f || theirs.sum < 0.f) {
+                squares = add_tiny_squares(mine, theirs);
+              } else {
+                const TripleSum both = add_sums(mine, theirs);
+                squares = both.sum < INFINITY ? nearest(both) : both.sum;  // infinite: nothing is left to correct
+              }
+              norm_half_row(y, squares, group < prm.heads ? prm.q_norm : prm.k_norm, prm.epsilon, share);
               if (form == kRopeBf16) {
                 const uint4 *table = static_cast<const uint4 *>(rope_row) + 12 * share;
 #pragma unroll

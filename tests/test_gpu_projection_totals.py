@@ -31,8 +31,9 @@ def _project(native_lib, weight, row_scale, summary_dtype, smooth_k):
     return {name: t.cpu() for name, t in out.items()}
 
 
-def _means(values, tile):
-    return torch.stack([piece.sum(0) / piece.shape[0] for piece in values.split(tile)])
+def _totals(weight, exponent, tile):
+    """Exact in 64 bits: the sum of a tile's scales first, then the weight."""
+    return torch.stack([(2.0 ** e.double()).sum() * weight.double() for e in exponent.split(tile)])
 
 
 @pytest.mark.parametrize("summary_dtype", [torch.float64, torch.float32, torch.bfloat16])
@@ -56,11 +57,10 @@ def test_totals_of_exact_partial_sums_are_exact(native_lib, smooth_k):
     weight = (torch.randint(-64, 64, (384,), generator=gen) * 2 + 1).to(torch.int8)
     exponent = torch.tensor([24.0, 2.0, -12.0, -19.0]).repeat_interleave(2).repeat(24)      # of row r: by (r % 8) // 2
     got = _project(native_lib, weight, 2.0 ** exponent, torch.float64, smooth_k)
-    values = weight.double()[None, :] * (2.0 ** exponent.double())[:, None]
-    assert torch.equal(got["q_summary"][0, 0], _means(values[:, :128], 128))
-    assert torch.equal(got["k_summary"][0, 0], _means(values[:, 128:256], 64))
+    assert torch.equal(got["q_summary"][0, 0], _totals(weight[:128], exponent, 128) / torch.tensor([[128.0], [64.0]]))
+    assert torch.equal(got["k_summary"][0, 0], _totals(weight[128:256], exponent, 64) / 64)
     if smooth_k:
-        assert torch.equal(got["stats"].view(torch.float64)[:128], values[:, 128:256].sum(0))
+        assert torch.equal(got["stats"].view(torch.float64)[:128], _totals(weight[128:256], exponent, 192)[0])
 
 
 def test_means_in_fp32_are_the_nearest(native_lib):
@@ -70,6 +70,5 @@ def test_means_in_fp32_are_the_nearest(native_lib):
     for exponents in ([24.0, 2.0, -12.0, -19.0], [0.0, -16.0, -16.0, -41.0], [0.0, -17.0, -25.0, -40.0]):
         exponent = torch.tensor(exponents).repeat_interleave(2).repeat(24)
         got = _project(native_lib, weight, 2.0 ** exponent, torch.float32, False)
-        values = weight.double()[None, :] * (2.0 ** exponent.double())[:, None]
-        assert torch.equal(got["q_summary"][0, 0], _means(values[:, :128], 128).float())
-        assert torch.equal(got["k_summary"][0, 0], _means(values[:, 128:256], 64).float())
+        assert torch.equal(got["q_summary"][0, 0], (_totals(weight[:128], exponent, 128) / torch.tensor([[128.0], [64.0]])).float())
+        assert torch.equal(got["k_summary"][0, 0], (_totals(weight[128:256], exponent, 64) / 64).float())
