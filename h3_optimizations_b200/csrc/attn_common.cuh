@@ -24,10 +24,9 @@ struct AttnParams {
   int32_t *status;
   int64_t out_stride_h, out_stride_s;
   int route_len, q_start, q_stop;
-  // A dense row's tile list may be cut into `parts` parts of `part_tiles` tiles, one CTA each (attn_half.cu);
-  // 1: not cut.  partial: per dense row and part 128 x 128 sums of P.V, 128 row sums and 128 reference points;
+  // A dense row's tile list may be cut into `parts` even parts, an item each (attn_half.cu); 1: not cut.  partial: per dense row and part 128 x 128 sums of P.V, 128 row sums and 128 reference points;
   // arrived: per dense row the number of parts that are in, zero at launch.
-  int parts, part_tiles;
+  int parts;
   float *partial;
   unsigned int *arrived;
   int heads, sequence, q_tiles, kv_tiles;

@@ -55,9 +55,8 @@
 // A CTA that is nearly through with an item takes over one that has not started (clusterlaunchcontrol), the long
 // ones first; the next item's Q, scales and first tile indices are fetched under the last tiles of this one.
 //
-// Dense rows (query tiles that see every key) are cut into parts where one of them is
-// longer than half of what an SM gets on average, i.e. where a few long rows would outlast
-// all others: see split_dense_rows.  Each part is an item with its own reference point; it
+// Dense rows (query tiles that see every key) are cut into parts where they would outlast
+// all others by more than the parts cost: see split_dense_rows.  Each part is an item with its own reference point; it
 // leaves its sums in memory and the part that comes last adds them up, in the order of
 // the list, so that the result does not depend on which one that was.
 //
@@ -217,8 +216,8 @@ __device__ __forceinline__ HalfWork work_item(const AttnParams &prm, int w) {
     it.head = it.dense_row / n_dense;
     const int i = it.dense_row - it.head * n_dense;
     it.tq = (n_sparse == 0 || i < prm.q_start) ? i : prm.q_stop + (i - prm.q_start);
-    it.first_tile = it.part * prm.part_tiles;
-    it.n_iter = min(prm.part_tiles, prm.kv_tiles - it.first_tile);
+    it.first_tile = it.part * prm.kv_tiles / prm.parts;  // even parts
+    it.n_iter = (it.part + 1) * prm.kv_tiles / prm.parts - it.first_tile;
   } else {
     const int v = w - dense_items;
     it.head = v / n_sparse;
@@ -868,24 +867,55 @@ __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v
   v16[2 * i + 1] = e4m3x8_to_half(make_uint2(codes.z, codes.w));
 }
 
-// Whether and how the dense rows' tile lists are cut.  An SM gets `share` tiles on average.  A dense row
-// that is longer ends after everything else has; parts of a quarter of the share even that out.  The line
-// is at half a share: there the parts cost nothing measurable (three heads of 33272 tokens at 30 %, 520
-// tiles of a share of 883: 384 us) and the order "long rows first" fills the SMs by itself further down.  Under 24
-// tiles a part's start and end would show.
-constexpr int kSlots = 148, kMinPartTiles = 24, kMaxParts = 16;
+// Whether and how the dense rows' tile lists are cut.  A row longer than half of what an SM gets on average may end after
+// everything else has, which parts even out; but parts are dear.  Beside its tiles (0.36 us each) a whole list takes an SM
+// about as long as twelve tiles, a part about 27: it writes 66 KB, waits until they are seen, and one of them
+// reads them all back.  So as many parts as end first by this estimate, every SM taking the next item as it gets free, and only if
+//  - that is earlier than with whole rows by more than 3 %, or
+//  - it is no later, and the parts' own cost is under 1 % of the work (three heads of 33272 tokens at 30 %: 376 us either way), or
+//  - nothing but dense rows is there, and dealt out evenly instead of in rounds the parts would end with the rows.
+//    Whole rows are the faster ones at this last line, for all that (3 x 4000: 33 us, 44 in parts).
+// Measured, us, with parts of a quarter of the average share as before / now:
+//   dense   1 x 5000 42 / 28, 1 x 9400 82 / 46, 1 x 33272 424 / 385, 2 x 9000 110 / 62, 3 x 12000 194 / 149, 4 x 9000 162 / 115,
+//           6 x 1545 34 / 18, 12 x 2000 53 / 37; 1 x 20000 190 either way (239 whole), 2 x 1537 20 (17 whole)
+//   routed  24 x 5000 at 10 % 87 / 74, 24 x 2362 at 20 % 56 / 40, 12 x 4540 at 20 % 65 / 51, 1 x 33272 at 10 % 79 / 61 (195 whole)
+constexpr int kMinPartTiles = 6, kMaxParts = 16;
+constexpr int kItemTiles = 12, kPartItemTiles = 27;
 
-static int split_dense_rows(int heads, int q_tiles, int kv_tiles, int n_sparse, int route_len, int *part_tiles) {
-  const int64_t n_dense = q_tiles - n_sparse;
-  const int64_t total = heads * (n_dense * kv_tiles + static_cast<int64_t>(n_sparse) * route_len);
-  *part_tiles = kv_tiles;
-  if (n_dense == 0 || static_cast<int64_t>(kv_tiles) * kSlots * 2 <= total) return 1;
-  int tiles = static_cast<int>(total / (4 * kSlots));
-  if (tiles < kMinPartTiles) tiles = kMinPartTiles;
-  if (tiles < ceil_div(kv_tiles, kMaxParts)) tiles = ceil_div(kv_tiles, kMaxParts);
-  const int parts = ceil_div(kv_tiles, tiles);
-  *part_tiles = ceil_div(kv_tiles, parts);  // even parts; none is empty
-  return ceil_div(kv_tiles, *part_tiles);
+// When the last item ends, in tiles: `dense` ones of `dense_cost` first, then `routed` ones of `routed_cost`
+static int64_t launch_span(int64_t dense, int64_t dense_cost, int64_t routed, int64_t routed_cost) {
+  const int64_t late = dense % kSmCount, early = kSmCount - late;  // SMs that get one dense item more, and the others
+  int64_t early_free = dense / kSmCount * dense_cost, late_free = early_free + dense_cost;
+  int64_t end = late > 0 ? late_free : early_free;
+  while (routed > 0) {
+    const bool first = late == 0 || early_free <= late_free;
+    int64_t &free = first ? early_free : late_free;
+    routed -= first ? early : late;
+    free += routed_cost;
+    if (free > end) end = free;
+  }
+  return end;
+}
+
+static int split_dense_rows(int heads, int q_tiles, int kv_tiles, int n_sparse, int route_len) {
+  const int64_t rows = static_cast<int64_t>(heads) * (q_tiles - n_sparse), routed = static_cast<int64_t>(heads) * n_sparse;
+  if (rows == 0 || static_cast<int64_t>(kv_tiles) * kSmCount * 2 <= rows * kv_tiles + routed * route_len) return 1;
+  const int64_t whole_cost = kv_tiles + kItemTiles, routed_cost = route_len + kItemTiles;
+  const int64_t whole_span = launch_span(rows, whole_cost, routed, routed_cost), whole_work = rows * whole_cost + routed * routed_cost;
+  int best = 1;
+  int64_t best_span = 0, best_work = 0;
+  bool even = false;
+  for (int parts = 2; parts <= kMaxParts && kv_tiles / parts >= kMinPartTiles; ++parts) {
+    const int64_t cost = ceil_div(kv_tiles, parts) + kPartItemTiles, work = rows * parts * cost + routed * routed_cost;
+    const int64_t span = launch_span(rows * parts, cost, routed, routed_cost);
+    if (best == 1 || span < best_span) { best = parts; best_span = span; best_work = work; }
+    const int64_t share = work / kSmCount;
+    even = even || (routed == 0 && 100 * (share > cost ? share : cost) <= 103 * whole_cost);
+  }
+  if (best == 1) return 1;
+  const bool earlier = 100 * best_span < 97 * whole_span;
+  const bool free = best_span <= whole_span && 100 * best_work <= 101 * whole_work;
+  return earlier || free || even ? best : 1;
 }
 
 static size_t split_bytes(int64_t dense_rows, int parts, size_t *arrived_bytes) {
@@ -924,8 +954,7 @@ extern "C" size_t h3s_sparse_attn_half_workspace_bytes(int heads, int sequence, 
   if (heads <= 0 || sequence <= 0) return 0;
   const int q_tiles = ceil_div(sequence, H3S_Q_TILE), kv_tiles = ceil_div(sequence, H3S_KV_TILE);
   const int n_sparse = route_len > 0 ? q_stop - q_start : 0;
-  int part_tiles;
-  const int parts = split_dense_rows(heads, q_tiles, kv_tiles, n_sparse, route_len, &part_tiles);
+  const int parts = split_dense_rows(heads, q_tiles, kv_tiles, n_sparse, route_len);
   size_t arrived_bytes;
   return parts > 1 ? split_bytes(static_cast<int64_t>(heads) * (q_tiles - n_sparse), parts, &arrived_bytes) : 0;
 }
@@ -955,17 +984,16 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
                              H3S_KV_TILE * 2, H3S_HEAD_DIM, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_half_fwd V map");
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  prm.parts = 1; prm.part_tiles = prm.kv_tiles; prm.partial = nullptr; prm.arrived = nullptr;
+  prm.parts = 1; prm.partial = nullptr; prm.arrived = nullptr;
   if (workspace != nullptr) {
     const int n_sparse = route != nullptr ? q_stop - q_start : 0;
-    int part_tiles;
-    const int parts = split_dense_rows(heads, prm.q_tiles, prm.kv_tiles, n_sparse, n_sparse ? route_len : 0, &part_tiles);
+    const int parts = split_dense_rows(heads, prm.q_tiles, prm.kv_tiles, n_sparse, n_sparse ? route_len : 0);
     size_t arrived_bytes;
     const size_t need = split_bytes(static_cast<int64_t>(heads) * (prm.q_tiles - n_sparse), parts, &arrived_bytes);
     if (parts > 1) {
       H3S_CHECK_ARG(workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
                     "sparse_attn_half_fwd: the workspace must be 16-byte aligned and hold %zu bytes, got %zu", need, workspace_bytes);
-      prm.parts = parts; prm.part_tiles = part_tiles;
+      prm.parts = parts;
       prm.arrived = static_cast<unsigned int *>(workspace);
       prm.partial = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + arrived_bytes);
       H3S_CHECK_CUDA(cudaMemsetAsync(workspace, 0, arrived_bytes, s));

@@ -31,6 +31,8 @@ int fail(int code, const char *fmt, ...);
 // (h3s_set_wait_budget_ns).
 unsigned long long wait_budget_ns();
 
+constexpr int kSmCount = 148;  // of a B200, for the rules that deal out work
+
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // ---- element loads: 8 consecutive channels of one row, widened to fp32 ----
