@@ -226,7 +226,9 @@ class B200SparseBackend:
     # -- device status word -------------------------------------------------
 
     ABORT_NAMES = {1: "Q tile load", 2: "K/V tile load", 3: "free K/V stage", 4: "QK^T result", 5: "P from the softmax warps",
-                   6: "free P buffer", 7: "P.V before a rescale", 8: "last P.V"}
+                   6: "free score slot", 7: "P.V of an earlier tile", 8: "last P.V", 9: "Q rows in tensor memory",
+                   10: "answer to the request for more work", 11: "end of a pass over the list", 12: "output sums being read",
+                   13: "first row maxima", 14: "output tile staged"}
 
     def _status_slot(self, device):
         key = device.index if device.index is not None else torch.cuda.current_device()

@@ -7,9 +7,10 @@
 
 namespace h3s {
 
+// A code names one kind of wait; backend.py and h3sparse.h have their texts
 enum AbortCode {
-  kAbortQFull = 1, kAbortKvFull, kAbortKvEmpty, kAbortSFull, kAbortPFull, kAbortPEmpty,
-  kAbortPvDone, kAbortFinal
+  kAbortQFull = 1, kAbortKvFull, kAbortKvEmpty, kAbortSFull, kAbortPFull, kAbortScoreSlot,
+  kAbortPvDone, kAbortFinal, kAbortQFree, kAbortNextItem, kAbortPass, kAbortOFree, kAbortFirstMax, kAbortStaged
 };
 
 constexpr float kIntBias = 12582912.0f;  // 1.5 * 2^23: float(kIntBias + s) has bits 0x4b400000 + s

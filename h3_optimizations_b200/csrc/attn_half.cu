@@ -313,7 +313,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
   };
   auto wait_pass = [&]() {
-    return warp_wait(&sh.pass_end, passes & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+    return warp_wait(&sh.pass_end, passes & 1u, abort_word, kAbortPass, 4 * prm.wait_budget_ns);
   };
   auto end_pass = [&]() {
     arrive_pass();
@@ -413,7 +413,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         ok = load_block(min(kHBlock, work.n_iter - i), [&]() { if (i + kHBlock < work.n_iter) fetch_block(work, i + kHBlock); });
       }
-      ok = ok && warp_wait(&sh.next_ready, items & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      ok = ok && warp_wait(&sh.next_ready, items & 1u, abort_word, kAbortNextItem, 4 * prm.wait_budget_ns);
       if (!ok) break;
       const int next = ptx::granted_block(&sh.next_reply);
       if (next >= 0) {
@@ -424,7 +424,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           if (lane == 0) to.q_scale = __ldg(prm.q_scale + it.head * prm.q_tiles + it.tq);
 #pragma unroll
           for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + it.head * H3S_HEAD_DIM + i * 32 + lane);
-          ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
+          ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortQFree, 4 * prm.wait_budget_ns);
           if (!ok) break;
           load_q(it);
         }
@@ -482,7 +482,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
             ok = ptx::mbar_wait(&sh.k_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
-                 ptx::mbar_wait(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortPEmpty, 3 * prm.wait_budget_ns);
+                 ptx::mbar_wait(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortScoreSlot, 3 * prm.wait_budget_ns);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(stage * (kHKBytes >> 4));
@@ -515,7 +515,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       int count = work.n_iter;
       for (int pass = 0;; ++pass) {
         arrive_pass();  // nothing of the pass's end depends on this warp
-        ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+        ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree, 4 * prm.wait_budget_ns);
         if (ok && ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
             const int j = done + i, g = j % kHGroups;
@@ -600,7 +600,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     auto meet = [&]() {  // all softmax warps
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&sh.staged);
-      return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortStaged, 4 * prm.wait_budget_ns);
     };
     // every P.V of the pass that has ended
     auto all_products = [&]() {
@@ -628,7 +628,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (!take(done + i, q_scale, s, c)) { ok = false; break; }
         if (i < kHGroups) {
           if (i < 2) leave_first(i, c * static_cast<float>(max_score(s)));  // c > 0
-          if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) { ok = false; break; }
+          if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) { ok = false; break; }
           m = first_reference();
         }
         const bool free_already = room_already(done + i);
