@@ -203,12 +203,15 @@ constexpr size_t route_smem(int rows, int pure_kv) {
   return sizeof(double) * (static_cast<size_t>(rows) * pure_kv + kRouteKBlock * kRouteKStride);
 }
 
+constexpr size_t kRouteMostSmem = 220 * 1024;
+
 template <typename T, int kRows>
 static int launch_route_rows(const void *q_summary, const void *k_summary, int heads, int q_tiles, int kv_tiles,
                              int q_start, int q_stop, int kv_start, int kv_stop, int retained, int route_len,
                              int32_t *route, cudaStream_t stream) {
   const size_t smem = route_smem(kRows, kv_stop - kv_start);
-  H3S_CHECK_CUDA(cudaFuncSetAttribute(route_topk_kernel<T, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  // one value for all callers: a thread with shorter rows would take away what another one is about to launch with
+  H3S_CHECK_CUDA(cudaFuncSetAttribute(route_topk_kernel<T, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRouteMostSmem)));
   dim3 grid(ceil_div(q_stop - q_start, kRows), heads);
   route_topk_kernel<T, kRows><<<grid, kRows * 32, smem, stream>>>(
       static_cast<const T *>(q_summary), static_cast<const T *>(k_summary), q_tiles, kv_tiles, q_start,
@@ -226,11 +229,10 @@ static int launch_route(const void *q_summary, const void *k_summary, int heads,
                         int q_start, int q_stop, int kv_start, int kv_stop, int retained, int route_len,
                         int32_t *route, cudaStream_t stream) {
   const int pure_kv = kv_stop - kv_start;
-  constexpr size_t kMost = 220 * 1024;
   const size_t least = route_smem(8, pure_kv) + sizeof(int) * 8 * 256;
-  H3S_CHECK_ARG(least <= kMost, "route_topk: %d pure-video KV tiles need %zu bytes of shared memory", pure_kv, least);
+  H3S_CHECK_ARG(least <= kRouteMostSmem, "route_topk: %d pure-video KV tiles need %zu bytes of shared memory", pure_kv, least);
   const int64_t ctas = static_cast<int64_t>(heads) * ceil_div(q_stop - q_start, 8);
-  if (ctas > 2 * 148 && route_smem(16, pure_kv) <= kMost)
+  if (ctas > 2 * 148 && route_smem(16, pure_kv) <= kRouteMostSmem)
     return launch_route_rows<T, 16>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
   return launch_route_rows<T, 8>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
 }
