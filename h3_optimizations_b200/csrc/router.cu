@@ -220,10 +220,26 @@ static int launch_route_rows(const void *q_summary, const void *k_summary, int h
   return H3S_OK;
 }
 
-// Sixteen rows where eight make more CTAs than run at once, two on each of 148 SMs: every CTA reads all K tile
-// means of its head (393 MB in all at 24 x 256 rows of 512 scores, 98 us; 85 with half of that).  Fewer
-// CTAs wait for their own chain, which is shorter with eight rows (3 x 256 rows 28.8 us, 30.4 with sixteen).  From 1233
-// pure-video KV tiles on, sixteen rows of scores do not fit beside a block.
+// Eight query tiles a CTA, or sixteen.  A CTA of eight is through sooner, so it is taken where no SM gets a second one.  Two of
+// them share an SM while their scores fit, beyond about 750 pure-video KV tiles they do not; sixteen query tiles take an SM for themselves,
+// but read the K tile means of their head once for all, with the next block's loads under the products.  us, eight / sixteen:
+//   one CTA of eight an SM         3 x 256 rows of 512 scores, fp32 22.2 / 27.7, FP64 28.1 / 30.0; 24 x 40 of 80, fp32 8.9 / 11.8
+//   two, side by side              8 x 256 of 512, fp32 31.0 / 27.7, FP64 35.6 / 30.1; 24 x 78 of 156, fp32 15.8 / 14.5
+//   two, one after the other       3 x 591 of 1181, fp32 88.7 / 57.1, FP64 115.5 / 65.2
+//   three, of which two share      10 x 256 of 512, fp32 49.0 / 51.3, FP64 59.0 / 56.5; 24 x 128 of 256, fp32 33.1 / 31.1
+//   more                           24 x 256 of 512, fp32 86.5 / 77.3, FP64 97.1 / 84.1; 24 x 591 of 1181, fp32 521 / 331
+// With three, sixteen leave most of a second round empty: there eight keep the rows of 384 scores and
+// more whose means are not in FP64 (12 x 200 of 400, fp32 42.7 / 44.1).  From 1233 pure-video KV tiles on, sixteen rows of scores do not fit
+// beside a block.
+template <typename T>
+static bool sixteen_rows(int heads, int rows, int pure_kv) {
+  if (route_smem(16, pure_kv) > kRouteMostSmem) return false;
+  const int64_t an_sm = (static_cast<int64_t>(heads) * ceil_div(rows, 8) + kSmCount - 1) / kSmCount;
+  const bool share = 2 * (route_smem(8, pure_kv) + 1024) <= 228 * 1024;
+  if (an_sm == 1 || (an_sm == 2 && rows <= 8)) return false;  // (half of sixteen would be empty)
+  return !(an_sm == 3 && share && pure_kv >= 384 && sizeof(T) < 8);
+}
+
 template <typename T>
 static int launch_route(const void *q_summary, const void *k_summary, int heads, int q_tiles, int kv_tiles,
                         int q_start, int q_stop, int kv_start, int kv_stop, int retained, int route_len,
@@ -231,8 +247,7 @@ static int launch_route(const void *q_summary, const void *k_summary, int heads,
   const int pure_kv = kv_stop - kv_start;
   const size_t least = route_smem(8, pure_kv) + sizeof(int) * 8 * 256;
   H3S_CHECK_ARG(least <= kRouteMostSmem, "route_topk: %d pure-video KV tiles need %zu bytes of shared memory", pure_kv, least);
-  const int64_t ctas = static_cast<int64_t>(heads) * ceil_div(q_stop - q_start, 8);
-  if (ctas > 2 * 148 && route_smem(16, pure_kv) <= kRouteMostSmem)
+  if (sixteen_rows<T>(heads, q_stop - q_start, pure_kv))
     return launch_route_rows<T, 16>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
   return launch_route_rows<T, 8>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
 }
