@@ -1,7 +1,7 @@
 """Attention kernel at the edges of its tile loop.  Needs a B200.
 
-Each softmax group takes every other KV tile and four stages are in flight, so lists of one to
-six tiles, odd and even, are the interesting lengths, with full and ragged last tiles.  The bound
+Each of four softmax groups takes every fourth KV tile, and three tiles of scores are ahead of them, so lists of
+one to six tiles are the interesting lengths, with full and ragged last tiles.  The bound
 is elementwise, 2^-8 * sum(p |v|) / sum(p) from the same oracle on |V|: room for probabilities of
 eight significant bits, or for FP16's where one key has nearly all the weight and the others lie
 close to its smallest value.  test_gpu_attention_precision has the close bound for FP16, and the
@@ -63,9 +63,9 @@ def test_scores_that_outgrow_the_first_tile(native_lib, tiles):
 
 
 def test_many_short_lists_that_are_walked_again(native_lib):
-    """The first of the tiles, walked last, is far above the others: nothing but the P.V warp's own arrival holds
-    back the pass behind it."""
-    sequence, heads = 187, 900                                                    # six waves of two CTAs on every SM
+    """The first of the tiles, walked last, is far above the others: three passes over a list of three tiles, one of which
+    is noted, in item after item."""
+    sequence, heads = 187, 900                                                    # 1800 items on 148 SMs
     spec = workloads.small_spec("edge", heads, 0, sequence)
     q, k, v = workloads.gaussian_qkv(spec, seed=12, widen=True)
     sign = -torch.ones(sequence)
