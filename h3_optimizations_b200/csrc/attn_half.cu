@@ -30,11 +30,11 @@
 // deviation, held over groups of 64 tokens, 2 to 14 % of the query tiles (27 % in a dense one of
 // 24792 tokens) came round again, with 0.03 to 0.5 % of all tiles; with the first tile of
 // the list and 2^-7 it was 17 to 61 % and 1.5 to 9 %.  What it costs at 24 heads x 33272
-// tokens, 30 %: 2.8 to 3.0 ms on the inputs above; 2.9 to 3.3 with one row of every query
-// tile 48 bits ahead in every 40th tile; 3.9 to 4.0 with a third of the rows ahead in every tenth;
+// tokens, 30 %, launches in a row: 3.11 ms on the inputs above; 3.32 with one row of every query
+// tile 48 bits ahead in every 40th tile; 3.78 with a third of the rows ahead in every tenth;
 // two E4M3 terms take 4.2 to 4.3 ms of each.  All but the first two tiles of a list
 // ahead is the worst: two walks, three where a sum overflows (120 bits): 24 heads x 9872,
-// dense, 0.83 ms, then 2.15 and 2.76, where two E4M3 terms take 1.13.
+// dense, 0.87 ms, then 2.18 and 2.86, where two E4M3 terms take 1.13.
 //
 // Without a running maximum the tiles of a row are independent but for the sum: the sixteen
 // softmax warps form four groups, group g takes every fourth tile, and each scheduler has one
@@ -62,12 +62,14 @@
 //
 // What bounds it: per tile and SM the ex2 pipe needs 512 cycles, the tensor pipe 453 (measured: 144 for QK^T with A
 // in TMEM, 258 with A in shared memory, 309 for P.V; at the nominal rates 384 in all), the softmax
-// instructions of four warps a scheduler together 535; a tile takes about 780.  Beside that an item has
-// about 7000 cycles of its own (last P.V, epilogue, first tiles), and the power cap holds the clock at 1.65 to
-// 1.75 GHz.  Attention alone, two CTAs of two groups an SM before and this now: 24 heads x 33272 tokens at 30 %, 3.08 ms
-// and 2.84 (3.38 and 3.26 in a loop); 24 x 9872 dense 866 us and 786; 3 x 33272 412 and 384; 7 x 10384 at 15 % 96.5 and
-// 88; 4 x 2304 28.7 and 22.9; 24 x 2304 43.6 and 43.1.  Tried and slower on the earlier form: a polynomial
-// for a share of the exponentials, two threads per row, one group per CTA.
+// instructions of four warps a scheduler together 535; a tile takes 700, an item 8100 beside its tiles (last P.V,
+// epilogue, first tiles), a launch 7100 (fit over lists of 4 to 296 tiles, one to four items an SM, time x sampled SM
+// clock, within 1.2 %; 24 heads x 9872 and x 33272 dense 713 and 699 a tile).  In a loop the power cap holds the clock at 1.6 to
+// 1.75 GHz.  Attention alone, launches in a row, two CTAs of two groups an SM and this: 24 heads x 33272 tokens at 30 %, 3.45 ms
+// and 3.15; 24 x 9872 dense 820 us and 780; 3 x 33272 at 30 % 409 and 376; 7 x 10384 at 15 % 93 and 84; 4 x 2304 at 30 % 27.7
+// and 20.8; 24 x 2304 45.7 and 44.2.  Tried and slower on the earlier form: a polynomial
+// for a share of the exponentials, two threads per row, one group per CTA.  Parts added up by a kernel of their own: 13 instead
+// of 27 tiles' time for a part, but another main loop by ptxas' choice, 3 to 8 % slower for every launch.
 #include "attn_common.cuh"
 #include "tma.cuh"
 

@@ -365,13 +365,14 @@ __device__ __forceinline__ void quantise8(const uint4 &raw, const SharedDivisor 
 // weight, then the split-half rotation of channels [0,48) against [48,96).
 // Same order of operations and roundings as the reference
 // (attention/sparse/fused_qkv.py:218-289); the sum of squares is accumulated
-// in FP64 so that it does not depend on the order of the additions.
+// in FP64 so that it does not depend on the order of the additions.  The staging
+// epilogue does this, a row to a thread; the carrier epilogue deals a row to two (HalfRow).
 //
 // The table is read 16 bytes at a time where it is stored as the model produces it; the
 // form is decided once per row, so that the loads of a batch are all in flight together
 // and the first batch travels while the norm is computed.  With the decision inside the
 // element loop, and one chain of dependent FP64 additions, a 4096-row chunk of the QKV
-// projection with norm and rotation took 197 us, 155 us now.
+// projection took 197 us for 155, when the carrier epilogue had this form.
 enum RopeForm { kRopeNone, kRopeBf16, kRopeF32, kRopeStrided };
 
 __device__ __forceinline__ void rotate_pair(uint32_t &first, uint32_t &second, const float (&f)[2][4]) {
