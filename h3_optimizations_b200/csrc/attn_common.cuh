@@ -32,6 +32,7 @@ struct AttnParams {
   unsigned int *arrived;
   int heads, sequence, q_tiles, kv_tiles;
   int out_dtype;
+  bool out_map;  // the output goes through TMA stores (attn_half.cu)
   // head-sharded runs: every output tile is also stored into these buffers
   // (the same slice of each peer GPU's full output, reached over NVLink with
   // plain stores), so no separate gather pass is needed

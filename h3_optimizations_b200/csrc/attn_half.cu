@@ -61,15 +61,20 @@
 // the list, so that the result does not depend on which one that was.
 //
 // What bounds it: per tile and SM the ex2 pipe needs 512 cycles, the tensor pipe 453 (measured: 144 for QK^T with A
-// in TMEM, 258 with A in shared memory, 309 for P.V; at the nominal rates 384 in all), the softmax
-// instructions of four warps a scheduler together 535; a tile takes 700, an item 8100 beside its tiles (last P.V,
-// epilogue, first tiles), a launch 7100 (fit over lists of 4 to 296 tiles, one to four items an SM, time x sampled SM
-// clock, within 1.2 %; 24 heads x 9872 and x 33272 dense 713 and 699 a tile).  In a loop the power cap holds the clock at 1.6 to
-// 1.75 GHz.  Attention alone, launches in a row, two CTAs of two groups an SM and this: 24 heads x 33272 tokens at 30 %, 3.45 ms
-// and 3.15; 24 x 9872 dense 820 us and 780; 3 x 33272 at 30 % 409 and 376; 7 x 10384 at 15 % 93 and 84; 4 x 2304 at 30 % 27.7
-// and 20.8; 24 x 2304 45.7 and 44.2.  Tried and slower on the earlier form: a polynomial
+// in TMEM, 258 with A in shared memory, 309 for P.V; at the nominal rates 384 in all), the softmax warps with their loads, stores
+// and barriers 565 (in a loop of their own; 572 beside issuing warps).  By the SM clock a tile takes 640 in the middle of a list:
+// the groups wait for one another's slots and for the slowest quarter of a group.  From an item's last P to the first
+// P of the next one it was 7600 cycles.  Cycles of a launch with the epilogue at the item's end, all first tiles in the loop / now, thousands:
+// 24 heads x 33272 tokens at 30 % 4856 / 4596; 24 x 9872 dense 1379 / 1298; 3 x 33272 at 30 % 621 / 595; 7 x 10384 at 15 % 113 / 108;
+// 24 x 5000 at 10 % 141 / 119.  In time, launches of many layers in a row: 1.03 to 1.05 of it is gained, as the power cap sets the clock
+// (1.49 GHz for the first of these after 200 launches, 1.75 for one by itself).
+// Tried and slower on the earlier form: a polynomial
 // for a share of the exponentials, two threads per row, one group per CTA.  Parts added up by a kernel of their own: 13 instead
-// of 27 tiles' time for a part, but another main loop by ptxas' choice, 3 to 8 % slower for every launch.
+// of 27 tiles' time for a part, but another main loop by ptxas' choice, 3 to 8 % slower for every launch.  On this form: groups kept
+// out of step by a barrier inside the exponentials (every form 5 to 45 % slower: it cuts the loop's schedule), waits of the
+// loading and issuing threads that sleep (1 to 13 % slower), eight orders of the exponentials' source (alike, or 1 % slower).
+#include <type_traits>
+
 #include "attn_common.cuh"
 #include "tma.cuh"
 
@@ -96,11 +101,12 @@ constexpr int kHNoted = 2048;          // bits of the note of tiles left out, ea
 
 enum { kAgainNoted = 1, kAgainFar = 2 };
 
-// What the warps need to know of an item before its first tile
-struct HalfItem {
-  int number;  // of the launch, -1: no more
-  float q_scale;
+// What the warps need to know of an item: left by the K loader, so that its place in the launch is worked out once
+struct alignas(16) HalfItem {
   float v_scale[H3S_HEAD_DIM];
+  int number;  // of the launch, -1: no more
+  int head, tq, n_iter;
+  int dense_row, part;  // of an item that is a part; -1 otherwise
 };
 
 struct alignas(16) HalfShared {
@@ -124,7 +130,7 @@ struct alignas(16) HalfShared {
   int again[4];                // per item in turn.  kAgainNoted: some row has left out a tile; kAgainFar: its sum
                                // there does not tell the maximum
   HalfItem item[3];            // in turn: an epilogue may still read the last one when the one after next is known
-  struct { int n_valid; float scale; } tile[kHMeta];  // keys of a tile inside the sequence, and its k_scale
+  struct { int n_valid; float scale; } tile[kHMeta];  // keys of a tile inside the sequence, and the factor of its scores
   int block[2][kHBlock];            // the next tiles of the list, for the threads that load K and V
   uint32_t noted[2][kHNoted / 32];  // tiles of the list that some row has left out, per item in turn
   float first[2][H3S_Q_TILE];
@@ -185,6 +191,23 @@ __device__ __forceinline__ int max_score(const uint32_t (&s)[H3S_KV_TILE]) {
   return max(__vimax3_s32(a, s[H3S_KV_TILE - 2], s[H3S_KV_TILE - 1]), b);
 }
 
+// 32 floats -> 16 (bf16, fp16) or 32 words
+template <typename OutT>
+__device__ __forceinline__ void pack_columns(const uint32_t (&o)[32], uint32_t (&packed)[8 * sizeof(OutT)]) {
+#pragma unroll
+  for (int e = 0; e < 32; e += 4 / static_cast<int>(sizeof(OutT))) {
+    const float lo = __uint_as_float(o[e]);
+    if constexpr (std::is_same<OutT, float>::value) {
+      packed[e] = __float_as_uint(lo);
+    } else if constexpr (std::is_same<OutT, __half>::value) {
+      packed[e / 2] = pack_half2(lo, __uint_as_float(o[e + 1]));
+    } else {
+      const __nv_bfloat162 pair = __floats2bfloat162_rn(lo, __uint_as_float(o[e + 1]));
+      packed[e / 2] = *reinterpret_cast<const uint32_t *>(&pair);
+    }
+  }
+}
+
 // Number of tiles the noted bits stand for (whole warp)
 __device__ __forceinline__ int noted_tiles(const uint32_t *noted, int n_iter, int coarse, int lane) {
   const uint32_t last = static_cast<uint32_t>(n_iter - 1) >> coarse;
@@ -198,7 +221,7 @@ __device__ __forceinline__ int noted_tiles(const uint32_t *noted, int n_iter, in
 // Item `w` of a launch: dense (long) rows first, then the routed rows
 struct HalfWork {
   int head, tq;
-  int dense_row, part;  // running number of a dense row, part of its list
+  int dense_row, part;  // running number of a dense row, part of its list where it is cut (-1: not)
   bool dense;
   int first_tile, n_iter;
   const int32_t *route_row;
@@ -210,16 +233,18 @@ __device__ __forceinline__ HalfWork work_item(const AttnParams &prm, int w) {
   const int n_dense = prm.q_tiles - n_sparse;
   const int dense_items = prm.heads * n_dense * prm.parts;
   it.dense = w < dense_items;
-  it.dense_row = it.part = it.first_tile = 0;
+  it.dense_row = it.first_tile = 0;
+  it.part = -1;
   it.route_row = nullptr;
   if (it.dense) {
     it.dense_row = w / prm.parts;
-    it.part = w - it.dense_row * prm.parts;
+    const int part = w - it.dense_row * prm.parts;
+    if (prm.parts > 1) it.part = part;
     it.head = it.dense_row / n_dense;
     const int i = it.dense_row - it.head * n_dense;
     it.tq = (n_sparse == 0 || i < prm.q_start) ? i : prm.q_stop + (i - prm.q_start);
-    it.first_tile = it.part * prm.kv_tiles / prm.parts;  // even parts
-    it.n_iter = (it.part + 1) * prm.kv_tiles / prm.parts - it.first_tile;
+    it.first_tile = part * prm.kv_tiles / prm.parts;  // even parts
+    it.n_iter = (part + 1) * prm.kv_tiles / prm.parts - it.first_tile;
   } else {
     const int v = w - dense_items;
     it.head = v / n_sparse;
@@ -242,7 +267,8 @@ __device__ __forceinline__ int note_scale(int n_iter) { return 32 - __clz((n_ite
 template <typename OutT>
 __global__ void __launch_bounds__(kHThreads, 1)
 sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                        const __grid_constant__ CUtensorMap map_v, const AttnParams prm) {
+                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
+                        const AttnParams prm) {
   using L = HalfLayout<OutT>;
   extern __shared__ unsigned char smem_dyn[];
   // SWIZZLE_128B tiles need 1024-byte alignment
@@ -284,7 +310,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     sh.abort_word = 0;
     sh.finish = 0;
     for (int i = 0; i < 4; ++i) sh.again[i] = 0;
-    sh.item[0].q_scale = __ldg(prm.q_scale + work.head * prm.q_tiles + work.tq);
+    sh.item[0].head = work.head;
+    sh.item[0].tq = work.tq;
     ptx::fence_mbar_init();
   }
   if (threadIdx.x < 2 * kHNoted / 32) (&sh.noted[0][0])[threadIdx.x] = 0u;
@@ -325,10 +352,14 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   // after an item's last pass: the next one, if there is one
   auto next_item = [&]() {
     ++items;
-    const int next = *static_cast<volatile int *>(&sh.item[items % 3u].number);
-    if (next < 0) return false;
-    item = next;
-    work = work_item(prm, item);
+    const HalfItem &next = sh.item[items % 3u];
+    item = next.number;
+    if (item < 0) return false;
+    work.head = next.head;
+    work.tq = next.tq;
+    work.n_iter = next.n_iter;
+    work.dense_row = next.dense_row;
+    work.part = next.part;
     return true;
   };
 
@@ -344,6 +375,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       ptx::prefetch_tensormap(map);
       if (keys) ptx::prefetch_tensormap(&map_q);
     }
+    // what an item's q_scale and k_scale are multiplied with: 1 / sqrt(128) / ln 2
+    auto scale_of = [&](const HalfWork &it) {
+      return __ldg(prm.q_scale + it.head * prm.q_tiles + it.tq) * (0.08838834764831845f * 1.4426950408889634f);
+    };
+    float item_scale = keys ? scale_of(work) : 0.f, coming_scale = 0.f;
     int next_tile = 0;  // of the block of the list that comes next, one per lane
     float next_scale = 0.f;
     auto fetch = [&](const HalfWork &it, int position) {
@@ -375,7 +411,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (keys && lane < tiles) {
         auto &tile = sh.tile[(seq + lane) % kHMeta];
         tile.n_valid = prm.sequence - next_tile * H3S_KV_TILE;
-        tile.scale = next_scale;
+        tile.scale = item_scale * next_scale;
       }
       seq += tiles;
       __syncwarp();
@@ -400,6 +436,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     };
     if (keys) load_q(work);
     fetch_block(work, 0);
+    HalfWork coming = work;
     while (ok) {
       for (int i = 0; ok && i < work.n_iter; i += kHBlock) {
         if (keys && i + kHBlock >= work.n_iter) {
@@ -419,16 +456,23 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (!ok) break;
       const int next = ptx::granted_block(&sh.next_reply);
       if (next >= 0) {
-        const HalfWork it = work_item(prm, next);
-        fetch_block(it, 0);
+        coming = work_item(prm, next);
+        fetch_block(coming, 0);
         if (keys) {
           HalfItem &to = sh.item[(items + 1) % 3u];
-          if (lane == 0) to.q_scale = __ldg(prm.q_scale + it.head * prm.q_tiles + it.tq);
+          coming_scale = scale_of(coming);
+          if (lane == 0) {
+            to.head = coming.head;
+            to.tq = coming.tq;
+            to.n_iter = coming.n_iter;
+            to.dense_row = coming.dense_row;
+            to.part = coming.part;
+          }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + it.head * H3S_HEAD_DIM + i * 32 + lane);
+          for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + coming.head * H3S_HEAD_DIM + i * 32 + lane);
           ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortQFree, 4 * prm.wait_budget_ns);
           if (!ok) break;
-          load_q(it);
+          load_q(coming);
         }
       }
       if (keys && lane == 0) sh.item[(items + 1) % 3u].number = next;
@@ -459,7 +503,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         next_tile = first_tile;
         next_scale = first_scale;
       }
-      if (!ok || !next_item()) break;
+      if (!ok || next < 0) break;
+      ++items;
+      item = next;
+      work = coming;
+      item_scale = coming_scale;
     }
   } else if (warp == kHScoreIssuer) {
     // =================== QK^T issuer ===================
@@ -554,7 +602,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const uint32_t tmem_p = tmem_o + kHTmemP + group * 32 + lane_addr;
 
     // scores of tile j -> registers, and the factor that belongs to them
-    auto take = [&](uint32_t j, float q_scale, uint32_t (&s)[H3S_KV_TILE], float &c) {
+    auto take = [&](uint32_t j, uint32_t (&s)[H3S_KV_TILE], float &c) {
       if (!warp_wait(&sh.s_full[group], (j / kHGroups) & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) return false;
       const uint32_t slot = j % kHScoreSlots;
       ptx::tc_fence_after();
@@ -562,7 +610,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       // left in shared memory by the K loader before the stage was handed to the tensor
       // pipe; the entry is written again when P.V of this tile is long complete
       const int n_valid = sh.tile[j % kHMeta].n_valid;
-      c = q_scale * sh.tile[j % kHMeta].scale;
+      c = sh.tile[j % kHMeta].scale;
       ptx::tmem_wait_ld(s);
       ptx::tc_fence_before();
       __syncwarp();
@@ -614,29 +662,83 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (lane == 0) ptx::mbar_arrive(&sh.o_free);
     };
 
+    // O / l * v_scale of an item whose sums are complete, 32 columns of a row to a thread
+    auto normalise = [&](uint32_t (&o)[32], float sum, const HalfItem &from) {
+      const float inv_l = 1.0f / sum;
+      const float2 inv2 = make_float2(inv_l, inv_l);
+      const float4 *v_scale = reinterpret_cast<const float4 *>(from.v_scale) + group * 8;
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        const float4 vs = v_scale[e / 4];
+        // |o / l| <= 448: nothing overflows
+        const float2 a = mul2(mul2(make_float2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), inv2), make_float2(vs.x, vs.y));
+        const float2 b = mul2(mul2(make_float2(__uint_as_float(o[e + 2]), __uint_as_float(o[e + 3])), inv2), make_float2(vs.z, vs.w));
+        o[e] = __float_as_uint(a.x); o[e + 1] = __float_as_uint(a.y);
+        o[e + 2] = __float_as_uint(b.x); o[e + 3] = __float_as_uint(b.y);
+      }
+    };
+    auto row_sum = [&]() {  // of the pass that has ended
+      const float *sums = &sh.row[(passes - 1) & 1][0][row];
+      return (sums[0] + sums[H3S_Q_TILE]) + (sums[2 * H3S_Q_TILE] + sums[3 * H3S_Q_TILE]);
+    };
+    // The epilogue of the item before, once this group's first tile of the next one is handed over: the softmax warps need
+    // not wait for the last P.V, and the next P.V comes later.  Every warp by itself: its 32 rows of 32 columns
+    // go through its own piece of shared memory to a TMA store, which also leaves out rows past the sequence.
+    bool pending = false;
+    auto finish_last = [&](const HalfItem &from) {
+      pending = false;
+      if (!all_products()) return false;
+      ptx::tc_fence_after();
+      uint32_t o[32];
+      H3S_TMEM_LD32(tmem_o + lane_addr + group * 32, o);
+      ptx::tmem_wait_ld(o);
+      release_o();
+      normalise(o, row_sum(), from);
+      constexpr int kRowBytes = 32 * static_cast<int>(sizeof(OutT)), kChunks = kRowBytes / 16;
+      uint32_t packed[4 * kChunks];
+      pack_columns<OutT>(o, packed);
+      unsigned char *piece = smem + L::kOffOut + warp * (32 * kRowBytes);
+      if (lane == 0) ptx::bulk_wait_read();  // the piece's last store has read it
+      __syncwarp();
+      // the map's swizzle: rows of 64 bytes take turns by pairs, rows of 128 bytes one by one
+      const int turn = sizeof(OutT) == 4 ? lane & 7 : (lane >> 1) & 3;
+#pragma unroll
+      for (int k = 0; k < kChunks; ++k)
+        *reinterpret_cast<uint4 *>(piece + lane * kRowBytes + ((k ^ turn) << 4)) =
+            make_uint4(packed[4 * k], packed[4 * k + 1], packed[4 * k + 2], packed[4 * k + 3]);
+      ptx::fence_proxy_async_smem();
+      __syncwarp();
+      const int first_row = from.tq * H3S_Q_TILE + quarter * 32;
+      if (lane == 0 && first_row < prm.sequence) {
+        ptx::tma_store_3d(&map_out, piece, group * kRowBytes, first_row, from.head);
+        ptx::bulk_commit();
+      }
+      return true;
+    };
+
     while (ok) {
       const int n_iter = work.n_iter;
       // Which of the four groups has the first tile depends on what the CTA has done before; sums are
       // added up in the order of the tiles all the same, so that a result does not depend on that.
       const int rank = (group - done) & (kHGroups - 1);
-      const float q_scale = sh.item[items % 3u].q_scale * (0.08838834764831845f * 1.4426950408889634f);
-      const int coarse = note_scale(n_iter);
       float m = 0.f, l = 0.f;
       sh.over[group][row] = 0.f;
       if (rank == 1 && n_iter == 1) leave_first(1, -INFINITY);
-      for (int i = rank; i < n_iter; i += kHGroups) {
+      // One tile.  A group's first one is a case of its own, so that the loop over the others holds neither the maxima nor the
+      // last item's epilogue: 24 heads x 33272 tokens at 30 % 4.89 -> 4.61 million cycles.
+      auto walk = [&](int i, auto first) {
         uint32_t s[H3S_KV_TILE];
         float c;
-        if (!take(done + i, q_scale, s, c)) { ok = false; break; }
-        if (i < kHGroups) {
+        if (!take(done + i, s, c)) return false;
+        if (decltype(first)::value) {
           if (i < 2) leave_first(i, c * static_cast<float>(max_score(s)));  // c > 0
-          if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) { ok = false; break; }
+          if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) return false;
           m = first_reference();
         }
         const bool free_already = room_already(done + i);
         uint32_t packed[H3S_KV_TILE / 2];
         float sum = exp_sum<true, false>(s, c, -fmaf(c, kIntBias, m), packed);
-        if (!__all_sync(0xffffffffu, free_already) && !room(done + i)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, free_already) && !room(done + i)) return false;
         put(packed);
         const bool out = !(sum <= kHSumLimit);
         if (__any_sync(0xffffffffu, out)) {  // these rows leave the tile out
@@ -650,14 +752,27 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
           put(packed);
           if (lane == 0) {
+            const int coarse = note_scale(work.n_iter);
             atomicOr(&sh.noted[items & 1][(i >> coarse) >> 5], 1u << ((i >> coarse) & 31));
             atomicOr(&sh.again[items & 3], far ? kAgainNoted | kAgainFar : kAgainNoted);
           }
         }
         l += sum;
         hand_over();
+        return true;
+      };
+      if (rank < n_iter) {
+        ok = walk(rank, std::true_type{});
+        if (ok && pending) ok = finish_last(sh.item[(items + 2) % 3u]);
+        for (int i = rank + kHGroups; ok && i < n_iter; i += kHGroups) ok = walk(i, std::false_type{});
       }
       if (!ok) break;
+      if (rank >= n_iter) {  // a group without a tile: the last item is not finished, and there is no reference point yet
+        ok = (!pending || finish_last(sh.item[(items + 2) % 3u])) &&
+             warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns);
+        if (!ok) break;
+        m = first_reference();
+      }
       done += n_iter;
       sh.row[passes & 1][rank][row] = l;
       // the word of the item after next: its last readers (two items ago) have all been at a pass's end since
@@ -665,7 +780,6 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       ok = end_pass();
       ++passes;
       if (!ok) break;
-      if (rank >= n_iter) m = first_reference();  // a group without a tile has none yet
       const int final_pass = last_pass();
       if (final_pass > 0) {
         const int count = count_noted();
@@ -681,7 +795,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           for (int i = (group - done) & (kHGroups - 1); ok && i < count; i += kHGroups) {
             uint32_t s[H3S_KV_TILE];
             float c;
-            ok = take(done + i, q_scale, s, c) && room(done + i);
+            ok = take(done + i, s, c) && room(done + i);
             if (!ok) break;
             top = fmaxf(top, c * static_cast<float>(max_score(s)));
             uint32_t none[H3S_KV_TILE / 2];  // O stays as it is
@@ -715,7 +829,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         for (int i = (group - done) & (kHGroups - 1); ok && i < count; i += kHGroups) {
           uint32_t s[H3S_KV_TILE];
           float c;
-          ok = take(done + i, q_scale, s, c) && room(done + i);
+          ok = take(done + i, s, c) && room(done + i);
           if (!ok) break;
           uint32_t packed[H3S_KV_TILE / 2];
           // the same sum as in the first pass, so the same tiles
@@ -739,18 +853,19 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // (this note's next item is the one after next, and its last reader has been at the pass's end)
         if (threadIdx.x < kHNoted / 32) sh.noted[items & 1][threadIdx.x] = 0u;
       }
-      {
-        const float *sums = &sh.row[(passes - 1) & 1][0][row];
-        l = (sums[0] + sums[H3S_Q_TILE]) + (sums[2 * H3S_Q_TILE] + sums[3 * H3S_Q_TILE]);
+      const bool split = work.part >= 0;
+      if (!split && prm.out_map) {
+        pending = true;
+        if (next_item()) continue;
+        ok = finish_last(sh.item[(items + 2) % 3u]);
+        break;
       }
+
+      // Parts of a row, and outputs that go to peers too: the softmax warps work together, at once
+      l = row_sum();
       ok = all_products();
       if (!ok) break;
-
-      // Epilogue: O / l * v_scale -> OutT, staged through shared memory.  A warp converts
-      // its 32 rows of 32 columns; the four warps of a row quarter then each write eight of the
-      // quarter's rows as full contiguous lines.
       ptx::tc_fence_after();
-      const bool split = work.dense && prm.parts > 1;
       uint32_t o[32];
       H3S_TMEM_LD32(tmem_o + lane_addr + group * 32, o);
       ptx::tmem_wait_ld(o);
@@ -809,28 +924,23 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
       }
       if (finish) {
-        const float inv_l = 1.0f / l;
+        // Staged through shared memory: the four warps of a row quarter each write eight of the quarter's rows as
+        // contiguous lines, and what goes to the peers is made of lines too.
+        normalise(o, l, sh.item[items % 3u]);
         constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
+        constexpr int kChunks = 32 * static_cast<int>(sizeof(OutT)) / 16;
         unsigned char *out_tile = smem + L::kOffOut;
-        unsigned char *my_row = out_tile + row * kRowBytes;
-        const float *v_scale = sh.item[items % 3u].v_scale + group * 32;
+        uint32_t packed[4 * kChunks];
+        pack_columns<OutT>(o, packed);
+        // a warp's own store of an earlier item may still be reading its piece, and the warps write each other's
+        if (lane == 0) ptx::bulk_wait_read();
+        ok = meet();
+        if (!ok) break;
+        // the chunk index is XORed with the row so that the 32 rows of a warp do not collide on banks
 #pragma unroll
-        for (int e0 = 0; e0 < 32; e0 += 8) {
-          float v[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            v[e] = __uint_as_float(o[e0 + e]) * inv_l * v_scale[e0 + e];  // |o / l| <= 448: nothing overflows
-          // 8 values = one (bf16/fp16) or two (fp32) 16-byte chunks; the chunk index is
-          // XORed with the row so that the 32 rows of a warp do not collide on banks
-          constexpr int kChunks8 = 8 * static_cast<int>(sizeof(OutT)) / 16;
-          const int chunk0 = (group * 32 + e0) * static_cast<int>(sizeof(OutT)) / 16;
-          __align__(16) OutT tmp[8];
-          store_out8<OutT>(tmp, v);
-#pragma unroll
-          for (int k = 0; k < kChunks8; ++k)
-            *reinterpret_cast<uint4 *>(my_row + (((chunk0 + k) ^ (row & 15)) << 4)) =
-                reinterpret_cast<const uint4 *>(tmp)[k];
-        }
+        for (int k = 0; k < kChunks; ++k)
+          *reinterpret_cast<uint4 *>(out_tile + row * kRowBytes + (((group * kChunks + k) ^ (row & 15)) << 4)) =
+              make_uint4(packed[4 * k], packed[4 * k + 1], packed[4 * k + 2], packed[4 * k + 3]);
         ok = meet();
         if (!ok) break;
         store_rows<OutT>(prm, out_tile, work.head, work.tq, quarter * 32 + group * 8, 8, lane);
@@ -838,6 +948,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
       if (!next_item()) break;
     }
+    if (lane == 0) ptx::bulk_wait();  // the last stores, before the CTA's shared memory goes
   }
 
   // ---- teardown ----
@@ -926,13 +1037,13 @@ static size_t split_bytes(int64_t dense_rows, int parts, size_t *arrived_bytes) 
 }
 
 template <typename OutT>
-static int launch_attn_half(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const AttnParams &prm,
-                            cudaStream_t stream) {
+static int launch_attn_half(const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const CUtensorMap &mo,
+                            const AttnParams &prm, cudaStream_t stream) {
   constexpr int kBytes = static_cast<int>(HalfLayout<OutT>::kBytes);
   H3S_CHECK_CUDA(cudaFuncSetAttribute(sparse_attn_half_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
   const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
   const int items = prm.heads * ((prm.q_tiles - n_sparse) * prm.parts + n_sparse);
-  sparse_attn_half_kernel<OutT><<<items, kHThreads, kBytes, stream>>>(mq, mk, mv, prm);
+  sparse_attn_half_kernel<OutT><<<items, kHThreads, kBytes, stream>>>(mq, mk, mv, mo, prm);
   H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
 }
@@ -987,6 +1098,15 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   prm.parts = 1; prm.partial = nullptr; prm.arrived = nullptr;
+  // One head's stride is never used and need not suit a map; with peers the tile is staged as a whole instead
+  const uint64_t size = out_dtype == H3S_F32 ? 4 : 2;
+  CUtensorMap mo;
+  const uint64_t stride_s = static_cast<uint64_t>(out_stride_s) * size;
+  const uint64_t stride_h = heads > 1 ? static_cast<uint64_t>(out_stride_h) * size : stride_s;
+  prm.out_map = n_peer_out == 0 && make_tensor_map_u8_3d(&mo, out, H3S_HEAD_DIM * size, S, heads, stride_s, stride_h, 32 * size, 32,
+                                                         size == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                                                         "sparse_attn_half_fwd output map") == H3S_OK;
+  if (!prm.out_map) mo = mq;
   if (workspace != nullptr) {
     const int n_sparse = route != nullptr ? q_stop - q_start : 0;
     const int parts = split_dense_rows(heads, prm.q_tiles, prm.kv_tiles, n_sparse, n_sparse ? route_len : 0);
@@ -1002,8 +1122,8 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
     }
   }
   switch (out_dtype) {
-    case H3S_F32: return launch_attn_half<float>(mq, mk, mv, prm, s);
-    case H3S_BF16: return launch_attn_half<__nv_bfloat16>(mq, mk, mv, prm, s);
-    default: return launch_attn_half<__half>(mq, mk, mv, prm, s);
+    case H3S_F32: return launch_attn_half<float>(mq, mk, mv, mo, prm, s);
+    case H3S_BF16: return launch_attn_half<__nv_bfloat16>(mq, mk, mv, mo, prm, s);
+    default: return launch_attn_half<__half>(mq, mk, mv, mo, prm, s);
   }
 }
