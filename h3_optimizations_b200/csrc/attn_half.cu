@@ -280,10 +280,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  int item = blockIdx.x;  // the first; more are asked for
-  HalfWork work = work_item(prm, item);
+  HalfWork work = work_item(prm, blockIdx.x);  // the first; more are asked for.  The loaders' own: the others read `sh.item`
+  int n_iter = work.n_iter;
 
   // ---- setup ----
+  let_next_start();
   if (threadIdx.x == 0) {
     ptx::mbar_init(&sh.next_ready, 1);
     ptx::mbar_init(&sh.q_full, 1);
@@ -310,16 +311,20 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     sh.abort_word = 0;
     sh.finish = 0;
     for (int i = 0; i < 4; ++i) sh.again[i] = 0;
+    sh.item[0].number = blockIdx.x;
     sh.item[0].head = work.head;
     sh.item[0].tq = work.tq;
+    sh.item[0].dense_row = work.dense_row;
+    sh.item[0].part = work.part;
     ptx::fence_mbar_init();
   }
   if (threadIdx.x < 2 * kHNoted / 32) (&sh.noted[0][0])[threadIdx.x] = 0u;
-  if (threadIdx.x < H3S_HEAD_DIM) sh.item[0].v_scale[threadIdx.x] = __ldg(prm.v_scale + work.head * H3S_HEAD_DIM + threadIdx.x);
   if (warp == kHValueIssuer) {
     ptx::tmem_alloc(&sh.tmem_base, kHTmemCols);
     ptx::tmem_relinquish();
   }
+  wait_for_previous();
+  if (threadIdx.x < H3S_HEAD_DIM) sh.item[0].v_scale[threadIdx.x] = __ldg(prm.v_scale + work.head * H3S_HEAD_DIM + threadIdx.x);
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -348,19 +353,13 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     arrive_pass();
     return wait_pass();
   };
-  auto count_noted = [&]() { return noted_tiles(sh.noted[items & 1], work.n_iter, note_scale(work.n_iter), lane); };
+  auto count_noted = [&]() { return noted_tiles(sh.noted[items & 1], n_iter, note_scale(n_iter), lane); };
   // after an item's last pass: the next one, if there is one
   auto next_item = [&]() {
     ++items;
     const HalfItem &next = sh.item[items % 3u];
-    item = next.number;
-    if (item < 0) return false;
-    work.head = next.head;
-    work.tq = next.tq;
-    work.n_iter = next.n_iter;
-    work.dense_row = next.dense_row;
-    work.part = next.part;
-    return true;
+    n_iter = next.n_iter;
+    return next.number >= 0;
   };
 
   if (warp == kHKeyLoader || warp == kHValueLoader) {
@@ -505,8 +504,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
       if (!ok || next < 0) break;
       ++items;
-      item = next;
       work = coming;
+      n_iter = work.n_iter;
       item_scale = coming_scale;
     }
   } else if (warp == kHScoreIssuer) {
@@ -526,7 +525,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         ptx::tc_commit(&sh.q_free);
       }
       __syncwarp();
-      int count = work.n_iter;
+      int count = n_iter;
       for (int pass = 0;; ++pass) {
         arrive_pass();  // nothing of the pass's end depends on this warp
         if (ptx::elect_one()) {
@@ -562,7 +561,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     int stage = 0;
     uint32_t round = 0;
     while (ok) {
-      int count = work.n_iter;
+      int count = n_iter;
       for (int pass = 0;; ++pass) {
         arrive_pass();  // nothing of the pass's end depends on this warp
         ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree, 4 * prm.wait_budget_ns);
@@ -624,8 +623,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
       return true;
     };
-    // whether the group's P columns are free, asked while there is other work; then certainly
-    auto room_already = [&](uint32_t j) { return ptx::mbar_test_wait(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u); };
+    // the group's P columns are free
     auto room = [&](uint32_t j) {
       return warp_wait(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
     };
@@ -717,7 +715,6 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     };
 
     while (ok) {
-      const int n_iter = work.n_iter;
       // Which of the four groups has the first tile depends on what the CTA has done before; sums are
       // added up in the order of the tiles all the same, so that a result does not depend on that.
       const int rank = (group - done) & (kHGroups - 1);
@@ -735,10 +732,9 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) return false;
           m = first_reference();
         }
-        const bool free_already = room_already(done + i);
         uint32_t packed[H3S_KV_TILE / 2];
         float sum = exp_sum<true, false>(s, c, -fmaf(c, kIntBias, m), packed);
-        if (!__all_sync(0xffffffffu, free_already) && !room(done + i)) return false;
+        if (!room(done + i)) return false;
         put(packed);
         const bool out = !(sum <= kHSumLimit);
         if (__any_sync(0xffffffffu, out)) {  // these rows leave the tile out
@@ -752,7 +748,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
           put(packed);
           if (lane == 0) {
-            const int coarse = note_scale(work.n_iter);
+            const int coarse = note_scale(n_iter);
             atomicOr(&sh.noted[items & 1][(i >> coarse) >> 5], 1u << ((i >> coarse) & 31));
             atomicOr(&sh.again[items & 3], far ? kAgainNoted | kAgainFar : kAgainNoted);
           }
@@ -764,7 +760,10 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (rank < n_iter) {
         ok = walk(rank, std::true_type{});
         if (ok && pending) ok = finish_last(sh.item[(items + 2) % 3u]);
-        for (int i = rank + kHGroups; ok && i < n_iter; i += kHGroups) ok = walk(i, std::false_type{});
+        if (ok) {
+          for (int i = rank + kHGroups; i < n_iter; i += kHGroups)
+            if (!walk(i, std::false_type{})) { ok = false; break; }
+        }
       }
       if (!ok) break;
       if (rank >= n_iter) {  // a group without a tile: the last item is not finished, and there is no reference point yet
@@ -853,6 +852,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // (this note's next item is the one after next, and its last reader has been at the pass's end)
         if (threadIdx.x < kHNoted / 32) sh.noted[items & 1][threadIdx.x] = 0u;
       }
+      const HalfItem &work = sh.item[items % 3u];
       const bool split = work.part >= 0;
       if (!split && prm.out_map) {
         pending = true;
@@ -926,7 +926,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (finish) {
         // Staged through shared memory: the four warps of a row quarter each write eight of the quarter's rows as
         // contiguous lines, and what goes to the peers is made of lines too.
-        normalise(o, l, sh.item[items % 3u]);
+        normalise(o, l, work);
         constexpr int kRowBytes = H3S_HEAD_DIM * static_cast<int>(sizeof(OutT));
         constexpr int kChunks = 32 * static_cast<int>(sizeof(OutT)) / 16;
         unsigned char *out_tile = smem + L::kOffOut;
@@ -959,9 +959,10 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     __nanosleep(200000);
     if (threadIdx.x == 0 && prm.status != nullptr) {
       if (atomicCAS(prm.status, 0, code) == 0) {
-        prm.status[1] = item;
-        prm.status[2] = work.head;
-        prm.status[3] = work.tq;
+        const HalfItem &at = sh.item[items % 3u];
+        prm.status[1] = at.number;
+        prm.status[2] = at.head;
+        prm.status[3] = at.tq;
       }
     }
   }
@@ -973,6 +974,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
 // E4M3 codes -> FP16 values: 16 per thread
 __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v8, uint4 *__restrict__ v16, int64_t chunks) {
+  let_next_start();
+  wait_for_previous();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= chunks) return;
   const uint4 codes = __ldg(v8 + i);
@@ -1043,8 +1046,7 @@ static int launch_attn_half(const CUtensorMap &mq, const CUtensorMap &mk, const 
   H3S_CHECK_CUDA(cudaFuncSetAttribute(sparse_attn_half_kernel<OutT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
   const int n_sparse = prm.route != nullptr ? prm.q_stop - prm.q_start : 0;
   const int items = prm.heads * ((prm.q_tiles - n_sparse) * prm.parts + n_sparse);
-  sparse_attn_half_kernel<OutT><<<items, kHThreads, kBytes, stream>>>(mq, mk, mv, mo, prm);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(sparse_attn_half_kernel<OutT>, items, kHThreads, kBytes, stream, mq, mk, mv, mo, prm));
   return H3S_OK;
 }
 
@@ -1056,9 +1058,8 @@ extern "C" int h3s_v_half(const uint8_t *v8t, void *v16t, int heads, int sequenc
   H3S_CHECK_ARG(heads > 0 && sequence > 0, "v_half: empty problem (heads=%d sequence=%d)", heads, sequence);
   H3S_CHECK_ARG(((reinterpret_cast<uintptr_t>(v8t) | reinterpret_cast<uintptr_t>(v16t)) & 15) == 0, "v_half: carriers must be 16-byte aligned");
   const int64_t chunks = static_cast<int64_t>(heads) * H3S_HEAD_DIM * (ceil_div(sequence, 128) * 128) / 16;
-  v_half_kernel<<<static_cast<unsigned>((chunks + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const uint4 *>(v8t), static_cast<uint4 *>(v16t), chunks);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(v_half_kernel, static_cast<unsigned>((chunks + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream),
+                             reinterpret_cast<const uint4 *>(v8t), static_cast<uint4 *>(v16t), chunks));
   return H3S_OK;
 }
 

@@ -35,6 +35,33 @@ constexpr int kSmCount = 148;  // of a B200, for the rules that deal out work
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// ---- launches that follow one another in a stream ----
+//
+// A kernel launched with `launch_next` may start while the kernel before it is still running: its blocks come as SMs get
+// free, set themselves up and stop at `wait_for_previous` until that kernel is complete and its writes are seen.  So every
+// thread of such a kernel calls it before it touches global memory, reads and writes alike; then a kernel is complete only
+// after all those before it are, whatever their kind.  `let_next_start` tells that this block does not mind; it stands at the
+// top, as the next kernel's blocks are only placed once every block of this one has been.  What is saved is the gap between
+// two kernels and the set-up of the second: MLP of 1000 x 3072 x 12288 (four kernels) 103 -> 95 us, of 33272 rows (36) 2595 ->
+// 2572, layer of 7 heads x 10384 tokens 141 -> 137, calls bound by the host unchanged.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = shared_bytes;
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 // ---- element loads: 8 consecutive channels of one row, widened to fp32 ----
 
 template <typename T>

@@ -67,6 +67,8 @@ __global__ void __launch_bounds__(kRotWarps * 32)
 convrot_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_stride, int rows, int hidden,
                           int8_t *__restrict__ out, float *__restrict__ scale_out) {
   extern __shared__ __align__(16) float rot_smem[];
+  let_next_start();
+  wait_for_previous();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = hidden / kRotGroup, stride = rot_stride(groups);
   float *mine = rot_smem + warp * 32 * stride;
@@ -685,6 +687,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int rank = ptx::cluster_rank();  // 0: issues the pair's MMAs
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
+  let_next_start();
   if (threadIdx.x == 0) {
     for (int i = 0; i < L::kStages; ++i) {
       ptx::mbar_init(&sh.full[i], 1);
@@ -704,6 +707,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     ptx::tmem_alloc_pair(&sh.tmem_base, kGemmTmemCols);
     ptx::tmem_relinquish_pair();
   }
+  wait_for_previous();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::cluster_sync();  // both CTAs' barriers are initialised
@@ -1313,9 +1317,8 @@ int h3s_convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hi
   const int smem = kRotWarps * 32 * rot_stride(hidden / kRotGroup) * static_cast<int>(sizeof(float));
   constexpr int kMostSmem = kRotWarps * 32 * rot_stride(32) * static_cast<int>(sizeof(float));  // 133 KB; one value for all callers
   H3S_CHECK_CUDA(cudaFuncSetAttribute(convrot_quant_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
-  convrot_quant_rows_kernel<<<ceil_div(rows, kRotWarps), kRotWarps * 32, smem, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16 *>(x), x_stride_row, rows, hidden, x_i8, x_scale);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(convrot_quant_rows_kernel, ceil_div(rows, kRotWarps), kRotWarps * 32, smem, static_cast<cudaStream_t>(stream),
+                             static_cast<const __nv_bfloat16 *>(x), x_stride_row, rows, hidden, x_i8, x_scale));
   return H3S_OK;
 }
 
@@ -1402,13 +1405,16 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
   if (carriers != nullptr) {
     H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeCarriers>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(GemmLayout<kModeCarriers>::kBytes)));
+    // Not `launch_next`: its blocks would take SMs one by one from the rotation of the rows that stands before it, whose last
+    // blocks share an SM four at a time (attention block of 33272 tokens 4995 us so, 4935 behind the complete rotation).
     qkv_gemm_kernel<kModeCarriers><<<grid, GemmWarps<kModeCarriers>::kThreads, GemmLayout<kModeCarriers>::kBytes, static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
+    H3S_CHECK_CUDA(cudaGetLastError());
   } else {
     H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeStaging>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(GemmLayout<kModeStaging>::kBytes)));
-    qkv_gemm_kernel<kModeStaging><<<grid, GemmWarps<kModeStaging>::kThreads, GemmLayout<kModeStaging>::kBytes, static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
+    H3S_CHECK_CUDA(launch_next(qkv_gemm_kernel<kModeStaging>, grid, GemmWarps<kModeStaging>::kThreads, GemmLayout<kModeStaging>::kBytes,
+                               static_cast<cudaStream_t>(stream), ma, mb, prm));
   }
-  H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
 }
 
@@ -1467,9 +1473,8 @@ int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_
   H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeDense>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(GemmLayout<kModeDense>::kBytes)));
   const int tiles = prm.m_pairs * prm.n_tiles;
-  qkv_gemm_kernel<kModeDense><<<2 * (tiles < sms / 2 ? tiles : sms / 2), GemmWarps<kModeDense>::kThreads, GemmLayout<kModeDense>::kBytes,
-                               static_cast<cudaStream_t>(stream)>>>(ma, mb, prm);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(qkv_gemm_kernel<kModeDense>, 2 * (tiles < sms / 2 ? tiles : sms / 2), GemmWarps<kModeDense>::kThreads,
+                             GemmLayout<kModeDense>::kBytes, static_cast<cudaStream_t>(stream), ma, mb, prm));
   return H3S_OK;
 }
 

@@ -26,6 +26,8 @@ column_stats_kernel(const T *__restrict__ k, int64_t k_stride_h, int64_t k_strid
                     int sequence, double *__restrict__ k_sum,
                     unsigned int *__restrict__ v_amax_bits) {
   __shared__ double red[kStatsThreads / 16][H3S_HEAD_DIM];
+  let_next_start();
+  wait_for_previous();
   const int head = blockIdx.y;
   const bool is_v = blockIdx.z == 1;
   const T *src = is_v ? v : k;
@@ -93,6 +95,8 @@ __global__ void column_stats_finalize_kernel(const double *__restrict__ k_sum,
                                              int total, int sequence, float v_bound,
                                              float *__restrict__ k_mean,
                                              float *__restrict__ v_scale) {
+  let_next_start();
+  wait_for_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   if (k_mean != nullptr) {
@@ -125,6 +129,8 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
   __shared__ float warp_amax[kThreads / 32];
   __shared__ double red[kSlots][H3S_HEAD_DIM];
 
+  let_next_start();
+  wait_for_previous();
   const int local_block = blockIdx.x;
   const int head = blockIdx.y;
   const int slot = threadIdx.x >> 4;
@@ -266,6 +272,8 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
                    const float *__restrict__ v_scale, uint8_t *__restrict__ out, uint16_t *__restrict__ out_half,
                    int rows, int row_start, int padded_total, float v_bound) {
   __shared__ __align__(16) uint8_t tile[H3S_HEAD_DIM * kVTile];
+  let_next_start();
+  wait_for_previous();
   const int head = blockIdx.y;
   const int first_row = blockIdx.x * kVTile;
   const int valid_rows = max(0, min(kVTile, rows - first_row));
@@ -389,6 +397,8 @@ template <int kChunks>  // 16-byte loads per lane
 __global__ void __launch_bounds__(kRowWarps * 32)
 quant_rows_fp8_warp_kernel(const __nv_bfloat16 *__restrict__ x, int64_t stride_row, int rows, int channels,
                            uint8_t *__restrict__ out, float *__restrict__ row_scale) {
+  let_next_start();
+  wait_for_previous();
   const int row = blockIdx.x * kRowWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const __nv_bfloat16 *src = x + row * stride_row;
@@ -430,6 +440,8 @@ __global__ void __launch_bounds__(kRowQuantThreads)
 quant_rows_fp8_kernel(const __nv_bfloat16 *__restrict__ x, int64_t stride_row, int rows, int channels,
                       uint8_t *__restrict__ out, float *__restrict__ row_scale) {
   __shared__ float warp_amax[kRowQuantThreads / 32];
+  let_next_start();
+  wait_for_previous();
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16 *src = x + row * stride_row;
     Elem<__nv_bfloat16>::Raw raw[kRowQuantMaxChunks];
@@ -492,13 +504,11 @@ static int launch_column_stats(const void *k, int64_t ksh, int64_t kss, const vo
   unsigned int *v_bits = reinterpret_cast<unsigned int *>(k_sum + heads * H3S_HEAD_DIM);
   H3S_CHECK_CUDA(cudaMemsetAsync(scratch, 0, h3s_column_stats_scratch_bytes(heads), stream));
   dim3 grid(ceil_div(sequence, kStatsRowsPerBlock), heads, 2);
-  column_stats_kernel<T><<<grid, kStatsThreads, 0, stream>>>(
-      static_cast<const T *>(k), ksh, kss, static_cast<const T *>(v), vsh, vss, sequence, k_sum, v_bits);
+  H3S_CHECK_CUDA(launch_next(column_stats_kernel<T>, grid, kStatsThreads, 0, stream, static_cast<const T *>(k), ksh, kss,
+                             static_cast<const T *>(v), vsh, vss, sequence, k_sum, v_bits));
   const int total = heads * H3S_HEAD_DIM;
-  column_stats_finalize_kernel<T><<<ceil_div(total, 256), 256, 0, stream>>>(
-      k_sum, v_bits, total, sequence, v_bound, k == nullptr ? nullptr : k_mean,
-      v == nullptr ? nullptr : v_scale);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(column_stats_finalize_kernel<T>, ceil_div(total, 256), 256, 0, stream, k_sum, v_bits, total, sequence,
+                             v_bound, k == nullptr ? nullptr : k_mean, v == nullptr ? nullptr : v_scale));
   return H3S_OK;
 }
 
@@ -510,16 +520,15 @@ static int launch_quant_qk(const void *x, int64_t sh, int64_t ss, const float *m
   const int blocks_total = ceil_div(sequence_total, block);
   dim3 grid(blocks, heads);
 #define H3S_LAUNCH_QK(BLOCK, HAS_MEAN)                                                               \
-  quant_qk_blocks_kernel<T, BLOCK, HAS_MEAN><<<grid, BLOCK * 2, 0, stream>>>(                         \
-      static_cast<const T *>(x), sh, ss, mean, out, scale, summary, summary_dtype, rows, row_start, \
-      sequence_total, blocks_total)
+  H3S_CHECK_CUDA(launch_next(quant_qk_blocks_kernel<T, BLOCK, HAS_MEAN>, grid, BLOCK * 2, 0, stream,                     \
+                             static_cast<const T *>(x), sh, ss, mean, out, scale, summary, summary_dtype, rows, row_start, \
+                             sequence_total, blocks_total))
   if (block == H3S_Q_TILE) {
     if (mean != nullptr) H3S_LAUNCH_QK(H3S_Q_TILE, true); else H3S_LAUNCH_QK(H3S_Q_TILE, false);
   } else {
     if (mean != nullptr) H3S_LAUNCH_QK(H3S_KV_TILE, true); else H3S_LAUNCH_QK(H3S_KV_TILE, false);
   }
 #undef H3S_LAUNCH_QK
-  H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
 }
 
@@ -532,9 +541,8 @@ static int launch_quant_v(const void *v, int64_t sh, int64_t ss, const float *v_
   const bool last = row_start + rows == sequence_total;
   const int covered = last ? padded_total - row_start : rows;
   dim3 grid(ceil_div(covered, kVTile), heads);
-  quant_v_fp8_kernel<T><<<grid, kVThreads, 0, stream>>>(static_cast<const T *>(v), sh, ss, v_scale, out,
-                                                        out_half, rows, row_start, padded_total, v_bound);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(quant_v_fp8_kernel<T>, grid, kVThreads, 0, stream, static_cast<const T *>(v), sh, ss, v_scale, out,
+                             out_half, rows, row_start, padded_total, v_bound));
   return H3S_OK;
 }
 
@@ -615,19 +623,17 @@ int h3s_quant_rows_fp8(const void *x_bf16, int64_t x_stride_row, int rows, int c
   H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(out) & 7) == 0, "quant_rows_fp8: output must be 8-byte aligned");
   const __nv_bfloat16 *bf16 = static_cast<const __nv_bfloat16 *>(x_bf16);
 #define H3S_LAUNCH_ROWS(CHUNKS)                                                                                  \
-  quant_rows_fp8_warp_kernel<CHUNKS><<<ceil_div(rows, kRowWarps), kRowWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>( \
-      bf16, x_stride_row, rows, channels, out, row_scale)
+  H3S_CHECK_CUDA(launch_next(quant_rows_fp8_warp_kernel<CHUNKS>, ceil_div(rows, kRowWarps), kRowWarps * 32, 0, \
+                             static_cast<cudaStream_t>(stream), bf16, x_stride_row, rows, channels, out, row_scale))
   if (channels <= 4096) {
     if (channels <= 1024) H3S_LAUNCH_ROWS(4); else if (channels <= 2048) H3S_LAUNCH_ROWS(8);
     else if (channels <= 3072) H3S_LAUNCH_ROWS(12); else H3S_LAUNCH_ROWS(16);
-    H3S_CHECK_CUDA(cudaGetLastError());
     return H3S_OK;
   }
 #undef H3S_LAUNCH_ROWS
   const int grid = rows < 148 * 8 ? rows : 148 * 8;
-  quant_rows_fp8_kernel<<<grid, kRowQuantThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16 *>(x_bf16), x_stride_row, rows, channels, out, row_scale);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(quant_rows_fp8_kernel, grid, kRowQuantThreads, 0, static_cast<cudaStream_t>(stream), bf16, x_stride_row,
+                             rows, channels, out, row_scale));
   return H3S_OK;
 }
 
@@ -644,11 +650,10 @@ int h3s_column_stats_finalize(const void *stats, int dtype, int heads, int seque
   const int total = heads * H3S_HEAD_DIM;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case H3S_F32: column_stats_finalize_kernel<float><<<ceil_div(total, 256), 256, 0, s>>>(k_sum, v_bits, total, sequence, v_bound, k_mean, v_scale); break;
-    case H3S_BF16: column_stats_finalize_kernel<__nv_bfloat16><<<ceil_div(total, 256), 256, 0, s>>>(k_sum, v_bits, total, sequence, v_bound, k_mean, v_scale); break;
-    default: column_stats_finalize_kernel<__half><<<ceil_div(total, 256), 256, 0, s>>>(k_sum, v_bits, total, sequence, v_bound, k_mean, v_scale); break;
+    case H3S_F32: H3S_CHECK_CUDA(launch_next(column_stats_finalize_kernel<float>, ceil_div(total, 256), 256, 0, s, k_sum, v_bits, total, sequence, v_bound, k_mean, v_scale)); break;
+    case H3S_BF16: H3S_CHECK_CUDA(launch_next(column_stats_finalize_kernel<__nv_bfloat16>, ceil_div(total, 256), 256, 0, s, k_sum, v_bits, total, sequence, v_bound, k_mean, v_scale)); break;
+    default: H3S_CHECK_CUDA(launch_next(column_stats_finalize_kernel<__half>, ceil_div(total, 256), 256, 0, s, k_sum, v_bits, total, sequence, v_bound, k_mean, v_scale)); break;
   }
-  H3S_CHECK_CUDA(cudaGetLastError());
   return H3S_OK;
 }
 

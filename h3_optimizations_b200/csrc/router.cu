@@ -41,6 +41,8 @@ route_topk_kernel(const T *__restrict__ q_summary, const T *__restrict__ k_summa
                   int kv_tiles, int q_start, int q_stop, int kv_start, int kv_stop, int retained,
                   int route_len, int32_t *__restrict__ route) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  let_next_start();
+  wait_for_previous();
   const int pure_q = q_stop - q_start;
   const int pure_kv = kv_stop - kv_start;
   double *scores = reinterpret_cast<double *>(smem_raw);              // [kRows][pure_kv]
@@ -213,10 +215,9 @@ static int launch_route_rows(const void *q_summary, const void *k_summary, int h
   // one value for all callers: a thread with shorter rows would take away what another one is about to launch with
   H3S_CHECK_CUDA(cudaFuncSetAttribute(route_topk_kernel<T, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRouteMostSmem)));
   dim3 grid(ceil_div(q_stop - q_start, kRows), heads);
-  route_topk_kernel<T, kRows><<<grid, kRows * 32, smem, stream>>>(
-      static_cast<const T *>(q_summary), static_cast<const T *>(k_summary), q_tiles, kv_tiles, q_start,
-      q_stop, kv_start, kv_stop, retained, route_len, route);
-  H3S_CHECK_CUDA(cudaGetLastError());
+  H3S_CHECK_CUDA(launch_next(route_topk_kernel<T, kRows>, grid, kRows * 32, smem, stream, static_cast<const T *>(q_summary),
+                             static_cast<const T *>(k_summary), q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained,
+                             route_len, route));
   return H3S_OK;
 }
 
