@@ -100,6 +100,10 @@ PROTOTYPES = {
     "h3s_sparse_attn_half_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                          c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
                                          c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "h3s_sparse_attn_half_fwd_mirrored": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                                  c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+                                                  c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p,
+                                                  c_void_p]),
     "h3s_sparse_attn_half_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
     "h3s_stream_order": (c_int, [c_void_p, c_void_p, c_void_p]),
     "h3s_quant_qkv": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,

@@ -18,9 +18,10 @@ the kernel return early and leave a code in a per-device status word that the
 backend hands to every launch.  Reading that word needs the stream to have
 drained, so it is not done on the hot path: ``check_status()`` reads it (and
 raises) whenever the caller synchronises anyway, ``forward_host`` calls it
-before it returns, and the next ``prepare`` on the device looks at the word
-through a pinned mirror filled by an asynchronous copy queued after the
-previous launch, without blocking.
+before it returns, and the next ``prepare`` on the device looks, without
+blocking, at a mirror of the word in pinned host memory that a kernel which
+gave up writes as well (with a copy behind every launch instead, the next
+call's kernels began 8 us later).
 """
 
 from __future__ import annotations
@@ -106,7 +107,7 @@ class B200SparseBackend:
 
             self.projector = ChunkedSparseQKVProjector()
         self.smooth_k = bool(smooth_k)
-        self._status = {}  # device index -> (device int32[4], pinned mirror, event of the last mirror copy)
+        self._status = {}  # device index -> (device int32[4], pinned mirror)
 
     # -- identity ---------------------------------------------------------
 
@@ -236,7 +237,7 @@ class B200SparseBackend:
         if slot is None:
             word = torch.zeros(4, dtype=torch.int32, device=device)
             mirror = torch.zeros(4, dtype=torch.int32).pin_memory()
-            slot = self._status[key] = (word, mirror, torch.cuda.Event())
+            slot = self._status[key] = (word, mirror)
         return slot
 
     @classmethod
@@ -249,11 +250,9 @@ class B200SparseBackend:
                 % (cls.ABORT_NAMES.get(code, "an unknown event"), code, cta, head, tile, where))
 
     def _poll_status(self, device):
-        """Non-blocking look at the mirror of the previous launch's status."""
-        if torch.cuda.is_current_stream_capturing():
-            return  # an event query is not allowed inside a capture; check_status() covers replays
+        """Non-blocking look at the mirror of the earlier launches' status."""
         slot = self._status.get(device.index if device.index is not None else torch.cuda.current_device())
-        if slot is not None and slot[2].query():
+        if slot is not None:
             self._raise_for(slot[1].tolist(), "reported by an earlier launch")
 
     def check_status(self, device=None):
@@ -377,21 +376,16 @@ class B200SparseBackend:
         route = sparse.route
         geometry = route.geometry
         device = sparse.q_int8.device
-        word, mirror, copied = self._status_slot(device)
+        word, mirror = self._status_slot(device)
         v = VCarrier.of(sparse)
         try:
             out_dtype = sparse.output_dtype
-            result = ops.sparse_attention(
+            return ops.sparse_attention(
                 sparse.q_int8, sparse.k_int8, v.codes, sparse.q_scale, sparse.k_scale,
                 sparse.v_scale, route.indices,
                 q_start=geometry.pure_video_q_start, q_stop=geometry.pure_video_q_stop,
-                out=out, out_dtype=out_dtype, status=word, peer_out_ptrs=peer_out_ptrs, v_half=v.half,
+                out=out, out_dtype=out_dtype, status=word, status_mirror=mirror, peer_out_ptrs=peer_out_ptrs, v_half=v.half,
             )
-            if not torch.cuda.is_current_stream_capturing():
-                # (an event recorded inside a capture could not be queried afterwards: replays are
-                # covered by check_status(), which reads the device word itself)
-                ops.status_mirror(word, mirror, copied, _native.stream_ptr(device))
-            return result
         except _native.NativeError as exc:
             raise SparseSageError(
                 "Sparse attention kernel failed: layer=%d sequence=%d heads=%d dtype=%s: %s"

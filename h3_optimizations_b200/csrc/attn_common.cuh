@@ -23,6 +23,7 @@ struct AttnParams {
   const int32_t *route;  // (heads, q_stop-q_start, route_len) or null
   void *out;
   int32_t *status;
+  int32_t *status_mirror;  // pinned host memory that gets the words too, or null (attn_half.cu)
   int64_t out_stride_h, out_stride_s;
   int route_len, q_start, q_stop;
   // A dense row's tile list may be cut into `parts` even parts, an item each (attn_half.cu); 1: not cut.  partial: per dense row and part 128 x 128 sums of P.V, 128 row sums and 128 reference points;

@@ -963,6 +963,14 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         prm.status[1] = at.number;
         prm.status[2] = at.head;
         prm.status[3] = at.tq;
+        if (prm.status_mirror != nullptr) {
+          volatile int32_t *mirror = prm.status_mirror;
+          mirror[1] = at.number;
+          mirror[2] = at.head;
+          mirror[3] = at.tq;
+          __threadfence_system();
+          mirror[0] = code;
+        }
       }
     }
   }
@@ -1073,12 +1081,12 @@ extern "C" size_t h3s_sparse_attn_half_workspace_bytes(int heads, int sequence, 
   return parts > 1 ? split_bytes(static_cast<int64_t>(heads) * (q_tiles - n_sparse), parts, &arrived_bytes) : 0;
 }
 
-extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, const void *v16t, const float *q_scale,
-                                        const float *k_scale, const float *v_scale, const int32_t *route,
-                                        int route_len, int q_start, int q_stop, void *out, void *const *peer_out,
-                                        int n_peer_out, int out_dtype, int64_t out_stride_h, int64_t out_stride_s,
-                                        int heads, int sequence, int flags, void *workspace, size_t workspace_bytes,
-                                        int32_t *status, h3s_stream_t stream) {
+extern "C" int h3s_sparse_attn_half_fwd_mirrored(const int8_t *q8, const int8_t *k8, const void *v16t, const float *q_scale,
+                                                 const float *k_scale, const float *v_scale, const int32_t *route,
+                                                 int route_len, int q_start, int q_stop, void *out, void *const *peer_out,
+                                                 int n_peer_out, int out_dtype, int64_t out_stride_h, int64_t out_stride_s,
+                                                 int heads, int sequence, int flags, void *workspace, size_t workspace_bytes,
+                                                 int32_t *status, int32_t *host_mirror, h3s_stream_t stream) {
   using namespace h3s;
   AttnParams prm;
   int rc = fill_attn_params(&prm, q8, k8, v16t, q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out,
@@ -1098,6 +1106,7 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
                              H3S_KV_TILE * 2, H3S_HEAD_DIM, CU_TENSOR_MAP_SWIZZLE_128B, "sparse_attn_half_fwd V map");
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  prm.status_mirror = host_mirror;
   prm.parts = 1; prm.partial = nullptr; prm.arrived = nullptr;
   // One head's stride is never used and need not suit a map; with peers the tile is staged as a whole instead
   const uint64_t size = out_dtype == H3S_F32 ? 4 : 2;
@@ -1127,4 +1136,15 @@ extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, cons
     case H3S_BF16: return launch_attn_half<__nv_bfloat16>(mq, mk, mv, mo, prm, s);
     default: return launch_attn_half<__half>(mq, mk, mv, mo, prm, s);
   }
+}
+
+extern "C" int h3s_sparse_attn_half_fwd(const int8_t *q8, const int8_t *k8, const void *v16t, const float *q_scale,
+                                        const float *k_scale, const float *v_scale, const int32_t *route,
+                                        int route_len, int q_start, int q_stop, void *out, void *const *peer_out,
+                                        int n_peer_out, int out_dtype, int64_t out_stride_h, int64_t out_stride_s,
+                                        int heads, int sequence, int flags, void *workspace, size_t workspace_bytes,
+                                        int32_t *status, h3s_stream_t stream) {
+  return h3s_sparse_attn_half_fwd_mirrored(q8, k8, v16t, q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out, peer_out,
+                                           n_peer_out, out_dtype, out_stride_h, out_stride_s, heads, sequence, flags, workspace,
+                                           workspace_bytes, status, nullptr, stream);
 }

@@ -614,7 +614,7 @@ def new_attention_output(heads, sequence, dtype, device):
 
 def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *, q_start=0, q_stop=0,
                      out=None, out_dtype=torch.bfloat16, status=None, legacy_mma=False, single_term_p=False,
-                     peer_out_ptrs=None, extra_flags=0, v_half=None, two_term_p=False):
+                     peer_out_ptrs=None, extra_flags=0, v_half=None, two_term_p=False, status_mirror=None):
     """Launch the attention kernel.  Returns ``out`` (HND).  ``single_term_p``
     carries the probabilities as one E4M3 term instead of in FP16, ``two_term_p``
     as two; both work on the carrier itself and make no copy of it.
@@ -622,7 +622,9 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
     keeps one; made here otherwise.
     ``peer_out_ptrs``: device addresses (ints) of up to 7 further buffers,
     addressed like ``out``, that receive every output tile as well (the slices
-    of the peer GPUs' full outputs in a head-sharded run)."""
+    of the peer GPUs' full outputs in a head-sharded run).
+    ``status_mirror``: pinned int32[4] that a launch which sets ``status`` writes too
+    (the FP16 kernel only)."""
     lib = _native.load()
     if out is None:
         out = new_attention_output(q8.shape[1], q8.shape[2], out_dtype, q8.device)
@@ -652,6 +654,6 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
             check_v_half(v_half, v_carrier)
         size = lib.h3s_sparse_attn_half_workspace_bytes(heads, sequence, route_len, int(q_start), int(q_stop))
         workspace = torch.empty(size, dtype=torch.uint8, device=q8.device) if size else None
-        check(lib.h3s_sparse_attn_half_fwd(ptr(q8), ptr(k8), ptr(v_half), *before, table, n_peers, *after,
-                                           ptr(workspace), size, ptr(status), stream), "h3s_sparse_attn_half_fwd")
+        check(lib.h3s_sparse_attn_half_fwd_mirrored(ptr(q8), ptr(k8), ptr(v_half), *before, table, n_peers, *after, ptr(workspace),
+                                                    size, ptr(status), ptr(status_mirror), stream), "h3s_sparse_attn_half_fwd")
     return out
