@@ -154,7 +154,7 @@ def check(status, what):
 
 
 def ptr(tensor):
-    return None if tensor is None else c_void_p(tensor.data_ptr())
+    return None if tensor is None else tensor.data_ptr()
 
 
 def stream_ptr(device=None):

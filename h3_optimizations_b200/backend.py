@@ -29,12 +29,16 @@ from __future__ import annotations
 import torch
 
 from . import _native, ops
-from .carriers import PreparedFusedQKV, PreparedHybrid, PreparedSparse, VCarrier, validate_prepared_fused_qkv
+from .carriers import PreparedFusedQKV, PreparedHybrid, PreparedLayer, PreparedSparse, VCarrier, validate_prepared_fused_qkv
 from .config import MODE_SAGE128_FUSED_QKV, HybridSparseConfig, resolve_video_budget
 from .errors import FusedQKVError, SparseRouterError, SparseSageError
 from .router import KV_TILE, Q_TILE, SparseTileRouter
 from .runtime import get_runtime_snapshot
 
+# Rows of all heads up to which a layer is prepared on one stream.  us a call, two streams / one: 1 head x 1128 tokens 106 / 90,
+# 4 x 2304 108 / 96, 6 x 4256 114 / 98, 24 x 1328 106 / 93, 4 x 9256 112 / 110, 12 x 4256 104 / 94; with the device waited for
+# after each call 126 / 110, 130 / 123, 140 / 133, 127 / 121, 170 / 165, 152 / 145.  Beyond, the kernels take longer than the host.
+ONE_STREAM_ROWS = 52000
 V_QUANT_BOUND = 448.0  # FP32 accumulation (reference: sparse_sage.py:296)
 
 
@@ -292,8 +296,9 @@ class B200SparseBackend:
             # buffer is allocated on the current stream, which both chains rejoin before
             # returning.  One native call issues all of it (4 heads x 2304
             # tokens, where host time is all there is: 236 -> 135 us).
+            # Short calls are over before the host has issued them: there one stream saves the host the events.
             stream = _native.stream_ptr(q.device)
-            side = self._side_stream(q.device)
+            side = self._side_stream(q.device) if heads * sequence > ONE_STREAM_ROWS else None
             buffers = ops.LayerBuffers(heads, sequence, q.device, smooth_k=self.smooth_k,
                                        summary_dtype=torch.float64 if need_route else None)
             try:
@@ -311,19 +316,17 @@ class B200SparseBackend:
             finally:
                 # on every exit path the main stream is ordered after the second one, so the
                 # allocator cannot hand these buffers to someone else while it still runs
-                side.join(stream)
+                if side is not None:
+                    side.join(stream)
         except SparseRouterError as exc:
             raise SparseSageError("sparse routing failed: %s" % exc) from exc
         except _native.NativeError as exc:
             raise SparseSageError("carrier preparation failed: layer=%d: %s" % (layer_index, exc)) from exc
-        sparse = PreparedSparse(
-            q_int8=buffers.q_int8, k_int8=buffers.k_int8, v_carrier=buffers.v_carrier, q_scale=buffers.q_scale,
-            k_scale=buffers.k_scale, v_scale=buffers.v_scale, route=route, output_dtype=q.dtype,
-            output_shape=tuple(q.shape), layer_index=int(layer_index), sequence=int(sequence), heads=int(heads),
-            metadata=self._metadata(route.metadata, layer_index, heads), v_half=buffers.v_half,
-        )
-        sparse.metadata["smooth_k"] = bool(self.smooth_k)
-        return PreparedHybrid(sparse=sparse)
+        buffers.release_call()
+        metadata = self._metadata(route.metadata, layer_index, heads)
+        metadata["smooth_k"] = self.smooth_k
+        return PreparedHybrid(sparse=PreparedLayer.over(
+            buffers, route=route, output_dtype=q.dtype, output_shape=tuple(q.shape), layer_index=int(layer_index), metadata=metadata))
 
     def prepare_projected(self, projected, *, layer_index, transformer_options):
         try:
@@ -375,11 +378,16 @@ class B200SparseBackend:
         sparse = prepared.sparse
         route = sparse.route
         geometry = route.geometry
-        device = sparse.q_int8.device
+        buffers = sparse.untouched() if isinstance(sparse, PreparedLayer) else None
+        device = sparse.q_int8.device if buffers is None else buffers.device
         word, mirror = self._status_slot(device)
-        v = VCarrier.of(sparse)
         try:
             out_dtype = sparse.output_dtype
+            if buffers is not None:
+                return ops.sparse_attention_of(
+                    buffers, route.indices, q_start=geometry.pure_video_q_start, q_stop=geometry.pure_video_q_stop, out=out,
+                    out_dtype=out_dtype, status=word, status_mirror=mirror, peer_out_ptrs=peer_out_ptrs)
+            v = VCarrier.of(sparse)
             return ops.sparse_attention(
                 sparse.q_int8, sparse.k_int8, v.codes, sparse.q_scale, sparse.k_scale,
                 sparse.v_scale, route.indices,

@@ -3,7 +3,7 @@ attention/sparse/sparse_sage.py:401-417)."""
 
 from __future__ import annotations
 
-from dataclasses import InitVar, dataclass, field
+from dataclasses import InitVar, dataclass, field, fields
 
 import torch
 
@@ -168,6 +168,40 @@ class PreparedSparse:
 
 
 PreparedSparse.v_carrier = VCarrier.field()
+
+
+class PreparedLayer(PreparedSparse):
+    """A ``PreparedSparse`` whose carriers are those of an ``ops.LayerBuffers`` (``over``).  Its tensors come into being
+    when they are asked for; until then (``untouched``) nobody can have written to them or put others in their place."""
+
+    _LAZY = frozenset(("q_int8", "k_int8", "q_scale", "k_scale", "v_scale", "_v"))
+
+    @classmethod
+    def over(cls, buffers, **rest):
+        prepared = object.__new__(cls)
+        prepared.__dict__.update(rest, sequence=buffers.sequence, heads=buffers.heads, _buffers=buffers)
+        return prepared
+
+    def __getattr__(self, name):  # of what the instance does not hold (yet)
+        buffers = self.__dict__.get("_buffers")
+        if buffers is None or name not in PreparedLayer._LAZY:
+            raise AttributeError("%r object has no attribute %r" % (type(self).__name__, name))
+        if name == "_v":
+            value, buffers.v_half = VCarrier(buffers.tensor("v_carrier"), buffers.v_half), None
+        else:
+            value = buffers.tensor(name)
+        self.__dict__[name] = value
+        return value
+
+    def untouched(self):
+        """The buffers, if no tensor of them has been handed out or replaced."""
+        buffers = self.__dict__.get("_buffers")
+        if buffers is None or buffers.v_half is None or not PreparedLayer._LAZY.isdisjoint(self.__dict__):
+            return None
+        return buffers
+
+    def __reduce_ex__(self, protocol):  # a copy is a PreparedSparse of its own tensors
+        return PreparedSparse, tuple(getattr(self, f.name) for f in fields(PreparedSparse))
 
 
 @dataclass

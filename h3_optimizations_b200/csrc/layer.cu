@@ -34,11 +34,12 @@ int h3s_quant_qkv(const h3s_layer_carriers *c, const void *q, const void *k, con
                   int dtype, int heads, int sequence, int smooth_k, float v_bound, int v_after_k, void *event,
                   h3s_stream_t stream, h3s_stream_t side_stream) {
   using namespace h3s;
-  H3S_CHECK_ARG(c != nullptr && strides != nullptr && event != nullptr, "quant_qkv: NULL argument");
+  const bool forked = side_stream != stream;  // else one stream does it all, in the same order
+  H3S_CHECK_ARG(c != nullptr && strides != nullptr && (event != nullptr || !forked), "quant_qkv: NULL argument");
   H3S_CHECK_ARG(q != nullptr && k != nullptr && v != nullptr, "quant_qkv: NULL input");
   cudaStream_t s = static_cast<cudaStream_t>(stream), side = static_cast<cudaStream_t>(side_stream);
   const float *mean = smooth_k ? c->k_mean : nullptr;
-  int rc = order_after(s, side, event);
+  int rc = forked ? order_after(s, side, event) : H3S_OK;
   if (rc) return rc;
   rc = h3s_column_stats(smooth_k ? k : nullptr, strides[2], strides[3], v, strides[4], strides[5], dtype, heads,
                         sequence, v_bound, smooth_k ? c->k_mean : nullptr, c->v_scale, c->scratch, side);
@@ -47,12 +48,12 @@ int h3s_quant_qkv(const h3s_layer_carriers *c, const void *q, const void *k, con
   rc = h3s_quant_qk_blocks(q, dtype, strides[0], strides[1], nullptr, c->q8, c->q_scale, c->q_summary,
                            c->summary_dtype, heads, sequence, 0, sequence, H3S_Q_TILE, s);
   if (rc) return rc;
-  rc = order_after(side, s, event);
+  rc = forked ? order_after(side, s, event) : H3S_OK;
   if (rc) return rc;
   rc = h3s_quant_qk_blocks(k, dtype, strides[2], strides[3], mean, c->k8, c->k_scale, c->k_summary, c->summary_dtype,
                            heads, sequence, 0, sequence, H3S_KV_TILE, s);
   if (rc) return rc;
-  if (v_after_k) {
+  if (v_after_k && forked) {
     rc = order_after(s, side, event);
     if (rc) return rc;
   }

@@ -232,31 +232,71 @@ class SideStream:
 
 class LayerBuffers:
     """Carriers, scales, tile means and scratch of one layer call (batch 1), as ``h3s_quant_qkv`` and
-    ``h3s_project_qkv`` fill them; all allocated on the current stream."""
+    ``h3s_project_qkv`` fill them; all allocated on the current stream.
+
+    Three allocations: the carriers and scales that outlive the call, the FP16 copy of V (which may be dropped
+    before them), and the tile means with what only the call needs.  The native calls go by addresses, so the tensors
+    ``q_int8``, ``k_int8``, ``v_carrier``, ``q_scale``, ``k_scale`` and ``v_scale`` come into being when somebody asks for them: all
+    of them, each in an allocation of its own, took 31 us of a call (4 heads x 2304 tokens, where host time is all there is)."""
 
     def __init__(self, heads, sequence, device, *, smooth_k, summary_dtype):
-        lib = _native.load()
-        q_blocks, k_blocks = _ceil_div(sequence, Q_TILE), _ceil_div(sequence, KV_TILE)
-        shape, small = (1, heads, sequence, HEAD_DIM), (1, heads, HEAD_DIM)
-        self.q_int8 = torch.empty(shape, dtype=torch.int8, device=device)
-        self.k_int8 = torch.empty(shape, dtype=torch.int8, device=device)
-        self.q_scale = torch.empty((1, heads, q_blocks), dtype=torch.float32, device=device)
-        self.k_scale = torch.empty((1, heads, k_blocks), dtype=torch.float32, device=device)
-        self.q_summary = self.k_summary = self.k_mean = None
+        q_blocks, k_blocks = -(-sequence // Q_TILE), -(-sequence // KV_TILE)
+        padded = -(-sequence // 128) * 128
+        codes, v_codes, column = heads * sequence * HEAD_DIM, heads * HEAD_DIM * padded, heads * HEAD_DIM
+        self.heads, self.sequence, self.device = heads, sequence, device
+        # byte offsets; every size is rounded up to 256
+        k_at = _round256(codes)
+        v_at = k_at + k_at
+        q_scale_at = v_at + _round256(v_codes)
+        k_scale_at = q_scale_at + _round256(4 * heads * q_blocks)
+        v_scale_at = k_scale_at + _round256(4 * heads * k_blocks)
+        self._at = {"q_int8": 0, "k_int8": k_at, "v_carrier": v_at, "q_scale": q_scale_at, "k_scale": k_scale_at, "v_scale": v_scale_at}
+        self._carriers = carriers = torch.empty(v_scale_at + _round256(4 * column), dtype=torch.int8, device=device)
+        self.v_half = torch.empty((1, heads, HEAD_DIM, padded), dtype=torch.float16, device=device)
+        # statistics scratch and the K mean in front, so that the tile means may have any element size
+        mean_at = _round256(_native.load().h3s_column_stats_scratch_bytes(heads))
+        means_at = mean_at + (_round256(4 * column) if smooth_k else 0)
+        size = 0 if summary_dtype is None else summary_dtype.itemsize
+        k_means_at = means_at + _round256(size * column * q_blocks)
+        self._call = call = torch.empty(k_means_at + _round256(size * column * k_blocks), dtype=torch.uint8, device=device)
+        self.q_summary = self.k_summary = None
         if summary_dtype is not None:
-            self.q_summary = torch.empty((1, heads, q_blocks, HEAD_DIM), dtype=summary_dtype, device=device)
-            self.k_summary = torch.empty((1, heads, k_blocks, HEAD_DIM), dtype=summary_dtype, device=device)
-        if smooth_k:
-            self.k_mean = torch.empty(small, dtype=torch.float32, device=device)
-        self.v_scale = torch.empty(small, dtype=torch.float32, device=device)
-        self.v_carrier = allocate_v_carrier(sequence, heads, device)
-        self.v_half = torch.empty(self.v_carrier.shape, dtype=torch.float16, device=device)
-        self.scratch = torch.empty(lib.h3s_column_stats_scratch_bytes(heads), dtype=torch.uint8, device=device)
+            means = call.view(summary_dtype)
+            self.q_summary = _view(means, (1, heads, q_blocks, HEAD_DIM), means_at // size)
+            self.k_summary = _view(means, (1, heads, k_blocks, HEAD_DIM), k_means_at // size)
+        base, own = carriers.data_ptr(), call.data_ptr()
         self.native = _native.LayerCarriers(
-            self.q_int8.data_ptr(), self.q_scale.data_ptr(), _address(self.q_summary),
-            self.k_int8.data_ptr(), self.k_scale.data_ptr(), _address(self.k_summary),
-            _address(self.k_mean), self.v_scale.data_ptr(), self.v_carrier.data_ptr(), self.v_half.data_ptr(),
-            self.scratch.data_ptr(), 0 if summary_dtype is None else dtype_code(summary_dtype))
+            base, base + q_scale_at, own + means_at if size else None,
+            base + k_at, base + k_scale_at, own + k_means_at if size else None,
+            own + mean_at if smooth_k else None, base + v_scale_at, base + v_at, self.v_half.data_ptr(),
+            own, 0 if summary_dtype is None else dtype_code(summary_dtype))
+
+    def release_call(self):
+        """Give up what only the call that fills the carriers needs (the caller's stream is behind it)."""
+        self._call = self.q_summary = self.k_summary = None
+
+    def tensor(self, name):
+        """The named carrier or scale."""
+        heads, sequence, at = self.heads, self.sequence, self._at[name]
+        if name == "v_carrier":
+            return _view(self._carriers.view(torch.float8_e4m3fn), (1, heads, HEAD_DIM, -(-sequence // 128) * 128), at)
+        if name in ("q_int8", "k_int8"):
+            return _view(self._carriers, (1, heads, sequence, HEAD_DIM), at)
+        last = {"q_scale": -(-sequence // Q_TILE), "k_scale": -(-sequence // KV_TILE), "v_scale": HEAD_DIM}[name]
+        return _view(self._carriers.view(torch.float32), (1, heads, last), at // 4)
+
+
+def _round256(n):
+    return (n + 255) & ~255
+
+
+def _view(base, shape, offset):
+    """A contiguous tensor of ``shape`` inside one-dimensional ``base``, ``offset`` elements behind its start."""
+    strides, step = [], 1
+    for n in reversed(shape):
+        strides.append(step)
+        step *= n
+    return base.as_strided(shape, strides[::-1], offset)
 
 
 def _address(tensor):
@@ -265,12 +305,13 @@ def _address(tensor):
 
 def quant_qkv(q, k, v, buffers, side, stream, *, smooth_k, v_after_k, v_bound=FP8_V_BOUND):
     """Carriers of HND ``q``, ``k``, ``v`` into ``buffers``, on ``stream`` (the raw handle of the current
-    stream) and ``side``.  The caller joins ``side`` on every path, before the buffers can be freed."""
+    stream) and, where given, ``side``.  The caller joins ``side`` on every path, before the buffers can be freed."""
     strides = (ctypes.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
     check(
         _native.load().h3s_quant_qkv(
             buffers.native, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, dtype_code(q.dtype), q.shape[1], q.shape[2],
-            int(smooth_k), v_bound, int(v_after_k), side.event_handle, stream, side.handle),
+            int(smooth_k), v_bound, int(v_after_k), None if side is None else side.event_handle, stream,
+            stream if side is None else side.handle),
         "h3s_quant_qkv",
     )
 
@@ -282,21 +323,21 @@ def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, s
     if x.stride(1) != 1:
         raise _native.NativeError("project_qkv: x must have contiguous rows")
     sequence, hidden = x.shape
-    device, rows = x.device, min(chunk_rows, sequence)
-    x_i8 = torch.empty((rows, hidden), dtype=torch.int8, device=device)
-    x_scale = torch.empty((rows,), dtype=torch.float32, device=device)
-    # bf16 staging of what needs whole-sequence statistics before it can be quantised
-    shape = (1, heads, sequence, HEAD_DIM)
-    v_stage = torch.empty(shape, dtype=torch.bfloat16, device=device)
-    k_stage = torch.empty(shape, dtype=torch.bfloat16, device=device) if smooth_k else None
+    rows = min(chunk_rows, sequence)
+    # one chunk's codes and scales, and bf16 staging of what needs whole-sequence statistics before it can be quantised
+    stage = _round256(2 * heads * sequence * HEAD_DIM)
+    scale_at = stage * (2 if smooth_k else 1)
+    codes_at = scale_at + _round256(4 * rows)
+    scratch = torch.empty(codes_at + rows * hidden, dtype=torch.uint8, device=x.device)
+    base = scratch.data_ptr()
     rope_code, strides = 0, None
     if rope is not None:
         rope_code = dtype_code(rope.dtype)
         strides = (ctypes.c_int64 * 4)(rope.stride(1), rope.stride(3), rope.stride(4), rope.stride(5))
     check(
         _native.load().h3s_project_qkv(
-            buffers.native, x.data_ptr(), x.stride(0), sequence, hidden, chunk_rows, x_i8.data_ptr(), x_scale.data_ptr(),
-            w_i8.data_ptr(), w_scale.data_ptr(), heads, int(smooth_k), _address(k_stage), v_stage.data_ptr(),
+            buffers.native, x.data_ptr(), x.stride(0), sequence, hidden, chunk_rows, base + codes_at, base + scale_at,
+            w_i8.data_ptr(), w_scale.data_ptr(), heads, int(smooth_k), base + stage if smooth_k else None, base,
             _address(q_norm), _address(k_norm), epsilon, _address(rope), rope_code, strides, v_bound, _address(status),
             side.event_handle, stream, side.handle),
         "h3s_project_qkv",
@@ -575,11 +616,7 @@ def _attn_args(q8, k8, v_carrier, q_scale, k_scale, v_scale, route, q_start, q_s
             or tuple(k_scale.shape) != (1, heads, _ceil_div(sequence, KV_TILE))
             or tuple(v_scale.shape) != (1, heads, HEAD_DIM)):
         raise _native.NativeError("sparse_attention: scale shapes do not agree")
-    route_len = 0
-    if route is not None:
-        if route.dtype != torch.int32 or not route.is_contiguous() or tuple(route.shape[:3]) != (1, heads, q_stop - q_start):
-            raise _native.NativeError("sparse_attention: route must be contiguous int32 (1,H,%d,len)" % (q_stop - q_start))
-        route_len = route.shape[-1]
+    route_len = _route_length(route, heads, q_stop - q_start)
     if out.shape != q8.shape or out.stride(-1) != 1:
         raise _native.NativeError("sparse_attention: output must be (1,H,S,128) with a contiguous last dimension")
     return heads, sequence, route_len
@@ -608,8 +645,42 @@ def check_v_half(v_half, v_carrier):
 def new_attention_output(heads, sequence, dtype, device):
     """HND view of a token-major ``(S, H*128)`` buffer, so the caller's
     transpose+reshape before ``out_proj`` (attention_forward.py:123-128) is free."""
-    base = torch.empty((1, sequence, heads, HEAD_DIM), dtype=dtype, device=device)
-    return base.permute(0, 2, 1, 3)
+    return torch.empty_strided((1, heads, sequence, HEAD_DIM), (sequence * heads * HEAD_DIM, HEAD_DIM, heads * HEAD_DIM, 1),
+                               dtype=dtype, device=device)
+
+
+def sparse_attention_of(buffers, route, *, q_start, q_stop, out, out_dtype, status, status_mirror, peer_out_ptrs):
+    """``sparse_attention`` on the carriers of ``LayerBuffers`` that nobody else has been handed: they are as they were
+    made, so that only the route and the output are looked at."""
+    heads, sequence, device = buffers.heads, buffers.sequence, buffers.device
+    if out is None:
+        out = new_attention_output(heads, sequence, out_dtype, device)
+    elif tuple(out.shape) != (1, heads, sequence, HEAD_DIM) or out.stride(-1) != 1:
+        raise _native.NativeError("sparse_attention: output must be (1,H,S,128) with a contiguous last dimension")
+    lib = _native.load()
+    route_len = _route_length(route, heads, q_stop - q_start)
+    table, n_peers = _peer_table(peer_out_ptrs)
+    size = lib.h3s_sparse_attn_half_workspace_bytes(heads, sequence, route_len, q_start, q_stop)
+    workspace = torch.empty(size, dtype=torch.uint8, device=device) if size else None
+    c = buffers.native
+    check(lib.h3s_sparse_attn_half_fwd_mirrored(
+        c.q8, c.k8, c.v16, c.q_scale, c.k_scale, c.v_scale, ptr(route), route_len, q_start, q_stop, out.data_ptr(), table, n_peers,
+        dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence, 0, ptr(workspace), size, status.data_ptr(),
+        status_mirror.data_ptr(), stream_ptr(device)), "h3s_sparse_attn_half_fwd")
+    return out
+
+
+def _route_length(route, heads, rows):
+    if route is None:
+        return 0
+    if route.dtype != torch.int32 or not route.is_contiguous() or tuple(route.shape[:3]) != (1, heads, rows):
+        raise _native.NativeError("sparse_attention: route must be contiguous int32 (1,H,%d,len)" % rows)
+    return route.shape[-1]
+
+
+def _peer_table(peer_out_ptrs):
+    n_peers = len(peer_out_ptrs or ())
+    return ((ctypes.c_void_p * n_peers)(*[ctypes.c_void_p(int(p)) for p in peer_out_ptrs]) if n_peers else None), n_peers
 
 
 def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *, q_start=0, q_stop=0,
@@ -630,11 +701,9 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
         out = new_attention_output(q8.shape[1], q8.shape[2], out_dtype, q8.device)
     heads, sequence, route_len = _attn_args(q8, k8, v_carrier, q_scale, k_scale, v_scale, route, q_start, q_stop, out)
     flags = (ATTN_P_SINGLE if single_term_p else 0) | int(extra_flags)
-    table, n_peers = None, len(peer_out_ptrs or ())
-    if n_peers:
-        if legacy_mma:
-            raise _native.NativeError("sparse_attention: the cross-check kernel does not scatter to peers")
-        table = (ctypes.c_void_p * n_peers)(*[ctypes.c_void_p(int(p)) for p in peer_out_ptrs])
+    table, n_peers = _peer_table(peer_out_ptrs)
+    if n_peers and legacy_mma:
+        raise _native.NativeError("sparse_attention: the cross-check kernel does not scatter to peers")
     before = (ptr(q_scale), ptr(k_scale), ptr(v_scale), ptr(route), route_len, int(q_start), int(q_stop), ptr(out))
     after = (dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence, flags)
     stream = stream_ptr(q8.device)

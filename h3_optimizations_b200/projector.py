@@ -157,9 +157,10 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
         raise FusedQKVError("chunked QKV projection failed: layer=%d: %s" % (layer_index, exc)) from exc
     return validate_prepared_fused_qkv(
         PreparedFusedQKV(
-            q_int8=buffers.q_int8, q_scale=buffers.q_scale, k_int8=buffers.k_int8, k_scale=buffers.k_scale, v=None,
+            q_int8=buffers.tensor("q_int8"), q_scale=buffers.tensor("q_scale"), k_int8=buffers.tensor("k_int8"),
+            k_scale=buffers.tensor("k_scale"), v=None,
             q_summary=buffers.q_summary, k_summary=buffers.k_summary, output_dtype=x.dtype, sequence=sequence,
             heads=heads, head_dim=HEAD_DIM, layer_index=int(layer_index), smooth_k=bool(smooth_k),
-            v_carrier=buffers.v_carrier, v_scale=buffers.v_scale, v_half=buffers.v_half,
+            v_carrier=buffers.tensor("v_carrier"), v_scale=buffers.tensor("v_scale"), v_half=buffers.v_half,
         )
     )
