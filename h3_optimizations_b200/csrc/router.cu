@@ -12,7 +12,7 @@
 // order, so no sort is needed.
 // It is bound by those reads, which go through L2, where there are many CTAs, and by latency where there are
 // few: 24 x 256 rows of 512 scores 85 us, 24 x 591 of 1181 370 us (98 and 685 with eight rows a CTA and no
-// block ahead; the latter then have one CTA of eight warps an SM), 3 x 256 of 512 29 us.
+// block ahead; the latter then have one CTA of eight warps an SM), 3 x 256 of 512 21 us (32 without the block ahead).
 #include "common.cuh"
 
 namespace h3s {
@@ -34,8 +34,9 @@ __device__ __forceinline__ unsigned long long score_key(double s) {
   return (bits >> 63) ? ~bits : (bits | 0x8000000000000000ull);
 }
 
-// kRows query tiles per CTA, as many warps
-template <typename T, int kRows>
+// kRows query tiles per CTA, as many warps.  kAhead: the next block's means are requested before this one's products, in up to
+// 64 registers a thread
+template <typename T, int kRows, bool kAhead>
 __global__ void __launch_bounds__(kRows * 32)
 route_topk_kernel(const T *__restrict__ q_summary, const T *__restrict__ k_summary, int q_tiles,
                   int kv_tiles, int q_start, int q_stop, int kv_start, int kv_stop, int retained,
@@ -79,7 +80,6 @@ route_topk_kernel(const T *__restrict__ q_summary, const T *__restrict__ k_summa
         ahead[i] = k_head[static_cast<int64_t>(tile) * H3S_HEAD_DIM + (e & 127)];
       }
     };
-    constexpr bool kAhead = kRows == 16;  // eight rows: two CTAs an SM instead, which leaves no registers for it
     if (kAhead) fetch(0);
     for (int base = 0; base < pure_kv; base += kRouteKBlock) {
       if (!kAhead) fetch(base);
@@ -207,15 +207,15 @@ constexpr size_t route_smem(int rows, int pure_kv) {
 
 constexpr size_t kRouteMostSmem = 220 * 1024;
 
-template <typename T, int kRows>
+template <typename T, int kRows, bool kAhead>
 static int launch_route_rows(const void *q_summary, const void *k_summary, int heads, int q_tiles, int kv_tiles,
                              int q_start, int q_stop, int kv_start, int kv_stop, int retained, int route_len,
                              int32_t *route, cudaStream_t stream) {
   const size_t smem = route_smem(kRows, kv_stop - kv_start);
   // one value for all callers: a thread with shorter rows would take away what another one is about to launch with
-  H3S_CHECK_CUDA(cudaFuncSetAttribute(route_topk_kernel<T, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRouteMostSmem)));
+  H3S_CHECK_CUDA(cudaFuncSetAttribute(route_topk_kernel<T, kRows, kAhead>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRouteMostSmem)));
   dim3 grid(ceil_div(q_stop - q_start, kRows), heads);
-  H3S_CHECK_CUDA(launch_next(route_topk_kernel<T, kRows>, grid, kRows * 32, smem, stream, static_cast<const T *>(q_summary),
+  H3S_CHECK_CUDA(launch_next(route_topk_kernel<T, kRows, kAhead>, grid, kRows * 32, smem, stream, static_cast<const T *>(q_summary),
                              static_cast<const T *>(k_summary), q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained,
                              route_len, route));
   return H3S_OK;
@@ -225,6 +225,7 @@ static int launch_route_rows(const void *q_summary, const void *k_summary, int h
 // them share an SM while their scores fit, beyond about 750 pure-video KV tiles they do not; sixteen query tiles take an SM for themselves,
 // but read the K tile means of their head once for all, with the next block's loads under the products.  us, eight / sixteen:
 //   one CTA of eight an SM         3 x 256 rows of 512 scores, fp32 22.2 / 27.7, FP64 28.1 / 30.0; 24 x 40 of 80, fp32 8.9 / 11.8
+//                                  (before that CTA had a block ahead, too)
 //   two, side by side              8 x 256 of 512, fp32 31.0 / 27.7, FP64 35.6 / 30.1; 24 x 78 of 156, fp32 15.8 / 14.5
 //   two, one after the other       3 x 591 of 1181, fp32 88.7 / 57.1, FP64 115.5 / 65.2
 //   three, of which two share      10 x 256 of 512, fp32 49.0 / 51.3, FP64 59.0 / 56.5; 24 x 128 of 256, fp32 33.1 / 31.1
@@ -249,8 +250,14 @@ static int launch_route(const void *q_summary, const void *k_summary, int heads,
   const size_t least = route_smem(8, pure_kv) + sizeof(int) * 8 * 256;
   H3S_CHECK_ARG(least <= kRouteMostSmem, "route_topk: %d pure-video KV tiles need %zu bytes of shared memory", pure_kv, least);
   if (sixteen_rows<T>(heads, q_stop - q_start, pure_kv))
-    return launch_route_rows<T, 16>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
-  return launch_route_rows<T, 8>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
+    return launch_route_rows<T, 16, true>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
+  // Eight rows where an SM gets one CTA: nothing runs beside it to hide the loads behind, and it has the registers (212 a thread with
+  // FP64 means, 176 with fp32); two share an SM without them.  us, without / with a block ahead, FP64 means: 3 x 256 rows of 512
+  // scores 31.8 / 20.8, 7 x 79 of 157 13.1 / 9.4, 1 x 591 of 1181 58.8 / 44.0, 24 x 40 of 80 11.0 / 7.4, 4 x 16 of 32 5.5 / 5.0; fp32:
+  // 27.7 / 19.8, 11.5 / 9.3, 45.0 / 41.6, 9.9 / 7.0, 4.9 / 4.9.
+  if (heads * ceil_div(q_stop - q_start, 8) <= kSmCount)
+    return launch_route_rows<T, 8, true>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
+  return launch_route_rows<T, 8, false>(q_summary, k_summary, heads, q_tiles, kv_tiles, q_start, q_stop, kv_start, kv_stop, retained, route_len, route, stream);
 }
 
 }  // namespace h3s
