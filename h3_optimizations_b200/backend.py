@@ -296,9 +296,11 @@ class B200SparseBackend:
             # buffer is allocated on the current stream, which both chains rejoin before
             # returning.  One native call issues all of it (4 heads x 2304
             # tokens, where host time is all there is: 236 -> 135 us).
-            # Short calls are over before the host has issued them: there one stream saves the host the events.
+            # Short calls are over before the host has issued them: there one stream saves the host the events.  A
+            # replay has no host in it (4 heads x 1341 tokens: 41 us on one stream, 35 on two).
             stream = _native.stream_ptr(q.device)
-            side = self._side_stream(q.device) if heads * sequence > ONE_STREAM_ROWS else None
+            forked = heads * sequence > ONE_STREAM_ROWS or torch.cuda.is_current_stream_capturing()
+            side = self._side_stream(q.device) if forked else None
             buffers = ops.LayerBuffers(heads, sequence, q.device, smooth_k=self.smooth_k,
                                        summary_dtype=torch.float64 if need_route else None)
             try:
