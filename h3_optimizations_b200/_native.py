@@ -111,6 +111,9 @@ PROTOTYPES = {
     "h3s_project_qkv": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p,
                                 c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_float,
                                 c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "h3s_project_qkv_norms": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p,
+                                      c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float,
+                                      c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p]),
     "h3s_status_mirror": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p]),
     "h3s_sparse_attn_fwd_mma": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                         c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int64,

@@ -31,6 +31,12 @@ int fail(int code, const char *fmt, ...);
 // (h3s_set_wait_budget_ns).
 unsigned long long wait_budget_ns();
 
+// h3s_qkv_gemm_chunk_carriers with norm weights of `norm_dtype`, fp32 or bf16 (qkv_gemm.cu)
+int qkv_gemm_carriers(const int8_t *x_i8, const float *x_scale, const int8_t *w_i8, const float *w_scale, int rows, int hidden,
+                      int heads, const h3s_qkv_carriers *carriers, const void *q_norm, const void *k_norm, int norm_dtype,
+                      float epsilon, const void *rope, int rope_dtype, const int64_t *rope_strides, int32_t *status,
+                      h3s_stream_t stream);
+
 constexpr int kSmCount = 148;  // of a B200, for the rules that deal out work
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -61,11 +61,11 @@ int h3s_quant_qkv(const h3s_layer_carriers *c, const void *q, const void *k, con
                               v_bound, side);
 }
 
-int h3s_project_qkv(const h3s_layer_carriers *c, const void *x_bf16, int64_t x_stride_row, int sequence, int hidden,
-                    int chunk_rows, int8_t *x_i8, float *x_scale, const int8_t *w_i8, const float *w_scale, int heads,
-                    int smooth_k, void *k_stage, void *v_stage, const float *q_norm, const float *k_norm,
-                    float epsilon, const void *rope, int rope_dtype, const int64_t *rope_strides, float v_bound,
-                    int32_t *status, void *event, h3s_stream_t stream, h3s_stream_t side_stream) {
+int h3s_project_qkv_norms(const h3s_layer_carriers *c, const void *x_bf16, int64_t x_stride_row, int sequence, int hidden,
+                          int chunk_rows, int8_t *x_i8, float *x_scale, const int8_t *w_i8, const float *w_scale, int heads,
+                          int smooth_k, void *k_stage, void *v_stage, const void *q_norm, const void *k_norm,
+                          int norm_dtype, float epsilon, const void *rope, int rope_dtype, const int64_t *rope_strides, float v_bound,
+                          int32_t *status, void *event, h3s_stream_t stream, h3s_stream_t side_stream) {
   using namespace h3s;
   H3S_CHECK_ARG(c != nullptr && event != nullptr, "project_qkv: NULL argument");
   H3S_CHECK_ARG(x_bf16 != nullptr && x_i8 != nullptr && x_scale != nullptr, "project_qkv: NULL input");
@@ -88,8 +88,8 @@ int h3s_project_qkv(const h3s_layer_carriers *c, const void *x_bf16, int64_t x_s
     if (rc) return rc;
     out.row_start = start;
     const void *rope_rows = rope == nullptr ? nullptr : static_cast<const char *>(rope) + start * rope_strides[0] * rope_size;
-    rc = h3s_qkv_gemm_chunk_carriers(x_i8, x_scale, w_i8, w_scale, rows, hidden, heads, &out, q_norm, k_norm, epsilon,
-                                     rope_rows, rope_dtype, rope_strides, status, s);
+    rc = qkv_gemm_carriers(x_i8, x_scale, w_i8, w_scale, rows, hidden, heads, &out, q_norm, k_norm, norm_dtype, epsilon,
+                           rope_rows, rope_dtype, rope_strides, status, s);
     if (rc) return rc;
   }
   rc = h3s_column_stats_finalize(c->scratch, H3S_BF16, heads, sequence, v_bound, smooth_k ? c->k_mean : nullptr,
@@ -110,6 +110,16 @@ int h3s_project_qkv(const h3s_layer_carriers *c, const void *x_bf16, int64_t x_s
   // joined wherever it was forked, and only there: a capture must not wait for a stream outside it
   const int joined = order_after(side, s, event);
   return rc ? rc : joined;
+}
+
+int h3s_project_qkv(const h3s_layer_carriers *c, const void *x_bf16, int64_t x_stride_row, int sequence, int hidden,
+                    int chunk_rows, int8_t *x_i8, float *x_scale, const int8_t *w_i8, const float *w_scale, int heads,
+                    int smooth_k, void *k_stage, void *v_stage, const float *q_norm, const float *k_norm,
+                    float epsilon, const void *rope, int rope_dtype, const int64_t *rope_strides, float v_bound,
+                    int32_t *status, void *event, h3s_stream_t stream, h3s_stream_t side_stream) {
+  return h3s_project_qkv_norms(c, x_bf16, x_stride_row, sequence, hidden, chunk_rows, x_i8, x_scale, w_i8, w_scale, heads, smooth_k, k_stage,
+                               v_stage, q_norm, k_norm, H3S_F32, epsilon, rope, rope_dtype, rope_strides, v_bound, status, event,
+                               stream, side_stream);
 }
 
 int h3s_status_mirror(const int32_t *status, int32_t *host_mirror, void *event, h3s_stream_t stream) {

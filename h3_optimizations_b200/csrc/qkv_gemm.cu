@@ -215,7 +215,8 @@ struct GemmLayout {
   static constexpr uint32_t kOffB = kStages * kGemmABytes;
   static constexpr uint32_t kOffTile = kOffB + kStages * kGemmBBytes;
   static constexpr uint32_t kOffExchange = kOffTile + (kCarriers ? 2 * kEpilogueTileBytes : 0);
-  static constexpr uint32_t kOffBar = kOffExchange + (kMode == kModeCarriers ? 2 * sizeof(EpilogueExchange) : 0);
+  static constexpr uint32_t kOffNorm = kOffExchange + (kMode == kModeCarriers ? 2 * sizeof(EpilogueExchange) : 0);  // weights of Q, of K
+  static constexpr uint32_t kOffBar = kOffNorm + (kMode == kModeCarriers ? 2 * H3S_HEAD_DIM * sizeof(float) : 0);
   static constexpr uint32_t kBytes = kOffBar + 256 + 1024;
   static_assert(sizeof(uint64_t) * (2 * 6 + 16) + 8 <= 256, "barriers");
   static_assert(kBytes <= 227 * 1024, "GEMM shared memory exceeds the per-CTA limit");
@@ -252,6 +253,7 @@ struct GemmParams {
   // optional per-head RMS norm (+ split-half rotation) of the Q and K groups
   const float *q_norm;    // (128) or null: no norm, no rotation
   const float *k_norm;    // (128)
+  int norm_dtype;         // carriers: type of both, which the epilogue reads from shared memory; else fp32
   const void *rope;       // (rows, 48, 2, 2) view with the strides below, or null
   int64_t rope_stride_seq, rope_stride_dim, rope_stride_rot, rope_stride_pair;
   int rope_dtype;         // H3S_F32 or H3S_BF16
@@ -617,7 +619,7 @@ __device__ __forceinline__ TripleSum half_row_squares(const HalfRow &y) {
 }
 
 __device__ __forceinline__ uint32_t norm_pair(uint32_t y, float2 inverse_rms, const float *__restrict__ weight) {
-  const float2 normed = mul2(mul2(bf16_pair(y), inverse_rms), __ldg(reinterpret_cast<const float2 *>(weight)));
+  const float2 normed = mul2(mul2(bf16_pair(y), inverse_rms), *reinterpret_cast<const float2 *>(weight));
   return pack_bf16x2(normed.x, normed.y);
 }
 
@@ -708,6 +710,13 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     ptx::tmem_relinquish_pair();
   }
   wait_for_previous();
+  float *norm_weights = reinterpret_cast<float *>(smem + L::kOffNorm);
+  if (kCarriers && prm.q_norm != nullptr) {
+    for (int i = threadIdx.x; i < 2 * H3S_HEAD_DIM; i += W::kThreads) {
+      const void *from = i < H3S_HEAD_DIM ? prm.q_norm : prm.k_norm;
+      norm_weights[i] = rope_load(from, i % H3S_HEAD_DIM, prm.norm_dtype);
+    }
+  }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::cluster_sync();  // both CTAs' barriers are initialised
@@ -988,7 +997,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 const TripleSum both = add_sums(mine, theirs);
                 squares = both.sum < INFINITY ? nearest(both) : both.sum;  // infinite: nothing is left to correct
               }
-              norm_half_row(y, squares, group < prm.heads ? prm.q_norm : prm.k_norm, prm.epsilon, share);
+              norm_half_row(y, squares, norm_weights + (group < prm.heads ? 0 : H3S_HEAD_DIM), prm.epsilon, share);
               if (form == kRopeBf16) {
                 const uint4 *table = static_cast<const uint4 *>(rope_row) + 12 * share;
 #pragma unroll
@@ -1326,7 +1335,8 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
                                int rows, int hidden, int n_out, void *out_bf16, int64_t out_stride_head,
                                const float *q_norm, const float *k_norm, float epsilon, const void *rope,
                                int rope_dtype, const int64_t *rope_strides, int heads, int32_t *status,
-                               h3s_stream_t stream, const char *who, const h3s_qkv_carriers *carriers = nullptr) {
+                               h3s_stream_t stream, const char *who, const h3s_qkv_carriers *carriers = nullptr,
+                               int norm_dtype = H3S_F32) {
   using namespace h3s;
   H3S_CHECK_ARG(x_i8 && x_scale && w_i8 && w_scale && (out_bf16 || carriers), "%s: NULL pointer", who);
   H3S_CHECK_ARG(rows > 0 && hidden > 0 && hidden % kGemmK == 0, "%s: hidden %d must be a positive multiple of 128", who, hidden);
@@ -1358,6 +1368,7 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
     H3S_CHECK_ARG(q_norm != nullptr && k_norm != nullptr, "%s: both norm weights are needed", who);
     H3S_CHECK_ARG(heads > 0 && n_out == 3 * heads * H3S_HEAD_DIM, "%s: n_out %d is not 3*heads*128 for %d heads", who, n_out, heads);
     H3S_CHECK_ARG(epsilon >= 0.f, "%s: negative epsilon", who);
+    H3S_CHECK_ARG(norm_dtype == H3S_F32 || norm_dtype == H3S_BF16, "%s: norm weights must be fp32 or bf16", who);
     if (rope != nullptr) {
       H3S_CHECK_ARG(rope_strides != nullptr, "%s: rope strides missing", who);
       H3S_CHECK_ARG(rope_dtype == H3S_F32 || rope_dtype == H3S_BF16, "%s: rope must be fp32 or bf16", who);
@@ -1379,7 +1390,7 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
   prm.q_norm = q_norm; prm.k_norm = k_norm; prm.rope = rope; prm.rope_dtype = rope_dtype;
   prm.rope_stride_seq = rope ? rope_strides[0] : 0; prm.rope_stride_dim = rope ? rope_strides[1] : 0;
   prm.rope_stride_rot = rope ? rope_strides[2] : 0; prm.rope_stride_pair = rope ? rope_strides[3] : 0;
-  prm.heads = heads; prm.epsilon = epsilon;
+  prm.heads = heads; prm.epsilon = epsilon; prm.norm_dtype = norm_dtype;
   prm.wait_budget_ns = wait_budget_ns();
   prm.q8 = prm.k8 = nullptr; prm.q_scale = prm.k_scale = nullptr; prm.q_summary = prm.k_summary = nullptr;
   prm.k_stage = prm.v_stage = nullptr; prm.k_sum = nullptr; prm.v_amax_bits = nullptr;
@@ -1483,10 +1494,18 @@ int h3s_qkv_gemm_chunk_carriers(const int8_t *x_i8, const float *x_scale, const 
                                 const h3s_qkv_carriers *carriers, const float *q_norm, const float *k_norm,
                                 float epsilon, const void *rope, int rope_dtype, const int64_t *rope_strides,
                                 int32_t *status, h3s_stream_t stream) {
-  H3S_CHECK_ARG(carriers != nullptr, "qkv_gemm_chunk_carriers: NULL carrier description");
-  return qkv_gemm_chunk_impl(x_i8, x_scale, w_i8, w_scale, rows, hidden, 3 * heads * H3S_HEAD_DIM, nullptr, 0, q_norm,
-                             k_norm, epsilon, rope, rope_dtype, rope_strides, heads, status, stream,
-                             "qkv_gemm_chunk_carriers", carriers);
+  return h3s::qkv_gemm_carriers(x_i8, x_scale, w_i8, w_scale, rows, hidden, heads, carriers, q_norm, k_norm, H3S_F32, epsilon, rope,
+                                rope_dtype, rope_strides, status, stream);
 }
 
 }  // extern "C"
+
+int h3s::qkv_gemm_carriers(const int8_t *x_i8, const float *x_scale, const int8_t *w_i8, const float *w_scale, int rows, int hidden,
+                           int heads, const h3s_qkv_carriers *carriers, const void *q_norm, const void *k_norm, int norm_dtype,
+                           float epsilon, const void *rope, int rope_dtype, const int64_t *rope_strides, int32_t *status,
+                           h3s_stream_t stream) {
+  H3S_CHECK_ARG(carriers != nullptr, "qkv_gemm_chunk_carriers: NULL carrier description");
+  return qkv_gemm_chunk_impl(x_i8, x_scale, w_i8, w_scale, rows, hidden, 3 * heads * H3S_HEAD_DIM, nullptr, 0,
+                             static_cast<const float *>(q_norm), static_cast<const float *>(k_norm), epsilon, rope, rope_dtype,
+                             rope_strides, heads, status, stream, "qkv_gemm_chunk_carriers", carriers, norm_dtype);
+}

@@ -322,6 +322,8 @@ def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, s
     ``quant_qkv``, but ``stream`` is behind ``side`` again when the call returns or raises."""
     if x.stride(1) != 1:
         raise _native.NativeError("project_qkv: x must have contiguous rows")
+    if q_norm is not None and (k_norm is None or k_norm.dtype != q_norm.dtype):
+        raise _native.NativeError("project_qkv: the norm weights must share a type")
     sequence, hidden = x.shape
     rows = min(chunk_rows, sequence)
     # one chunk's codes and scales, and bf16 staging of what needs whole-sequence statistics before it can be quantised
@@ -335,10 +337,10 @@ def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, s
         rope_code = dtype_code(rope.dtype)
         strides = (ctypes.c_int64 * 4)(rope.stride(1), rope.stride(3), rope.stride(4), rope.stride(5))
     check(
-        _native.load().h3s_project_qkv(
+        _native.load().h3s_project_qkv_norms(
             buffers.native, x.data_ptr(), x.stride(0), sequence, hidden, chunk_rows, base + codes_at, base + scale_at,
             w_i8.data_ptr(), w_scale.data_ptr(), heads, int(smooth_k), base + stage if smooth_k else None, base,
-            _address(q_norm), _address(k_norm), epsilon, _address(rope), rope_code, strides, v_bound, _address(status),
+            _address(q_norm), _address(k_norm), 0 if q_norm is None else dtype_code(q_norm.dtype), epsilon, _address(rope), rope_code, strides, v_bound, _address(status),
             side.event_handle, stream, side.handle),
         "h3s_project_qkv",
     )

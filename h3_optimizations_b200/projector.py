@@ -132,8 +132,10 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
     epsilon = 0.0
     if norm is not None:
         q_norm, k_norm, epsilon = norm
-        q_norm = q_norm.detach().to(device=device, dtype=torch.float32).contiguous()
-        k_norm = k_norm.detach().to(device=device, dtype=torch.float32).contiguous()
+        # bf16 weights go to the kernel as they are: two launches and two tensors fewer
+        dtype = torch.bfloat16 if q_norm.dtype == k_norm.dtype == torch.bfloat16 else torch.float32
+        q_norm = q_norm.detach().to(device=device, dtype=dtype).contiguous()
+        k_norm = k_norm.detach().to(device=device, dtype=dtype).contiguous()
         if tuple(q_norm.shape) != (HEAD_DIM,) or tuple(k_norm.shape) != (HEAD_DIM,):
             raise FusedQKVError("q_norm / k_norm weights must have 128 elements")
     if rope_freqs is not None:
