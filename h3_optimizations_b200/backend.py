@@ -300,7 +300,9 @@ class B200SparseBackend:
             # replay has no host in it (4 heads x 1341 tokens: 41 us on one stream, 35 on two).
             stream = _native.stream_ptr(q.device)
             forked = heads * sequence > ONE_STREAM_ROWS or torch.cuda.is_current_stream_capturing()
-            side = self._side_stream(q.device) if forked else None
+            side = self._side_stream(q.device)  # there from the first call on: a capture must not bring it into being
+            if not forked:
+                side = None
             buffers = ops.LayerBuffers(heads, sequence, q.device, smooth_k=self.smooth_k,
                                        summary_dtype=torch.float64 if need_route else None)
             try:

@@ -77,3 +77,10 @@ def test_one_stream_and_two_prepare_the_same(layer, monkeypatch, budget, smooth_
         torch.cuda.synchronize()
         assert torch.equal(out, expected)
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_a_short_call_leaves_nothing_to_a_capture(layer):
+    """The second stream is there before a capture, which uses it, although the calls before it did not."""
+    backend, prepare = layer()
+    backend.execute(prepare())
+    assert len(backend._side_streams) == 1
