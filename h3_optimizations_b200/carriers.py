@@ -193,6 +193,12 @@ class PreparedLayer(PreparedSparse):
         self.__dict__[name] = value
         return value
 
+    @property
+    def device(self):
+        """Where the carriers are, without asking for one."""
+        buffers = self.__dict__.get("_buffers")
+        return self.q_int8.device if buffers is None else buffers.device
+
     def untouched(self):
         """The buffers, if no tensor of them has been handed out or replaced."""
         buffers = self.__dict__.get("_buffers")

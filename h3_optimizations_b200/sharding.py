@@ -16,6 +16,8 @@ from __future__ import annotations
 import torch
 import torch.distributed as dist
 
+from .carriers import PreparedLayer
+
 
 def head_partition(heads, world_size, rank):
     """Contiguous ``[start, stop)`` head range of ``rank``; the first
@@ -208,7 +210,7 @@ class HeadShardedBackend:
         ``kernel_done``: optional CUDA event recorded between the attention
         kernel and the reassembly step (benchmarks time the two apart)."""
         sparse = prepared.sparse
-        self._setup(sparse.sequence, sparse.output_dtype, sparse.q_int8.device)
+        self._setup(sparse.sequence, sparse.output_dtype, sparse.device if isinstance(sparse, PreparedLayer) else sparse.q_int8.device)
         a, b = self.head_range
         local = self._full[:, a:b]
         if self.exchange == "peer":

@@ -41,3 +41,19 @@ def test_stores_are_the_same(native_lib, layout, sequence, dtype):
     torch.cuda.synchronize()
     assert torch.isfinite(out).all() and not (out == 77.0).all(dim=-1).any()
     assert torch.equal(whole[0], whole[1]) and torch.equal(whole[0], whole[2])
+
+
+def test_an_output_in_pinned_host_memory(native_lib):
+    from h3_optimizations_b200 import ops
+
+    spec = workloads.small_spec("output", 2, 0, 200)
+    q, k, v = (t.cuda() for t in workloads.gaussian_qkv(spec, seed=7))
+    k_mean, v_scale = ops.column_stats(k, v)
+    q8, qs, _ = ops.quant_qk_blocks(q, 128)
+    k8, ks, _ = ops.quant_qk_blocks(k, 64, mean=k_mean)
+    vc, _ = ops.quant_v_fp8(v, v_scale)
+    host = torch.zeros((1, 2, 200, 128), dtype=torch.bfloat16).pin_memory()
+    ops.sparse_attention(q8, k8, vc, qs, ks, v_scale, out=host)
+    out = ops.sparse_attention(q8, k8, vc, qs, ks, v_scale)
+    torch.cuda.synchronize()
+    assert torch.equal(host, out.cpu())
