@@ -993,8 +993,9 @@ __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v
 
 // Whether and how the dense rows' tile lists are cut.  A row longer than half of what an SM gets on average may end after
 // everything else has, which parts even out; but parts are dear.  Beside its tiles (0.36 us each) a whole list takes an SM
-// about as long as twelve tiles, a part about 27: it writes 66 KB, waits until they are seen, and one of them
-// reads them all back.  So as many parts as end first by this estimate, every SM taking the next item as it gets free, and only if
+// about as long as twelve tiles (before its epilogue ran under the next item's tiles), a part about 27: it writes 66 KB, waits
+// until they are seen, and one of them reads them all back.  So as many parts as end first by this estimate, every SM taking the
+// next item as it gets free, and only if
 //  - that is earlier than with whole rows by more than 3 %, or
 //  - it is no later, and the parts' own cost is under 1 % of the work (three heads of 33272 tokens at 30 %: 376 us either way), or
 //  - nothing but dense rows is there, and dealt out evenly instead of in rounds the parts would end with the rows.
