@@ -19,12 +19,16 @@ int fail(int code, const char *fmt, ...);
     if (!(cond)) return ::h3s::fail(H3S_EINVAL, __VA_ARGS__); \
   } while (0)
 
+// The error is reported here, so the runtime's note of it goes too: a later cudaGetLastError() would take it for that of a
+// launch of its own.
 #define H3S_CHECK_CUDA(expr)                                                   \
   do {                                                                         \
     cudaError_t err__ = (expr);                                                \
-    if (err__ != cudaSuccess)                                                  \
+    if (err__ != cudaSuccess) {                                                \
+      (void)cudaGetLastError();                                                \
       return ::h3s::fail(H3S_ECUDA, "%s failed: %s", #expr,                    \
                          cudaGetErrorString(err__));                           \
+    }                                                                          \
   } while (0)
 
 // Upper bound of every device-side wait of the kernels launched from now on
