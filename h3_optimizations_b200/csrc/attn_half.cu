@@ -125,7 +125,8 @@ struct alignas(16) HalfShared {
   uint64_t pass_end;           // the rows' values of a pass are in `row`, `noted` is complete; all warps arrive and wait
   uint64_t staged;             // softmax warps only: the output tile is in shared memory (and steps before that)
   uint32_t tmem_base;
-  int abort_word;
+  int abort_word;              // code of the wait that ran out, and 256 times the warp it was in
+  int stopped[kHWarps];        // turn (of three) of the item that a warp gave up in
   int finish;                  // of an item that is a part: this CTA writes the output tile
   int again[4];                // per item in turn.  kAgainNoted: some row has left out a tile; kAgainFar: its sum
                                // there does not tell the maximum
@@ -347,7 +348,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
   };
   auto wait_pass = [&]() {
-    return warp_wait(&sh.pass_end, passes & 1u, abort_word, kAbortPass, 4 * prm.wait_budget_ns);
+    return warp_wait<true>(&sh.pass_end, passes & 1u, abort_word, kAbortPass, 4 * prm.wait_budget_ns);
   };
   auto end_pass = [&]() {
     arrive_pass();
@@ -403,7 +404,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     uint32_t seq = 0;    // tiles so far
     int stage = 0;       // state of the loading thread ...
     uint32_t round = 1;  // ... parity of the ring's previous use
-    bool drop = prm.drop_kv_load == 0;
+    int drop = prm.drop_kv_load;  // running number of the tile that is not loaded, -1: none
     // the fetched block's first `tiles` tiles into the next stages; `meanwhile` may fetch again
     auto load_block = [&](int tiles, auto meanwhile) {
       if (lane < tiles) block[lane] = next_tile;
@@ -420,13 +421,13 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int head = work.head;
         for (int i = 0; i < tiles; ++i) {
           const int t = block[i];
-          fine = ptx::mbar_wait(&empty[stage], round, abort_word, kAbortKvEmpty, 4 * prm.wait_budget_ns);
+          fine = ptx::mbar_wait<true>(&empty[stage], round, abort_word, kAbortKvEmpty, 4 * prm.wait_budget_ns);
           if (!fine) break;
-          if (!drop) {
+          if (drop != 0) {
             ptx::mbar_arrive_expect_tx(&full[stage], bytes);
             ptx::tma_load_3d(ring + stage * bytes, map, &full[stage], keys ? 0 : t * H3S_KV_TILE * 2, keys ? t * H3S_KV_TILE : 0, head);
           }
-          drop = false;
+          if (drop >= 0) --drop;
           if (++stage == stages) { stage = 0; round ^= 1u; }
         }
       }
@@ -437,6 +438,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     fetch_block(work, 0);
     HalfWork coming = work;
     while (ok) {
+      if (prm.drop_last_v_load && !keys) drop = work.n_iter - 1;
       for (int i = 0; ok && i < work.n_iter; i += kHBlock) {
         if (keys && i + kHBlock >= work.n_iter) {
           // Not before the last block: an item that is taken over waits until this one is through, while other
@@ -451,7 +453,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         ok = load_block(min(kHBlock, work.n_iter - i), [&]() { if (i + kHBlock < work.n_iter) fetch_block(work, i + kHBlock); });
       }
-      ok = ok && warp_wait(&sh.next_ready, items & 1u, abort_word, kAbortNextItem, 4 * prm.wait_budget_ns);
+      ok = ok && warp_wait<true>(&sh.next_ready, items & 1u, abort_word, kAbortNextItem, 4 * prm.wait_budget_ns);
       if (!ok) break;
       const int next = ptx::granted_block(&sh.next_reply);
       if (next >= 0) {
@@ -469,7 +471,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + coming.head * H3S_HEAD_DIM + i * 32 + lane);
-          ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortQFree, 4 * prm.wait_budget_ns);
+          ok = warp_wait<true>(&sh.q_free, items & 1u, abort_word, kAbortQFree, 4 * prm.wait_budget_ns);
           if (!ok) break;
           load_q(coming);
         }
@@ -517,7 +519,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     uint32_t round = 0, slot_round = 0;
     while (ok) {
       const uint32_t tmem_q = tmem_o + kHTmemQ + (items & 1) * 32;
-      ok = warp_wait(&sh.q_full, items & 1u, abort_word, kAbortQFull, prm.wait_budget_ns);
+      ok = warp_wait<true>(&sh.q_full, items & 1u, abort_word, kAbortQFull, prm.wait_budget_ns);
       if (!ok) break;
       if (ptx::elect_one()) {
 #pragma unroll
@@ -530,8 +532,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         arrive_pass();  // nothing of the pass's end depends on this warp
         if (ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
-            ok = ptx::mbar_wait(&sh.k_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
-                 ptx::mbar_wait(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortScoreSlot, 3 * prm.wait_budget_ns);
+            ok = ptx::mbar_wait<true>(&sh.k_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
+                 ptx::mbar_wait<true>(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortScoreSlot, 3 * prm.wait_budget_ns);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(stage * (kHKBytes >> 4));
@@ -564,12 +566,12 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       int count = n_iter;
       for (int pass = 0;; ++pass) {
         arrive_pass();  // nothing of the pass's end depends on this warp
-        ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree, 4 * prm.wait_budget_ns);
+        ok = warp_wait<true>(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree, 4 * prm.wait_budget_ns);
         if (ok && ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
             const int j = done + i, g = j % kHGroups;
-            ok = ptx::mbar_wait(&sh.v_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
-                 ptx::mbar_wait(&sh.p_full[g], (j / kHGroups) & 1u, abort_word, kAbortPFull, 3 * prm.wait_budget_ns);
+            ok = ptx::mbar_wait<true>(&sh.v_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
+                 ptx::mbar_wait<true>(&sh.p_full[g], (j / kHGroups) & 1u, abort_word, kAbortPFull, 3 * prm.wait_budget_ns);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t v_desc = v_desc0 + static_cast<uint64_t>(stage * (kHVBytes >> 4));
@@ -602,7 +604,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
     // scores of tile j -> registers, and the factor that belongs to them
     auto take = [&](uint32_t j, uint32_t (&s)[H3S_KV_TILE], float &c) {
-      if (!warp_wait(&sh.s_full[group], (j / kHGroups) & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) return false;
+      if (!warp_wait<true>(&sh.s_full[group], (j / kHGroups) & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) return false;
       const uint32_t slot = j % kHScoreSlots;
       ptx::tc_fence_after();
       H3S_TMEM_LD64(tmem_o + kHTmemS + slot * 64 + lane_addr, s);
@@ -625,7 +627,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     };
     // the group's P columns are free
     auto room = [&](uint32_t j) {
-      return warp_wait(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
+      return warp_wait<true>(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
     };
     // behind `room`: the fence orders the store after P.V's reads of the same columns
     auto put = [&](const uint32_t (&packed)[H3S_KV_TILE / 2]) {
@@ -648,11 +650,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     auto meet = [&]() {  // all softmax warps
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&sh.staged);
-      return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortStaged, 4 * prm.wait_budget_ns);
+      return warp_wait<true>(&sh.staged, staged_uses++ & 1u, abort_word, kAbortStaged, 4 * prm.wait_budget_ns);
     };
     // every P.V of the pass that has ended
     auto all_products = [&]() {
-      return warp_wait(&sh.o_full, (passes - 1) & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      return warp_wait<true>(&sh.o_full, (passes - 1) & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
     };
     auto release_o = [&]() {
       ptx::tc_fence_before();
@@ -683,9 +685,10 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // not wait for the last P.V, and the next P.V comes later.  Every warp by itself: its 32 rows of 32 columns
     // go through its own piece of shared memory to a TMA store, which also leaves out rows past the sequence.
     bool pending = false;
-    auto finish_last = [&](const HalfItem &from) {
+    auto finish_last = [&]() {
+      const HalfItem &from = sh.item[(items + 2) % 3u];
       pending = false;
-      if (!all_products()) return false;
+      if (!all_products()) { items += 2; return false; }  // given up in that item
       ptx::tc_fence_after();
       uint32_t o[32];
       H3S_TMEM_LD32(tmem_o + lane_addr + group * 32, o);
@@ -729,7 +732,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (!take(done + i, s, c)) return false;
         if (decltype(first)::value) {
           if (i < 2) leave_first(i, c * static_cast<float>(max_score(s)));  // c > 0
-          if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) return false;
+          if (!warp_wait<true>(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) return false;
           m = first_reference();
         }
         uint32_t packed[H3S_KV_TILE / 2];
@@ -759,7 +762,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       };
       if (rank < n_iter) {
         ok = walk(rank, std::true_type{});
-        if (ok && pending) ok = finish_last(sh.item[(items + 2) % 3u]);
+        if (ok && pending) ok = finish_last();
         if (ok) {
           for (int i = rank + kHGroups; i < n_iter; i += kHGroups)
             if (!walk(i, std::false_type{})) { ok = false; break; }
@@ -767,8 +770,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
       if (!ok) break;
       if (rank >= n_iter) {  // a group without a tile: the last item is not finished, and there is no reference point yet
-        ok = (!pending || finish_last(sh.item[(items + 2) % 3u])) &&
-             warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns);
+        ok = (!pending || finish_last()) &&
+             warp_wait<true>(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns);
         if (!ok) break;
         m = first_reference();
       }
@@ -857,7 +860,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (!split && prm.out_map) {
         pending = true;
         if (next_item()) continue;
-        ok = finish_last(sh.item[(items + 2) % 3u]);
+        ok = finish_last();
         break;
       }
 
@@ -952,14 +955,15 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   }
 
   // ---- teardown ----
+  if (!ok && lane == 0) sh.stopped[warp] = items % 3u;
   __syncthreads();
-  const int code = sh.abort_word;
+  const int code = sh.abort_word & 255;
   if (code != 0) {
     // leave time for copies / MMAs still in flight before releasing TMEM and shared memory
     __nanosleep(200000);
     if (threadIdx.x == 0 && prm.status != nullptr) {
       if (atomicCAS(prm.status, 0, code) == 0) {
-        const HalfItem &at = sh.item[items % 3u];
+        const HalfItem &at = sh.item[sh.stopped[sh.abort_word >> 8]];
         prm.status[1] = at.number;
         prm.status[2] = at.head;
         prm.status[3] = at.tq;

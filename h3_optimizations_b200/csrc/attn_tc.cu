@@ -511,6 +511,7 @@ int fill_attn_params(AttnParams *params, const int8_t *q8, const int8_t *k8, con
   prm.n_peer_out = n_peer_out;
   prm.wait_budget_ns = wait_budget_ns();
   prm.drop_kv_load = (flags & H3S_ATTN_TEST_DROP_KV_LOAD) ? 0 : -1;
+  prm.drop_last_v_load = (flags & H3S_ATTN_TEST_DROP_LAST_V_LOAD) != 0;
   for (int i = 0; i < H3S_MAX_PEER_OUTPUTS; ++i) prm.peer_out[i] = i < n_peer_out ? peer_out[i] : nullptr;
   return H3S_OK;
 }

@@ -95,8 +95,9 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
 }
 
 // Waits for the phase with the given parity.  Returns false (and raises
-// *abort_word with `code`) when the budget expires or another waiter already
-// gave up.  `abort_word` lives in shared memory.
+// *abort_word with `code`, with kNameWarp + 256 * warp) when the budget expires or another waiter
+// already gave up.  `abort_word` lives in shared memory.
+template <bool kNameWarp = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_word,
                                           int code, unsigned long long budget_ns) {
   // a phase that is already complete costs one test_wait (a try_wait with a
@@ -110,6 +111,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     if ((++spins & 15u) == 0u) {
       if (*abort_word != 0) return false;
       if (global_timer_ns() - start > budget_ns) {
+        if (kNameWarp) code |= static_cast<int>(threadIdx.x >> 5) << 8;
         atomicCAS(const_cast<int *>(abort_word), 0, code);
         return false;
       }

@@ -22,6 +22,7 @@ FP8_V_BOUND = 448.0
 ATTN_P_SINGLE = 1
 ATTN_PLAIN_STORES = 2
 ATTN_TEST_DROP_KV_LOAD = 0x4000
+ATTN_TEST_DROP_LAST_V_LOAD = 0x8000
 
 
 def _ceil_div(a, b):
