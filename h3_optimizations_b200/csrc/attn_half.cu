@@ -276,7 +276,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   // (offset arithmetic, so that the compiler still sees shared memory)
   unsigned char *smem = smem_dyn + ((1024u - (ptx::smem_u32(smem_dyn) & 1023u)) & 1023u);
   HalfShared &sh = *reinterpret_cast<HalfShared *>(smem + L::kOffShared);
-  volatile int *abort_word = &sh.abort_word;
+  const ptx::WarpAbort abort_word{&sh.abort_word};
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -348,7 +348,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
   };
   auto wait_pass = [&]() {
-    return warp_wait<true>(&sh.pass_end, passes & 1u, abort_word, kAbortPass, 4 * prm.wait_budget_ns);
+    return warp_wait(&sh.pass_end, passes & 1u, abort_word, kAbortPass, 4 * prm.wait_budget_ns);
   };
   auto end_pass = [&]() {
     arrive_pass();
@@ -421,7 +421,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int head = work.head;
         for (int i = 0; i < tiles; ++i) {
           const int t = block[i];
-          fine = ptx::mbar_wait<true>(&empty[stage], round, abort_word, kAbortKvEmpty, 4 * prm.wait_budget_ns);
+          fine = ptx::mbar_wait(&empty[stage], round, abort_word, kAbortKvEmpty, 4 * prm.wait_budget_ns);
           if (!fine) break;
           if (drop != 0) {
             ptx::mbar_arrive_expect_tx(&full[stage], bytes);
@@ -453,7 +453,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         ok = load_block(min(kHBlock, work.n_iter - i), [&]() { if (i + kHBlock < work.n_iter) fetch_block(work, i + kHBlock); });
       }
-      ok = ok && warp_wait<true>(&sh.next_ready, items & 1u, abort_word, kAbortNextItem, 4 * prm.wait_budget_ns);
+      ok = ok && warp_wait(&sh.next_ready, items & 1u, abort_word, kAbortNextItem, 4 * prm.wait_budget_ns);
       if (!ok) break;
       const int next = ptx::granted_block(&sh.next_reply);
       if (next >= 0) {
@@ -471,7 +471,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + coming.head * H3S_HEAD_DIM + i * 32 + lane);
-          ok = warp_wait<true>(&sh.q_free, items & 1u, abort_word, kAbortQFree, 4 * prm.wait_budget_ns);
+          ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortQFree, 4 * prm.wait_budget_ns);
           if (!ok) break;
           load_q(coming);
         }
@@ -519,7 +519,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     uint32_t round = 0, slot_round = 0;
     while (ok) {
       const uint32_t tmem_q = tmem_o + kHTmemQ + (items & 1) * 32;
-      ok = warp_wait<true>(&sh.q_full, items & 1u, abort_word, kAbortQFull, prm.wait_budget_ns);
+      ok = warp_wait(&sh.q_full, items & 1u, abort_word, kAbortQFull, prm.wait_budget_ns);
       if (!ok) break;
       if (ptx::elect_one()) {
 #pragma unroll
@@ -532,8 +532,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         arrive_pass();  // nothing of the pass's end depends on this warp
         if (ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
-            ok = ptx::mbar_wait<true>(&sh.k_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
-                 ptx::mbar_wait<true>(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortScoreSlot, 3 * prm.wait_budget_ns);
+            ok = ptx::mbar_wait(&sh.k_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
+                 ptx::mbar_wait(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortScoreSlot, 3 * prm.wait_budget_ns);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(stage * (kHKBytes >> 4));
@@ -566,12 +566,12 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       int count = n_iter;
       for (int pass = 0;; ++pass) {
         arrive_pass();  // nothing of the pass's end depends on this warp
-        ok = warp_wait<true>(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree, 4 * prm.wait_budget_ns);
+        ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree, 4 * prm.wait_budget_ns);
         if (ok && ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
             const int j = done + i, g = j % kHGroups;
-            ok = ptx::mbar_wait<true>(&sh.v_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
-                 ptx::mbar_wait<true>(&sh.p_full[g], (j / kHGroups) & 1u, abort_word, kAbortPFull, 3 * prm.wait_budget_ns);
+            ok = ptx::mbar_wait(&sh.v_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
+                 ptx::mbar_wait(&sh.p_full[g], (j / kHGroups) & 1u, abort_word, kAbortPFull, 3 * prm.wait_budget_ns);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t v_desc = v_desc0 + static_cast<uint64_t>(stage * (kHVBytes >> 4));
@@ -604,7 +604,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
     // scores of tile j -> registers, and the factor that belongs to them
     auto take = [&](uint32_t j, uint32_t (&s)[H3S_KV_TILE], float &c) {
-      if (!warp_wait<true>(&sh.s_full[group], (j / kHGroups) & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) return false;
+      if (!warp_wait(&sh.s_full[group], (j / kHGroups) & 1u, abort_word, kAbortSFull, 2 * prm.wait_budget_ns)) return false;
       const uint32_t slot = j % kHScoreSlots;
       ptx::tc_fence_after();
       H3S_TMEM_LD64(tmem_o + kHTmemS + slot * 64 + lane_addr, s);
@@ -627,7 +627,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     };
     // the group's P columns are free
     auto room = [&](uint32_t j) {
-      return warp_wait<true>(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
+      return warp_wait(&sh.pv_done[group], ((j / kHGroups) & 1u) ^ 1u, abort_word, kAbortPvDone, 4 * prm.wait_budget_ns);
     };
     // behind `room`: the fence orders the store after P.V's reads of the same columns
     auto put = [&](const uint32_t (&packed)[H3S_KV_TILE / 2]) {
@@ -650,11 +650,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     auto meet = [&]() {  // all softmax warps
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&sh.staged);
-      return warp_wait<true>(&sh.staged, staged_uses++ & 1u, abort_word, kAbortStaged, 4 * prm.wait_budget_ns);
+      return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortStaged, 4 * prm.wait_budget_ns);
     };
     // every P.V of the pass that has ended
     auto all_products = [&]() {
-      return warp_wait<true>(&sh.o_full, (passes - 1) & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+      return warp_wait(&sh.o_full, (passes - 1) & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
     };
     auto release_o = [&]() {
       ptx::tc_fence_before();
@@ -732,7 +732,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (!take(done + i, s, c)) return false;
         if (decltype(first)::value) {
           if (i < 2) leave_first(i, c * static_cast<float>(max_score(s)));  // c > 0
-          if (!warp_wait<true>(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) return false;
+          if (!warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns)) return false;
           m = first_reference();
         }
         uint32_t packed[H3S_KV_TILE / 2];
@@ -771,7 +771,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (!ok) break;
       if (rank >= n_iter) {  // a group without a tile: the last item is not finished, and there is no reference point yet
         ok = (!pending || finish_last()) &&
-             warp_wait<true>(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns);
+             warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns);
         if (!ok) break;
         m = first_reference();
       }
