@@ -33,7 +33,7 @@ struct AttnParams {
   unsigned int *arrived;
   int heads, sequence, q_tiles, kv_tiles;
   int out_dtype;
-  bool out_map;  // the output goes through TMA stores (attn_half.cu)
+  bool out_map;  // the output may go, and in attn_half.cu does go, through TMA stores
   // head-sharded runs: every output tile is also stored into these buffers
   // (the same slice of each peer GPU's full output, reached over NVLink with
   // plain stores), so no separate gather pass is needed
@@ -49,6 +49,10 @@ struct AttnParams {
   int drop_kv_load;                   // iteration index, -1 = none
   bool drop_last_v_load;              // H3S_ATTN_TEST_DROP_LAST_V_LOAD: that of every item's last tile (attn_half.cu)
 };
+
+// 1: `out` is memory of this device; 0: other memory that the device can write to (pinned host memory, managed
+// memory, a peer's), which keeps plain stores; else a status (attn_tc.cu)
+int output_home(const void *out, const char *who);
 
 // Checks the arguments of an attention launch and fills `params` (attn_tc.cu).  `v` is the V
 // carrier the kernel reads, E4M3 or its FP16 copy.

@@ -1118,7 +1118,7 @@ extern "C" int h3s_sparse_attn_half_fwd_mirrored(const int8_t *q8, const int8_t 
   CUtensorMap mo;
   const uint64_t stride_s = static_cast<uint64_t>(out_stride_s) * size;
   const uint64_t stride_h = heads > 1 ? static_cast<uint64_t>(out_stride_h) * size : stride_s;
-  prm.out_map = n_peer_out == 0 && (flags & H3S_ATTN_PLAIN_STORES) == 0 &&
+  prm.out_map = prm.out_map && n_peer_out == 0 && (flags & H3S_ATTN_PLAIN_STORES) == 0 &&
                 make_tensor_map_u8_3d(&mo, out, H3S_HEAD_DIM * size, S, heads, stride_s, stride_h, 32 * size, 32,
                                       size == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                                       "sparse_attn_half_fwd output map") == H3S_OK;

@@ -22,6 +22,7 @@ int check_attn_args(const int8_t *q8, const int8_t *k8, const uint8_t *v8t, cons
                     const float *k_scale, const float *v_scale, const int32_t *route, int route_len,
                     int q_start, int q_stop, void *out, int out_dtype, int64_t out_stride_h,
                     int64_t out_stride_s, int heads, int sequence, const char *who);
+int output_home(const void *out, const char *who);
 
 constexpr int kMmaThreads = 256;
 constexpr int kKPitch = H3S_HEAD_DIM + 16;   // bytes per key row
@@ -293,6 +294,8 @@ extern "C" int h3s_sparse_attn_fwd_mma(const int8_t *q8, const int8_t *k8, const
     int rc = check_attn_args(q8, k8, v8t, q_scale, k_scale, v_scale, route, route_len, q_start, q_stop, out,
                              out_dtype, out_stride_h, out_stride_s, heads, sequence, "sparse_attn_fwd_mma");
     if (rc) return rc;
+    rc = output_home(out, "sparse_attn_fwd_mma");
+    if (rc < 0) return rc;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool sp = (flags & H3S_ATTN_P_SINGLE) == 0;

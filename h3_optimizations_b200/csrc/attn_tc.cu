@@ -483,6 +483,16 @@ int check_attn_args(const int8_t *q8, const int8_t *k8, const uint8_t *v8t, cons
   return H3S_OK;
 }
 
+int output_home(const void *out, const char *who) {
+  int device = 0;
+  cudaPointerAttributes at;
+  H3S_CHECK_CUDA(cudaGetDevice(&device));
+  H3S_CHECK_CUDA(cudaPointerGetAttributes(&at, out));
+  H3S_CHECK_ARG(at.type != cudaMemoryTypeUnregistered && at.devicePointer != nullptr,
+                "%s: the output is not memory that device %d can write to", who, device);
+  return at.type == cudaMemoryTypeDevice && at.device == device;
+}
+
 int fill_attn_params(AttnParams *params, const int8_t *q8, const int8_t *k8, const void *v, const float *q_scale,
                      const float *k_scale, const float *v_scale, const int32_t *route, int route_len, int q_start,
                      int q_stop, void *out, void *const *peer_out, int n_peer_out, int out_dtype, int64_t out_stride_h,
@@ -500,7 +510,10 @@ int fill_attn_params(AttnParams *params, const int8_t *q8, const int8_t *k8, con
   const int cap = h3s_device_capability();
   if (cap < 0) return cap;
   if (cap / 10 != 10) return fail(H3S_EARCH, "%s: needs an sm_100 device, found sm_%d", who, cap);
+  const int home = output_home(out, who);
+  if (home < 0) return home;
   AttnParams &prm = *params;
+  prm.out_map = home == 1;
   prm.q_scale = q_scale; prm.k_scale = k_scale; prm.v_scale = v_scale;
   prm.route = route; prm.out = out; prm.status = status;
   prm.out_stride_h = out_stride_h; prm.out_stride_s = out_stride_s;

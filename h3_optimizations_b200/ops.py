@@ -20,7 +20,6 @@ KV_TILE = 64
 HEAD_DIM = 128
 FP8_V_BOUND = 448.0
 ATTN_P_SINGLE = 1
-ATTN_PLAIN_STORES = 2
 ATTN_TEST_DROP_KV_LOAD = 0x4000
 ATTN_TEST_DROP_LAST_V_LOAD = 0x8000
 
@@ -669,7 +668,7 @@ def sparse_attention_of(buffers, route, *, q_start, q_stop, out, out_dtype, stat
     c = buffers.native
     check(lib.h3s_sparse_attn_half_fwd_mirrored(
         c.q8, c.k8, c.v16, c.q_scale, c.k_scale, c.v_scale, ptr(route), route_len, q_start, q_stop, out.data_ptr(), table, n_peers,
-        dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence, 0 if out.is_cuda else ATTN_PLAIN_STORES, ptr(workspace), size, status.data_ptr(),
+        dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence, 0, ptr(workspace), size, status.data_ptr(),
         status_mirror.data_ptr(), stream_ptr(device)), "h3s_sparse_attn_half_fwd")
     return out
 
@@ -725,8 +724,6 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
             v_half = v_half_copy(v_carrier)
         else:
             check_v_half(v_half, v_carrier)
-        if not out.is_cuda:  # pinned host memory
-            after = after[:-1] + (flags | ATTN_PLAIN_STORES,)
         size = lib.h3s_sparse_attn_half_workspace_bytes(heads, sequence, route_len, int(q_start), int(q_stop))
         workspace = torch.empty(size, dtype=torch.uint8, device=q8.device) if size else None
         check(lib.h3s_sparse_attn_half_fwd_mirrored(ptr(q8), ptr(k8), ptr(v_half), *before, table, n_peers, *after, ptr(workspace),
