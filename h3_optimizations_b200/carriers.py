@@ -3,7 +3,7 @@ attention/sparse/sparse_sage.py:401-417)."""
 
 from __future__ import annotations
 
-from dataclasses import InitVar, dataclass, field, fields
+from dataclasses import InitVar, dataclass, field
 
 import torch
 
@@ -29,6 +29,9 @@ class VCarrier:
         """The pair that ``prepared`` holds; its codes alone where it is no class of this module."""
         pair = getattr(prepared, "_v", None)
         return pair if isinstance(pair, cls) else cls(prepared.v_carrier)
+
+    def __reduce__(self):
+        return VCarrier, (self.codes, self.half)
 
     @classmethod
     def field(cls):
@@ -170,6 +173,10 @@ class PreparedSparse:
 PreparedSparse.v_carrier = VCarrier.field()
 
 
+def _unfilled(cls):
+    return object.__new__(cls)
+
+
 class PreparedLayer(PreparedSparse):
     """A ``PreparedSparse`` whose carriers are those of an ``ops.LayerBuffers`` (``over``).  Its tensors come into being
     when they are asked for; until then (``untouched``) nobody can have written to them or put others in their place."""
@@ -206,8 +213,11 @@ class PreparedLayer(PreparedSparse):
             return None
         return buffers
 
-    def __reduce_ex__(self, protocol):  # a copy is a PreparedSparse of its own tensors
-        return PreparedSparse, tuple(getattr(self, f.name) for f in fields(PreparedSparse))
+    def __reduce_ex__(self, protocol):
+        """A copy is a ``PreparedSparse``.  A shallow one shares the tensors, and the pair of codes and FP16 copy as such."""
+        state = {name: getattr(self, name) for name in PreparedLayer._LAZY}
+        state.update((name, value) for name, value in self.__dict__.items() if name != "_buffers")
+        return _unfilled, (PreparedSparse,), state
 
 
 @dataclass
