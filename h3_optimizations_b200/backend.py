@@ -269,6 +269,8 @@ class B200SparseBackend:
             if slot is None:
                 continue
             words = slot[0].cpu().tolist()
+            if words[0] == 0:
+                words = slot[1].tolist()  # a kernel of another stream may have got to the mirror after both were cleared
             if words[0] != 0:
                 slot[0].zero_()
                 slot[1].zero_()
