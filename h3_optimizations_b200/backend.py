@@ -18,7 +18,7 @@ the kernel return early and leave a code in a per-device status word that the
 backend hands to every launch.  Reading that word needs the stream to have
 drained, so it is not done on the hot path: ``check_status()`` reads it (and
 raises) whenever the caller synchronises anyway, ``forward_host`` calls it
-before it returns, and the next ``prepare`` on the device looks, without
+before it returns, and the next ``prepare`` or ``prepare_projected`` on the device looks, without
 blocking, at a mirror of the word in pinned host memory that a kernel which
 gave up writes as well (with a copy behind every launch instead, the next
 call's kernels began 8 us later).
@@ -346,6 +346,7 @@ class B200SparseBackend:
         heads, sequence = int(projected.heads), int(projected.sequence)
         if not projected.q_int8.is_cuda:
             raise SparseSageError("fused H3 Sparse Sage requires CUDA")
+        self._poll_status(projected.q_int8.device)
         try:
             route = self.router.build_route_from_summaries(
                 projected.q_summary, projected.k_summary, snapshot.layout, video_budget,

@@ -47,3 +47,25 @@ def test_the_next_prepare_raises_until_the_words_are_cleared(short_budget):  # n
         backend.check_status()
     backend.execute(prepare())
     backend.check_status()
+
+
+def test_the_projected_way_looks_at_it_too(native_lib):
+    from h3_optimizations_b200 import B200SparseBackend, HybridSparseConfig, runtime_options, workloads
+    from h3_optimizations_b200.errors import SparseSageError
+    from h3_optimizations_b200.projector import run_chunked_sparse_qkv
+
+    spec = workloads.small_spec("mirror", 1, 64, 192)
+    options = runtime_options(spec.layout(), step_index=5, total_steps=20)
+    x = torch.ones((256, 256), dtype=torch.bfloat16, device="cuda")
+    w = torch.ones((384, 256), dtype=torch.int8, device="cuda")
+    projected = run_chunked_sparse_qkv(x, w, torch.full((384,), 0.01, device="cuda"), heads=1)
+    backend = B200SparseBackend(HybridSparseConfig(video_budget=0.3))
+    backend.execute(backend.prepare_projected(projected, layer_index=0, transformer_options=options))
+    torch.cuda.synchronize()
+    backend._status_slot(x.device)[1].copy_(torch.tensor([K_V_TILE_LOAD, 0, 0, 1], dtype=torch.int32))
+    with pytest.raises(SparseSageError, match="K/V tile load.*reported by an earlier launch"):
+        backend.prepare_projected(projected, layer_index=0, transformer_options=options)
+    with pytest.raises(SparseSageError, match="found by check_status"):
+        backend.check_status()
+    backend.execute(backend.prepare_projected(projected, layer_index=0, transformer_options=options))
+    backend.check_status()
