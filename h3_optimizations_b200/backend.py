@@ -39,6 +39,12 @@ from .runtime import get_runtime_snapshot
 # 4 x 2304 108 / 96, 6 x 4256 114 / 98, 24 x 1328 106 / 93, 4 x 9256 112 / 110, 12 x 4256 104 / 94; with the device waited for
 # after each call 126 / 110, 130 / 123, 140 / 133, 127 / 121, 170 / 165, 152 / 145.  Beyond, the kernels take longer than the host.
 ONE_STREAM_ROWS = 52000
+# Output copies of ``forward_host`` are cut into pieces of this size.  A copy out that runs beside the next chunk's copies in
+# slows them down, by how much depends on which of them it meets; between pieces the two directions are dealt out anew.
+# us a call, whole / pieces of 3, 2, 1.6 and 1.25 MB: 24 heads x 9881 tokens 4189 / 3928, 3934, 3973, 3988; 12 x 8512 1940 / 1936, 1827,
+# 1851, 1854; 24 x 6512 2995 / 3007, 2802, 2806, 2866; 4 x 33512 2545 / 2466, 2474, 2467, 2474; 8 x 33272 4486 / 4424, 4393, 4382, 4384;
+# 8 x 4512 (2.3 MB a chunk) 930 / 936, 929, 915, 994; 24 x 11512 dense 4740 / 4704, 4687, 4683, 4681.
+COPY_OUT_BYTES = 1.6 * 2**20
 V_QUANT_BOUND = 448.0  # FP32 accumulation (reference: sparse_sage.py:296)
 
 
@@ -511,7 +517,7 @@ class B200SparseBackend:
             slot["computed"].record(main)
             with torch.cuda.stream(d2h):
                 d2h.wait_event(slot["computed"])
-                out[:, a:b].copy_(slot["out"][:, :n], non_blocking=True)
+                self._copy_out(out[:, a:b], slot["out"][:, :n], last=b == heads)
                 slot["stored"].record(d2h)
         main.wait_stream(d2h)
         main.wait_stream(h2d)
@@ -529,6 +535,16 @@ class B200SparseBackend:
             return [(a, min(a + chunk, heads)) for a in range(0, heads, chunk)]
         pairs = (heads - 1) // 2
         return [(2 * i, 2 * i + 2) for i in range(pairs)] + [(a, a + 1) for a in range(2 * pairs, heads)]
+
+    @staticmethod
+    def _copy_out(to, source, last=False):
+        """One chunk's output to host memory, in pieces of about ``COPY_OUT_BYTES`` unless nothing comes in any more."""
+        pieces = 1 if last else max(1, round(to.numel() * to.element_size() / COPY_OUT_BYTES))
+        if pieces == 1:
+            to.copy_(source, non_blocking=True)
+            return
+        for part, rows in zip(to.view(-1, 128).tensor_split(pieces), source.view(-1, 128).tensor_split(pieces)):
+            part.copy_(rows, non_blocking=True)
 
     def _host_pipeline(self, device, chunk, sequence, dtype, n_slots):
         key = (device.index, int(chunk), int(sequence), dtype, int(n_slots))
