@@ -38,7 +38,14 @@ from .runtime import get_runtime_snapshot
 # Rows of all heads up to which a layer is prepared on one stream.  us a call, two streams / one: 1 head x 1128 tokens 106 / 90,
 # 4 x 2304 108 / 96, 6 x 4256 114 / 98, 24 x 1328 106 / 93, 4 x 9256 112 / 110, 12 x 4256 104 / 94; with the device waited for
 # after each call 126 / 110, 130 / 123, 140 / 133, 127 / 121, 170 / 165, 152 / 145.  Beyond, the kernels take longer than the host.
+# It holds for the chunks of host calls as well: 8 heads x 2512 tokens in pairs 908 / 848, 24 x 3512 2398 / 2325; longer ones are
+# alike (8 x 8512 1311 / 1316, 24 x 11512 4481 / 4486, 4 x 33512 2440 / 2461, 12 x 12512 2560 / 2550).
 ONE_STREAM_ROWS = 52000
+# Bytes of a head's q, k and v from which ``forward_host`` ends with single heads: as long as they take to copy a chunk more is
+# paid for by a shorter end, below that it costs the host's time.  us a call, pairs to the end / single heads at the end, 8 heads,
+# bf16: 1212 tokens 818 / 1001, 4512 933 / 1046, 6512 1080 / 1130, 7512 1155 / 1181, 8512 1316 / 1313, 10512 1594 / 1555, 33272 4575 /
+# 4374; fp32: 3512 1113 / 1157, 4512 1389 / 1389, 10512 2918 / 2845; 24 heads, bf16: 1212 2203 / 2384, 6512 2755 / 2769, 11512 4486 / 4458.
+LONE_HEAD_BYTES = 6_500_000
 # Output copies of ``forward_host`` are cut into pieces of this size.  A copy out that runs beside the next chunk's copies in
 # slows them down, by how much depends on which of them it meets; between pieces the two directions are dealt out anew.
 # us a call, whole / pieces of 3, 2, 1.6 and 1.25 MB: 24 heads x 9881 tokens 4189 / 3928, 3934, 3973, 3988; 12 x 8512 1940 / 1936, 1827,
@@ -474,7 +481,10 @@ class B200SparseBackend:
         is the longest of the three, so the call takes about as long as that
         copy alone.  Returns ``out`` (host, HND ``(1, H, S, 128)``; allocated
         pinned when not given).  With a route sink installed the heads are not
-        split (the sink expects one call per layer).  The call returns once the
+        split (the sink expects one call per layer).  How many heads go through
+        at a time decides into how many parts the attention kernel cuts the rows that
+        see every key, and so the order of their FP32 sums: the last bits of a head may
+        differ between chunk sizes, and from those of a whole layer.  The call returns once the
         output is in host memory and raises if a launch reported an expired
         device wait."""
         if q.is_cuda or k.is_cuda or v.is_cuda:
@@ -491,7 +501,7 @@ class B200SparseBackend:
             raise SparseSageError("forward_host: out must be a contiguous host tensor shaped and typed like q")
         recorder = (transformer_options or {}).get("h3_optimizations_attention_route")
         whole = getattr(recorder, "sink", None) is not None
-        bounds = [(0, heads)] if whole else self._head_chunks(heads, heads_per_chunk)
+        bounds = [(0, heads)] if whole else self._head_chunks(heads, heads_per_chunk, 3 * sequence * 128 * q.element_size())
         chunk = max((b - a for a, b in bounds), default=1)
         device = torch.device("cuda", torch.cuda.current_device())
         main = torch.cuda.current_stream(device)
@@ -526,12 +536,14 @@ class B200SparseBackend:
         return out
 
     @staticmethod
-    def _head_chunks(heads, heads_per_chunk):
+    def _head_chunks(heads, heads_per_chunk, head_bytes=LONE_HEAD_BYTES):
         """The heads ``forward_host`` takes through at a time, as (first, stop).  By itself it takes two where that leaves
-        at least four chunks, so that copy-in, kernels and copy-out overlap, and ends with single heads: what the last chunk's
-        kernels and copy-out take comes on top of the copies in (8 heads x 33272 tokens 4746 -> 4440 us)."""
-        if heads_per_chunk is not None or heads < 8:
-            chunk = max(1, min(int(heads_per_chunk or 1), heads))
+        at least four chunks, so that copy-in, kernels and copy-out overlap, and ends with single heads where a head's q, k and v
+        (``head_bytes``) are many: what the last chunk's kernels and copy-out take comes on top of the copies in."""
+        if heads_per_chunk is not None or heads < 8 or head_bytes < LONE_HEAD_BYTES:
+            if heads_per_chunk is None:
+                heads_per_chunk = 2 if heads >= 8 else 1
+            chunk = max(1, min(int(heads_per_chunk), heads))
             return [(a, min(a + chunk, heads)) for a in range(0, heads, chunk)]
         pairs = (heads - 1) // 2
         return [(2 * i, 2 * i + 2) for i in range(pairs)] + [(a, a + 1) for a in range(2 * pairs, heads)]

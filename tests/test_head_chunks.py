@@ -19,6 +19,15 @@ def test_chunks_cover_the_heads_once(heads, asked):
         assert max(sizes) == (2 if heads >= 8 else 1) and sizes[-1] == 1
 
 
+@pytest.mark.parametrize("heads", [1, 2, 7, 8, 9, 24, 25])
+@pytest.mark.parametrize("asked", [None, 1, 3])
+def test_short_heads_stay_in_pairs(heads, asked):
+    chunks = B200SparseBackend._head_chunks(heads, asked, module.LONE_HEAD_BYTES - 1)
+    assert [h for a, b in chunks for h in range(a, b)] == list(range(heads))
+    size = min(heads, asked or (2 if heads >= 8 else 1))
+    assert [b - a for a, b in chunks] == [size] * (heads // size) + [heads % size] * (heads % size > 0)
+
+
 @pytest.mark.parametrize("size", [1, 512, 5000, 10**9])
 @pytest.mark.parametrize("last", [False, True])
 @pytest.mark.parametrize("heads,sequence", [(1, 1), (1, 7), (2, 13), (3, 64)])
