@@ -347,14 +347,6 @@ def project_qkv(x, w_i8, w_scale, buffers, side, stream, *, heads, chunk_rows, s
     )
 
 
-def status_mirror(word, mirror, event, stream):
-    """Queue the copy of the status words into pinned ``mirror`` and ``event`` behind it."""
-    if not event.cuda_event:
-        event.record()  # brings the native event into being
-    check(_native.load().h3s_status_mirror(word.data_ptr(), mirror.data_ptr(), event.cuda_event, stream),
-          "h3s_status_mirror")
-
-
 def convrot_quant_rows(x, x_i8=None, x_scale=None):
     """ConvRot (Hadamard-256) + per-row INT8 of ``x`` (rows, hidden) bf16.
     Returns ``(codes int8 (rows, hidden), scale fp32 (rows,))``."""

@@ -1,0 +1,57 @@
+"""C entry points that the package itself does not call: those with fewer arguments do what the longer ones do, and the
+copy of the status words.  Needs a B200."""
+
+import pytest
+import torch
+
+from h3_optimizations_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def test_attention_without_a_mirror(native_lib, monkeypatch):
+    from h3_optimizations_b200 import ops
+
+    spec = workloads.small_spec("entries", 2, 0, 500)
+    q, k, v = (t.cuda() for t in workloads.gaussian_qkv(spec, seed=2))
+    k_mean, v_scale = ops.column_stats(k, v)
+    q8, qs, _ = ops.quant_qk_blocks(q, 128)
+    k8, ks, _ = ops.quant_qk_blocks(k, 64, mean=k_mean)
+    vc, _ = ops.quant_v_fp8(v, v_scale)
+    expected = ops.sparse_attention(q8, k8, vc, qs, ks, v_scale)
+    calls = []
+    monkeypatch.setattr(native_lib, "h3s_sparse_attn_half_fwd_mirrored",
+                        lambda *args: calls.append(1) or native_lib.h3s_sparse_attn_half_fwd(*args[:-2], args[-1]))
+    assert torch.equal(ops.sparse_attention(q8, k8, vc, qs, ks, v_scale), expected) and calls
+
+
+def test_projection_with_fp32_norms(native_lib, monkeypatch):
+    from h3_optimizations_b200.projector import run_chunked_sparse_qkv
+
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn((300, 256), generator=gen, device="cuda").bfloat16()
+    w = torch.randint(-127, 128, (3 * 2 * 128, 256), generator=gen, device="cuda", dtype=torch.int8)
+    w_scale = torch.rand(3 * 2 * 128, generator=gen, device="cuda") / 2000
+    norm = (*(torch.rand(128, generator=gen, device="cuda") + 0.5 for _ in range(2)), 1e-6)
+
+    def carriers():
+        p = run_chunked_sparse_qkv(x, w, w_scale, heads=2, chunk_rows=128, norm=norm)
+        return [p.q_int8, p.k_int8, p.q_scale, p.k_scale, p.v_scale, p.q_summary, p.v_carrier.view(torch.uint8)]
+
+    expected = carriers()
+    calls = []
+    monkeypatch.setattr(native_lib, "h3s_project_qkv_norms",
+                        lambda *args: calls.append(1) or native_lib.h3s_project_qkv(*args[:16], *args[17:]))
+    assert all(torch.equal(a, b) for a, b in zip(carriers(), expected)) and calls
+
+
+def test_copy_of_the_status_words(native_lib):
+    from h3_optimizations_b200 import _native
+
+    word = torch.tensor([2, 5, 1, 3], dtype=torch.int32, device="cuda")
+    mirror = torch.zeros(4, dtype=torch.int32).pin_memory()
+    event = torch.cuda.Event()
+    event.record()
+    _native.check(native_lib.h3s_status_mirror(word.data_ptr(), mirror.data_ptr(), event.cuda_event, _native.stream_ptr()), "h3s_status_mirror")
+    event.synchronize()
+    assert mirror.tolist() == [2, 5, 1, 3]
