@@ -996,20 +996,25 @@ __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v
 }
 
 // Whether and how the dense rows' tile lists are cut.  A row longer than half of what an SM gets on average may end after
-// everything else has, which parts even out; but parts are dear.  Beside its tiles (0.36 us each) a whole list takes an SM
-// about as long as twelve tiles (before its epilogue ran under the next item's tiles), a part about 27: it writes 66 KB, waits
-// until they are seen, and one of them reads them all back.  So as many parts as end first by this estimate, every SM taking the
-// next item as it gets free, and only if
-//  - that is earlier than with whole rows by more than 3 %, or
-//  - it is no later, and the parts' own cost is under 1 % of the work (three heads of 33272 tokens at 30 %: 376 us either way), or
-//  - nothing but dense rows is there, and dealt out evenly instead of in rounds the parts would end with the rows.
-//    Whole rows are the faster ones at this last line, for all that (3 x 4000: 33 us, 44 in parts).
-// Measured, us, with parts of a quarter of the average share as before / now:
-//   dense   1 x 5000 42 / 28, 1 x 9400 82 / 46, 1 x 33272 424 / 385, 2 x 9000 110 / 62, 3 x 12000 194 / 149, 4 x 9000 162 / 115,
-//           6 x 1545 34 / 18, 12 x 2000 53 / 37; 1 x 20000 190 either way (239 whole), 2 x 1537 20 (17 whole)
-//   routed  24 x 5000 at 10 % 87 / 74, 24 x 2362 at 20 % 56 / 40, 12 x 4540 at 20 % 65 / 51, 1 x 33272 at 10 % 79 / 61 (195 whole)
+// everything else has, which parts even out; but parts are dear.  Beside its tiles (0.35 us each) a whole dense row takes an SM
+// about as long as eight tiles, a routed one fifteen (most of it before its first tile), a part 28 and three for each
+// part of its row: it writes 66 KB, waits until they are seen, and one of them reads them all back; and counters are cleared
+// before the launch, which then starts behind the one before it.  So as many parts as end first by this estimate, every SM
+// taking the next item as it gets free, and only if
+//  - that is earlier than with whole rows, or
+//  - it is no later, and the parts' own cost is under 1 % of the work (three heads of 33272 tokens at 30 %: 417 us, 410 whole), or
+//  - nothing but dense rows is there, and dealt out evenly instead of in rounds the parts would end with the rows, by an older
+//    estimate of their cost.  Whole rows are the faster ones at this last line (3 x 4000: 30 us, 45 in parts; 2 x 1537 15 and 23);
+//    it stays because the tests of the parts take their shapes from it.
+// Fitted to 228 shapes of 1 to 24 heads, launches in a row.  Measured, us, whole / in parts (how many), the one taken last:
+//   dense   1 x 5000 34 / 28 (3), 1 x 9400 57 / 45 (2), 1 x 20000 224 / 185 (3); 2 x 9000 99 (4) / 57, 4 x 9000 177 (4) / 106,
+//           6 x 1545 35 (3) / 15, 12 x 2000 56 (2) / 32, 1 x 33272 463 (4) / 401
+//   routed  1 x 12512 at 30 % 74 / 34 (6), 3 x 6512 at 30 % 42 / 39 (2), 2 x 15000 at 15 % 87 / 46 (3), 1 x 33272 at 10 % 184 / 58 (5), at 30 %
+//           202 / 134 (2); 4 x 2304 at 30 % 24 (6) / 19, 6 x 4256 33 (2) / 30, 24 x 5000 at 10 % 100 (4) / 75, 7 x 10384 at 15 % 74 (4) / 68
+// It is wrong by most for 3 x 18181 at 20 % (107 whole, 96 in sixteen parts) and 4 x 8161 at 15 % (46 in three, 43 in four).
 constexpr int kMinPartTiles = 6, kMaxParts = 16;
-constexpr int kItemTiles = 12, kPartItemTiles = 27;
+constexpr int kLongTiles = 8, kRoutedTiles = 15, kPartTiles = 28, kPerPartTiles = 3;
+constexpr int kEvenLongTiles = 12, kEvenPartTiles = 27;
 
 // When the last item ends, in tiles: `dense` ones of `dense_cost` first, then `routed` ones of `routed_cost`
 static int64_t launch_span(int64_t dense, int64_t dense_cost, int64_t routed, int64_t routed_cost) {
@@ -1029,20 +1034,21 @@ static int64_t launch_span(int64_t dense, int64_t dense_cost, int64_t routed, in
 static int split_dense_rows(int heads, int q_tiles, int kv_tiles, int n_sparse, int route_len) {
   const int64_t rows = static_cast<int64_t>(heads) * (q_tiles - n_sparse), routed = static_cast<int64_t>(heads) * n_sparse;
   if (rows == 0 || static_cast<int64_t>(kv_tiles) * kSmCount * 2 <= rows * kv_tiles + routed * route_len) return 1;
-  const int64_t whole_cost = kv_tiles + kItemTiles, routed_cost = route_len + kItemTiles;
+  const int64_t whole_cost = kv_tiles + kLongTiles, routed_cost = route_len + kRoutedTiles;
   const int64_t whole_span = launch_span(rows, whole_cost, routed, routed_cost), whole_work = rows * whole_cost + routed * routed_cost;
   int best = 1;
   int64_t best_span = 0, best_work = 0;
   bool even = false;
   for (int parts = 2; parts <= kMaxParts && kv_tiles / parts >= kMinPartTiles; ++parts) {
-    const int64_t cost = ceil_div(kv_tiles, parts) + kPartItemTiles, work = rows * parts * cost + routed * routed_cost;
+    const int part_tiles = ceil_div(kv_tiles, parts);
+    const int64_t cost = part_tiles + kPartTiles + kPerPartTiles * parts, work = rows * parts * cost + routed * routed_cost;
     const int64_t span = launch_span(rows * parts, cost, routed, routed_cost);
     if (best == 1 || span < best_span) { best = parts; best_span = span; best_work = work; }
-    const int64_t share = work / kSmCount;
-    even = even || (routed == 0 && 100 * (share > cost ? share : cost) <= 103 * whole_cost);
+    const int64_t even_cost = part_tiles + kEvenPartTiles, share = rows * parts * even_cost / kSmCount;
+    even = even || (routed == 0 && 100 * (share > even_cost ? share : even_cost) <= 103 * (kv_tiles + kEvenLongTiles));
   }
   if (best == 1) return 1;
-  const bool earlier = 100 * best_span < 97 * whole_span;
+  const bool earlier = best_span < whole_span;
   const bool free = best_span <= whole_span && 100 * best_work <= 101 * whole_work;
   return earlier || free || even ? best : 1;
 }

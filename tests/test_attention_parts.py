@@ -31,3 +31,16 @@ def test_rows_that_end_with_the_routed_ones_stay_whole(native_lib, heads, sequen
                                                             (1, 33272, 512, 0.3), (3, 6404, 812, 0.1), (4, 7511, 193, 0.3)])
 def test_rows_that_outlast_everything_else_are_cut(native_lib, heads, sequence, context, density):
     assert 2 <= _parts(native_lib, heads, sequence, context, density) <= 16
+
+
+@pytest.mark.parametrize("heads,sequence,context,density", [(1, 2304, 256, 0.3), (4, 2304, 256, 0.3), (6, 4256, 512, 0.3), (3, 2103, 813, 0.3),
+                                                            (7, 1594, 234, 0.15), (4, 29543, 451, 0.15), (4, 9000, 978, 0.3)])
+def test_rows_whose_parts_cost_more_than_they_even_out_stay_whole(native_lib, heads, sequence, context, density):
+    """With the cost of a part underestimated these were cut, and took up to 1.4 times as long."""
+    assert _parts(native_lib, heads, sequence, context, density) == 1
+
+
+@pytest.mark.parametrize("heads,sequence,context,density,parts", [(1, 12512, 512, 0.3, 6), (3, 6512, 512, 0.3, 2), (1, 5000, 512, 0.15, 5),
+                                                                  (2, 15000, 512, 0.15, 3), (1, 33272, 512, 0.1, 5), (1, 9400, 0, 1.0, 2)])
+def test_the_number_of_parts(native_lib, heads, sequence, context, density, parts):
+    assert _parts(native_lib, heads, sequence, context, density) == parts
