@@ -70,8 +70,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // Every lane polls the barrier; the warp then agrees on the outcome so that
 // the .sync.aligned tcgen05 instructions that follow stay convergent even if
 // the abort word was raised between two lanes' polls.
-template <typename Abort>
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, Abort abort_word, int code,
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_word, int code,
                                           unsigned long long budget_ns) {
   if (__all_sync(0xffffffffu, ptx::mbar_test_wait(bar, parity))) return true;  // the usual case, kept short
   const bool ok = ptx::mbar_wait(bar, parity, abort_word, code, budget_ns);

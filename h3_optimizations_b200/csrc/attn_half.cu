@@ -101,6 +101,9 @@ constexpr int kHNoted = 2048;          // bits of the note of tiles left out, ea
 
 enum { kAgainNoted = 1, kAgainFar = 2 };
 
+// Beside the code of a wait: whose item it was about.  Constants, as what stands behind a wait is code in the loops.
+constexpr int kInScoreIssuer = kHScoreIssuer << 8, kInValueIssuer = kHValueIssuer << 8, kItemBefore = 1 << 15;
+
 // What the warps need to know of an item: left by the K loader, so that its place in the launch is worked out once
 struct alignas(16) HalfItem {
   float v_scale[H3S_HEAD_DIM];
@@ -125,8 +128,8 @@ struct alignas(16) HalfShared {
   uint64_t pass_end;           // the rows' values of a pass are in `row`, `noted` is complete; all warps arrive and wait
   uint64_t staged;             // softmax warps only: the output tile is in shared memory (and steps before that)
   uint32_t tmem_base;
-  int abort_word;              // code of the wait that ran out, and 256 times the warp it was in
-  int stopped[kHWarps];        // turn (of three) of the item that a warp gave up in
+  int abort_word;              // code of the wait that ran out, 256 times the warp it was in (softmax: 0), kItemBefore
+  int stopped[kHWarps];        // turn (of three) of the item that a warp ended at
   int finish;                  // of an item that is a part: this CTA writes the output tile
   int again[4];                // per item in turn.  kAgainNoted: some row has left out a tile; kAgainFar: its sum
                                // there does not tell the maximum
@@ -276,7 +279,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   // (offset arithmetic, so that the compiler still sees shared memory)
   unsigned char *smem = smem_dyn + ((1024u - (ptx::smem_u32(smem_dyn) & 1023u)) & 1023u);
   HalfShared &sh = *reinterpret_cast<HalfShared *>(smem + L::kOffShared);
-  const ptx::WarpAbort abort_word{&sh.abort_word};
+  volatile int *abort_word = &sh.abort_word;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -348,7 +351,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (lane == 0) ptx::mbar_arrive(&sh.pass_end);
   };
   auto wait_pass = [&]() {
-    return warp_wait(&sh.pass_end, passes & 1u, abort_word, kAbortPass, 4 * prm.wait_budget_ns);
+    return warp_wait(&sh.pass_end, passes & 1u, abort_word, kAbortPass | warp << 8, 4 * prm.wait_budget_ns);
   };
   auto end_pass = [&]() {
     arrive_pass();
@@ -421,7 +424,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int head = work.head;
         for (int i = 0; i < tiles; ++i) {
           const int t = block[i];
-          fine = ptx::mbar_wait(&empty[stage], round, abort_word, kAbortKvEmpty, 4 * prm.wait_budget_ns);
+          fine = ptx::mbar_wait(&empty[stage], round, abort_word, kAbortKvEmpty | warp << 8, 4 * prm.wait_budget_ns);
           if (!fine) break;
           if (drop != 0) {
             ptx::mbar_arrive_expect_tx(&full[stage], bytes);
@@ -453,7 +456,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         ok = load_block(min(kHBlock, work.n_iter - i), [&]() { if (i + kHBlock < work.n_iter) fetch_block(work, i + kHBlock); });
       }
-      ok = ok && warp_wait(&sh.next_ready, items & 1u, abort_word, kAbortNextItem, 4 * prm.wait_budget_ns);
+      ok = ok && warp_wait(&sh.next_ready, items & 1u, abort_word, kAbortNextItem | warp << 8, 4 * prm.wait_budget_ns);
       if (!ok) break;
       const int next = ptx::granted_block(&sh.next_reply);
       if (next >= 0) {
@@ -471,7 +474,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + coming.head * H3S_HEAD_DIM + i * 32 + lane);
-          ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortQFree, 4 * prm.wait_budget_ns);
+          ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortQFree | warp << 8, 4 * prm.wait_budget_ns);
           if (!ok) break;
           load_q(coming);
         }
@@ -519,7 +522,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     uint32_t round = 0, slot_round = 0;
     while (ok) {
       const uint32_t tmem_q = tmem_o + kHTmemQ + (items & 1) * 32;
-      ok = warp_wait(&sh.q_full, items & 1u, abort_word, kAbortQFull, prm.wait_budget_ns);
+      ok = warp_wait(&sh.q_full, items & 1u, abort_word, kAbortQFull | kInScoreIssuer, prm.wait_budget_ns);
       if (!ok) break;
       if (ptx::elect_one()) {
 #pragma unroll
@@ -532,8 +535,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         arrive_pass();  // nothing of the pass's end depends on this warp
         if (ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
-            ok = ptx::mbar_wait(&sh.k_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
-                 ptx::mbar_wait(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortScoreSlot, 3 * prm.wait_budget_ns);
+            ok = ptx::mbar_wait(&sh.k_full[stage], round, abort_word, kAbortKvFull | kInScoreIssuer, prm.wait_budget_ns) &&
+                 ptx::mbar_wait(&sh.s_taken[slot], slot_round ^ 1u, abort_word, kAbortScoreSlot | kInScoreIssuer, 3 * prm.wait_budget_ns);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t k_desc = k_desc0 + static_cast<uint64_t>(stage * (kHKBytes >> 4));
@@ -566,12 +569,12 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       int count = n_iter;
       for (int pass = 0;; ++pass) {
         arrive_pass();  // nothing of the pass's end depends on this warp
-        ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree, 4 * prm.wait_budget_ns);
+        ok = warp_wait(&sh.o_free, (passes & 1u) ^ 1u, abort_word, kAbortOFree | kInValueIssuer, 4 * prm.wait_budget_ns);
         if (ok && ptx::elect_one()) {
           for (int i = 0; i < count; ++i) {
             const int j = done + i, g = j % kHGroups;
-            ok = ptx::mbar_wait(&sh.v_full[stage], round, abort_word, kAbortKvFull, prm.wait_budget_ns) &&
-                 ptx::mbar_wait(&sh.p_full[g], (j / kHGroups) & 1u, abort_word, kAbortPFull, 3 * prm.wait_budget_ns);
+            ok = ptx::mbar_wait(&sh.v_full[stage], round, abort_word, kAbortKvFull | kInValueIssuer, prm.wait_budget_ns) &&
+                 ptx::mbar_wait(&sh.p_full[g], (j / kHGroups) & 1u, abort_word, kAbortPFull | kInValueIssuer, 3 * prm.wait_budget_ns);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t v_desc = v_desc0 + static_cast<uint64_t>(stage * (kHVBytes >> 4));
@@ -653,8 +656,8 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       return warp_wait(&sh.staged, staged_uses++ & 1u, abort_word, kAbortStaged, 4 * prm.wait_budget_ns);
     };
     // every P.V of the pass that has ended
-    auto all_products = [&]() {
-      return warp_wait(&sh.o_full, (passes - 1) & 1u, abort_word, kAbortFinal, 4 * prm.wait_budget_ns);
+    auto all_products = [&](int whose = 0) {
+      return warp_wait(&sh.o_full, (passes - 1) & 1u, abort_word, kAbortFinal | whose, 4 * prm.wait_budget_ns);
     };
     auto release_o = [&]() {
       ptx::tc_fence_before();
@@ -685,10 +688,9 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // not wait for the last P.V, and the next P.V comes later.  Every warp by itself: its 32 rows of 32 columns
     // go through its own piece of shared memory to a TMA store, which also leaves out rows past the sequence.
     bool pending = false;
-    auto finish_last = [&]() {
-      const HalfItem &from = sh.item[(items + 2) % 3u];
+    auto finish_last = [&](const HalfItem &from) {
       pending = false;
-      if (!all_products()) { items += 2; return false; }  // given up in that item
+      if (!all_products(kItemBefore)) return false;
       ptx::tc_fence_after();
       uint32_t o[32];
       H3S_TMEM_LD32(tmem_o + lane_addr + group * 32, o);
@@ -762,7 +764,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       };
       if (rank < n_iter) {
         ok = walk(rank, std::true_type{});
-        if (ok && pending) ok = finish_last();
+        if (ok && pending) ok = finish_last(sh.item[(items + 2) % 3u]);
         if (ok) {
           for (int i = rank + kHGroups; i < n_iter; i += kHGroups)
             if (!walk(i, std::false_type{})) { ok = false; break; }
@@ -770,7 +772,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
       if (!ok) break;
       if (rank >= n_iter) {  // a group without a tile: the last item is not finished, and there is no reference point yet
-        ok = (!pending || finish_last()) &&
+        ok = (!pending || finish_last(sh.item[(items + 2) % 3u])) &&
              warp_wait(&sh.first_max, items & 1u, abort_word, kAbortFirstMax, 2 * prm.wait_budget_ns);
         if (!ok) break;
         m = first_reference();
@@ -860,7 +862,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (!split && prm.out_map) {
         pending = true;
         if (next_item()) continue;
-        ok = finish_last();
+        ok = finish_last(sh.item[(items + 2) % 3u]);
         break;
       }
 
@@ -955,15 +957,17 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   }
 
   // ---- teardown ----
-  if (!ok && lane == 0) sh.stopped[warp] = items % 3u;
+  if (lane == 0) sh.stopped[warp] = items % 3u;
   __syncthreads();
-  const int code = sh.abort_word & 255;
+  const int word = sh.abort_word, code = word & 255;
   if (code != 0) {
     // leave time for copies / MMAs still in flight before releasing TMEM and shared memory
     __nanosleep(200000);
     if (threadIdx.x == 0 && prm.status != nullptr) {
       if (atomicCAS(prm.status, 0, code) == 0) {
-        const HalfItem &at = sh.item[sh.stopped[sh.abort_word >> 8]];
+        int turn = (sh.stopped[(word >> 8) & 31] + ((word & kItemBefore) != 0 ? 2 : 0)) % 3;
+        if (sh.item[turn].number < 0) turn = (turn + 2) % 3;  // a warp that was through
+        const HalfItem &at = sh.item[turn];
         prm.status[1] = at.number;
         prm.status[2] = at.head;
         prm.status[3] = at.tq;

@@ -94,19 +94,10 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
   return done != 0;
 }
 
-// The abort word of a kernel that also wants to know which warp gave up: code + 256 * warp
-struct WarpAbort {
-  volatile int *word;
-  __device__ __forceinline__ int operator*() const { return *word; }
-};
-__device__ __forceinline__ void raise_abort(volatile int *word, int code) { atomicCAS(const_cast<int *>(word), 0, code); }
-__device__ __forceinline__ void raise_abort(WarpAbort at, int code) { raise_abort(at.word, code | static_cast<int>(threadIdx.x >> 5) << 8); }
-
 // Waits for the phase with the given parity.  Returns false (and raises
 // *abort_word with `code`) when the budget expires or another waiter already
-// gave up.  The word lives in shared memory.
-template <typename Abort>
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, Abort abort_word,
+// gave up.  `abort_word` lives in shared memory.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_word,
                                           int code, unsigned long long budget_ns) {
   // a phase that is already complete costs one test_wait (a try_wait with a
   // suspend hint takes about twice as long even when it succeeds at once)
@@ -119,7 +110,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, Abort 
     if ((++spins & 15u) == 0u) {
       if (*abort_word != 0) return false;
       if (global_timer_ns() - start > budget_ns) {
-        raise_abort(abort_word, code);
+        atomicCAS(const_cast<int *>(abort_word), 0, code);
         return false;
       }
     }
