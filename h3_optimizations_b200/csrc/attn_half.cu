@@ -30,11 +30,11 @@
 // deviation, held over groups of 64 tokens, 2 to 14 % of the query tiles (27 % in a dense one of
 // 24792 tokens) came round again, with 0.03 to 0.5 % of all tiles; with the first tile of
 // the list and 2^-7 it was 17 to 61 % and 1.5 to 9 %.  What it costs at 24 heads x 33272
-// tokens, 30 %, launches in a row: 3.11 ms on the inputs above; 3.32 with one row of every query
-// tile 48 bits ahead in every 40th tile; 3.78 with a third of the rows ahead in every tenth;
-// two E4M3 terms take 4.2 to 4.3 ms of each.  All but the first two tiles of a list
+// tokens, 30 %, launches in a row: 2.82 ms on inputs with a rank-8 part; 3.00 with one row of every query
+// tile 48 bits ahead in every 40th tile; 3.43 with a third of the rows ahead in every tenth;
+// two E4M3 terms take 4.4 to 4.5 ms of each.  All but the first two tiles of a list
 // ahead is the worst: two walks, three where a sum overflows (120 bits): 24 heads x 9872,
-// dense, 0.87 ms, then 2.18 and 2.86, where two E4M3 terms take 1.13.
+// dense, 0.85 ms, then 2.21 and 2.86, where two E4M3 terms take 1.31, 1.12 and 1.10.
 //
 // Without a running maximum the tiles of a row are independent but for the sum: the sixteen
 // softmax warps form four groups, group g takes every fourth tile, and each scheduler has one

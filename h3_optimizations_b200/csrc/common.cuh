@@ -52,8 +52,9 @@ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // thread of such a kernel calls it before it touches global memory, reads and writes alike; then a kernel is complete only
 // after all those before it are, whatever their kind.  `let_next_start` tells that this block does not mind; it stands at the
 // top, as the next kernel's blocks are only placed once every block of this one has been.  What is saved is the gap between
-// two kernels and the set-up of the second: MLP of 1000 x 3072 x 12288 (four kernels) 103 -> 95 us, of 33272 rows (36) 2595 ->
-// 2572, layer of 7 heads x 10384 tokens 141 -> 137, calls bound by the host unchanged.
+// two kernels and the set-up of the second.  us, the same kernels launched without / with it, in turn: MLP of 1000 x 3072 x 12288 (four
+// kernels) 102 / 94, of 33272 rows (36) 2612 / 2567, of 33130 x 1024 x 4096 623 / 558; layer of 7 heads x 10384 tokens 133 / 131, of
+// 24 x 33272 alike.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
