@@ -270,7 +270,9 @@ class B200SparseBackend:
         """Non-blocking look at the mirror of the earlier launches' status."""
         slot = self._status.get(device.index if device.index is not None else torch.cuda.current_device())
         if slot is not None:
-            self._raise_for(slot[1].tolist(), "reported by an earlier launch")
+            words = slot[1].tolist()
+            if words[0] != 0:
+                self._raise_for(words, "reported by an earlier launch")
 
     def check_status(self, device=None):
         """Synchronise with the device and raise ``SparseSageError`` if a

@@ -510,7 +510,7 @@ int fill_attn_params(AttnParams *params, const int8_t *q8, const int8_t *k8, con
   const int cap = h3s_device_capability();
   if (cap < 0) return cap;
   if (cap / 10 != 10) return fail(H3S_EARCH, "%s: needs an sm_100 device, found sm_%d", who, cap);
-  const int home = output_home(out, who);
+  const int home = (flags & H3S_ATTN_DEVICE_OUTPUT) != 0 ? 1 : output_home(out, who);
   if (home < 0) return home;
   AttnParams &prm = *params;
   prm.out_map = home == 1;

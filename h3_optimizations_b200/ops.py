@@ -20,6 +20,7 @@ KV_TILE = 64
 HEAD_DIM = 128
 FP8_V_BOUND = 448.0
 ATTN_P_SINGLE = 1
+ATTN_DEVICE_OUTPUT = 4
 ATTN_TEST_DROP_KV_LOAD = 0x4000
 ATTN_TEST_DROP_LAST_V_LOAD = 0x8000
 
@@ -648,10 +649,13 @@ def sparse_attention_of(buffers, route, *, q_start, q_stop, out, out_dtype, stat
     """``sparse_attention`` on the carriers of ``LayerBuffers`` that nobody else has been handed: they are as they were
     made, so that only the route and the output are looked at."""
     heads, sequence, device = buffers.heads, buffers.sequence, buffers.device
+    flags = ATTN_DEVICE_OUTPUT
     if out is None:
         out = new_attention_output(heads, sequence, out_dtype, device)
     elif tuple(out.shape) != (1, heads, sequence, HEAD_DIM) or out.stride(-1) != 1:
         raise _native.NativeError("sparse_attention: output must be (1,H,S,128) with a contiguous last dimension")
+    elif out.device != device:
+        flags = 0  # the library asks CUDA where it is
     lib = _native.load()
     route_len = _route_length(route, heads, q_stop - q_start)
     table, n_peers = _peer_table(peer_out_ptrs)
@@ -660,7 +664,7 @@ def sparse_attention_of(buffers, route, *, q_start, q_stop, out, out_dtype, stat
     c = buffers.native
     check(lib.h3s_sparse_attn_half_fwd_mirrored(
         c.q8, c.k8, c.v16, c.q_scale, c.k_scale, c.v_scale, ptr(route), route_len, q_start, q_stop, out.data_ptr(), table, n_peers,
-        dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence, 0, ptr(workspace), size, status.data_ptr(),
+        dtype_code(out.dtype), out.stride(1), out.stride(2), heads, sequence, flags, ptr(workspace), size, status.data_ptr(),
         status_mirror.data_ptr(), stream_ptr(device)), "h3s_sparse_attn_half_fwd")
     return out
 
@@ -692,10 +696,13 @@ def sparse_attention(q8, k8, v_carrier, q_scale, k_scale, v_scale, route=None, *
     ``status_mirror``: pinned int32[4] that a launch which sets ``status`` writes too
     (the FP16 kernel only)."""
     lib = _native.load()
+    flags = (ATTN_P_SINGLE if single_term_p else 0) | int(extra_flags)
     if out is None:
         out = new_attention_output(q8.shape[1], q8.shape[2], out_dtype, q8.device)
+        flags |= ATTN_DEVICE_OUTPUT
+    elif out.device == q8.device:
+        flags |= ATTN_DEVICE_OUTPUT
     heads, sequence, route_len = _attn_args(q8, k8, v_carrier, q_scale, k_scale, v_scale, route, q_start, q_stop, out)
-    flags = (ATTN_P_SINGLE if single_term_p else 0) | int(extra_flags)
     table, n_peers = _peer_table(peer_out_ptrs)
     if n_peers and legacy_mma:
         raise _native.NativeError("sparse_attention: the cross-check kernel does not scatter to peers")
