@@ -51,7 +51,9 @@ LONE_HEAD_BYTES = 6_500_000
 # us a call, whole / pieces of 3, 2, 1.6 and 1.25 MB: 24 heads x 9881 tokens 4189 / 3928, 3934, 3973, 3988; 12 x 8512 1940 / 1936, 1827,
 # 1851, 1854; 24 x 6512 2995 / 3007, 2802, 2806, 2866; 4 x 33512 2545 / 2466, 2474, 2467, 2474; 8 x 33272 4486 / 4424, 4393, 4382, 4384;
 # 8 x 4512 (2.3 MB a chunk) 930 / 936, 929, 915, 994; 24 x 11512 dense 4740 / 4704, 4687, 4683, 4681.
-COPY_OUT_BYTES = 1.6 * 2**20
+# A chunk of less than two pieces goes in one copy, as does the last one: there the host's time for a copy more (10 to 20 us) shows,
+# 6 heads x 4923 fp32 (2.5 MB each) 1302 / 1431 in two.
+COPY_OUT_BYTES = 1_600_000
 V_QUANT_BOUND = 448.0  # FP32 accumulation (reference: sparse_sage.py:296)
 
 
@@ -503,7 +505,8 @@ class B200SparseBackend:
             raise SparseSageError("forward_host: out must be a contiguous host tensor shaped and typed like q")
         recorder = (transformer_options or {}).get("h3_optimizations_attention_route")
         whole = getattr(recorder, "sink", None) is not None
-        bounds = [(0, heads)] if whole else self._head_chunks(heads, heads_per_chunk, 3 * sequence * 128 * q.element_size())
+        head_bytes = sequence * 128 * q.element_size()
+        bounds = [(0, heads)] if whole else self._head_chunks(heads, heads_per_chunk, 3 * head_bytes)
         chunk = max((b - a for a, b in bounds), default=1)
         device = torch.device("cuda", torch.cuda.current_device())
         main = torch.cuda.current_stream(device)
@@ -529,7 +532,10 @@ class B200SparseBackend:
             slot["computed"].record(main)
             with torch.cuda.stream(d2h):
                 d2h.wait_event(slot["computed"])
-                self._copy_out(out[:, a:b], slot["out"][:, :n], last=b == heads)
+                if b < heads and n * head_bytes >= 2 * COPY_OUT_BYTES:
+                    self._copy_out(out[:, a:b], slot["out"][:, :n])
+                else:
+                    out[:, a:b].copy_(slot["out"][:, :n], non_blocking=True)
                 slot["stored"].record(d2h)
         main.wait_stream(d2h)
         main.wait_stream(h2d)
@@ -551,12 +557,9 @@ class B200SparseBackend:
         return [(2 * i, 2 * i + 2) for i in range(pairs)] + [(a, a + 1) for a in range(2 * pairs, heads)]
 
     @staticmethod
-    def _copy_out(to, source, last=False):
-        """One chunk's output to host memory, in pieces of about ``COPY_OUT_BYTES`` unless nothing comes in any more."""
-        pieces = 1 if last else max(1, round(to.numel() * to.element_size() / COPY_OUT_BYTES))
-        if pieces == 1:
-            to.copy_(source, non_blocking=True)
-            return
+    def _copy_out(to, source):
+        """One chunk's output to host memory, in pieces of ``COPY_OUT_BYTES`` or a little more."""
+        pieces = max(1, int(to.numel() * to.element_size() / COPY_OUT_BYTES))
         for part, rows in zip(to.view(-1, 128).tensor_split(pieces), source.view(-1, 128).tensor_split(pieces)):
             part.copy_(rows, non_blocking=True)
 

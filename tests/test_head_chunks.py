@@ -29,12 +29,11 @@ def test_short_heads_stay_in_pairs(heads, asked):
 
 
 @pytest.mark.parametrize("size", [1, 512, 5000, 10**9])
-@pytest.mark.parametrize("last", [False, True])
 @pytest.mark.parametrize("heads,sequence", [(1, 1), (1, 7), (2, 13), (3, 64)])
-def test_the_output_arrives_whole(monkeypatch, heads, sequence, last, size):
+def test_the_output_arrives_whole(monkeypatch, heads, sequence, size):
     monkeypatch.setattr(module, "COPY_OUT_BYTES", size)
     slot = torch.randn((1, 3, sequence, 128)).bfloat16()
     out = torch.full((1, 5, sequence, 128), 77.0, dtype=torch.bfloat16)
-    B200SparseBackend._copy_out(out[:, 1:1 + heads], slot[:, :heads], last)
+    B200SparseBackend._copy_out(out[:, 1:1 + heads], slot[:, :heads])
     assert torch.equal(out[:, 1:1 + heads], slot[:, :heads])
     assert bool((out[:, :1] == 77.0).all()) and bool((out[:, 1 + heads:] == 77.0).all())
