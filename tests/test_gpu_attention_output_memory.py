@@ -59,3 +59,21 @@ def test_execute_refuses_it_too(native_lib):
         torch.cuda.synchronize()
         assert torch.equal(pinned, out.cpu())
     backend.check_status()
+
+
+def test_pinned_memory_in_a_capture(native_lib):
+    """Asking where an output is does not disturb a capture of any mode."""
+    from h3_optimizations_b200 import ops
+
+    args = _carriers(ops)
+    half = ops.v_half_copy(args[2])
+    out = ops.sparse_attention(*args, v_half=half)
+    for mode in ("global", "thread_local", "relaxed"):
+        pinned = torch.zeros((1, 2, 200, 128), dtype=torch.bfloat16).pin_memory()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, capture_error_mode=mode):
+            ops.sparse_attention(*args, out=pinned, v_half=half)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(pinned, out.cpu())
