@@ -274,6 +274,7 @@ struct GemmParams {
   const float *col_scale;          // (n_out) or null
   const float *bias;               // (n_out) or null
   int activation;                  // H3S_ACT_NONE / H3S_ACT_GELU_TANH
+  int tile_n;                      // columns of a tile: kGemmN or less, a multiple of 32
   bool vector_columns;             // col_scale and bias, where given, are 16-byte aligned
   __nv_bfloat16 *dense_out;        // (rows, ldc)
   int64_t ldc;
@@ -692,6 +693,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int total_tiles = prm.m_pairs * prm.n_tiles;
   const int rank = ptx::cluster_rank();  // 0: issues the pair's MMAs
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  const int tile_n = kMode == kModeDense ? prm.tile_n : kGemmN;
 
   let_next_start();
   if (threadIdx.x == 0) {
@@ -741,11 +743,11 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       for (int tile = first_tile; ok && tile < total_tiles; tile += tile_step) {
         int pair, tn;
         tile_position(prm, tile, pair, tn);
-        const int row0 = pair * kGemmPairM + rank * kGemmM, col0 = tn * kGemmN + rank * (kGemmN / 2);
+        const int row0 = pair * kGemmPairM + rank * kGemmM, col0 = tn * tile_n + rank * (tile_n / 2);
         for (int k = 0; k < prm.hidden; k += kGemmK) {
           if (!ptx::mbar_wait(&sh.empty[stage], previous, abort_word, kGemmAbortEmpty, prm.wait_budget_ns)) { ok = false; break; }
           const uint32_t full = full0 + stage * sizeof(uint64_t);
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&sh.full[stage], 2 * (kGemmABytes + kGemmBBytes));
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&sh.full[stage], 2 * kGemmABytes + tile_n * kGemmK);
           ptx::tma_load_2d_pair(smem + stage * kGemmABytes, &map_a, full, k, row0);
           ptx::tma_load_2d_pair(smem + L::kOffB + stage * kGemmBBytes, &map_b, full, k, col0);
           ++it;
@@ -786,10 +788,10 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       auto i8 = [](uint32_t d, uint64_t x, uint64_t y, uint32_t i, uint32_t accumulate) { ptx::umma_i8_pair(d, x, y, i, accumulate); };
       auto f8 = [](uint32_t d, uint64_t x, uint64_t y, uint32_t i, uint32_t accumulate) { ptx::umma_f8_pair(d, x, y, i, accumulate); };
       auto f16 = [](uint32_t d, uint64_t x, uint64_t y, uint32_t i, uint32_t accumulate) { ptx::umma_f16_pair(d, x, y, i, accumulate); };
-      if (kind == H3S_GEMM_I8) issue(ptx::umma_idesc(2, 1, 1, kGemmPairM, kGemmN), i8);
-      else if (kind == H3S_GEMM_E4M3) issue(ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN), f8);
-      else if (kind == H3S_GEMM_BF16) issue(ptx::umma_idesc(1, 1, 1, kGemmPairM, kGemmN), f16);
-      else issue(ptx::umma_idesc(1, 0, 0, kGemmPairM, kGemmN), f16);
+      if (kind == H3S_GEMM_I8) issue(ptx::umma_idesc(2, 1, 1, kGemmPairM, tile_n), i8);
+      else if (kind == H3S_GEMM_E4M3) issue(ptx::umma_idesc(1, 0, 0, kGemmPairM, tile_n), f8);
+      else if (kind == H3S_GEMM_BF16) issue(ptx::umma_idesc(1, 1, 1, kGemmPairM, tile_n), f16);
+      else issue(ptx::umma_idesc(1, 0, 0, kGemmPairM, tile_n), f16);
     }
   } else if (W::epilogue(warp)) {
     // epilogue: warp group <-> 128-column half of the tile, thread <-> accumulator row (carriers: half a row)
@@ -817,9 +819,10 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const bool row_ok = row < prm.rows;
       const float xs = prm.x_scale == nullptr ? 1.0f : (row_ok ? __ldg(prm.x_scale + row) : 0.f);
       {
-        const int group_col0 = tn * kGemmN + gi * H3S_HEAD_DIM;
+        const int group_col0 = tn * tile_n + gi * H3S_HEAD_DIM;
         const int group = group_col0 >> 7;  // 128-column group == (kind, head)
-        const bool group_ok = group_col0 < prm.n_out && tm * kGemmM < prm.rows;
+        const int columns_end = min(prm.n_out, (tn + 1) * tile_n);  // of the tile
+        const bool group_ok = group_col0 < columns_end && tm * kGemmM < prm.rows;
         const bool normed = prm.q_norm != nullptr && group < 2 * prm.heads;
         if (kMode == kModeDense) {
           // ---- dense epilogue: scaled, biased, activated bf16 rows, staged for coalesced stores ----
@@ -829,9 +832,10 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           const bool integer = prm.operand_kind == H3S_GEMM_I8;
           uint4 *my_row = reinterpret_cast<uint4 *>(tile + local_row * (H3S_HEAD_DIM * 2));
           const bool gelu = prm.activation == H3S_ACT_GELU_TANH;
+          const int blocks = min(H3S_HEAD_DIM, tile_n - gi * H3S_HEAD_DIM) / 32;  // of 32 columns; none or less: nothing of this half
           auto convert = [&](auto scale_tag, auto bias_tag, auto gelu_tag) {
 #pragma unroll 1
-            for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
+            for (int cc = 0; cc < blocks; ++cc) {
               uint32_t acc[32], y[16];
               H3S_TMEM_LD32(tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM + cc * 32, acc);
               ptx::tmem_wait_ld(acc);
@@ -854,7 +858,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             }
           } else {
 #pragma unroll 1
-          for (int cc = 0; cc < H3S_HEAD_DIM / 32; ++cc) {
+          for (int cc = 0; cc < blocks; ++cc) {
             uint32_t acc[32];
             H3S_TMEM_LD32(tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM + cc * 32, acc);
             ptx::tmem_wait_ld(acc);
@@ -910,7 +914,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           }
           const int valid = min(kGemmM, prm.rows - tm * kGemmM);
           const int col = group_col0 + c * 8;
-          if (col < prm.n_out) {  // n_out is a multiple of 8: a 16-byte chunk is inside or outside as a whole
+          if (col < columns_end) {  // a multiple of 8: a 16-byte chunk is inside or outside as a whole
             __nv_bfloat16 *dst = prm.dense_out + static_cast<int64_t>(tm) * kGemmM * prm.ldc + col;
 #pragma unroll
             for (int p = 0; p < 16; ++p) {
@@ -1400,7 +1404,7 @@ static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const i
   prm.k_stage = prm.v_stage = nullptr; prm.k_sum = nullptr; prm.v_amax_bits = nullptr;
   prm.summary_dtype = H3S_F32; prm.sequence_total = rows; prm.row_start = 0;
   prm.operand_kind = H3S_GEMM_I8; prm.row_scale = nullptr; prm.col_scale = nullptr; prm.bias = nullptr;
-  prm.activation = H3S_ACT_NONE; prm.vector_columns = false; prm.dense_out = nullptr; prm.ldc = 0;
+  prm.activation = H3S_ACT_NONE; prm.tile_n = kGemmN; prm.vector_columns = false; prm.dense_out = nullptr; prm.ldc = 0;
   if (carriers != nullptr) {
     const h3s_qkv_carriers &c = *carriers;
     prm.q8 = c.q8; prm.k8 = c.k8; prm.q_scale = c.q_scale; prm.k_scale = c.k_scale;
@@ -1451,6 +1455,27 @@ int h3s_qkv_gemm_chunk_norm_rope(const int8_t *x_i8, const float *x_scale, const
                              stream, "qkv_gemm_chunk_norm_rope");
 }
 
+// Columns of a dense tile.  Every pair of SMs takes as long as the most tiles that one of them gets, a round of tiles; narrower
+// tiles may need no more rounds, or make up for one more.  A tile's time goes with its columns and a part that does not: per step of
+// K its 128 rows of A are loaded whatever the width (96 bytes a clock and SM with 128 columns, 64 with 256), and what the MMAs leave
+// idle the SM clock makes up for, as the power allows.  96 columns' worth of such time is where the line fits 52 shapes; the rule's
+// choice is the fastest width of each or within 4 % of it.  us, 256 columns / the rule's, launches in a row:
+//   fp8    64 x 3072 x 12288 33.2 / 17.8 (96), 300 x 3072 x 12288 33.7 / 19.8 (96), 700 x 3072 x 12288 34.0 / 23.8 (128), 1000 x 3072 x 12288
+//          38.0 / 30.5 (192), 1000 x 12288 x 3072 34.2 / 31.3 (224), 2000 x 3072 x 12288 80.6 / 66.1 (192), 1500 x 3072 x 12288 42.2 (256)
+//   bf16   64 x 1024 x 1024 10.0 / 6.9 (64), 900 x 3072 x 3072 21.2 / 17.4 (192), 2304 x 3072 x 3072 35.3 / 30.4 (192), 8000 x 3072 x 3072
+//          128.5 / 120.9 (192), 33272 x 3072 x 3072 462.3 (256; 224: 477, 128: 603)
+static int dense_tile_columns(int m_pairs, int n_out, int pairs_of_sms) {
+  constexpr int kStep = 32, kLeast = 64, kFixed = 96;
+  int best = h3s::kGemmN;
+  int64_t best_cost = 0;
+  for (int width = h3s::kGemmN; width >= kLeast; width -= kStep) {
+    const int64_t tiles = static_cast<int64_t>(m_pairs) * h3s::ceil_div(n_out, width);
+    const int64_t cost = (tiles + pairs_of_sms - 1) / pairs_of_sms * (kFixed + width);
+    if (best_cost == 0 || cost < best_cost) { best = width; best_cost = cost; }
+  }
+  return best;
+}
+
 int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_bytes, int operand_kind, int rows,
                    int n_out, int k_bytes, const float *row_scale, const float *col_scale, const float *bias,
                    int activation, void *out_bf16, int64_t ldc, int32_t *status, h3s_stream_t stream) {
@@ -1471,20 +1496,21 @@ int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_
   CUtensorMap ma, mb;
   int rc = make_tensor_map_u8_2d(&ma, a, k_bytes, rows, lda_bytes, kGemmK, kGemmM, "dense_gemm A map");
   if (rc) return rc;
-  rc = make_tensor_map_u8_2d(&mb, b, k_bytes, n_out, ldb_bytes, kGemmK, kGemmN / 2, "dense_gemm B map");
+  int device = 0, sms = 0;
+  H3S_CHECK_CUDA(cudaGetDevice(&device));
+  H3S_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  const int tile_n = dense_tile_columns(ceil_div(rows, kGemmPairM), n_out, sms / 2);
+  rc = make_tensor_map_u8_2d(&mb, b, k_bytes, n_out, ldb_bytes, kGemmK, tile_n / 2, "dense_gemm B map");
   if (rc) return rc;
   GemmParams prm;
   memset(&prm, 0, sizeof(prm));
   prm.x_scale = row_scale; prm.status = status;
   prm.rows = rows; prm.n_out = n_out; prm.hidden = k_bytes;
-  prm.m_pairs = ceil_div(rows, kGemmPairM); prm.n_tiles = ceil_div(n_out, kGemmN);
+  prm.m_pairs = ceil_div(rows, kGemmPairM); prm.n_tiles = ceil_div(n_out, tile_n); prm.tile_n = tile_n;
   prm.heads = 1; prm.wait_budget_ns = wait_budget_ns();
   prm.operand_kind = operand_kind; prm.row_scale = row_scale; prm.col_scale = col_scale; prm.bias = bias;
   prm.vector_columns = ((reinterpret_cast<uintptr_t>(col_scale) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0;
   prm.activation = activation; prm.dense_out = static_cast<__nv_bfloat16 *>(out_bf16); prm.ldc = ldc;
-  int device = 0, sms = 0;
-  H3S_CHECK_CUDA(cudaGetDevice(&device));
-  H3S_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   H3S_CHECK_CUDA(cudaFuncSetAttribute(qkv_gemm_kernel<kModeDense>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(GemmLayout<kModeDense>::kBytes)));
   const int tiles = prm.m_pairs * prm.n_tiles;
