@@ -19,38 +19,30 @@ namespace h3s {
 constexpr int kStatsThreads = 256;
 constexpr int kStatsRowsPerBlock = 512;
 
-template <typename T>
-__global__ void __launch_bounds__(kStatsThreads)
-column_stats_kernel(const T *__restrict__ k, int64_t k_stride_h, int64_t k_stride_s,
-                    const T *__restrict__ v, int64_t v_stride_h, int64_t v_stride_s,
-                    int sequence, double *__restrict__ k_sum,
-                    unsigned int *__restrict__ v_amax_bits) {
-  __shared__ double red[kStatsThreads / 16][H3S_HEAD_DIM];
-  let_next_start();
-  wait_for_previous();
-  const int head = blockIdx.y;
-  const bool is_v = blockIdx.z == 1;
-  const T *src = is_v ? v : k;
-  if (src == nullptr) return;
-  const int64_t stride_h = is_v ? v_stride_h : k_stride_h;
-  const int64_t stride_s = is_v ? v_stride_s : k_stride_s;
+// Rows [row_begin, row_end) of one head: column sums of K, or column maxima of V, added to the head's totals.  Where registers are plenty
+// (80 here) the choice is left to run time: as two bodies the compiler made do with 52, and three heads of 33272 tokens took 20 us beside the
+// Q quantiser instead of 15; a kernel of 64 registers spills with one body for both.
+enum StatsOf { kStatsOfK, kStatsOfV, kStatsOfEither };
+template <typename T, StatsOf kOf, int kAhead = 8>
+__device__ __forceinline__ void column_stats_rows(const T *__restrict__ src, int64_t stride_s, int row_begin, int row_end, bool v_now,
+                                                  double (&red)[kStatsThreads / 16][H3S_HEAD_DIM], double *__restrict__ k_sum,
+                                                  unsigned int *__restrict__ v_amax_bits) {
+  const bool is_v = kOf == kStatsOfEither ? v_now : kOf == kStatsOfV;
   const int slot = threadIdx.x >> 4;
   const int c0 = (threadIdx.x & 15) * 8;
-  const int row_begin = blockIdx.x * kStatsRowsPerBlock;
-  const int row_end = min(row_begin + kStatsRowsPerBlock, sequence);
   double acc[8];
   float amax[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) { acc[i] = 0.0; amax[i] = 0.f; }
-  const T *base = src + head * stride_h + c0;
-  // eight rows are requested before the first is used (rows past the end count as zeros):
+  const T *base = src + c0;
+  // kAhead rows are requested before the first is used (rows past the end count as zeros), eight for one:
   // 24 heads x 33272 tokens 117 -> 85 us, 3 heads 32 -> 22 us
-  constexpr int kAhead = 8, kStep = kStatsThreads / 16;
+  constexpr int kStep = kStatsThreads / 16;
   for (int row = row_begin + slot; row < row_end; row += kStep * kAhead) {
     typename Elem<T>::Raw raw[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u)
-      raw[u] = row + u * kStep < row_end ? Elem<T>::load_raw(base + (row + u * kStep) * stride_s) : Elem<T>::zero_raw();
+      raw[u] = Elem<T>::load_raw_if(base + (row + u * kStep) * stride_s, row + u * kStep < row_end);
     if (is_v) {
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
@@ -79,14 +71,40 @@ column_stats_kernel(const T *__restrict__ k, int64_t k_stride_h, int64_t k_strid
 #pragma unroll
       for (int s = 0; s < kStatsThreads / 16; ++s) m = fmax(m, red[s][d]);
       // non-negative floats order like their bit patterns
-      atomicMax(&v_amax_bits[head * H3S_HEAD_DIM + d], __float_as_uint(static_cast<float>(m)));
+      atomicMax(&v_amax_bits[d], __float_as_uint(static_cast<float>(m)));
     } else {
       double s = 0.0;
 #pragma unroll
       for (int i = 0; i < kStatsThreads / 16; ++i) s += red[i][d];
-      atomicAdd(&k_sum[head * H3S_HEAD_DIM + d], s);
+      atomicAdd(&k_sum[d], s);
     }
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kStatsThreads)
+column_stats_kernel(const T *__restrict__ k, int64_t k_stride_h, int64_t k_stride_s,
+                    const T *__restrict__ v, int64_t v_stride_h, int64_t v_stride_s,
+                    int sequence, double *__restrict__ k_sum,
+                    unsigned int *__restrict__ v_amax_bits) {
+  __shared__ double red[kStatsThreads / 16][H3S_HEAD_DIM];
+  let_next_start();
+  wait_for_previous();
+  const int head = blockIdx.y;
+  const bool is_v = blockIdx.z == 1;
+  const T *src = is_v ? v : k;
+  if (src == nullptr) return;
+  const int row_begin = blockIdx.x * kStatsRowsPerBlock;
+  column_stats_rows<T, kStatsOfEither>(src + head * (is_v ? v_stride_h : k_stride_h), is_v ? v_stride_s : k_stride_s, row_begin,
+                    min(row_begin + kStatsRowsPerBlock, sequence), is_v, red, k_sum + head * H3S_HEAD_DIM, v_amax_bits + head * H3S_HEAD_DIM);
+}
+
+template <typename T>
+__device__ __forceinline__ float finalize_mean(double sum, int sequence) {
+  return Elem<T>::round_trip(static_cast<float>(sum / static_cast<double>(sequence)));
+}
+__device__ __forceinline__ float finalize_scale(unsigned int amax_bits, float v_bound) {
+  return fmaxf(__fdiv_rn(__uint_as_float(amax_bits), v_bound), 1.0e-20f);
 }
 
 template <typename T>
@@ -99,14 +117,8 @@ __global__ void column_stats_finalize_kernel(const double *__restrict__ k_sum,
   wait_for_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
-  if (k_mean != nullptr) {
-    const float mean = static_cast<float>(k_sum[i] / static_cast<double>(sequence));
-    k_mean[i] = Elem<T>::round_trip(mean);
-  }
-  if (v_scale != nullptr) {
-    const float amax = __uint_as_float(v_amax_bits[i]);
-    v_scale[i] = fmaxf(__fdiv_rn(amax, v_bound), 1.0e-20f);
-  }
+  if (k_mean != nullptr) k_mean[i] = finalize_mean<T>(k_sum[i], sequence);
+  if (v_scale != nullptr) v_scale[i] = finalize_scale(v_amax_bits[i], v_bound);
 }
 
 // ---------------------------------------------------------------------------
@@ -116,51 +128,37 @@ __global__ void column_stats_finalize_kernel(const double *__restrict__ k_sum,
 // reduction and the store, so it is read from memory exactly once.
 // ---------------------------------------------------------------------------
 
-template <typename T, int BLOCK, bool kHasMean>
-__global__ void __launch_bounds__(BLOCK * 2, (sizeof(T) == 2 ? 1024 : 512) / (BLOCK * 2))
-quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride_s,
-                       const float *__restrict__ mean, int8_t *__restrict__ out,
-                       float *__restrict__ scale_out, void *__restrict__ summary,
-                       int summary_dtype, int rows, int row_start, int sequence_total,
-                       int blocks_total) {
+template <int BLOCK>
+struct QkShared {
+  float warp_amax[BLOCK / 16];
+  double red[BLOCK / 8][H3S_HEAD_DIM];
+};
+
+// One block of BLOCK rows by 2 * BLOCK threads, of which this is the t-th.  `x` is the block's first row, `out` the carrier's.  `sync` lets
+// these threads meet; `minus_mean(m)` gives this thread's eight channels of the mean, negated (x - mu == x + (-mu)), and is called when the
+// block's loads have been issued.
+template <typename T, int BLOCK, bool kHasMean, typename Sync, typename Mean>
+__device__ __forceinline__ void quant_qk_block(const T *__restrict__ x, int64_t stride_s, int valid_rows, int8_t *__restrict__ out,
+                                               float *__restrict__ scale_out, void *__restrict__ summary, int summary_dtype,
+                                               int64_t summary_at, int t, QkShared<BLOCK> &sh, Sync sync, Mean minus_mean) {
   constexpr int kThreads = BLOCK * 2;
   constexpr int kSlots = kThreads / 16;  // rows per pass
   constexpr int kPasses = BLOCK / kSlots;  // == 8
-  __shared__ float warp_amax[kThreads / 32];
-  __shared__ double red[kSlots][H3S_HEAD_DIM];
-
-  let_next_start();
-  wait_for_previous();
-  const int local_block = blockIdx.x;
-  const int head = blockIdx.y;
-  const int slot = threadIdx.x >> 4;
-  const int c0 = (threadIdx.x & 15) * 8;
-  const int first_row = local_block * BLOCK;  // within this chunk
-  const int valid_rows = min(BLOCK, rows - first_row);
-
-  float2 minus_mu[4];  // x - mu == x + (-mu)
-#pragma unroll
-  for (int i = 0; i < 4; ++i) minus_mu[i] = make_float2(0.f, 0.f);
-  if (kHasMean) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float *mu = mean + head * H3S_HEAD_DIM + c0 + 2 * i;
-      minus_mu[i] = make_float2(-__ldg(mu), -__ldg(mu + 1));
-    }
-  }
-
+  const int slot = t >> 4;
+  const int c0 = (t & 15) * 8;
   typename Elem<T>::Raw raw[kPasses];
   float2 col[4];  // this thread's rows (at most 8) summed in fp32, widened once
 #pragma unroll
   for (int i = 0; i < 4; ++i) col[i] = make_float2(0.f, 0.f);
   float amax = 0.f;
-  const T *base = x + head * stride_h + c0;
+  const T *base = x + c0;
 #pragma unroll
   for (int p = 0; p < kPasses; ++p) {
     const int r = p * kSlots + slot;
-    raw[p] = r < valid_rows ? Elem<T>::load_raw(base + static_cast<int64_t>(first_row + r) * stride_s)
-                            : Elem<T>::zero_raw();
+    raw[p] = Elem<T>::load_raw_if(base + r * stride_s, r < valid_rows);
   }
+  float2 minus_mu[4];
+  minus_mean(minus_mu);
 #pragma unroll
   for (int p = 0; p < kPasses; ++p) {
     const int r = p * kSlots + slot;
@@ -177,26 +175,24 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
     }
   }
   amax = warp_max(amax);
-  if ((threadIdx.x & 31) == 0) warp_amax[threadIdx.x >> 5] = amax;
+  if ((t & 31) == 0) sh.warp_amax[t >> 5] = amax;
   if (summary != nullptr) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      red[slot][c0 + 2 * i] = static_cast<double>(col[i].x);
-      red[slot][c0 + 2 * i + 1] = static_cast<double>(col[i].y);
+      sh.red[slot][c0 + 2 * i] = static_cast<double>(col[i].x);
+      sh.red[slot][c0 + 2 * i + 1] = static_cast<double>(col[i].y);
     }
   }
-  __syncthreads();
-  amax = warp_amax[0];
+  sync();
+  amax = sh.warp_amax[0];
 #pragma unroll
-  for (int w = 1; w < kThreads / 32; ++w) amax = fmaxf(amax, warp_amax[w]);
+  for (int w = 1; w < kThreads / 32; ++w) amax = fmaxf(amax, sh.warp_amax[w]);
   const float scale = __fadd_rn(__fdiv_rn(amax, 127.0f), 1.0e-7f);
   const SharedDivisor by_scale = make_divisor(scale);
 
-  const int global_block = row_start / BLOCK + local_block;
-  if (threadIdx.x == 0 && scale_out != nullptr) scale_out[head * blocks_total + global_block] = scale;
+  if (t == 0 && scale_out != nullptr) *scale_out = scale;
 
-  int8_t *dst = out + (static_cast<int64_t>(head) * sequence_total + row_start + first_row) *
-                          H3S_HEAD_DIM + c0;
+  int8_t *dst = out + c0;
   // code = trunc(v/scale +- 0.5): the half carries the quotient's sign bit, the four
   // codes of a word are gathered with byte permutes.  The divisor's exactness is
   // tested once, around the whole loop (see divide<>).
@@ -219,20 +215,19 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
         for (int w = 0; w < 2; ++w)
           packed[w] = __byte_perm(__byte_perm(code[4 * w], code[4 * w + 1], 0x0040),
                                   __byte_perm(code[4 * w + 2], code[4 * w + 3], 0x0040), 0x5410);
-        *reinterpret_cast<uint2 *>(dst + static_cast<int64_t>(r) * H3S_HEAD_DIM) =
-            make_uint2(packed[0], packed[1]);
+        *reinterpret_cast<uint2 *>(dst + static_cast<int64_t>(r) * H3S_HEAD_DIM) = make_uint2(packed[0], packed[1]);
       }
     }
   };
   if (by_scale.exact) emit(std::true_type{}); else emit(std::false_type{});
 
-  if (summary != nullptr && threadIdx.x < H3S_HEAD_DIM) {
-    const int d = threadIdx.x;
+  if (summary != nullptr && t < H3S_HEAD_DIM) {
+    const int d = t;
     double s = 0.0;
 #pragma unroll
-    for (int i = 0; i < kSlots; ++i) s += red[i][d];
-    const double m = s / static_cast<double>(valid_rows);
-    const int64_t at = (static_cast<int64_t>(head) * blocks_total + global_block) * H3S_HEAD_DIM + d;
+    for (int i = 0; i < kSlots; ++i) s += sh.red[i][d];
+    const double m = valid_rows == BLOCK ? s * (1.0 / BLOCK) : s / static_cast<double>(valid_rows);  // a power of two divides exactly
+    const int64_t at = summary_at + d;
     switch (summary_dtype) {
       case H3S_F64: static_cast<double *>(summary)[at] = m; break;
       case H3S_F32: static_cast<float *>(summary)[at] = static_cast<float>(m); break;
@@ -244,6 +239,32 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
         break;
     }
   }
+}
+
+template <typename T, int BLOCK, bool kHasMean>
+__global__ void __launch_bounds__(BLOCK * 2, (sizeof(T) == 2 ? 1024 : 512) / (BLOCK * 2))
+quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride_s,
+                       const float *__restrict__ mean, int8_t *__restrict__ out,
+                       float *__restrict__ scale_out, void *__restrict__ summary,
+                       int summary_dtype, int rows, int row_start, int sequence_total,
+                       int blocks_total) {
+  __shared__ QkShared<BLOCK> sh;
+  let_next_start();
+  wait_for_previous();
+  const int head = blockIdx.y;
+  const int first_row = blockIdx.x * BLOCK;  // within this chunk
+  const int64_t block = static_cast<int64_t>(head) * blocks_total + row_start / BLOCK + blockIdx.x;
+  auto minus_mean = [&](float2 (&m)[4]) {
+    if (!kHasMean) return;
+    const float *mu = mean + head * H3S_HEAD_DIM + (threadIdx.x & 15) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = make_float2(-__ldg(mu + 2 * i), -__ldg(mu + 2 * i + 1));
+  };
+  quant_qk_block<T, BLOCK, kHasMean>(
+      x + head * stride_h + first_row * stride_s, stride_s, min(BLOCK, rows - first_row),
+      out == nullptr ? nullptr : out + (static_cast<int64_t>(head) * sequence_total + row_start + first_row) * H3S_HEAD_DIM,
+      scale_out == nullptr ? nullptr : scale_out + block, summary, summary_dtype, block * H3S_HEAD_DIM, threadIdx.x, sh,
+      []() { __syncthreads(); }, minus_mean);
 }
 
 // ---------------------------------------------------------------------------
@@ -266,34 +287,15 @@ __device__ __forceinline__ int v_tile_offset(int d, int s) {
   return d * kVTile + chunk * 16 + (s & 15);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kVThreads)
-quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
-                   const float *__restrict__ v_scale, uint8_t *__restrict__ out, uint16_t *__restrict__ out_half,
-                   int rows, int row_start, int padded_total, float v_bound) {
-  __shared__ __align__(16) uint8_t tile[H3S_HEAD_DIM * kVTile];
-  let_next_start();
-  wait_for_previous();
-  const int head = blockIdx.y;
-  const int first_row = blockIdx.x * kVTile;
-  const int valid_rows = max(0, min(kVTile, rows - first_row));
+// One tile of 128 sequence rows by 256 threads.  `v` is its first row, `out` and `out_half` the tile's first column of the head's carrier;
+// `scales(s)` gives this thread's eight channels' scales and is called when the tile's loads have been issued.
+template <typename T, typename Scales>
+__device__ __forceinline__ void quant_v_tile(const T *__restrict__ v, int64_t stride_s, int valid_rows, uint8_t *__restrict__ out,
+                                             uint16_t *__restrict__ out_half, int padded_total, float v_bound,
+                                             uint8_t (&tile)[H3S_HEAD_DIM * kVTile], Scales scales) {
   const int slot = threadIdx.x >> 4;
   const int c0 = (threadIdx.x & 15) * 8;
-
-  float2 sc[4], rc[4], minus_sc[4];
-  bool all_exact = true;
-  const bool clamp = v_bound < 448.0f;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float *scale = v_scale + head * H3S_HEAD_DIM + c0 + 2 * i;
-    const SharedDivisor a = make_divisor(fmaxf(__ldg(scale), 1.0e-20f)), b = make_divisor(fmaxf(__ldg(scale + 1), 1.0e-20f));
-    sc[i] = make_float2(a.b, b.b);
-    minus_sc[i] = make_float2(-a.b, -b.b);
-    rc[i] = make_float2(a.r, b.r);
-    all_exact = all_exact && a.exact && b.exact;
-  }
-
-  const T *base = v + head * stride_h + c0;
+  const T *base = v + c0;
   constexpr int kPasses = kVTile / (kVThreads / 16 * 4);
   typename Elem<T>::Raw raw[kPasses][4];
 #pragma unroll
@@ -301,8 +303,21 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int r = (p * (kVThreads / 16) + slot) * 4 + j;  // four consecutive rows
-      raw[p][j] = r < valid_rows ? Elem<T>::load_raw(base + static_cast<int64_t>(first_row + r) * stride_s)
-                                 : Elem<T>::zero_raw();  // 0 / scale is the padding's code
+      raw[p][j] = Elem<T>::load_raw_if(base + r * stride_s, r < valid_rows);  // 0 / scale is the padding's code
+    }
+  }
+  float2 minus_sc[4], rc[4];
+  bool all_exact = true;
+  const bool clamp = v_bound < 448.0f;
+  {
+    float scale[8];
+    scales(scale);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const SharedDivisor a = make_divisor(fmaxf(scale[2 * i], 1.0e-20f)), b = make_divisor(fmaxf(scale[2 * i + 1], 1.0e-20f));
+      minus_sc[i] = make_float2(-a.b, -b.b);
+      rc[i] = make_float2(a.r, b.r);
+      all_exact = all_exact && a.exact && b.exact;
     }
   }
   // the divisors' exactness is tested once, around the whole loop (see divide<>)
@@ -326,7 +341,7 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
           const float2 q0 = mul2(pair, rc[i]);
           y = fma2(fma2(minus_sc[i], q0, pair), rc[i], q0);
         } else {
-          y = make_float2(__fdiv_rn(pair.x, sc[i].x), __fdiv_rn(pair.y, sc[i].y));
+          y = make_float2(__fdiv_rn(pair.x, -minus_sc[i].x), __fdiv_rn(pair.y, -minus_sc[i].y));
         }
         // the conversion saturates at +-448 by itself; a tighter bound is applied here
         if (clamp) y = make_float2(fminf(fmaxf(y.x, -v_bound), v_bound), fminf(fmaxf(y.y, -v_bound), v_bound));
@@ -349,13 +364,12 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
   };
   if (all_exact) fill(std::true_type{}); else fill(std::false_type{});
   __syncthreads();
-  const int64_t base_at = static_cast<int64_t>(head) * H3S_HEAD_DIM * padded_total + row_start + first_row;
 #pragma unroll
   for (int p = 0; p < H3S_HEAD_DIM / (kVThreads / 8); ++p) {
     const int d = p * (kVThreads / 8) + (threadIdx.x >> 3);
     const int chunk = threadIdx.x & 7;
     const uint4 data = *reinterpret_cast<const uint4 *>(&tile[v_tile_offset(d, chunk * 16)]);
-    const int64_t at = base_at + static_cast<int64_t>(d) * padded_total + chunk * 16;
+    const int64_t at = static_cast<int64_t>(d) * padded_total + chunk * 16;
     *reinterpret_cast<uint4 *>(out + at) = data;
   }
   if (out_half != nullptr) {  // the copy the attention kernel multiplies with FP16 probabilities
@@ -363,9 +377,27 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
     for (int p = 0; p < H3S_HEAD_DIM / (kVThreads / 16); ++p) {
       const int d = p * (kVThreads / 16) + slot, s = (threadIdx.x & 15) * 8;
       const uint2 data = *reinterpret_cast<const uint2 *>(&tile[v_tile_offset(d, s)]);
-      *reinterpret_cast<uint4 *>(out_half + base_at + static_cast<int64_t>(d) * padded_total + s) = e4m3x8_to_half(data);
+      *reinterpret_cast<uint4 *>(out_half + static_cast<int64_t>(d) * padded_total + s) = e4m3x8_to_half(data);
     }
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kVThreads)
+quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
+                   const float *__restrict__ v_scale, uint8_t *__restrict__ out, uint16_t *__restrict__ out_half,
+                   int rows, int row_start, int padded_total, float v_bound) {
+  __shared__ __align__(16) uint8_t tile[H3S_HEAD_DIM * kVTile];
+  let_next_start();
+  wait_for_previous();
+  const int head = blockIdx.y;
+  const int first_row = blockIdx.x * kVTile;
+  const int64_t at = static_cast<int64_t>(head) * H3S_HEAD_DIM * padded_total + row_start + first_row;
+  quant_v_tile(v + head * stride_h + first_row * stride_s, stride_s, max(0, min(kVTile, rows - first_row)), out + at,
+               out_half == nullptr ? nullptr : out_half + at, padded_total, v_bound, tile, [&](float (&scale)[8]) {
+#pragma unroll
+                 for (int i = 0; i < 8; ++i) scale[i] = __ldg(v_scale + head * H3S_HEAD_DIM + (threadIdx.x & 15) * 8 + i);
+               });
 }
 
 // ---------------------------------------------------------------------------
