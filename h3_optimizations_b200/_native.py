@@ -105,6 +105,9 @@ PROTOTYPES = {
                                                   c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p,
                                                   c_void_p]),
     "h3s_sparse_attn_half_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "h3s_prepare_layer_counter_bytes": (c_size_t, [c_int]),
+    "h3s_prepare_layer": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                  c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p]),
     "h3s_stream_order": (c_int, [c_void_p, c_void_p, c_void_p]),
     "h3s_quant_qkv": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                               c_int, c_float, c_int, c_void_p, c_void_p, c_void_p]),

@@ -35,12 +35,13 @@ from .errors import FusedQKVError, SparseRouterError, SparseSageError
 from .router import KV_TILE, Q_TILE, SparseTileRouter
 from .runtime import get_runtime_snapshot
 
-# Rows of all heads up to which a layer is prepared on one stream.  us a call, two streams / one: 1 head x 1128 tokens 106 / 90,
-# 4 x 2304 108 / 96, 6 x 4256 114 / 98, 24 x 1328 106 / 93, 4 x 9256 112 / 110, 12 x 4256 104 / 94; with the device waited for
-# after each call 126 / 110, 130 / 123, 140 / 133, 127 / 121, 170 / 165, 152 / 145.  Beyond, the kernels take longer than the host.
-# It holds for the chunks of host calls as well: 8 heads x 2512 tokens in pairs 908 / 848, 24 x 3512 2398 / 2325; longer ones are
-# alike (8 x 8512 1311 / 1316, 24 x 11512 4481 / 4486, 4 x 33512 2440 / 2461, 12 x 12512 2560 / 2550).
-ONE_STREAM_ROWS = 52000
+# One kernel makes all carriers of a layer, on one stream, up to this many rows of all heads if no head has more than SHORT_HEAD_ROWS.
+# Beyond, kernels of their own on two streams do without the bookkeeping of jobs, and V goes beside the router, which takes longer the more
+# KV tiles a head has.  us a call, two streams / one kernel: 1 head x 1128 tokens 105 / 81, 4 x 2304 fp32 103 / 81, 24 x 1756 96 / 81, 12 x 4256
+# 97 / 83, 24 x 2304 96 / 81, 7 x 10384 127 / 127, 24 x 4000 135 / 132, 24 x 6012 197 / 192, 4 x 13512 157 / 161, 1 x 33272 177 / 182; replayed:
+# 37 / 29, 50 / 44, 66 / 64, 85 / 83, 75 / 75, 123 / 124, 128 / 127, 185 / 184, 156 / 161, 180 / 183.
+ONE_STREAM_ROWS = 150_000
+SHORT_HEAD_ROWS = 12_000
 # Bytes of a head's q, k and v from which ``forward_host`` ends with single heads: as long as they take to copy a chunk more is
 # paid for by a shorter end, below that it costs the host's time.  us a call, pairs to the end / single heads at the end, 8 heads,
 # bf16: 1212 tokens 818 / 1001, 4512 933 / 1046, 6512 1080 / 1130, 7512 1155 / 1181, 8512 1316 / 1313, 10512 1594 / 1555, 33272 4575 /
@@ -248,7 +249,7 @@ class B200SparseBackend:
     ABORT_NAMES = {1: "Q tile load", 2: "K/V tile load", 3: "free K/V stage", 4: "QK^T result", 5: "P from the softmax warps",
                    6: "free score slot", 7: "P.V of an earlier tile", 8: "last P.V", 9: "Q rows in tensor memory",
                    10: "answer to the request for more work", 11: "end of a pass over the list", 12: "output sums being read",
-                   13: "first row maxima", 14: "output tile staged"}
+                   13: "first row maxima", 14: "output tile staged", 15: "whole-sequence statistics"}
 
     def _status_slot(self, device):
         key = device.index if device.index is not None else torch.cuda.current_device()
@@ -306,27 +307,25 @@ class B200SparseBackend:
             geometry = self.router.geometry(snapshot.layout)
             retained = self.router._retained(video_budget, geometry)
             need_route = retained < geometry.pure_video_kv_tiles
-            # Two streams share the GPU.  The column statistics (K mean, V scale) run on a
-            # second stream while the Q quantiser, which needs neither, starts at once on the
-            # current one; the K quantiser joins when the statistics are in.  The V carrier
-            # is held back until the K quantiser is through, so that this memory-bound
-            # kernel runs beside the router, which is latency bound and leaves the memory
-            # system idle, instead of sharing the bandwidth with the K quantiser.  Every
-            # buffer is allocated on the current stream, which both chains rejoin before
-            # returning.  One native call issues all of it (4 heads x 2304
-            # tokens, where host time is all there is: 236 -> 135 us).
-            # Short calls are over before the host has issued them: there one stream saves the host the events.  A
-            # replay has no host in it (4 heads x 1341 tokens: 41 us on one stream, 35 on two).
+            # Where layers are short one kernel makes all carriers.  Else every carrier has its own, on two streams: the column
+            # statistics (K mean, V scale) run on the second one while the Q quantiser, which needs neither, starts at once on the
+            # current one; the K quantiser joins when the statistics are in, and the V carrier is held back until the K quantiser
+            # is through, so that this memory-bound kernel runs beside the router, which leaves the memory system idle.  Every
+            # buffer is allocated on the current stream, which both chains rejoin before returning.
             stream = _native.stream_ptr(q.device)
-            forked = heads * sequence > ONE_STREAM_ROWS or torch.cuda.is_current_stream_capturing()
             side = self._side_stream(q.device)  # there from the first call on: a capture must not bring it into being
-            if not forked:
+            if heads * sequence <= ONE_STREAM_ROWS and sequence <= SHORT_HEAD_ROWS:
                 side = None
             buffers = ops.LayerBuffers(heads, sequence, q.device, smooth_k=self.smooth_k,
                                        summary_dtype=torch.float64 if need_route else None)
             try:
-                ops.quant_qkv(q, k, v, buffers, side, stream, smooth_k=self.smooth_k, v_after_k=need_route,
-                              v_bound=V_QUANT_BOUND)
+                if side is None:
+                    word, mirror = self._status_slot(q.device)
+                    ops.prepare_layer(q, k, v, buffers, stream, smooth_k=self.smooth_k, status=word, status_mirror=mirror,
+                                      v_bound=V_QUANT_BOUND)
+                else:
+                    ops.quant_qkv(q, k, v, buffers, side, stream, smooth_k=self.smooth_k, v_after_k=need_route,
+                                  v_bound=V_QUANT_BOUND)
                 if need_route:
                     route = self.router.build_route_from_summaries(
                         buffers.q_summary, buffers.k_summary, snapshot.layout, video_budget,

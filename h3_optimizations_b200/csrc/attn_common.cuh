@@ -10,8 +10,24 @@ namespace h3s {
 // A code names one kind of wait; backend.py and h3sparse.h have their texts
 enum AbortCode {
   kAbortQFull = 1, kAbortKvFull, kAbortKvEmpty, kAbortSFull, kAbortPFull, kAbortScoreSlot,
-  kAbortPvDone, kAbortFinal, kAbortQFree, kAbortNextItem, kAbortPass, kAbortOFree, kAbortFirstMax, kAbortStaged
+  kAbortPvDone, kAbortFinal, kAbortQFree, kAbortNextItem, kAbortPass, kAbortOFree, kAbortFirstMax, kAbortStaged,
+  kAbortStatistics
 };
+
+// The words of the first launch that gives up, and their copy in pinned host memory (either may be null); one thread
+__device__ __forceinline__ void report_status(int32_t *status, int32_t *status_mirror, int code, int number, int head, int tile) {
+  if (status == nullptr || atomicCAS(status, 0, code) != 0) return;
+  status[1] = number;
+  status[2] = head;
+  status[3] = tile;
+  if (status_mirror == nullptr) return;
+  volatile int32_t *mirror = status_mirror;
+  mirror[1] = number;
+  mirror[2] = head;
+  mirror[3] = tile;
+  __threadfence_system();
+  mirror[0] = code;
+}
 
 constexpr float kIntBias = 12582912.0f;  // 1.5 * 2^23: float(kIntBias + s) has bits 0x4b400000 + s
 constexpr uint32_t kIntBiasBits = 0x4b400000u;

@@ -963,23 +963,11 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   if (code != 0) {
     // leave time for copies / MMAs still in flight before releasing TMEM and shared memory
     __nanosleep(200000);
-    if (threadIdx.x == 0 && prm.status != nullptr) {
-      if (atomicCAS(prm.status, 0, code) == 0) {
-        int turn = (sh.stopped[(word >> 8) & 31] + ((word & kItemBefore) != 0 ? 2 : 0)) % 3;
-        if (sh.item[turn].number < 0) turn = (turn + 2) % 3;  // a warp that was through
-        const HalfItem &at = sh.item[turn];
-        prm.status[1] = at.number;
-        prm.status[2] = at.head;
-        prm.status[3] = at.tq;
-        if (prm.status_mirror != nullptr) {
-          volatile int32_t *mirror = prm.status_mirror;
-          mirror[1] = at.number;
-          mirror[2] = at.head;
-          mirror[3] = at.tq;
-          __threadfence_system();
-          mirror[0] = code;
-        }
-      }
+    if (threadIdx.x == 0) {
+      int turn = (sh.stopped[(word >> 8) & 31] + ((word & kItemBefore) != 0 ? 2 : 0)) % 3;
+      if (sh.item[turn].number < 0) turn = (turn + 2) % 3;  // a warp that was through
+      const HalfItem &at = sh.item[turn];
+      report_status(prm.status, prm.status_mirror, code, at.number, at.head, at.tq);
     }
   }
   if (warp == kHValueIssuer) {

@@ -7,7 +7,7 @@
 #include <mutex>
 #include <type_traits>
 
-#include "common.cuh"
+#include "attn_common.cuh"
 
 namespace h3s {
 
@@ -401,6 +401,171 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
 }
 
 // ---------------------------------------------------------------------------
+// Carriers of a layer in one launch: statistics of K and V, and the carriers of a head as soon as its statistics are complete.  Where
+// layers are short, the chain of kernels for statistics, their end, Q, K and V is bound by latency, of the host and of the kernels: each fills
+// the chip for a few microseconds and waits for the last block of the one before.  Here blocks take jobs in order, by a counter, and only K and
+// V of a head wait for that head's statistics.  us, the chain on two streams / this with the clearing before it: 1 head x 1200 tokens 19.5 /
+// 9.2, 4 x 2304 fp32 20.5 / 12.8, 24 x 2304 32.3 / 27.1, 7 x 10384 37.9 / 33.8, 24 x 9872 90.1 / 85.0.  Long layers 24 x 33272 269 / 263 by
+// themselves, but it is the slower one behind an attention kernel, which leaves a lower SM clock: a job's bookkeeping is half as many
+// instructions again as its work.  Sixty-four registers, four blocks an SM: with three and no spills 24 x 76112 692 for 650.  Measured and not
+// kept: four steps of 128 rows to a job (24 x 76112 3 % faster, all short layers slower), a head's means and scales made by its last
+// statistics job (4 x 2304 15.9 for 13.8), K and V right behind their head's statistics, with streaming hints (re-reads still miss L2).
+// ---------------------------------------------------------------------------
+
+constexpr int kCarrierThreads = 256, kCarrierRows = 128;  // rows of a step: one Q block, two K blocks or a tile of V
+enum CarrierKind { kCarrierKStats, kCarrierVStats, kCarrierQ, kCarrierK, kCarrierV };
+
+struct CarrierParams {
+  const void *q, *k, *v;
+  int64_t q_stride_h, q_stride_s, k_stride_h, k_stride_s, v_stride_h, v_stride_s;
+  int8_t *q8, *k8;
+  uint8_t *v8;
+  uint16_t *v16;
+  float *q_scale, *k_scale, *v_scale, *k_mean;
+  void *q_summary, *k_summary;
+  int summary_dtype;
+  int heads, sequence, padded, steps;
+  float v_bound;
+  double *k_sum;                    // (heads, 128), and
+  unsigned int *v_amax_bits;        // (heads, 128): totals, cleared before the launch with the counters below, or complete
+  unsigned int *next, *stats_done;  // the next job; per head: statistics jobs that are through
+  int32_t *status, *status_mirror;
+  unsigned long long wait_budget_ns;
+  int stats_rows;                                // of a statistics job
+  int k_stats, v_stats, q_jobs, k_jobs, v_jobs;  // jobs of a head
+};
+
+struct CarrierJob {
+  int kind, head, index;
+};
+
+// Jobs in the order in which they are taken: head by head the statistics and Q, which needs none, then head by head K and V.  What a job
+// waits for comes before it, so whoever has the first job that is not through can go on, however many blocks run at a time.
+__host__ __device__ inline CarrierJob carrier_job(const CarrierParams &p, int t) {
+  const int early = p.k_stats + p.v_stats + p.q_jobs, late = p.k_jobs + p.v_jobs;
+  if (t < p.heads * early) {
+    const int head = t / early;
+    t -= head * early;
+    if (t < p.k_stats) return {kCarrierKStats, head, t};
+    t -= p.k_stats;
+    return t < p.v_stats ? CarrierJob{kCarrierVStats, head, t} : CarrierJob{kCarrierQ, head, t - p.v_stats};
+  }
+  t -= p.heads * early;
+  const int head = t / late;
+  t -= head * late;
+  return t < p.k_jobs ? CarrierJob{kCarrierK, head, t} : CarrierJob{kCarrierV, head, t - p.k_jobs};
+}
+
+union CarrierShared {
+  double red[kStatsThreads / 16][H3S_HEAD_DIM];
+  QkShared<H3S_Q_TILE> q;
+  QkShared<H3S_KV_TILE> k[2];
+  uint8_t tile[H3S_HEAD_DIM * kVTile];
+};
+static_assert(kStatsThreads == kCarrierThreads && kVThreads == kCarrierThreads && kVTile == kCarrierRows, "carrier jobs");
+
+// Until the count has reached `target`: what was written before the arrivals is visible to this thread then
+__device__ __forceinline__ bool wait_for_count(const unsigned int *count, unsigned int target, unsigned long long budget_ns) {
+  if (ptx::load_acquire(count) >= target) return true;
+  const unsigned long long start = ptx::global_timer_ns();
+  while (ptx::load_acquire(count) < target)
+    if (ptx::global_timer_ns() - start > budget_ns) return false;
+  return true;
+}
+
+template <typename T, bool kSmooth>
+__global__ void __launch_bounds__(kCarrierThreads, sizeof(T) == 2 ? 4 : 2)
+layer_carriers_kernel(const __grid_constant__ CarrierParams p) {
+  __shared__ __align__(16) CarrierShared sh;
+  __shared__ __align__(16) float head_values[H3S_HEAD_DIM];
+  __shared__ int jobs[2];
+  __shared__ int gave_up;
+  let_next_start();
+  if (threadIdx.x == 0) gave_up = 0;
+  wait_for_previous();
+  const int total = p.heads * (p.k_stats + p.v_stats + p.q_jobs + p.k_jobs + p.v_jobs);
+  const int t = threadIdx.x, c0 = (t & 15) * 8;
+  int next = t == 0 ? static_cast<int>(atomicAdd(p.next, 1u)) : 0;
+  for (int turn = 0;; turn ^= 1) {
+    if (t == 0) jobs[turn] = next;
+    __syncthreads();  // and the job before this one has left shared memory
+    const int number = jobs[turn];
+    if (number >= total || gave_up != 0) break;
+    if (t == 0) next = static_cast<int>(atomicAdd(p.next, 1u));  // asked for ahead of its use
+    const CarrierJob job = carrier_job(p, number);
+    const int head = job.head;
+    if (job.kind <= kCarrierVStats) {
+      constexpr int kAhead = sizeof(T) == 4 ? 4 : 8;  // as the registers allow
+      const int begin = job.index * p.stats_rows, end = min(begin + p.stats_rows, p.sequence);
+      if (job.kind == kCarrierKStats)
+        column_stats_rows<T, kStatsOfK, kAhead>(static_cast<const T *>(p.k) + head * p.k_stride_h, p.k_stride_s, begin, end, false, sh.red,
+                                                p.k_sum + head * H3S_HEAD_DIM, nullptr);
+      else
+        column_stats_rows<T, kStatsOfV, kAhead>(static_cast<const T *>(p.v) + head * p.v_stride_h, p.v_stride_s, begin, end, true, sh.red,
+                                                nullptr, p.v_amax_bits + head * H3S_HEAD_DIM);
+      __syncthreads();
+      if (t == 0) {
+        __threadfence();
+        ptx::add_release(p.stats_done + head, 1u);
+      }
+      continue;
+    }
+    const int step = job.index, row = step * kCarrierRows;
+    // the head's K mean or V scale, when its statistics are in; every thread calls it
+    auto wait_for_head = [&](bool is_v) {
+      if (t == 0 && !wait_for_count(p.stats_done + head, p.k_stats + p.v_stats, p.wait_budget_ns)) {
+        gave_up = 1;
+        report_status(p.status, p.status_mirror, kAbortStatistics, number, head, step);
+      }
+      __syncthreads();
+      if (t < H3S_HEAD_DIM) {
+        const int at = head * H3S_HEAD_DIM + t;
+        const float value = is_v ? finalize_scale(__ldcg(p.v_amax_bits + at), p.v_bound) : finalize_mean<T>(__ldcg(p.k_sum + at), p.sequence);
+        head_values[t] = value;
+        if (step == 0) (is_v ? p.v_scale : p.k_mean)[at] = value;
+      }
+      __syncthreads();
+    };
+    if (job.kind == kCarrierQ) {
+      const int64_t block = static_cast<int64_t>(head) * p.steps + step;
+      quant_qk_block<T, H3S_Q_TILE, false>(
+          static_cast<const T *>(p.q) + head * p.q_stride_h + row * p.q_stride_s, p.q_stride_s, min(kCarrierRows, p.sequence - row),
+          p.q8 + (static_cast<int64_t>(head) * p.sequence + row) * H3S_HEAD_DIM, p.q_scale + block, p.q_summary, p.summary_dtype,
+          block * H3S_HEAD_DIM, t, sh.q, []() { __syncthreads(); }, [](float2 (&)[4]) {});
+    } else if (job.kind == kCarrierK) {
+      const int half = t >> 7, blocks = (p.sequence + H3S_KV_TILE - 1) / H3S_KV_TILE;
+      const int half_row = row + half * H3S_KV_TILE;
+      const int64_t block = static_cast<int64_t>(head) * blocks + 2 * step + half;
+      const bool some = half_row < p.sequence;  // the last step's second block may be past the end: it is gone through, nothing is stored
+      quant_qk_block<T, H3S_KV_TILE, kSmooth>(
+          static_cast<const T *>(p.k) + head * p.k_stride_h + half_row * p.k_stride_s, p.k_stride_s, min(H3S_KV_TILE, p.sequence - half_row),
+          some ? p.k8 + (static_cast<int64_t>(head) * p.sequence + half_row) * H3S_HEAD_DIM : nullptr, some ? p.k_scale + block : nullptr,
+          some ? p.k_summary : nullptr, p.summary_dtype, block * H3S_HEAD_DIM, t & 127, sh.k[half], []() { __syncthreads(); },
+          [&](float2 (&minus_mu)[4]) {
+            if (!kSmooth) return;
+            wait_for_head(false);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) minus_mu[i] = make_float2(-head_values[c0 + 2 * i], -head_values[c0 + 2 * i + 1]);
+          });
+    } else {
+      const int64_t at = static_cast<int64_t>(head) * H3S_HEAD_DIM * p.padded + row;
+      quant_v_tile(static_cast<const T *>(p.v) + head * p.v_stride_h + row * p.v_stride_s, p.v_stride_s, min(kVTile, p.sequence - row),
+                   p.v8 + at, p.v16 == nullptr ? nullptr : p.v16 + at, p.padded, p.v_bound, sh.tile, [&](float (&scale)[8]) {
+                     wait_for_head(true);
+#pragma unroll
+                     for (int i = 0; i < 8; ++i) scale[i] = head_values[c0 + i];
+                   });
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) clear_words_kernel(unsigned int *words, int n) {
+  let_next_start();
+  wait_for_previous();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) words[i] = 0u;
+}
+
+// ---------------------------------------------------------------------------
 // Per-row FP8-E4M3 quantisation of a bf16 matrix (activations of the FP8 MLP).
 // Kept in registers between the amax reduction and the store.  Rows of up to 4096
 // channels: one warp each, no barrier, all loads of the row in flight (4096 x 3072: 23 -> 13 us);
@@ -578,6 +743,26 @@ static int launch_quant_v(const void *v, int64_t sh, int64_t ss, const float *v_
   return H3S_OK;
 }
 
+// Rows of a statistics job: as many as leave enough jobs for all SMs at once, since everything but Q waits for the last of them.  us,
+// both kernels, jobs of 128 / 256 / 512 / 1024 rows: 4 heads x 2304 tokens, fp32 13 / 16 / 22 / 32, 7 x 10384 37 / 35 / 38 / 46, 24 x 2304
+// 30 / 29 / 31 / 36, 8 x 20000 71 / 66 / 64 / 69, 24 x 33272 315 / 289 / 279 / 276.
+static int carrier_stats_rows(int heads, int sequence, bool smooth_k) {
+  constexpr int64_t kEnough = 380;
+  int rows = 1024;
+  while (rows > 64 && static_cast<int64_t>(heads) * ceil_div(sequence, rows) * (smooth_k ? 2 : 1) < kEnough) rows /= 2;
+  return rows;
+}
+
+template <typename T>
+static int launch_layer_carriers(const CarrierParams &p, bool smooth_k, cudaStream_t stream) {
+  constexpr int kResident = kSmCount * (sizeof(T) == 2 ? 4 : 2);
+  const int jobs = p.heads * (p.k_stats + p.v_stats + p.q_jobs + p.k_jobs + p.v_jobs);
+  const int grid = jobs < kResident ? jobs : kResident;
+  if (smooth_k) H3S_CHECK_CUDA(launch_next(layer_carriers_kernel<T, true>, grid, kCarrierThreads, 0, stream, p));
+  else H3S_CHECK_CUDA(launch_next(layer_carriers_kernel<T, false>, grid, kCarrierThreads, 0, stream, p));
+  return H3S_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Scratch that lives inside the library image, for hosts that cannot hand
 // h3s_column_stats a scratch buffer of their own (see h3s_column_stats_static).
@@ -640,6 +825,53 @@ int h3s_column_stats(const void *k, int64_t k_stride_h, int64_t k_stride_s, cons
     case H3S_F32: return launch_column_stats<float>(k, k_stride_h, k_stride_s, v, v_stride_h, v_stride_s, heads, sequence, v_bound, k_mean, v_scale, scratch, s);
     case H3S_BF16: return launch_column_stats<__nv_bfloat16>(k, k_stride_h, k_stride_s, v, v_stride_h, v_stride_s, heads, sequence, v_bound, k_mean, v_scale, scratch, s);
     default: return launch_column_stats<__half>(k, k_stride_h, k_stride_s, v, v_stride_h, v_stride_s, heads, sequence, v_bound, k_mean, v_scale, scratch, s);
+  }
+}
+
+size_t h3s_prepare_layer_counter_bytes(int heads) { return (static_cast<size_t>(heads) + 1) * sizeof(unsigned int); }
+
+int h3s_prepare_layer(const h3s_layer_carriers *c, const void *q, const void *k, const void *v, const int64_t *strides, int dtype,
+                           int heads, int sequence, int smooth_k, float v_bound, void *counters, int32_t *status,
+                           int32_t *host_mirror, h3s_stream_t stream) {
+  using namespace h3s;
+  H3S_CHECK_ARG(c != nullptr && strides != nullptr && counters != nullptr, "prepare_layer: NULL argument");
+  H3S_CHECK_ARG(q != nullptr && k != nullptr && v != nullptr, "prepare_layer: NULL input");
+  H3S_CHECK_ARG(heads > 0 && sequence > 0 && v_bound > 0.f, "prepare_layer: empty problem (heads=%d sequence=%d)", heads, sequence);
+  H3S_CHECK_ARG(c->q8 && c->q_scale && c->k8 && c->k_scale && c->v8 && c->v_scale && c->scratch && (!smooth_k || c->k_mean), "prepare_layer: NULL output");
+  H3S_CHECK_ARG((c->q_summary != nullptr) == (c->k_summary != nullptr) &&
+                (c->q_summary == nullptr || (c->summary_dtype >= H3S_F32 && c->summary_dtype <= H3S_F64)), "prepare_layer: bad tile means");
+  H3S_CHECK_ARG(((reinterpret_cast<uintptr_t>(c->q8) | reinterpret_cast<uintptr_t>(c->k8) | reinterpret_cast<uintptr_t>(c->scratch)) & 7) == 0 &&
+                ((reinterpret_cast<uintptr_t>(c->v8) | reinterpret_cast<uintptr_t>(c->v16)) & 15) == 0, "prepare_layer: misaligned buffers");
+  H3S_CHECK_ARG(static_cast<char *>(counters) == static_cast<char *>(c->scratch) + h3s_column_stats_scratch_bytes(heads),
+                "prepare_layer: the counters stand right behind the scratch");
+  { int rc = check_view(q, dtype, strides[0], strides[1], "prepare_layer q"); if (rc) return rc; }
+  { int rc = check_view(k, dtype, strides[2], strides[3], "prepare_layer k"); if (rc) return rc; }
+  { int rc = check_view(v, dtype, strides[4], strides[5], "prepare_layer v"); if (rc) return rc; }
+  CarrierParams p;
+  p.q = q; p.k = k; p.v = v;
+  p.q_stride_h = strides[0]; p.q_stride_s = strides[1]; p.k_stride_h = strides[2]; p.k_stride_s = strides[3];
+  p.v_stride_h = strides[4]; p.v_stride_s = strides[5];
+  p.q8 = c->q8; p.k8 = c->k8; p.v8 = c->v8; p.v16 = static_cast<uint16_t *>(c->v16);
+  p.q_scale = c->q_scale; p.k_scale = c->k_scale; p.v_scale = c->v_scale; p.k_mean = c->k_mean;
+  p.q_summary = c->q_summary; p.k_summary = c->k_summary; p.summary_dtype = c->summary_dtype;
+  p.heads = heads; p.sequence = sequence; p.padded = ceil_div(sequence, kVTile) * kVTile; p.v_bound = v_bound;
+  p.k_sum = static_cast<double *>(c->scratch);
+  p.v_amax_bits = reinterpret_cast<unsigned int *>(p.k_sum + heads * H3S_HEAD_DIM);
+  p.next = static_cast<unsigned int *>(counters); p.stats_done = p.next + 1;
+  p.status = status; p.status_mirror = host_mirror; p.wait_budget_ns = wait_budget_ns();
+  p.steps = ceil_div(sequence, kCarrierRows);
+  p.q_jobs = p.k_jobs = p.v_jobs = p.steps;
+  p.stats_rows = carrier_stats_rows(heads, sequence, smooth_k != 0);
+  p.v_stats = ceil_div(sequence, p.stats_rows);
+  p.k_stats = smooth_k ? p.v_stats : 0;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int words = static_cast<int>((h3s_column_stats_scratch_bytes(heads) + h3s_prepare_layer_counter_bytes(heads)) / sizeof(unsigned int));
+  const int clears = ceil_div(words, 1024);
+  H3S_CHECK_CUDA(launch_next(clear_words_kernel, clears < 64 ? clears : 64, 256, 0, s, reinterpret_cast<unsigned int *>(c->scratch), words));
+  switch (dtype) {
+    case H3S_F32: return launch_layer_carriers<float>(p, smooth_k != 0, s);
+    case H3S_BF16: return launch_layer_carriers<__nv_bfloat16>(p, smooth_k != 0, s);
+    default: return launch_layer_carriers<__half>(p, smooth_k != 0, s);
   }
 }
 

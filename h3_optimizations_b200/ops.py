@@ -255,8 +255,10 @@ class LayerBuffers:
         self._at = {"q_int8": 0, "k_int8": k_at, "v_carrier": v_at, "q_scale": q_scale_at, "k_scale": k_scale_at, "v_scale": v_scale_at}
         self._carriers = carriers = torch.empty(v_scale_at + _round256(4 * column), dtype=torch.int8, device=device)
         self.v_half = torch.empty((1, heads, HEAD_DIM, padded), dtype=torch.float16, device=device)
-        # statistics scratch and the K mean in front, so that the tile means may have any element size
-        mean_at = _round256(_native.load().h3s_column_stats_scratch_bytes(heads))
+        # statistics scratch with the counters of ``h3s_prepare_layer`` and the K mean in front, so that the tile means may have any element size
+        lib = _native.load()
+        self.counters_at = lib.h3s_column_stats_scratch_bytes(heads)
+        mean_at = _round256(self.counters_at + lib.h3s_prepare_layer_counter_bytes(heads))
         means_at = mean_at + (_round256(4 * column) if smooth_k else 0)
         size = 0 if summary_dtype is None else summary_dtype.itemsize
         k_means_at = means_at + _round256(size * column * q_blocks)
@@ -305,15 +307,25 @@ def _address(tensor):
     return None if tensor is None else tensor.data_ptr()
 
 
+def prepare_layer(q, k, v, buffers, stream, *, smooth_k, status, status_mirror, v_bound=FP8_V_BOUND):
+    """Carriers of HND ``q``, ``k``, ``v`` into ``buffers``, on ``stream`` (the raw handle of the current stream)."""
+    strides = (ctypes.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
+    check(
+        _native.load().h3s_prepare_layer(
+            buffers.native, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, dtype_code(q.dtype), q.shape[1], q.shape[2],
+            int(smooth_k), v_bound, buffers.native.scratch + buffers.counters_at, status.data_ptr(), status_mirror.data_ptr(), stream),
+        "h3s_prepare_layer",
+    )
+
+
 def quant_qkv(q, k, v, buffers, side, stream, *, smooth_k, v_after_k, v_bound=FP8_V_BOUND):
-    """Carriers of HND ``q``, ``k``, ``v`` into ``buffers``, on ``stream`` (the raw handle of the current
-    stream) and, where given, ``side``.  The caller joins ``side`` on every path, before the buffers can be freed."""
+    """The same as ``prepare_layer`` with kernels of their own, on ``stream`` and ``side``.  The caller joins ``side`` on every
+    path, before the buffers can be freed."""
     strides = (ctypes.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
     check(
         _native.load().h3s_quant_qkv(
             buffers.native, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, dtype_code(q.dtype), q.shape[1], q.shape[2],
-            int(smooth_k), v_bound, int(v_after_k), None if side is None else side.event_handle, stream,
-            stream if side is None else side.handle),
+            int(smooth_k), v_bound, int(v_after_k), side.event_handle, stream, side.handle),
         "h3s_quant_qkv",
     )
 

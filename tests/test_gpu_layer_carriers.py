@@ -1,0 +1,60 @@
+"""The carriers of a layer from one kernel against the kernels of their own, bit for bit.  Needs a B200."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CARRIERS = ("q_int8", "k_int8", "v_carrier", "q_scale", "k_scale", "v_scale")
+
+
+# one row; a K block and its first row more; a last step without a second K block; as many statistics jobs as fit one wave and more; heads of
+# one short block each
+@pytest.mark.parametrize("heads,sequence,dtype", [
+    (2, 1, torch.bfloat16), (3, 64, torch.float32), (1, 65, torch.float16), (2, 129, torch.bfloat16), (5, 1100, torch.float32),
+    (4, 2304, torch.bfloat16), (7, 10384, torch.float16), (3, 33272, torch.bfloat16), (200, 70, torch.bfloat16)])
+@pytest.mark.parametrize("token_major", [False, True])
+@pytest.mark.parametrize("smooth_k,means", [(True, True), (False, True), (True, False)])
+def test_one_kernel_gives_what_the_others_give(native_lib, heads, sequence, dtype, token_major, smooth_k, means):
+    from h3_optimizations_b200 import _native, ops
+
+    gen = torch.Generator(device="cuda").manual_seed(heads * sequence)
+    qkv = []
+    for offset in (0.0, 0.7, -0.2):
+        x = (torch.randn((1, heads, sequence, 128), generator=gen, device="cuda") + offset).to(dtype)
+        qkv.append(x.transpose(1, 2).contiguous().transpose(1, 2) if token_major else x)
+    device = qkv[0].device
+    stream, side = _native.stream_ptr(device), ops.SideStream(device)
+    word, mirror = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.zeros(4, dtype=torch.int32).pin_memory()
+    results = []
+    for one in (False, True, True):
+        buffers = ops.LayerBuffers(heads, sequence, device, smooth_k=smooth_k, summary_dtype=torch.float64 if means else None)
+        buffers._carriers.fill_(77)
+        buffers.v_half.fill_(3.0)
+        buffers._call.fill_(91)  # scratch and counters come as they are
+        if one:
+            ops.prepare_layer(*qkv, buffers, stream, smooth_k=smooth_k, status=word, status_mirror=mirror)
+        else:
+            ops.quant_qkv(*qkv, buffers, side, stream, smooth_k=smooth_k, v_after_k=True)
+            side.join(stream)
+        torch.cuda.synchronize()
+        tensors = [buffers.tensor(name) for name in CARRIERS] + [buffers.v_half]
+        results.append([t.view(torch.uint8).clone() for t in tensors + ([buffers.q_summary, buffers.k_summary] if means else [])])
+    assert word.tolist() == mirror.tolist() == [0, 0, 0, 0]
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+
+
+def test_what_the_kernel_cannot_take_is_refused(native_lib):
+    from h3_optimizations_b200 import _native, ops
+
+    q, k, v = (torch.zeros((1, 2, 128, 136), device="cuda", dtype=torch.bfloat16)[..., :128] for _ in range(3))
+    buffers = ops.LayerBuffers(2, 128, q.device, smooth_k=True, summary_dtype=None)
+    word, mirror = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.zeros(4, dtype=torch.int32).pin_memory()
+    call = lambda *qkv: ops.prepare_layer(*qkv, buffers, _native.stream_ptr(q.device), smooth_k=True, status=word, status_mirror=mirror)
+    call(q, k, v)
+    odd = torch.zeros((2 * 128 * 132 + 4,), device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(_native.NativeError, match="multiples of 8"):
+        call(q, odd[: 2 * 128 * 132].view(1, 2, 128, 132)[..., :128], v)
+    with pytest.raises(_native.NativeError, match="aligned"):
+        call(q, k, odd[4:].view(-1)[: 2 * 128 * 128].view(1, 2, 128, 128))
