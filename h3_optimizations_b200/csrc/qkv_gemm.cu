@@ -216,7 +216,8 @@ struct GemmLayout {
   static constexpr uint32_t kOffTile = kOffB + kStages * kGemmBBytes;
   static constexpr uint32_t kOffExchange = kOffTile + (kCarriers ? 2 * kEpilogueTileBytes : 0);
   static constexpr uint32_t kOffNorm = kOffExchange + (kMode == kModeCarriers ? 2 * sizeof(EpilogueExchange) : 0);  // weights of Q, of K
-  static constexpr uint32_t kOffBar = kOffNorm + (kMode == kModeCarriers ? 2 * H3S_HEAD_DIM * sizeof(float) : 0);
+  static constexpr uint32_t kOffScale = kOffNorm + (kMode == kModeCarriers ? 2 * H3S_HEAD_DIM * sizeof(float) : 0);  // a warp's 64 column scales
+  static constexpr uint32_t kOffBar = kOffScale + (kMode == kModeCarriers ? 16 * 64 * sizeof(float) : 0);
   static constexpr uint32_t kBytes = kOffBar + 256 + 1024;
   static_assert(sizeof(uint64_t) * (2 * 6 + 16) + 8 <= 256, "barriers");
   static_assert(kBytes <= 227 * 1024, "GEMM shared memory exceeds the per-CTA limit");
@@ -810,16 +811,23 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int tm = 2 * pair + rank;  // this CTA's 128 rows; may lie past the last row
       const int a = local & 1;
       const uint32_t acc_use = local >> 1;
+      const int row = tm * kGemmM + quarter * 32 + lane;
+      const bool row_ok = row < prm.rows;
+      const int group_col0 = tn * tile_n + gi * H3S_HEAD_DIM;
+      // scales come while the MMAs are still at it
+      const float xs = prm.x_scale == nullptr ? 1.0f : (row_ok ? __ldg(prm.x_scale + row) : 0.f);
+      float *my_scales = reinterpret_cast<float *>(smem + L::kOffScale) + warp * 64;
+      if (kCarriers) {  // without a group nothing is stored
+        const int i = 2 * lane, channel = i < 24 ? 24 * share + i : i < 48 ? 24 + 24 * share + i : 48 + 16 * share + i;
+        reinterpret_cast<float2 *>(my_scales)[lane] = __ldg(reinterpret_cast<const float2 *>(prm.w_scale + (group_col0 < prm.n_out ? group_col0 : 0) + channel));
+        __syncwarp();
+      }
       {
         const bool got = ptx::mbar_wait(&sh.acc_full[a], acc_use & 1u, abort_word, kGemmAbortAccFull, prm.wait_budget_ns);
         if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
       }
       ptx::tc_fence_after();
-      const int row = tm * kGemmM + quarter * 32 + lane;
-      const bool row_ok = row < prm.rows;
-      const float xs = prm.x_scale == nullptr ? 1.0f : (row_ok ? __ldg(prm.x_scale + row) : 0.f);
       {
-        const int group_col0 = tn * tile_n + gi * H3S_HEAD_DIM;
         const int group = group_col0 >> 7;  // 128-column group == (kind, head)
         const int columns_end = min(prm.n_out, (tn + 1) * tile_n);  // of the tile
         const bool group_ok = group_col0 < columns_end && tm * kGemmM < prm.rows;
@@ -936,33 +944,32 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           {
             HalfRow y;
             const float2 xs2 = make_float2(xs, xs);
-            const float *w_scale = prm.w_scale + (group_ok ? group_col0 : 0);  // without a group nothing is stored
             const uint32_t columns = tmem_base + lane_addr + a * kGemmN + gi * H3S_HEAD_DIM;
-            auto dequantise = [&](uint32_t lo, uint32_t hi, int channel) {
-              const float2 ws = __ldg(reinterpret_cast<const float2 *>(w_scale + channel));
+            auto dequantise = [&](uint32_t lo, uint32_t hi, int i) {  // the i-th and the next of this share's channels
+              const float2 ws = *reinterpret_cast<const float2 *>(my_scales + i);
               const float2 value = mul2(make_float2(static_cast<float>(static_cast<int>(lo)),
                                                     static_cast<float>(static_cast<int>(hi))), mul2(xs2, ws));
               return pack_bf16x2(value.x, value.y);
             };
-            auto read24 = [&](uint32_t (&to)[12], int channel) {
+            auto read24 = [&](uint32_t (&to)[12], int channel, int first) {
               uint32_t acc[16], more[8];
               H3S_TMEM_LD16(columns + channel, acc);
               H3S_TMEM_LD8(columns + channel + 16, more);
               ptx::tmem_wait_ld(acc);
               ptx::tmem_wait_ld(more);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) to[i] = dequantise(acc[2 * i], acc[2 * i + 1], channel + 2 * i);
+              for (int i = 0; i < 8; ++i) to[i] = dequantise(acc[2 * i], acc[2 * i + 1], first + 2 * i);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) to[8 + i] = dequantise(more[2 * i], more[2 * i + 1], channel + 16 + 2 * i);
+              for (int i = 0; i < 4; ++i) to[8 + i] = dequantise(more[2 * i], more[2 * i + 1], first + 16 + 2 * i);
             };
-            read24(y.first, 24 * share);
-            read24(y.second, 48 + 24 * share);
+            read24(y.first, 24 * share, 0);
+            read24(y.second, 48 + 24 * share, 24);
             {
               uint32_t acc[16];
               H3S_TMEM_LD16(columns + 96 + 16 * share, acc);
               ptx::tmem_wait_ld(acc);
 #pragma unroll
-              for (int i = 0; i < 8; ++i) y.rest[i] = dequantise(acc[2 * i], acc[2 * i + 1], 96 + 16 * share + 2 * i);
+              for (int i = 0; i < 8; ++i) y.rest[i] = dequantise(acc[2 * i], acc[2 * i + 1], 48 + 2 * i);
             }
             // the accumulator is in registers: the MMA warp may refill it
             ptx::tc_fence_before();
