@@ -29,7 +29,7 @@ from __future__ import annotations
 import torch
 
 from . import _native, ops
-from .carriers import PreparedFusedQKV, PreparedHybrid, PreparedLayer, PreparedSparse, VCarrier, validate_prepared_fused_qkv
+from .carriers import PreparedFusedQKV, PreparedHybrid, PreparedLayer, PreparedSparse, ProjectedLayer, VCarrier, validate_prepared_fused_qkv
 from .config import MODE_SAGE128_FUSED_QKV, HybridSparseConfig, resolve_video_budget
 from .errors import FusedQKVError, SparseRouterError, SparseSageError
 from .router import KV_TILE, Q_TILE, SparseTileRouter
@@ -360,18 +360,24 @@ class B200SparseBackend:
             self.config, snapshot.step_index, snapshot.total_steps, layer_index
         )
         heads, sequence = int(projected.heads), int(projected.sequence)
-        if not projected.q_int8.is_cuda:
+        lazy = isinstance(projected, ProjectedLayer)
+        device = projected.device if lazy else projected.q_int8.device
+        if device.type != "cuda":
             raise SparseSageError("fused H3 Sparse Sage requires CUDA")
-        self._poll_status(projected.q_int8.device)
+        self._poll_status(device)
         try:
             route = self.router.build_route_from_summaries(
                 projected.q_summary, projected.k_summary, snapshot.layout, video_budget,
                 **self._sink(transformer_options, layer_index),
             )
-            v_carrier, v_scale = VCarrier.of(projected), projected.v_scale
-            prepacked = v_carrier.codes is not None
-            if not prepacked:
-                v_carrier, v_scale = ops.quant_v_fp8(projected.v, None, V_QUANT_BOUND)
+            # after the route: a route sink may have been handed the carriers meanwhile
+            buffers = projected.untouched() if lazy else None
+            prepacked = True
+            if buffers is None:
+                v_carrier, v_scale = VCarrier.of(projected), projected.v_scale
+                prepacked = v_carrier.codes is not None
+                if not prepacked:
+                    v_carrier, v_scale = ops.quant_v_fp8(projected.v, None, V_QUANT_BOUND)
         except SparseRouterError as exc:
             raise SparseSageError("sparse routing failed: %s" % exc) from exc
         except _native.NativeError as exc:
@@ -384,6 +390,10 @@ class B200SparseBackend:
                 "prepacked_fp8_v": prepacked,
             }
         )
+        if buffers is not None:
+            return PreparedHybrid(sparse=PreparedLayer.over(
+                buffers, route=route, output_dtype=projected.output_dtype, output_shape=(1, heads, sequence, projected.head_dim),
+                layer_index=int(projected.layer_index), metadata=metadata))
         sparse = PreparedSparse(
             q_int8=projected.q_int8, k_int8=projected.k_int8, v_carrier=v_carrier,
             q_scale=projected.q_scale, k_scale=projected.k_scale, v_scale=v_scale, route=route,
@@ -440,7 +450,8 @@ class B200SparseBackend:
         weight = getattr(linear, "weight", None)
         sparse = prepared.sparse
         if (weight is None or weight.ndim != 2 or weight.dtype != torch.bfloat16
-                or weight.dtype != sparse.output_dtype or weight.device != sparse.q_int8.device
+                or weight.dtype != sparse.output_dtype
+                or weight.device != (sparse.device if isinstance(sparse, PreparedLayer) else sparse.q_int8.device)
                 or weight.shape[1] != sparse.heads * 128 or weight.shape[0] % 8 or weight.stride(1) != 1):
             return None
         out_hnd = self.execute(prepared)                                   # (1, H, S, 128) view of (S, H, 128)

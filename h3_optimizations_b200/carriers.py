@@ -124,7 +124,10 @@ def validate_prepared_fused_qkv(prepared):
     (attention/sparse/fused_qkv.py:95-154: same conditions, same
     ``FusedQKVError`` texts) and hand it back.  The conditions are a table
     (``_carrier_spec``) walked once; device and contiguity are checked over
-    every tensor the table names."""
+    every tensor the table names.  Carriers that nobody has been handed yet are
+    as ``ops.LayerBuffers`` laid them out."""
+    if isinstance(prepared, ProjectedLayer) and prepared.untouched() is not None:
+        return prepared
     if int(prepared.head_dim) != HEAD_DIM:
         raise FusedQKVError("fused H3 QKV requires head_dim 128")
     seen = {}
@@ -177,11 +180,13 @@ def _unfilled(cls):
     return object.__new__(cls)
 
 
-class PreparedLayer(PreparedSparse):
-    """A ``PreparedSparse`` whose carriers are those of an ``ops.LayerBuffers`` (``over``).  Its tensors come into being
-    when they are asked for; until then (``untouched``) nobody can have written to them or put others in their place."""
+class _OverBuffers:
+    """The lazy part of a class whose carriers are those of an ``ops.LayerBuffers`` (``over``).  Its tensors come into being
+    when they are asked for; until then (``untouched``) nobody can have written to them or put others in their place.
+    Objects over the same buffers share the pair of codes and FP16 copy as such, through the buffers."""
 
     _LAZY = frozenset(("q_int8", "k_int8", "q_scale", "k_scale", "v_scale", "_v"))
+    _copied_as = None  # the class of a copy
 
     @classmethod
     def over(cls, buffers, **rest):
@@ -191,10 +196,13 @@ class PreparedLayer(PreparedSparse):
 
     def __getattr__(self, name):  # of what the instance does not hold (yet)
         buffers = self.__dict__.get("_buffers")
-        if buffers is None or name not in PreparedLayer._LAZY:
+        if buffers is None or name not in _OverBuffers._LAZY:
             raise AttributeError("%r object has no attribute %r" % (type(self).__name__, name))
         if name == "_v":
-            value, buffers.v_half = VCarrier(buffers.tensor("v_carrier"), buffers.v_half), None
+            value = getattr(buffers, "v_pair", None)
+            if value is None:
+                value = buffers.v_pair = VCarrier(buffers.tensor("v_carrier"), buffers.v_half)
+                buffers.v_half = None
         else:
             value = buffers.tensor(name)
         self.__dict__[name] = value
@@ -209,15 +217,50 @@ class PreparedLayer(PreparedSparse):
     def untouched(self):
         """The buffers, if no tensor of them has been handed out or replaced."""
         buffers = self.__dict__.get("_buffers")
-        if buffers is None or buffers.v_half is None or not PreparedLayer._LAZY.isdisjoint(self.__dict__):
+        if buffers is None or buffers.v_half is None or not _OverBuffers._LAZY.isdisjoint(self.__dict__):
             return None
         return buffers
 
     def __reduce_ex__(self, protocol):
-        """A copy is a ``PreparedSparse``.  A shallow one shares the tensors, and the pair of codes and FP16 copy as such."""
-        state = {name: getattr(self, name) for name in PreparedLayer._LAZY}
+        """A copy is of the plain class.  A shallow one shares the tensors, and the pair of codes and FP16 copy as such."""
+        state = {name: getattr(self, name) for name in _OverBuffers._LAZY}
         state.update((name, value) for name, value in self.__dict__.items() if name != "_buffers")
-        return _unfilled, (PreparedSparse,), state
+        return _unfilled, (self._copied_as,), state
+
+
+class PreparedLayer(_OverBuffers, PreparedSparse):
+    """A ``PreparedSparse`` over an ``ops.LayerBuffers``."""
+
+    _copied_as = PreparedSparse
+
+
+class ProjectedLayer(_OverBuffers, PreparedFusedQKV):
+    """A ``PreparedFusedQKV`` over an ``ops.LayerBuffers``: what a backend of this package is handed by its projector, and
+    hands on to the attention kernel by addresses.  Making the seven tensors, looking at each of them at both ends and taking
+    them apart again for the launches took 27 of the 213 us for which the host is busy with an attention block, and at 24 heads x
+    2304 tokens that is what bounds it: 186 -> 170 us a block."""
+
+    _copied_as = PreparedFusedQKV
+
+    @property
+    def v_scale(self):  # the plain class has a default, which would be found before ``__getattr__``
+        held = self.__dict__
+        return held["v_scale"] if "v_scale" in held else self.__getattr__("v_scale")
+
+    @v_scale.setter
+    def v_scale(self, value):
+        self.__dict__["v_scale"] = value
+
+    def untouched(self):
+        """The buffers, if besides their tensors also what describes them, and the tile means, is as the contract wants it."""
+        buffers = super().untouched()
+        if buffers is None or (self.sequence, self.heads, self.head_dim) != (buffers.sequence, buffers.heads, HEAD_DIM):
+            return None
+        for means, tile in ((self.q_summary, Q_TILE), (self.k_summary, KV_TILE)):
+            if (means.shape != (1, buffers.heads, -(-buffers.sequence // tile), HEAD_DIM) or means.device != buffers.device
+                    or not means.is_contiguous()):
+                return None
+        return buffers
 
 
 @dataclass

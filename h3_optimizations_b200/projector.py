@@ -37,7 +37,7 @@ import math
 import torch
 
 from . import _native, ops
-from .carriers import PreparedFusedQKV, validate_prepared_fused_qkv
+from .carriers import ProjectedLayer
 from .errors import FusedQKVError
 from .router import KV_TILE, Q_TILE
 
@@ -157,12 +157,8 @@ def run_chunked_sparse_qkv(x, w_i8, w_scale, *, heads, head_dim=HEAD_DIM, layer_
                         epsilon=float(epsilon), rope=rope_freqs, status=status, v_bound=V_QUANT_BOUND)
     except _native.NativeError as exc:
         raise FusedQKVError("chunked QKV projection failed: layer=%d: %s" % (layer_index, exc)) from exc
-    return validate_prepared_fused_qkv(
-        PreparedFusedQKV(
-            q_int8=buffers.tensor("q_int8"), q_scale=buffers.tensor("q_scale"), k_int8=buffers.tensor("k_int8"),
-            k_scale=buffers.tensor("k_scale"), v=None,
-            q_summary=buffers.q_summary, k_summary=buffers.k_summary, output_dtype=x.dtype, sequence=sequence,
-            heads=heads, head_dim=HEAD_DIM, layer_index=int(layer_index), smooth_k=bool(smooth_k),
-            v_carrier=buffers.tensor("v_carrier"), v_scale=buffers.tensor("v_scale"), v_half=buffers.v_half,
-        )
-    )
+    q_summary, k_summary = buffers.q_summary, buffers.k_summary
+    buffers.release_call()
+    return ProjectedLayer.over(
+        buffers, v=None, q_summary=q_summary, k_summary=k_summary, output_dtype=x.dtype, head_dim=HEAD_DIM,
+        layer_index=int(layer_index), smooth_k=bool(smooth_k))
