@@ -41,6 +41,13 @@ int qkv_gemm_carriers(const int8_t *x_i8, const float *x_scale, const int8_t *w_
                       float epsilon, const void *rope, int rope_dtype, const int64_t *rope_strides, int32_t *status,
                       h3s_stream_t stream);
 
+// K (with smooth_k) and V of the projection from their staging and the totals in `c->scratch`
+int staged_carriers(const h3s_layer_carriers *c, const void *k_stage, const void *v_stage, int heads, int sequence, bool smooth_k,
+                    float v_bound, cudaStream_t stream);
+// h3s_convrot_quant_rows, whose first launch of a call may also clear `words` 32-bit words
+int convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hidden, int8_t *x_i8, float *x_scale, uint32_t *clear, int words,
+                       cudaStream_t stream);
+
 constexpr int kSmCount = 148;  // of a B200, for the rules that deal out work
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }

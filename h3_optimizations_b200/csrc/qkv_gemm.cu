@@ -65,10 +65,11 @@ __host__ __device__ constexpr int rot_stride(int groups) { return 8 * groups + 4
 
 __global__ void __launch_bounds__(kRotWarps * 32)
 convrot_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_stride, int rows, int hidden,
-                          int8_t *__restrict__ out, float *__restrict__ scale_out) {
+                          int8_t *__restrict__ out, float *__restrict__ scale_out, uint32_t *__restrict__ clear, int words) {
   extern __shared__ __align__(16) float rot_smem[];
   let_next_start();
   wait_for_previous();
+  for (int i = blockIdx.x * (kRotWarps * 32) + threadIdx.x; i < words; i += gridDim.x * (kRotWarps * 32)) clear[i] = 0u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = hidden / kRotGroup, stride = rot_stride(groups);
   float *mine = rot_smem + warp * 32 * stride;
@@ -1325,13 +1326,8 @@ inline int make_tensor_map_u8_2d(CUtensorMap *map, const void *base, uint64_t di
   return H3S_OK;
 }
 
-}  // namespace h3s
-
-extern "C" {
-
-int h3s_convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hidden, int8_t *x_i8,
-                           float *x_scale, h3s_stream_t stream) {
-  using namespace h3s;
+int convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hidden, int8_t *x_i8, float *x_scale, uint32_t *clear, int words,
+                       cudaStream_t stream) {
   H3S_CHECK_ARG(x != nullptr && x_i8 != nullptr && x_scale != nullptr, "convrot_quant_rows: NULL pointer");
   H3S_CHECK_ARG(rows > 0 && hidden > 0 && hidden % kRotGroup == 0 && hidden / kRotGroup <= 32,
                 "convrot_quant_rows: hidden %d must be a multiple of 256 and at most 8192", hidden);
@@ -1341,9 +1337,18 @@ int h3s_convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hi
   const int smem = kRotWarps * 32 * rot_stride(hidden / kRotGroup) * static_cast<int>(sizeof(float));
   constexpr int kMostSmem = kRotWarps * 32 * rot_stride(32) * static_cast<int>(sizeof(float));  // 133 KB; one value for all callers
   H3S_CHECK_CUDA(cudaFuncSetAttribute(convrot_quant_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
-  H3S_CHECK_CUDA(launch_next(convrot_quant_rows_kernel, ceil_div(rows, kRotWarps), kRotWarps * 32, smem, static_cast<cudaStream_t>(stream),
-                             static_cast<const __nv_bfloat16 *>(x), x_stride_row, rows, hidden, x_i8, x_scale));
+  H3S_CHECK_CUDA(launch_next(convrot_quant_rows_kernel, ceil_div(rows, kRotWarps), kRotWarps * 32, smem, stream,
+                             static_cast<const __nv_bfloat16 *>(x), x_stride_row, rows, hidden, x_i8, x_scale, clear, words));
   return H3S_OK;
+}
+
+}  // namespace h3s
+
+extern "C" {
+
+int h3s_convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hidden, int8_t *x_i8,
+                           float *x_scale, h3s_stream_t stream) {
+  return h3s::convrot_quant_rows(x, x_stride_row, rows, hidden, x_i8, x_scale, nullptr, 0, static_cast<cudaStream_t>(stream));
 }
 
 static int qkv_gemm_chunk_impl(const int8_t *x_i8, const float *x_scale, const int8_t *w_i8, const float *w_scale,

@@ -559,6 +559,62 @@ layer_carriers_kernel(const __grid_constant__ CarrierParams p) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Second phase of the projection in one launch: K without its mean and V by its scale, from bf16 staging and complete totals.  For short
+// sequences, which are bound by latency: every block makes its head's means or scales itself, from totals that it asks for before its rows, so
+// that no kernel stands between the last projection tile and this one, and no second stream.  Long sequences go the other way, figures at
+// h3s_project_qkv_norms; of the 19 us that they would lose 5 are the 64-bit divisions of every block.
+// ---------------------------------------------------------------------------
+
+template <bool kSmooth>
+__global__ void __launch_bounds__(kCarrierThreads, 4)
+staged_carriers_kernel(const __grid_constant__ CarrierParams p) {
+  using T = __nv_bfloat16;
+  __shared__ __align__(16) CarrierShared sh;
+  __shared__ __align__(16) float head_values[H3S_HEAD_DIM];
+  let_next_start();
+  wait_for_previous();
+  const int t = threadIdx.x, c0 = (t & 15) * 8;
+  constexpr int kKinds = kSmooth ? 2 : 1;
+  const int place = blockIdx.x / kKinds, head = place / p.steps;
+  const int step = place - head * p.steps, row = step * kCarrierRows;
+  const bool is_v = !kSmooth || blockIdx.x % kKinds != 0;
+  const int at_value = head * H3S_HEAD_DIM + (t & (H3S_HEAD_DIM - 1));
+  // asked for before the rows
+  const double k_total = is_v ? 0.0 : __ldg(p.k_sum + at_value);
+  const unsigned int v_top = is_v ? __ldg(p.v_amax_bits + at_value) : 0u;
+  auto make_values = [&]() {
+    if (t < H3S_HEAD_DIM) {
+      const float value = is_v ? finalize_scale(v_top, p.v_bound) : finalize_mean<T>(k_total, p.sequence);
+      head_values[t] = value;
+      if (step == 0) (is_v ? p.v_scale : p.k_mean)[at_value] = value;
+    }
+    __syncthreads();
+  };
+  if (kSmooth && !is_v) {
+    const int half = t >> 7, blocks = (p.sequence + H3S_KV_TILE - 1) / H3S_KV_TILE;
+    const int half_row = row + half * H3S_KV_TILE;
+    const bool some = half_row < p.sequence;  // the last step's second block may be past the end: it is gone through, nothing is stored
+    quant_qk_block<T, H3S_KV_TILE, true>(
+        static_cast<const T *>(p.k) + head * p.k_stride_h + half_row * p.k_stride_s, p.k_stride_s, min(H3S_KV_TILE, p.sequence - half_row),
+        some ? p.k8 + (static_cast<int64_t>(head) * p.sequence + half_row) * H3S_HEAD_DIM : nullptr,
+        some ? p.k_scale + static_cast<int64_t>(head) * blocks + 2 * step + half : nullptr, nullptr, H3S_F32, 0, t & 127, sh.k[half],
+        []() { __syncthreads(); }, [&](float2 (&minus_mu)[4]) {
+          make_values();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) minus_mu[i] = make_float2(-head_values[c0 + 2 * i], -head_values[c0 + 2 * i + 1]);
+        });
+  } else {
+    const int64_t at = static_cast<int64_t>(head) * H3S_HEAD_DIM * p.padded + row;
+    quant_v_tile(static_cast<const T *>(p.v) + head * p.v_stride_h + row * p.v_stride_s, p.v_stride_s, min(kVTile, p.sequence - row),
+                 p.v8 + at, p.v16 == nullptr ? nullptr : p.v16 + at, p.padded, p.v_bound, sh.tile, [&](float (&scale)[8]) {
+                   make_values();
+#pragma unroll
+                   for (int i = 0; i < 8; ++i) scale[i] = head_values[c0 + i];
+                 });
+  }
+}
+
 __global__ void __launch_bounds__(256) clear_words_kernel(unsigned int *words, int n) {
   let_next_start();
   wait_for_previous();
@@ -760,6 +816,33 @@ static int launch_layer_carriers(const CarrierParams &p, bool smooth_k, cudaStre
   const int grid = jobs < kResident ? jobs : kResident;
   if (smooth_k) H3S_CHECK_CUDA(launch_next(layer_carriers_kernel<T, true>, grid, kCarrierThreads, 0, stream, p));
   else H3S_CHECK_CUDA(launch_next(layer_carriers_kernel<T, false>, grid, kCarrierThreads, 0, stream, p));
+  return H3S_OK;
+}
+
+int staged_carriers(const h3s_layer_carriers *c, const void *k_stage, const void *v_stage, int heads, int sequence, bool smooth_k,
+                    float v_bound, cudaStream_t stream) {
+  H3S_CHECK_ARG(v_bound > 0.f, "project_qkv: v_bound must be positive");
+  H3S_CHECK_ARG(c->v8 && c->v_scale && v_stage && (!smooth_k || (c->k8 && c->k_scale && c->k_mean && k_stage)), "project_qkv: NULL carrier");
+  H3S_CHECK_ARG(((reinterpret_cast<uintptr_t>(c->k8) | reinterpret_cast<uintptr_t>(c->scratch)) & 7) == 0 &&
+                ((reinterpret_cast<uintptr_t>(c->v8) | reinterpret_cast<uintptr_t>(c->v16)) & 15) == 0, "project_qkv: misaligned buffers");
+  CarrierParams p = {};
+  p.k = k_stage; p.v = v_stage;
+  p.k_stride_h = p.v_stride_h = static_cast<int64_t>(sequence) * H3S_HEAD_DIM;
+  p.k_stride_s = p.v_stride_s = H3S_HEAD_DIM;
+  if (smooth_k) {
+    int rc = check_view(k_stage, H3S_BF16, p.k_stride_h, p.k_stride_s, "project_qkv k_stage");
+    if (rc) return rc;
+  }
+  { int rc = check_view(v_stage, H3S_BF16, p.v_stride_h, p.v_stride_s, "project_qkv v_stage"); if (rc) return rc; }
+  p.k8 = c->k8; p.v8 = c->v8; p.v16 = static_cast<uint16_t *>(c->v16);
+  p.k_scale = c->k_scale; p.v_scale = c->v_scale; p.k_mean = c->k_mean;
+  p.heads = heads; p.sequence = sequence; p.padded = ceil_div(sequence, kVTile) * kVTile; p.v_bound = v_bound;
+  p.k_sum = static_cast<double *>(c->scratch);
+  p.v_amax_bits = reinterpret_cast<unsigned int *>(p.k_sum + heads * H3S_HEAD_DIM);
+  p.steps = ceil_div(sequence, kCarrierRows);
+  const int grid = heads * p.steps * (smooth_k ? 2 : 1);
+  if (smooth_k) H3S_CHECK_CUDA(launch_next(staged_carriers_kernel<true>, grid, kCarrierThreads, 0, stream, p));
+  else H3S_CHECK_CUDA(launch_next(staged_carriers_kernel<false>, grid, kCarrierThreads, 0, stream, p));
   return H3S_OK;
 }
 
