@@ -36,110 +36,139 @@ namespace h3s {
 constexpr int kRotGroup = 256;
 
 // In-register part of the transform: butterflies over the three low index bits.
-__device__ __forceinline__ void fwht8(float (&v)[8]) {
+// The stages of a Walsh-Hadamard transform behind the first, on pairs of neighbouring values; a - b as the exactly rounded a + (-1) * b
+template <int kPairs>
+__device__ __forceinline__ void fwht_pairs(float2 (&v)[kPairs]) {
 #pragma unroll
-  for (int stride = 1; stride < 8; stride <<= 1) {
+  for (int stride = 1; stride < kPairs; stride <<= 1) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kPairs; ++i) {
       if ((i & stride) == 0) {
-        const float a = v[i], b = v[i + stride];
-        v[i] = __fadd_rn(a, b);
-        v[i + stride] = __fsub_rn(a, b);
+        const float2 a = v[i], b = v[i + stride];
+        v[i] = add2(a, b);
+        v[i + stride] = fma2(b, make_float2(-1.f, -1.f), a);
       }
     }
   }
+}
+
+// The larger magnitude, with some sign; a NaN stays one
+__device__ __forceinline__ float larger_magnitude(float a, float b) {
+  float d;
+  asm("max.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
 }
 
 // One warp per row.  The three low index bits are transformed as loaded (8 channels a lane);
 // the row then crosses shared memory once, so that a lane holds the 32 values that share
 // their low bits and the five remaining stages are additions of its own registers.  With
 // those stages as warp shuffles (40 per 8 channels) and a row spread over all warps of a CTA
-// (two barriers a row), 4096 rows of 3072 channels took
-// 24.5 us, 21.4 us now.
+// (two barriers a row), 4096 rows of 3072 channels took 24.5 us and 21.4 so.  Instructions bound it then, two for each that
+// the transform needs: with packed additions, the integer taken from the low bits of a shifted quotient, and NaN looked for once a
+// row instead of a clamp for each code, 15.1 -> 13.0 us behind one another (2.9 TB/s; 2304 rows 9.0 -> 8.0, 900 rows 8.1 -> 7.1).
+// What is left is sixteen warps an SM, as many as shared memory has rows for, that wait for their loads.
 // Shared memory of a warp: [32 upper indices][8 * groups + 4 floats]; the padding puts
 // the 16-byte stores of eight lanes into different banks.
-constexpr int kRotWarps = 4;    // rows (warps) per CTA
-constexpr int kRotAhead = 6;    // 16-byte loads of a lane in flight
+constexpr int kRotWarps = 4;  // rows (warps) per CTA, at most
 
 __host__ __device__ constexpr int rot_stride(int groups) { return 8 * groups + 4; }
 
+template <int kAhead>  // 16-byte loads of a lane in flight
 __global__ void __launch_bounds__(kRotWarps * 32)
 convrot_quant_rows_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_stride, int rows, int hidden,
                           int8_t *__restrict__ out, float *__restrict__ scale_out, uint32_t *__restrict__ clear, int words) {
   extern __shared__ __align__(16) float rot_smem[];
   let_next_start();
   wait_for_previous();
-  for (int i = blockIdx.x * (kRotWarps * 32) + threadIdx.x; i < words; i += gridDim.x * (kRotWarps * 32)) clear[i] = 0u;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) clear[i] = 0u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = hidden / kRotGroup, stride = rot_stride(groups);
   float *mine = rot_smem + warp * 32 * stride;
-  const int row = blockIdx.x * kRotWarps + warp;
+  const int row = blockIdx.x * (blockDim.x >> 5) + warp;
   if (row >= rows) return;  // warps of a CTA do not meet
   const __nv_bfloat16 *src = x + row * x_stride + lane * 8;
-  for (int g0 = 0; g0 < groups; g0 += kRotAhead) {
-    Elem<__nv_bfloat16>::Raw raw[kRotAhead];
+  for (int g0 = 0; g0 < groups; g0 += kAhead) {
+    Elem<__nv_bfloat16>::Raw raw[kAhead];
 #pragma unroll
-    for (int i = 0; i < kRotAhead; ++i)
+    for (int i = 0; i < kAhead; ++i)
       raw[i] = g0 + i < groups ? Elem<__nv_bfloat16>::load_raw(src + (g0 + i) * kRotGroup) : Elem<__nv_bfloat16>::zero_raw();
 #pragma unroll
-    for (int i = 0; i < kRotAhead; ++i) {
+    for (int i = 0; i < kAhead; ++i) {
       if (g0 + i < groups) {
-        float v[8];
-        Elem<__nv_bfloat16>::unpack(raw[i], v);
-        fwht8(v);
+        float x[8];
+        Elem<__nv_bfloat16>::unpack(raw[i], x);
+        float2 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = make_float2(__fadd_rn(x[2 * k], x[2 * k + 1]), __fsub_rn(x[2 * k], x[2 * k + 1]));
+        fwht_pairs(v);
         float4 *dst = reinterpret_cast<float4 *>(mine + lane * stride + (g0 + i) * 8);
-        dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-        dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+        dst[0] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+        dst[1] = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
       }
     }
   }
   __syncwarp();
   float amax = 0.f;
   for (int c = lane; c < 8 * groups; c += 32) {  // (group, low bits)
-    float v[32];
+    float2 v[16];  // two upper indices at a time
 #pragma unroll
-    for (int l = 0; l < 32; ++l) v[l] = mine[l * stride + c];
-#pragma unroll
-    for (int step = 1; step < 32; step <<= 1) {
-#pragma unroll
-      for (int l = 0; l < 32; ++l) {
-        if ((l & step) == 0) {
-          const float a = v[l], b = v[l + step];
-          v[l] = __fadd_rn(a, b);
-          v[l + step] = __fsub_rn(a, b);
-        }
-      }
+    for (int i = 0; i < 16; ++i) {
+      const float a = mine[(2 * i) * stride + c], b = mine[(2 * i + 1) * stride + c];
+      v[i] = make_float2(__fadd_rn(a, b), __fsub_rn(a, b));
     }
+    fwht_pairs(v);
 #pragma unroll
-    for (int l = 0; l < 32; ++l) {
-      v[l] *= 0.0625f;  // 1/sqrt(256), exact
-      amax = fmaxf(amax, fabsf(v[l]));
-      mine[l * stride + c] = v[l];
+    for (int i = 0; i < 16; ++i) {
+      v[i] = mul2(v[i], make_float2(0.0625f, 0.0625f));  // 1/sqrt(256), exact
+      amax = larger_magnitude(larger_magnitude(amax, v[i].x), v[i].y);
+      mine[(2 * i) * stride + c] = v[i].x;
+      mine[(2 * i + 1) * stride + c] = v[i].y;
     }
   }
-  amax = warp_max(amax);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = larger_magnitude(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  amax = fabsf(amax);
   __syncwarp();
+  const bool some_nan = amax != amax;
+  if (some_nan) {  // it counts as nothing
+    amax = 0.f;
+    for (int c = lane; c < 8 * groups; c += 32)
+      for (int l = 0; l < 32; ++l) amax = fmaxf(amax, fabsf(mine[l * stride + c]));
+    amax = warp_max(amax);
+  }
   const float scale = amax > 0.f ? __fdiv_rn(amax, 127.0f) : 1.0f;
   if (lane == 0) scale_out[row] = scale;
   const SharedDivisor by_scale = make_divisor(scale);  // exact v/scale without a divide per element
   int8_t *dst = out + static_cast<int64_t>(row) * hidden + lane * 8;
   auto emit = [&](auto exact_tag) {
+    constexpr bool kExact = decltype(exact_tag)::value;
 #pragma unroll 2
     for (int g = 0; g < groups; ++g) {
       const float4 *at = reinterpret_cast<const float4 *>(mine + lane * stride + g * 8);
       const float4 lo = at[0], hi = at[1];
-      const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-      uint32_t packed[2] = {0u, 0u};
+      const float2 v[4] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y), make_float2(hi.z, hi.w)};
+      uint32_t code[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        int code = __float2int_rn(divide<decltype(exact_tag)::value>(by_scale, v[i]));
-        code = max(-127, min(127, code));
-        packed[i >> 2] |= (static_cast<uint32_t>(code) & 0xffu) << ((i & 3) * 8);
+      for (int i = 0; i < 4; ++i) {
+        const float2 q = divide2<kExact>(by_scale, v[i]);
+        if (kExact) {  // |q| <= 127.0001: the nearest integer is in the low bits of q + 1.5 * 2^23
+          const float2 shifted = add2(q, make_float2(12582912.0f, 12582912.0f));
+          code[2 * i] = __float_as_uint(shifted.x);
+          code[2 * i + 1] = __float_as_uint(shifted.y);
+        } else {
+          code[2 * i] = static_cast<uint32_t>(max(-127, min(127, __float2int_rn(q.x))));
+          code[2 * i + 1] = static_cast<uint32_t>(max(-127, min(127, __float2int_rn(q.y))));
+        }
       }
+      uint32_t packed[2];
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        packed[w] = __byte_perm(__byte_perm(code[4 * w], code[4 * w + 1], 0x0040),
+                                __byte_perm(code[4 * w + 2], code[4 * w + 3], 0x0040), 0x5410);
       *reinterpret_cast<uint2 *>(dst + g * kRotGroup) = make_uint2(packed[0], packed[1]);
     }
   };
-  if (by_scale.exact) emit(std::true_type{}); else emit(std::false_type{});
+  if (by_scale.exact && !some_nan) emit(std::true_type{}); else emit(std::false_type{});
 }
 
 // ---------------------------------------------------------------------------
@@ -1334,12 +1363,17 @@ int convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hidden
   H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(x) & 15) == 0 && x_stride_row % 8 == 0 && x_stride_row >= hidden,
                 "convrot_quant_rows: input must be 16-byte aligned with a row stride that is a multiple of 8");
   H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(x_i8) & 7) == 0, "convrot_quant_rows: output must be 8-byte aligned");
-  const int smem = kRotWarps * 32 * rot_stride(hidden / kRotGroup) * static_cast<int>(sizeof(float));
-  constexpr int kMostSmem = kRotWarps * 32 * rot_stride(32) * static_cast<int>(sizeof(float));  // 133 KB; one value for all callers
-  H3S_CHECK_CUDA(cudaFuncSetAttribute(convrot_quant_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
-  H3S_CHECK_CUDA(launch_next(convrot_quant_rows_kernel, ceil_div(rows, kRotWarps), kRotWarps * 32, smem, stream,
-                             static_cast<const __nv_bfloat16 *>(x), x_stride_row, rows, hidden, x_i8, x_scale, clear, words));
-  return H3S_OK;
+  const int row_bytes = 32 * rot_stride(hidden / kRotGroup) * static_cast<int>(sizeof(float));  // of shared memory, 33 KB at most
+  auto launch = [&](auto kernel, int warps) {
+    H3S_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRotWarps * 32 * rot_stride(32) * static_cast<int>(sizeof(float))));
+    H3S_CHECK_CUDA(launch_next(kernel, ceil_div(rows, warps), warps * 32, warps * row_bytes, stream, static_cast<const __nv_bfloat16 *>(x),
+                               x_stride_row, rows, hidden, x_i8, x_scale, clear, words));
+    return H3S_OK;
+  };
+  // Of wide rows shared memory holds few: as many as go in with one to a CTA, and more loads to each.  us for 4096 rows, four to a CTA with
+  // six loads ahead / one with six / one with twelve: 5120 channels 28.7 / 23.4 / 21.6, 8192 64.9 / 49.1 / 42.0; 3072 12.9 / 13.0 / 13.4,
+  // 1024 5.8 / 6.3 / 6.0.
+  return hidden > 3072 ? launch(convrot_quant_rows_kernel<12>, 1) : launch(convrot_quant_rows_kernel<6>, kRotWarps);
 }
 
 }  // namespace h3s

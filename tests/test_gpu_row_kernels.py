@@ -56,3 +56,29 @@ def test_a_batch_equals_its_elements(native_lib, batch):
         one = backend.forward(q[b:b + 1], k[b:b + 1], v[b:b + 1], layer_index=0, transformer_options=options)
         # the K mean's FP64 sum is gathered with atomics, in any order: its rounding is the same but for ties
         assert (out[b:b + 1].float() - one.float()).abs().max() <= 2.0 ** -8 * one.float().abs().max()
+
+
+@pytest.mark.parametrize("hidden", [512, 3328])
+def test_rotated_codes_of_unusual_rows(native_lib, hidden):
+    """A NaN counts as nothing and takes code 0, as whatever an infinite scale divides; scales down to the smallest."""
+    from h3_optimizations_b200 import ops
+
+    gen = torch.Generator().manual_seed(hidden)
+    x = torch.randn((8, hidden), generator=gen).to(torch.bfloat16)
+    x[0], x[1], x[2] = 0.0, x[1] * 2.0 ** -120, x[2] * 2.0 ** 120
+    x[3] = 0.0
+    x[3, 7] = 2.0 ** -133  # a scale below the smallest normal number
+    without = x.clone()
+    x[4, 5], without[4, :256] = float("nan"), 0.0
+    x[5, 300] = float("inf")
+    x[6, 3], x[6, 4] = float("inf"), float("nan")
+    codes, scale = (t.cpu() for t in ops.convrot_quant_rows(x.cuda()))
+    want_codes, want_scale = oracle.convrot_quantize_rows(without)
+    rows = [0, 1, 2, 3, 4, 7]
+    assert torch.equal(scale[rows], want_scale[rows]) and torch.equal(codes[rows], want_codes[rows])
+    assert scale[5] == float("inf") and not codes[5].any()
+    # the group of row 6 has nothing but NaN; the others are quantised by their own largest magnitude
+    other = x[6:7].clone()
+    other[0, :256] = 0.0
+    want_codes, want_scale = oracle.convrot_quantize_rows(other)
+    assert torch.equal(codes[6:7], want_codes) and torch.equal(scale[6:7], want_scale)
