@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("smooth_k", [True, False])
-@pytest.mark.parametrize("heads,sequence", [(1, 1), (3, 63), (2, 65), (3, 129), (2, 1000), (1, 150_000), (1, 150_001)])
+@pytest.mark.parametrize("heads,sequence", [(1, 1), (3, 63), (2, 65), (3, 129), (2, 1000), (1, 100_000), (1, 100_001)])
 def test_against_the_oracle(native_lib, heads, sequence, smooth_k):
     from h3_optimizations_b200 import ops
     from h3_optimizations_b200.projector import run_chunked_sparse_qkv
