@@ -108,6 +108,8 @@ PROTOTYPES = {
     "h3s_prepare_layer_counter_bytes": (c_size_t, [c_int]),
     "h3s_prepare_layer": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                   c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "h3s_prepare_layer_flags": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                        c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "h3s_stream_order": (c_int, [c_void_p, c_void_p, c_void_p]),
     "h3s_quant_qkv": (c_int, [ctypes.POINTER(LayerCarriers), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                               c_int, c_float, c_int, c_void_p, c_void_p, c_void_p]),

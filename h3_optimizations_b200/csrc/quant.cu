@@ -431,6 +431,7 @@ struct CarrierParams {
   unsigned int *next, *stats_done;  // the next job; per head: statistics jobs that are through
   int32_t *status, *status_mirror;
   unsigned long long wait_budget_ns;
+  int missing;                                   // self-test of the wait: statistics jobs of a head that it expects and nobody does
   int stats_rows;                                // of a statistics job
   int k_stats, v_stats, q_jobs, k_jobs, v_jobs;  // jobs of a head
 };
@@ -479,18 +480,18 @@ layer_carriers_kernel(const __grid_constant__ CarrierParams p) {
   __shared__ __align__(16) CarrierShared sh;
   __shared__ __align__(16) float head_values[H3S_HEAD_DIM];
   __shared__ int jobs[2];
-  __shared__ int gave_up;
+  __shared__ bool late;  // the first thread's alone: its wait has run out
   let_next_start();
-  if (threadIdx.x == 0) gave_up = 0;
   wait_for_previous();
   const int total = p.heads * (p.k_stats + p.v_stats + p.q_jobs + p.k_jobs + p.v_jobs);
   const int t = threadIdx.x, c0 = (t & 15) * 8;
   int next = t == 0 ? static_cast<int>(atomicAdd(p.next, 1u)) : 0;
+  if (t == 0) late = false;
   for (int turn = 0;; turn ^= 1) {
     if (t == 0) jobs[turn] = next;
     __syncthreads();  // and the job before this one has left shared memory
     const int number = jobs[turn];
-    if (number >= total || gave_up != 0) break;
+    if (number >= total) break;
     if (t == 0) next = static_cast<int>(atomicAdd(p.next, 1u));  // asked for ahead of its use
     const CarrierJob job = carrier_job(p, number);
     const int head = job.head;
@@ -511,10 +512,11 @@ layer_carriers_kernel(const __grid_constant__ CarrierParams p) {
       continue;
     }
     const int step = job.index, row = step * kCarrierRows;
-    // the head's K mean or V scale, when its statistics are in; every thread calls it
+    // The head's K mean or V scale, when its statistics are in; every thread calls it.  After a wait that has run out the block goes through
+    // its jobs without another one: nobody else takes them, and what reads the carriers next is to find values, if wrong ones.
     auto wait_for_head = [&](bool is_v) {
-      if (t == 0 && !wait_for_count(p.stats_done + head, p.k_stats + p.v_stats, p.wait_budget_ns)) {
-        gave_up = 1;
+      if (t == 0 && !late && !wait_for_count(p.stats_done + head, p.k_stats + p.v_stats + p.missing, p.wait_budget_ns)) {
+        late = true;
         report_status(p.status, p.status_mirror, kAbortStatistics, number, head, step);
       }
       __syncthreads();
@@ -914,8 +916,14 @@ int h3s_column_stats(const void *k, int64_t k_stride_h, int64_t k_stride_s, cons
 size_t h3s_prepare_layer_counter_bytes(int heads) { return (static_cast<size_t>(heads) + 1) * sizeof(unsigned int); }
 
 int h3s_prepare_layer(const h3s_layer_carriers *c, const void *q, const void *k, const void *v, const int64_t *strides, int dtype,
-                           int heads, int sequence, int smooth_k, float v_bound, void *counters, int32_t *status,
-                           int32_t *host_mirror, h3s_stream_t stream) {
+                      int heads, int sequence, int smooth_k, float v_bound, void *counters, int32_t *status,
+                      int32_t *host_mirror, h3s_stream_t stream) {
+  return h3s_prepare_layer_flags(c, q, k, v, strides, dtype, heads, sequence, smooth_k, v_bound, 0, counters, status, host_mirror, stream);
+}
+
+int h3s_prepare_layer_flags(const h3s_layer_carriers *c, const void *q, const void *k, const void *v, const int64_t *strides, int dtype,
+                            int heads, int sequence, int smooth_k, float v_bound, int flags, void *counters, int32_t *status,
+                            int32_t *host_mirror, h3s_stream_t stream) {
   using namespace h3s;
   H3S_CHECK_ARG(c != nullptr && strides != nullptr && counters != nullptr, "prepare_layer: NULL argument");
   H3S_CHECK_ARG(q != nullptr && k != nullptr && v != nullptr, "prepare_layer: NULL input");
@@ -942,6 +950,7 @@ int h3s_prepare_layer(const h3s_layer_carriers *c, const void *q, const void *k,
   p.v_amax_bits = reinterpret_cast<unsigned int *>(p.k_sum + heads * H3S_HEAD_DIM);
   p.next = static_cast<unsigned int *>(counters); p.stats_done = p.next + 1;
   p.status = status; p.status_mirror = host_mirror; p.wait_budget_ns = wait_budget_ns();
+  p.missing = (flags & H3S_PREPARE_TEST_MISSING_STATISTICS) != 0;
   p.steps = ceil_div(sequence, kCarrierRows);
   p.q_jobs = p.k_jobs = p.v_jobs = p.steps;
   p.stats_rows = carrier_stats_rows(heads, sequence, smooth_k != 0);

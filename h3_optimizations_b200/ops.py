@@ -23,6 +23,7 @@ ATTN_P_SINGLE = 1
 ATTN_DEVICE_OUTPUT = 4
 ATTN_TEST_DROP_KV_LOAD = 0x4000
 ATTN_TEST_DROP_LAST_V_LOAD = 0x8000
+PREPARE_TEST_MISSING_STATISTICS = 1
 
 
 def _ceil_div(a, b):
@@ -307,13 +308,13 @@ def _address(tensor):
     return None if tensor is None else tensor.data_ptr()
 
 
-def prepare_layer(q, k, v, buffers, stream, *, smooth_k, status, status_mirror, v_bound=FP8_V_BOUND):
+def prepare_layer(q, k, v, buffers, stream, *, smooth_k, status, status_mirror, v_bound=FP8_V_BOUND, extra_flags=0):
     """Carriers of HND ``q``, ``k``, ``v`` into ``buffers``, on ``stream`` (the raw handle of the current stream)."""
     strides = (ctypes.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
     check(
-        _native.load().h3s_prepare_layer(
+        _native.load().h3s_prepare_layer_flags(
             buffers.native, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, dtype_code(q.dtype), q.shape[1], q.shape[2],
-            int(smooth_k), v_bound, buffers.native.scratch + buffers.counters_at, status.data_ptr(), status_mirror.data_ptr(), stream),
+            int(smooth_k), v_bound, extra_flags, buffers.native.scratch + buffers.counters_at, status.data_ptr(), status_mirror.data_ptr(), stream),
         "h3s_prepare_layer",
     )
 

@@ -58,3 +58,57 @@ def test_what_the_kernel_cannot_take_is_refused(native_lib):
         call(q, odd[: 2 * 128 * 132].view(1, 2, 128, 132)[..., :128], v)
     with pytest.raises(_native.NativeError, match="aligned"):
         call(q, k, odd[4:].view(-1)[: 2 * 128 * 128].view(1, 2, 128, 128))
+
+
+# fewer jobs than blocks, and more than twice as many
+@pytest.mark.parametrize("heads,sequence,dtype", [(2, 200, torch.bfloat16), (1, 1, torch.float32), (24, 2304, torch.bfloat16), (9, 5000, torch.float32)])
+@pytest.mark.parametrize("smooth_k", [True, False])
+def test_statistics_that_do_not_come_are_given_up(native_lib, heads, sequence, dtype, smooth_k):
+    """The wait expects a statistics job that nobody does, with a limit of 1 ms: the launch says so and ends, every block with one wait,
+    all jobs are done (the statistics are there by then, so with the right result), and the next launch is as ever."""
+    from h3_optimizations_b200 import _native, ops
+
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    qkv = [torch.randn((1, heads, sequence, 128), generator=gen, device="cuda").to(dtype) for _ in range(3)]
+    device = qkv[0].device
+    word, mirror = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.zeros(4, dtype=torch.int32).pin_memory()
+    start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+
+    def carriers(flags):
+        buffers = ops.LayerBuffers(heads, sequence, device, smooth_k=smooth_k, summary_dtype=torch.float64)
+        buffers._carriers.fill_(77)
+        buffers.v_half.fill_(3.0)
+        buffers._call.fill_(91)
+        torch.cuda.synchronize()
+        start.record()
+        ops.prepare_layer(*qkv, buffers, _native.stream_ptr(device), smooth_k=smooth_k, status=word, status_mirror=mirror, extra_flags=flags)
+        stop.record()
+        torch.cuda.synchronize()  # returns: the kernel ended by itself
+        return [t.view(torch.uint8).clone() for t in [buffers.tensor(name) for name in CARRIERS] + [buffers.v_half, buffers.q_summary, buffers.k_summary]]
+
+    good = carriers(0)
+    assert word.tolist() == mirror.tolist() == [0, 0, 0, 0]
+    previous = ops.set_wait_budget_ns(1_000_000)
+    try:
+        late = carriers(ops.PREPARE_TEST_MISSING_STATISTICS)
+    finally:
+        ops.set_wait_budget_ns(previous)
+    assert 0.9 < start.elapsed_time(stop) < 50.0
+    code, job, head, step = word.tolist()
+    assert code == 15 and mirror.tolist() == [code, job, head, step]
+    steps = -(-sequence // 128)
+    job -= _early_jobs(heads, sequence, smooth_k)
+    assert 0 <= job < heads * 2 * steps and (head, step) == (job // (2 * steps), job % steps)
+    assert all(torch.equal(a, b) for a, b in zip(good, late))
+    word.zero_()
+    mirror.zero_()
+    assert all(torch.equal(a, b) for a, b in zip(good, carriers(0)))
+    assert word.tolist() == mirror.tolist() == [0, 0, 0, 0]
+
+
+def _early_jobs(heads, sequence, smooth_k):
+    """Jobs that wait for nothing: statistics, of as many rows a job as leave 380 of them where there are so many, and Q blocks."""
+    rows = 1024
+    while rows > 64 and heads * -(-sequence // rows) * (2 if smooth_k else 1) < 380:
+        rows //= 2
+    return heads * (-(-sequence // rows) * (2 if smooth_k else 1) + -(-sequence // 128))
