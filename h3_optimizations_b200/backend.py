@@ -250,6 +250,8 @@ class B200SparseBackend:
                    6: "free score slot", 7: "P.V of an earlier tile", 8: "last P.V", 9: "Q rows in tensor memory",
                    10: "answer to the request for more work", 11: "end of a pass over the list", 12: "output sums being read",
                    13: "first row maxima", 14: "output tile staged", 15: "whole-sequence statistics"}
+    # where another kernel than the attention waited, and what the words behind the code are
+    ABORT_PLACES = {15: ("Layer carrier", "job %d, head %d, block %d of 128 rows")}
 
     def _status_slot(self, device):
         key = device.index if device.index is not None else torch.cuda.current_device()
@@ -262,12 +264,12 @@ class B200SparseBackend:
 
     @classmethod
     def _raise_for(cls, words, where):
-        code, cta, head, tile = (int(x) for x in words)
+        code, number, head, tile = (int(x) for x in words)
         if code != 0:
+            kernel, places = cls.ABORT_PLACES.get(code, ("Sparse attention", "CTA %d, head %d, query tile %d"))
             raise SparseSageError(
-                "Sparse attention kernel gave up waiting for %s (code %d) in CTA %d, head %d, query tile %d (%s); "
-                "the output of that launch is invalid"
-                % (cls.ABORT_NAMES.get(code, "an unknown event"), code, cta, head, tile, where))
+                "%s kernel gave up waiting for %s (code %d) in %s (%s); the output of that launch is invalid"
+                % (kernel, cls.ABORT_NAMES.get(code, "an unknown event"), code, places % (number, head, tile), where))
 
     def _poll_status(self, device):
         """Non-blocking look at the mirror of the earlier launches' status."""
@@ -279,7 +281,7 @@ class B200SparseBackend:
 
     def check_status(self, device=None):
         """Synchronise with the device and raise ``SparseSageError`` if a
-        bounded device wait ran out in any attention launch since the last
+        bounded device wait ran out in any launch of a layer call since the last
         check.  Clears the word."""
         devices = list(self._status) if device is None else [torch.device(device).index]
         for key in devices:
