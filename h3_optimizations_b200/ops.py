@@ -320,13 +320,14 @@ def prepare_layer(q, k, v, buffers, stream, *, smooth_k, status, status_mirror, 
 
 
 def quant_qkv(q, k, v, buffers, side, stream, *, smooth_k, v_after_k, v_bound=FP8_V_BOUND):
-    """The same as ``prepare_layer`` with kernels of their own, on ``stream`` and ``side``.  The caller joins ``side`` on every
-    path, before the buffers can be freed."""
+    """The same as ``prepare_layer`` with kernels of their own, on ``stream`` and, where given, ``side``.  The caller joins ``side``
+    on every path, before the buffers can be freed."""
     strides = (ctypes.c_int64 * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
     check(
         _native.load().h3s_quant_qkv(
             buffers.native, q.data_ptr(), k.data_ptr(), v.data_ptr(), strides, dtype_code(q.dtype), q.shape[1], q.shape[2],
-            int(smooth_k), v_bound, int(v_after_k), side.event_handle, stream, side.handle),
+            int(smooth_k), v_bound, int(v_after_k), None if side is None else side.event_handle, stream,
+            stream if side is None else side.handle),
         "h3s_quant_qkv",
     )
 

@@ -55,3 +55,22 @@ def test_copy_of_the_status_words(native_lib):
     _native.check(native_lib.h3s_status_mirror(word.data_ptr(), mirror.data_ptr(), event.cuda_event, _native.stream_ptr()), "h3s_status_mirror")
     event.synchronize()
     assert mirror.tolist() == [2, 5, 1, 3]
+
+
+@pytest.mark.parametrize("smooth_k", [True, False])
+@pytest.mark.parametrize("v_after_k", [True, False])
+def test_carriers_by_kernels_of_their_own_on_one_stream(native_lib, smooth_k, v_after_k):
+    from h3_optimizations_b200 import _native, ops
+
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    qkv = [torch.randn((1, 3, 1100, 128), generator=gen, device="cuda").bfloat16() for _ in range(3)]
+    stream, second = _native.stream_ptr(qkv[0].device), ops.SideStream(qkv[0].device)
+    results = []
+    for side in (second, None):
+        buffers = ops.LayerBuffers(3, 1100, qkv[0].device, smooth_k=smooth_k, summary_dtype=torch.float32)
+        ops.quant_qkv(*qkv, buffers, side, stream, smooth_k=smooth_k, v_after_k=v_after_k)
+        if side is not None:
+            side.join(stream)
+        names = ("q_int8", "k_int8", "v_carrier", "q_scale", "k_scale", "v_scale")
+        results.append([buffers.tensor(name).view(torch.uint8) for name in names] + [buffers.v_half, buffers.q_summary, buffers.k_summary])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
