@@ -617,10 +617,10 @@ staged_carriers_kernel(const __grid_constant__ CarrierParams p) {
   }
 }
 
-__global__ void __launch_bounds__(256) clear_words_kernel(unsigned int *words, int n) {
+__global__ void __launch_bounds__(256) clear_words_kernel(unsigned int *words, int n, unsigned int *more, int m) {
   let_next_start();
   wait_for_previous();
-  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) words[i] = 0u;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n + m; i += gridDim.x * 256) (i < n ? words[i] : more[i - n]) = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -933,8 +933,7 @@ int h3s_prepare_layer_flags(const h3s_layer_carriers *c, const void *q, const vo
                 (c->q_summary == nullptr || (c->summary_dtype >= H3S_F32 && c->summary_dtype <= H3S_F64)), "prepare_layer: bad tile means");
   H3S_CHECK_ARG(((reinterpret_cast<uintptr_t>(c->q8) | reinterpret_cast<uintptr_t>(c->k8) | reinterpret_cast<uintptr_t>(c->scratch)) & 7) == 0 &&
                 ((reinterpret_cast<uintptr_t>(c->v8) | reinterpret_cast<uintptr_t>(c->v16)) & 15) == 0, "prepare_layer: misaligned buffers");
-  H3S_CHECK_ARG(static_cast<char *>(counters) == static_cast<char *>(c->scratch) + h3s_column_stats_scratch_bytes(heads),
-                "prepare_layer: the counters stand right behind the scratch");
+  H3S_CHECK_ARG((reinterpret_cast<uintptr_t>(counters) & 3) == 0, "prepare_layer: misaligned counters");
   { int rc = check_view(q, dtype, strides[0], strides[1], "prepare_layer q"); if (rc) return rc; }
   { int rc = check_view(k, dtype, strides[2], strides[3], "prepare_layer k"); if (rc) return rc; }
   { int rc = check_view(v, dtype, strides[4], strides[5], "prepare_layer v"); if (rc) return rc; }
@@ -957,9 +956,9 @@ int h3s_prepare_layer_flags(const h3s_layer_carriers *c, const void *q, const vo
   p.v_stats = ceil_div(sequence, p.stats_rows);
   p.k_stats = smooth_k ? p.v_stats : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int words = static_cast<int>((h3s_column_stats_scratch_bytes(heads) + h3s_prepare_layer_counter_bytes(heads)) / sizeof(unsigned int));
-  const int clears = ceil_div(words, 1024);
-  H3S_CHECK_CUDA(launch_next(clear_words_kernel, clears < 64 ? clears : 64, 256, 0, s, reinterpret_cast<unsigned int *>(c->scratch), words));
+  const int words = static_cast<int>(h3s_column_stats_scratch_bytes(heads) / sizeof(unsigned int)), clears = ceil_div(words + heads + 1, 1024);
+  H3S_CHECK_CUDA(launch_next(clear_words_kernel, clears < 64 ? clears : 64, 256, 0, s, reinterpret_cast<unsigned int *>(c->scratch), words,
+                             p.next, heads + 1));
   switch (dtype) {
     case H3S_F32: return launch_layer_carriers<float>(p, smooth_k != 0, s);
     case H3S_BF16: return launch_layer_carriers<__nv_bfloat16>(p, smooth_k != 0, s);

@@ -74,3 +74,30 @@ def test_carriers_by_kernels_of_their_own_on_one_stream(native_lib, smooth_k, v_
         names = ("q_int8", "k_int8", "v_carrier", "q_scale", "k_scale", "v_scale")
         results.append([buffers.tensor(name).view(torch.uint8) for name in names] + [buffers.v_half, buffers.q_summary, buffers.k_summary])
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("heads", [1, 5, 600])
+def test_layer_carriers_with_counters_of_their_own(native_lib, heads):
+    import ctypes
+
+    from h3_optimizations_b200 import _native, ops
+
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    qkv = [torch.randn((1, heads, 150, 128), generator=gen, device="cuda").bfloat16() for _ in range(3)]
+    strides = (ctypes.c_int64 * 6)(*(150 * 128, 128) * 3)
+    guard = torch.full((heads + 9,), 7, dtype=torch.int32, device="cuda")
+    results = []
+    for own in (False, True):
+        buffers = ops.LayerBuffers(heads, 150, qkv[0].device, smooth_k=True, summary_dtype=torch.float64)
+        buffers._call.fill_(91)
+        counters = guard.data_ptr() + 4 * 5 if own else buffers.native.scratch + buffers.counters_at
+        _native.check(native_lib.h3s_prepare_layer(
+            buffers.native, *(t.data_ptr() for t in qkv), strides, _native.H3S_BF16, heads, 150, 1, 448.0, counters, None, None,
+            _native.stream_ptr(qkv[0].device)), "h3s_prepare_layer")
+        names = ("q_int8", "k_int8", "v_carrier", "q_scale", "k_scale", "v_scale")
+        results.append([buffers.tensor(name).view(torch.uint8) for name in names] + [buffers.v_half, buffers.q_summary, buffers.k_summary])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    assert guard[:5].tolist() + guard[heads + 6:].tolist() == [7] * 8
+    assert native_lib.h3s_prepare_layer_counter_bytes(heads) == 4 * (heads + 1)
+    assert native_lib.h3s_prepare_layer(buffers.native, *(t.data_ptr() for t in qkv), strides, _native.H3S_BF16, heads, 150, 1, 448.0,
+                                        counters + 2, None, None, None) == -1
