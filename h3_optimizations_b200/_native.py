@@ -84,6 +84,7 @@ PROTOTYPES = {
                                             c_int, c_void_p, c_void_p, c_void_p]),
     "h3s_dense_gemm": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p]),
+    "h3s_dense_gemm_columns": (c_int, [c_int, c_int, c_int, c_int]),
     "h3s_quant_rows_fp8": (c_int, [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "h3s_column_stats_finalize": (c_int, [c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p]),
     "h3s_route_topk": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,

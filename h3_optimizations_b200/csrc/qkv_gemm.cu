@@ -275,7 +275,7 @@ struct GemmParams {
   int64_t out_stride_head;  // elements between consecutive 128-column groups
   int32_t *status;
   int rows, n_out, hidden;
-  int m_pairs, n_tiles;  // pairs of 128-row tiles, 256-column tiles
+  int m_pairs, n_tiles;  // pairs of 128-row tiles, tiles of tile_n columns
   // Column tiles are visited in the order of the weight rows, [Q | K | V]: the tiles that are
   // dearer in the epilogue (norm, rotation, quantisation) are dealt out first, the cheap
   // V tiles even out what is left.  Alternating between the kinds, as suits a kernel that is
@@ -1506,16 +1506,26 @@ int h3s_qkv_gemm_chunk_norm_rope(const int8_t *x_i8, const float *x_scale, const
 // K its 128 rows of A are loaded whatever the width (96 bytes a clock and SM with 128 columns, 64 with 256), and what the MMAs leave
 // idle the SM clock makes up for, as the power allows.  96 columns' worth of such time is where the line fits 52 shapes; the rule's
 // choice is the fastest width of each or within 4 % of it.  us, 256 columns / the rule's, launches in a row:
-//   fp8    64 x 3072 x 12288 33.2 / 17.8 (96), 300 x 3072 x 12288 33.7 / 19.8 (96), 700 x 3072 x 12288 34.0 / 23.8 (128), 1000 x 3072 x 12288
+//   fp8    64 x 3072 x 12288 32.7 / 17.6 (64), 300 x 3072 x 12288 33.7 / 19.8 (96), 700 x 3072 x 12288 34.0 / 23.8 (128), 1000 x 3072 x 12288
 //          38.0 / 30.5 (192), 1000 x 12288 x 3072 34.2 / 31.3 (224), 2000 x 3072 x 12288 80.6 / 66.1 (192), 1500 x 3072 x 12288 42.2 (256)
 //   bf16   64 x 1024 x 1024 10.0 / 6.9 (64), 900 x 3072 x 3072 21.2 / 17.4 (192), 2304 x 3072 x 3072 35.3 / 30.4 (192), 8000 x 3072 x 3072
 //          128.5 / 120.9 (192), 33272 x 3072 x 3072 462.3 (256; 224: 477, 128: 603)
-static int dense_tile_columns(int m_pairs, int n_out, int pairs_of_sms) {
-  constexpr int kStep = 32, kLeast = 64, kFixed = 96;
+// Where A is all but nothing (up to 20 rows of 6 KB, 8 of 12 KB) every CTA waits for the same few lines of it at the same time, and 32 tiles
+// and more beside one another take longer than 24.  us, 256 columns / as many as leave 24 tiles / 64: fp8 1 x 3072 x 12288 32.6 / 26.9
+// (128) / 38.4, 8 rows 32.6 / 25.2 / 39.3, 12 rows 32.6 / 18.9 / 17.5; bf16 1 x 3072 x 3072 19.2 / 17.0 (128) / 23.2, 20 rows 19.2 / 13.8 / 21.2,
+// 24 rows 19.2 / 12.0 / 11.3; 1 x 4096 x 1024 10.3 / 10.3 (192) / 11.9, 48 rows 10.3 / 9.4 / 10.3, 64 rows 10.3 / 9.0 / 7.5; 1 x 2048 x 2048
+// 14.7 / 14.2 (96) / 16.3, 24 rows 14.7 / 11.4 / 13.4, 32 rows 14.7 / 9.3 / 9.0; with 264 columns 64 are the fastest throughout.
+int h3s_dense_gemm_columns(int rows, int n_out, int k_bytes, int sms) {
+  constexpr int kStep = 32, kLeast = 64, kFixed = 96, kTilesOfLittle = 24;
+  constexpr int64_t kLittle = 128 * 1024;  // bytes of A that a row of tiles reads
+  const int m_pairs = h3s::ceil_div(rows, h3s::kGemmPairM), pairs_of_sms = sms < 2 ? 1 : sms / 2;
+  const bool little = static_cast<int64_t>(rows < h3s::kGemmPairM ? rows : h3s::kGemmPairM) * k_bytes < kLittle;
   int best = h3s::kGemmN;
   int64_t best_cost = 0;
   for (int width = h3s::kGemmN; width >= kLeast; width -= kStep) {
-    const int64_t tiles = static_cast<int64_t>(m_pairs) * h3s::ceil_div(n_out, width);
+    const int columns = h3s::ceil_div(n_out, width);
+    if (little && columns > kTilesOfLittle) break;
+    const int64_t tiles = static_cast<int64_t>(m_pairs) * columns;
     const int64_t cost = (tiles + pairs_of_sms - 1) / pairs_of_sms * (kFixed + width);
     if (best_cost == 0 || cost < best_cost) { best = width; best_cost = cost; }
   }
@@ -1545,7 +1555,7 @@ int h3s_dense_gemm(const void *a, int64_t lda_bytes, const void *b, int64_t ldb_
   int device = 0, sms = 0;
   H3S_CHECK_CUDA(cudaGetDevice(&device));
   H3S_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const int tile_n = dense_tile_columns(ceil_div(rows, kGemmPairM), n_out, sms / 2);
+  const int tile_n = h3s_dense_gemm_columns(rows, n_out, k_bytes, sms);
   rc = make_tensor_map_u8_2d(&mb, b, k_bytes, n_out, ldb_bytes, kGemmK, tile_n / 2, "dense_gemm B map");
   if (rc) return rc;
   GemmParams prm;
