@@ -1373,7 +1373,14 @@ int convrot_quant_rows(const void *x, int64_t x_stride_row, int rows, int hidden
   // Of wide rows shared memory holds few: as many as go in with one to a CTA, and more loads to each.  us for 4096 rows, four to a CTA with
   // six loads ahead / one with six / one with twelve: 5120 channels 28.7 / 23.4 / 21.6, 8192 64.9 / 49.1 / 42.0; 3072 12.9 / 13.0 / 13.4,
   // 1024 5.8 / 6.3 / 6.0.
-  return hidden > 3072 ? launch(convrot_quant_rows_kernel<12>, 1) : launch(convrot_quant_rows_kernel<6>, kRotWarps);
+  // But where one round of CTAs with four holds all rows, more than two for each SM, nothing is won by that, and a quarter of the CTAs
+  // start sooner.  us with the GEMM behind it (8 heads), one / four to a CTA: 592 x 3328 21.6 / 20.6, 2304 x 3328 33.9 / 31.5, 888 x 4096
+  // 26.0 / 24.3, 1776 x 4096 34.6 / 33.3, 592 x 5120 26.8 / 25.5, 1184 x 5120 28.0 / 26.3, 592 x 8192 35.7 / 33.3; beyond one round 1480 x
+  // 5120 28.7 / 30.1, 888 x 8192 36.4 / 40.4.  By itself 64 x 8192 7.2 / 7.8, 300 x 5120 5.5 / 5.9.
+  constexpr int kSharedPerSm = 228 * 1024, kReserved = 1024;  // of a CTA
+  const int one_round = kSmCount * kRotWarps * (kSharedPerSm / (kRotWarps * row_bytes + kReserved));
+  const bool one_to_a_cta = hidden > 3072 && (rows <= 2 * kSmCount || rows > one_round);
+  return one_to_a_cta ? launch(convrot_quant_rows_kernel<12>, 1) : launch(convrot_quant_rows_kernel<6>, kRotWarps);
 }
 
 }  // namespace h3s

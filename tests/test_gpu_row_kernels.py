@@ -41,6 +41,18 @@ def test_rotated_codes(native_lib, rows, hidden):
     assert torch.equal(scale.cpu(), want_scale) and torch.equal(codes.cpu(), want_codes)
 
 
+# wide rows, on both sides of the lines between one and four to a block
+@pytest.mark.parametrize("rows,hidden", [(296, 8192), (297, 8192), (592, 8192), (593, 8192), (299, 3328), (2368, 3328), (2369, 3328)])
+def test_rotated_codes_of_wide_rows(native_lib, rows, hidden):
+    from h3_optimizations_b200 import ops
+
+    gen = torch.Generator().manual_seed(hidden + rows)
+    x = torch.randn((rows, hidden), generator=gen).to(torch.bfloat16)
+    codes, scale = ops.convrot_quant_rows(x.cuda())
+    want_codes, want_scale = oracle.convrot_quantize_rows(x)
+    assert torch.equal(scale.cpu(), want_scale) and torch.equal(codes.cpu(), want_codes)
+
+
 @pytest.mark.parametrize("batch", [1, 2, 3])
 def test_a_batch_equals_its_elements(native_lib, batch):
     from h3_optimizations_b200 import B200SparseBackend, HybridSparseConfig, runtime_options
