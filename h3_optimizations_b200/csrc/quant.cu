@@ -254,11 +254,18 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
   const int head = blockIdx.y;
   const int first_row = blockIdx.x * BLOCK;  // within this chunk
   const int64_t block = static_cast<int64_t>(head) * blocks_total + row_start / BLOCK + blockIdx.x;
-  auto minus_mean = [&](float2 (&m)[4]) {
-    if (!kHasMean) return;
+  // Here the mean is complete, and asked for before the rows.  us, behind the rows / before them: fp32 24 heads x 1000 tokens 4.9 / 4.6, 3 x
+  // 33272 13.3 / 13.1, bf16 3 x 33272 9.5 / 9.2, 24 x 33272 66.9 / 66.7.
+  float2 minus_mu[4];
+  if (kHasMean) {
     const float *mu = mean + head * H3S_HEAD_DIM + (threadIdx.x & 15) * 8;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = make_float2(-__ldg(mu + 2 * i), -__ldg(mu + 2 * i + 1));
+    for (int i = 0; i < 4; ++i) minus_mu[i] = make_float2(-__ldg(mu + 2 * i), -__ldg(mu + 2 * i + 1));
+  }
+  auto minus_mean = [&](float2 (&m)[4]) {
+    if (!kHasMean) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = minus_mu[i];
   };
   quant_qk_block<T, BLOCK, kHasMean>(
       x + head * stride_h + first_row * stride_s, stride_s, min(BLOCK, rows - first_row),
