@@ -35,13 +35,24 @@ from .errors import FusedQKVError, SparseRouterError, SparseSageError
 from .router import KV_TILE, Q_TILE, SparseTileRouter
 from .runtime import get_runtime_snapshot
 
-# One kernel makes all carriers of a layer, on one stream, up to this many rows of all heads if no head has more than SHORT_HEAD_ROWS.
-# Beyond, kernels of their own on two streams do without the bookkeeping of jobs, and V goes beside the router, which takes longer the more
-# KV tiles a head has.  us a call, two streams / one kernel: 1 head x 1128 tokens 105 / 81, 4 x 2304 fp32 103 / 81, 24 x 1756 96 / 81, 12 x 4256
-# 97 / 83, 24 x 2304 96 / 81, 7 x 10384 127 / 127, 24 x 4000 135 / 132, 24 x 6012 197 / 192, 4 x 13512 157 / 161, 1 x 33272 177 / 182; replayed:
-# 37 / 29, 50 / 44, 66 / 64, 85 / 83, 75 / 75, 123 / 124, 128 / 127, 185 / 184, 156 / 161, 180 / 183.
+# Where one kernel makes all carriers of a layer, on one stream, and where kernels of their own do it on two.  Long layers do without the
+# bookkeeping of jobs, and where a head has many KV tiles V goes beside the router, which takes longer the more they are.  Of the others a
+# call that the host issues waits for the host first, and one kernel saves it a dozen calls; while that is so (``HOST_BOUND``) it is the faster.
+# Replays have no host in them: up to a few rows it saves launches, from there on V is better off beside the router, until the
+# router fills the chip by itself (``MANY_ROWS``).  us a call, two streams / one kernel, from the host (bf16, fp32) and replayed (bf16, fp32):
+#   1 head x 3000    113 / 88   101 / 87    49.9 / 43.5  51.0 / 44.4      8 x 6000     102 / 87   102 / 100   86.0 / 89.1  97.1 / 98.0
+#   4 x 4500          98 / 83    98 / 83    65.2 / 62.4  66.0 / 64.6      3 x 10500    102 / 94   102 / 97    91.8 / 91.2  97.1 / 101.9
+#   2 x 9000         101 / 88   101 / 87    76.2 / 74.8  79.1 / 79.0      4 x 11900    119 / 119  129 / 136   115 / 122    125 / 134
+#   4 x 6000         108 / 90   102 / 87    70.6 / 71.4  74.5 / 77.0      6 x 9000     118 / 122  135 / 134   116 / 120    129 / 132
+#   8 x 4500          99 / 83    97 / 83    72.9 / 73.5  78.7 / 81.2      10 x 9000    171 / 172  194 / 201   165 / 167    188 / 189
+#   24 x 2304        100 / 81    99 / 90    74.6 / 74.5  87.5 / 87.1      24 x 4500    150 / 149  184 / 183   144 / 144    169 / 169
+#   24 x 3000         98 / 93   118 / 120   93.7 / 91.8  109 / 112        24 x 6000    211 / 209  249 / 252   202 / 199    234 / 231
+#   16 x 4500        113 / 111  132 / 135   108 / 108    123 / 128        12 x 11900   300 / 298  340 / 344   291 / 284    323 / 319
+# (heads of 13512 tokens: 4 of them 157 / 161, replayed 156 / 161; one of 33272 177 / 182, 180 / 183.)
 ONE_STREAM_ROWS = 150_000
 SHORT_HEAD_ROWS = 12_000
+FEW_ROWS, MANY_ROWS = 20_000, 105_000  # of all heads
+HOST_BOUND = 335_000_000  # rows of all heads, times the rows of one
 # Bytes of a head's q, k and v from which ``forward_host`` ends with single heads: as long as they take to copy a chunk more is
 # paid for by a shorter end, below that it costs the host's time.  us a call, pairs to the end / single heads at the end, 8 heads,
 # bf16: 1212 tokens 818 / 1001, 4512 933 / 1046, 6512 1080 / 1130, 7512 1155 / 1181, 8512 1316 / 1313, 10512 1594 / 1555, 33272 4575 /
@@ -72,11 +83,24 @@ def preflight():
     return capability
 
 
+def one_carrier_kernel(heads, sequence, element_size):
+    """Whether the carriers of a layer call on the current stream are made by one kernel."""
+    rows = heads * sequence
+    if rows > ONE_STREAM_ROWS or sequence > SHORT_HEAD_ROWS:
+        return False
+    if rows <= FEW_ROWS:
+        return True
+    replayed = torch.cuda.is_current_stream_capturing()
+    if rows >= MANY_ROWS:
+        return replayed or element_size == 2
+    return not replayed and rows * sequence <= HOST_BOUND
+
+
 class CapturedLayerCall:
     """``prepare`` + ``execute`` of one layer call on fixed input tensors, captured
     once into a CUDA graph.  A sampler calls the same layer with the same shapes
     and the same budget step after step; replaying the graph takes the host out
-    of the step (four launches of a short layer, eight and half a dozen stream operations of a long one otherwise) and
+    of the step (four launches of most short layers, eight and half a dozen stream operations of the others otherwise) and
     closes the gaps between the small carrier kernels.  Every kernel still runs on
     every replay - statistics, carriers, router, attention (and, for a sharded
     owner, the exchange) - on whatever ``q``, ``k``, ``v`` hold at that moment; the
@@ -309,14 +333,14 @@ class B200SparseBackend:
             geometry = self.router.geometry(snapshot.layout)
             retained = self.router._retained(video_budget, geometry)
             need_route = retained < geometry.pure_video_kv_tiles
-            # Where layers are short one kernel makes all carriers.  Else every carrier has its own, on two streams: the column
+            # One kernel makes all carriers of most short layers.  Else every carrier has its own, on two streams: the column
             # statistics (K mean, V scale) run on the second one while the Q quantiser, which needs neither, starts at once on the
             # current one; the K quantiser joins when the statistics are in, and the V carrier is held back until the K quantiser
             # is through, so that this memory-bound kernel runs beside the router, which leaves the memory system idle.  Every
             # buffer is allocated on the current stream, which both chains rejoin before returning.
             stream = _native.stream_ptr(q.device)
             side = self._side_stream(q.device)  # there from the first call on: a capture must not bring it into being
-            if heads * sequence <= ONE_STREAM_ROWS and sequence <= SHORT_HEAD_ROWS:
+            if one_carrier_kernel(heads, sequence, q.element_size()):
                 side = None
             buffers = ops.LayerBuffers(heads, sequence, q.device, smooth_k=self.smooth_k,
                                        summary_dtype=torch.float64 if need_route else None)
