@@ -3,6 +3,8 @@
 import pytest
 import torch
 
+from oracle import h3_oracle as oracle
+
 pytestmark = pytest.mark.gpu
 
 CARRIERS = ("q_int8", "k_int8", "v_carrier", "q_scale", "k_scale", "v_scale")
@@ -58,6 +60,91 @@ def test_what_the_kernel_cannot_take_is_refused(native_lib):
         call(q, odd[: 2 * 128 * 132].view(1, 2, 128, 132)[..., :128], v)
     with pytest.raises(_native.NativeError, match="aligned"):
         call(q, k, odd[4:].view(-1)[: 2 * 128 * 128].view(1, 2, 128, 128))
+
+
+def _one_zero(codes):
+    """E4M3 codes with -0, which the quantiser writes as 0, as 0."""
+    return torch.where(codes == 0x80, torch.zeros_like(codes), codes)
+
+
+UNUSUAL = ["zeros", "zero column", "equal rows", "tiny", "huge", "steps", "infinity", "NaN"]
+
+
+@pytest.mark.parametrize("how", UNUSUAL)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("one", [True, False])
+@pytest.mark.parametrize("heads,sequence", [(2, 300), (1, 1)])
+def test_unusual_values_against_the_oracle(native_lib, heads, sequence, one, dtype, how):
+    """K mean, codes, scales and tile means by plain torch.  A NaN counts as nothing where a maximum is taken; codes of it are 0 in
+    Q and K and NaN in V, as are those of an infinity by an infinite scale."""
+    from h3_optimizations_b200 import _native, ops
+
+    gen = torch.Generator().manual_seed(sequence)
+    q, k, v = ((torch.randn((1, heads, sequence, 128), generator=gen) + offset).to(dtype) for offset in (0.0, 0.7, -0.2))
+    row = sequence // 2
+    for x in (q, k, v):
+        if how == "zeros":
+            x.zero_()
+        elif how == "zero column":
+            x[:, 0, :, 9] = 0.0
+            x[:, -1, :, 70] = -0.0
+        elif how == "equal rows":
+            x[:] = x[:, :, :1].clone()
+        elif how == "tiny":
+            x *= 2.0 ** -125
+        elif how == "huge":
+            x *= 2.0 ** 120
+        elif how == "steps":
+            x[:, :, ::7] *= 2.0 ** 20
+    plain = [x.clone() for x in (q, k, v)]
+    bad = {"infinity": float("inf"), "NaN": float("nan")}.get(how)
+    if bad is not None:  # not in K, whose mean would be so
+        q[0, 0, row, 3] = v[0, 0, row, 5] = bad
+    device = torch.device("cuda", torch.cuda.current_device())
+    stream, side = _native.stream_ptr(device), ops.SideStream(device)
+    word, mirror = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.zeros(4, dtype=torch.int32).pin_memory()
+    buffers = ops.LayerBuffers(heads, sequence, device, smooth_k=True, summary_dtype=torch.float64)
+    inputs = [x.cuda() for x in (q, k, v)]
+    if one:
+        ops.prepare_layer(*inputs, buffers, stream, smooth_k=True, status=word, status_mirror=mirror)
+    else:
+        ops.quant_qkv(*inputs, buffers, side, stream, smooth_k=True, v_after_k=True)
+        side.join(stream)
+    got = {name: buffers.tensor(name).cpu() for name in CARRIERS}
+    q_means, k_means = buffers.q_summary.cpu(), buffers.k_summary.cpu()
+
+    mean = k.double().mean(dim=2).to(torch.float32).to(dtype).float()
+    k_codes, k_scale = oracle.quantize_blocks(k, 64, mean=mean)
+    assert torch.equal(got["k_int8"], k_codes) and torch.equal(got["k_scale"], k_scale)
+    q_codes, q_scale = oracle.quantize_blocks(plain[0], 128)
+    v_codes, v_scale = oracle.v_fp8_carrier(plain[2])
+    v_codes = v_codes.view(torch.uint8)
+    if how == "infinity":
+        block = slice(row // 128 * 128, row // 128 * 128 + 128)
+        q_codes[0, 0, block], q_scale[0, 0, row // 128] = 0, bad
+        v_codes[0, 0, 5, :sequence] = 0
+        v_scale[0, 0, 5] = bad
+    if how == "NaN":
+        for x, tile in ((plain[0], 128), (plain[2], None)):
+            x[0, 0, row, 3 if tile else 5] = 0.0  # counts as nothing
+        q_codes, q_scale = oracle.quantize_blocks(plain[0], 128)
+        v_codes, v_scale = oracle.v_fp8_carrier(plain[2])
+        v_codes = v_codes.view(torch.uint8)
+    if bad is not None:
+        assert got["v_carrier"].view(torch.uint8)[0, 0, 5, row] & 0x7F == 0x7F  # NaN
+        v_codes[0, 0, 5, row] = got["v_carrier"].view(torch.uint8)[0, 0, 5, row]
+    assert torch.equal(got["q_int8"], q_codes) and torch.equal(got["q_scale"], q_scale)
+    assert torch.equal(_one_zero(got["v_carrier"].view(torch.uint8)), _one_zero(v_codes)) and torch.equal(got["v_scale"], v_scale)
+    half = buffers.v_half.cpu()
+    want_half = got["v_carrier"].to(torch.float16)
+    assert torch.equal(torch.isnan(half), torch.isnan(want_half)) and torch.equal(half.nan_to_num(0.0), want_half.nan_to_num(0.0))
+    for x, means, tile in ((q, q_means, 128), (k, k_means, 64)):
+        want = oracle.mean_pool(x.double(), tile)
+        largest = oracle.mean_pool(x.double().abs(), tile)
+        fine = torch.isfinite(want)
+        # up to eight rows are added up in fp32
+        assert bool(((means - want).abs()[fine] <= 8 * 2.0 ** -24 * largest[fine]).all()) and not bool(torch.isfinite(means[~fine]).any())
+    assert word.tolist() == [0, 0, 0, 0]
 
 
 # fewer jobs than blocks, and more than twice as many
