@@ -35,7 +35,6 @@ namespace h3s {
 
 constexpr int kRotGroup = 256;
 
-// In-register part of the transform: butterflies over the three low index bits.
 // The stages of a Walsh-Hadamard transform behind the first, on pairs of neighbouring values; a - b as the exactly rounded a + (-1) * b
 template <int kPairs>
 __device__ __forceinline__ void fwht_pairs(float2 (&v)[kPairs]) {
