@@ -328,7 +328,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     ptx::tmem_relinquish();
   }
   wait_for_previous();
-  if (threadIdx.x < H3S_HEAD_DIM) sh.item[0].v_scale[threadIdx.x] = __ldg(prm.v_scale + work.head * H3S_HEAD_DIM + threadIdx.x);
+  if (threadIdx.x < H3S_HEAD_DIM) sh.item[0].v_scale[threadIdx.x] = load_written(prm.v_scale + work.head * H3S_HEAD_DIM + threadIdx.x);
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -380,14 +380,14 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     }
     // what an item's q_scale and k_scale are multiplied with: 1 / sqrt(128) / ln 2
     auto scale_of = [&](const HalfWork &it) {
-      return __ldg(prm.q_scale + it.head * prm.q_tiles + it.tq) * (0.08838834764831845f * 1.4426950408889634f);
+      return load_written(prm.q_scale + it.head * prm.q_tiles + it.tq) * (0.08838834764831845f * 1.4426950408889634f);
     };
     float item_scale = keys ? scale_of(work) : 0.f, coming_scale = 0.f;
     int next_tile = 0;  // of the block of the list that comes next, one per lane
     float next_scale = 0.f;
     auto fetch = [&](const HalfWork &it, int position) {
-      next_tile = it.dense ? it.first_tile + position : __ldg(it.route_row + position);
-      if (keys) next_scale = __ldg(prm.k_scale + static_cast<int64_t>(it.head) * prm.kv_tiles + next_tile);
+      next_tile = it.dense ? it.first_tile + position : load_written(it.route_row + position);
+      if (keys) next_scale = load_written(prm.k_scale + static_cast<int64_t>(it.head) * prm.kv_tiles + next_tile);
     };
     auto fetch_block = [&](const HalfWork &it, int i) {  // from the i-th tile on
       fetch(it, list_position(min(i + lane % kHBlock, it.n_iter - 1), it.n_iter));
@@ -473,7 +473,7 @@ sparse_attn_half_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             to.part = coming.part;
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = __ldg(prm.v_scale + coming.head * H3S_HEAD_DIM + i * 32 + lane);
+          for (int i = 0; i < 4; ++i) to.v_scale[i * 32 + lane] = load_written(prm.v_scale + coming.head * H3S_HEAD_DIM + i * 32 + lane);
           ok = warp_wait(&sh.q_free, items & 1u, abort_word, kAbortQFree | warp << 8, 4 * prm.wait_budget_ns);
           if (!ok) break;
           load_q(coming);
@@ -982,7 +982,7 @@ __global__ void __launch_bounds__(256) v_half_kernel(const uint4 *__restrict__ v
   wait_for_previous();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= chunks) return;
-  const uint4 codes = __ldg(v8 + i);
+  const uint4 codes = load_written(v8 + i);
   v16[2 * i] = e4m3x8_to_half(make_uint2(codes.x, codes.y));
   v16[2 * i + 1] = e4m3x8_to_half(make_uint2(codes.z, codes.w));
 }

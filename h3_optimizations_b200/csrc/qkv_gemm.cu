@@ -364,8 +364,8 @@ __device__ __forceinline__ float4 column4(const float *base, int col, int n_out,
 }
 
 __device__ __forceinline__ float rope_load(const void *base, int64_t index, int dtype) {
-  return dtype == H3S_F32 ? __ldg(static_cast<const float *>(base) + index)
-                          : __bfloat162float(__ldg(static_cast<const __nv_bfloat16 *>(base) + index));
+  return dtype == H3S_F32 ? load_written(static_cast<const float *>(base) + index)
+                          : __bfloat162float(load_written(static_cast<const __nv_bfloat16 *>(base) + index));
 }
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
@@ -844,11 +844,11 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const bool row_ok = row < prm.rows;
       const int group_col0 = tn * tile_n + gi * H3S_HEAD_DIM;
       // scales come while the MMAs are still at it
-      const float xs = prm.x_scale == nullptr ? 1.0f : (row_ok ? __ldg(prm.x_scale + row) : 0.f);
+      const float xs = prm.x_scale == nullptr ? 1.0f : (row_ok ? load_written(prm.x_scale + row) : 0.f);
       float *my_scales = reinterpret_cast<float *>(smem + L::kOffScale) + warp * 64;
       if (kCarriers) {  // without a group nothing is stored
         const int i = 2 * lane, channel = i < 24 ? 24 * share + i : i < 48 ? 24 + 24 * share + i : 48 + 16 * share + i;
-        reinterpret_cast<float2 *>(my_scales)[lane] = __ldg(reinterpret_cast<const float2 *>(prm.w_scale + (group_col0 < prm.n_out ? group_col0 : 0) + channel));
+        reinterpret_cast<float2 *>(my_scales)[lane] = load_written(reinterpret_cast<const float2 *>(prm.w_scale + (group_col0 < prm.n_out ? group_col0 : 0) + channel));
         __syncwarp();
       }
       {

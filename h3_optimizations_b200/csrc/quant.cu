@@ -117,8 +117,8 @@ __global__ void column_stats_finalize_kernel(const double *__restrict__ k_sum,
   wait_for_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
-  if (k_mean != nullptr) k_mean[i] = finalize_mean<T>(k_sum[i], sequence);
-  if (v_scale != nullptr) v_scale[i] = finalize_scale(v_amax_bits[i], v_bound);
+  if (k_mean != nullptr) k_mean[i] = finalize_mean<T>(load_written(k_sum + i), sequence);
+  if (v_scale != nullptr) v_scale[i] = finalize_scale(load_written(v_amax_bits + i), v_bound);
 }
 
 // ---------------------------------------------------------------------------
@@ -260,7 +260,7 @@ quant_qk_blocks_kernel(const T *__restrict__ x, int64_t stride_h, int64_t stride
   if (kHasMean) {
     const float *mu = mean + head * H3S_HEAD_DIM + (threadIdx.x & 15) * 8;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) minus_mu[i] = make_float2(-__ldg(mu + 2 * i), -__ldg(mu + 2 * i + 1));
+    for (int i = 0; i < 4; ++i) minus_mu[i] = make_float2(-load_written(mu + 2 * i), -load_written(mu + 2 * i + 1));
   }
   auto minus_mean = [&](float2 (&m)[4]) {
     if (!kHasMean) return;
@@ -403,7 +403,7 @@ quant_v_fp8_kernel(const T *__restrict__ v, int64_t stride_h, int64_t stride_s,
   quant_v_tile(v + head * stride_h + first_row * stride_s, stride_s, max(0, min(kVTile, rows - first_row)), out + at,
                out_half == nullptr ? nullptr : out_half + at, padded_total, v_bound, tile, [&](float (&scale)[8]) {
 #pragma unroll
-                 for (int i = 0; i < 8; ++i) scale[i] = __ldg(v_scale + head * H3S_HEAD_DIM + (threadIdx.x & 15) * 8 + i);
+                 for (int i = 0; i < 8; ++i) scale[i] = load_written(v_scale + head * H3S_HEAD_DIM + (threadIdx.x & 15) * 8 + i);
                });
 }
 
@@ -590,8 +590,8 @@ staged_carriers_kernel(const __grid_constant__ CarrierParams p) {
   const bool is_v = !kSmooth || blockIdx.x % kKinds != 0;
   const int at_value = head * H3S_HEAD_DIM + (t & (H3S_HEAD_DIM - 1));
   // asked for before the rows
-  const double k_total = is_v ? 0.0 : __ldg(p.k_sum + at_value);
-  const unsigned int v_top = is_v ? __ldg(p.v_amax_bits + at_value) : 0u;
+  const double k_total = is_v ? 0.0 : load_written(p.k_sum + at_value);
+  const unsigned int v_top = is_v ? load_written(p.v_amax_bits + at_value) : 0u;
   auto make_values = [&]() {
     if (t < H3S_HEAD_DIM) {
       const float value = is_v ? finalize_scale(v_top, p.v_bound) : finalize_mean<T>(k_total, p.sequence);

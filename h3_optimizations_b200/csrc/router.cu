@@ -38,12 +38,14 @@ __device__ __forceinline__ unsigned long long score_key(double s) {
 // 64 registers a thread
 template <typename T, int kRows, bool kAhead>
 __global__ void __launch_bounds__(kRows * 32)
-route_topk_kernel(const T *__restrict__ q_summary, const T *__restrict__ k_summary, int q_tiles,
+route_topk_kernel(const T *q_summary, const T *k_summary, int q_tiles,
                   int kv_tiles, int q_start, int q_stop, int kv_start, int kv_stop, int retained,
                   int route_len, int32_t *__restrict__ route) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   let_next_start();
   wait_for_previous();
+  q_summary = written_before(q_summary);
+  k_summary = written_before(k_summary);
   const int pure_q = q_stop - q_start;
   const int pure_kv = kv_stop - kv_start;
   double *scores = reinterpret_cast<double *>(smem_raw);              // [kRows][pure_kv]
