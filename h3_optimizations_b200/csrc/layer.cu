@@ -95,8 +95,8 @@ int h3s_project_qkv_norms(const h3s_layer_carriers *c, const void *x_bf16, int64
     if (rc) return rc;
   }
   // One launch for short sequences, in whose kernels and between whose kernels the chip waits more than it works: from the last projection
-  // tile to the end 11.9 us for 12.9 at 24 heads x 2304 tokens, and the host issues three calls for nine; a whole block of 4 x 900 164 ->
-  // 147 us, 24 x 2304 173 -> 170, 12 x 8000 294 -> 292.  For long ones, kernels of their own are the faster: 24 x 33272 151 us for 169.  Replayed
+  // tile to the end 11.9 us for 12.9 at 24 heads x 2304 tokens, and the host issues three calls for nine; whole blocks of 4 x 900 139 ->
+  // 129 us, 24 x 900 140 -> 130, 24 x 2304 168 and 167, 12 x 8000 372 and 371.  For long ones, kernels of their own are the faster: 24 x 33272 151 us for 169.  Replayed
   // from a graph, without the host, whole projections several / one: 24 x 900 41.2 / 41.3, 24 x 2304 80.3 / 79.0, 24 x 4500 154.0 / 154.4,
   // 24 x 6000 199.1 / 200.5, 4 x 36000 226 / 230, 24 x 8000 255 / 259, 24 x 16000 496 / 509.
   if (static_cast<int64_t>(heads) * sequence <= kStagedOneLaunchRows)

@@ -312,7 +312,7 @@ struct GemmParams {
 
 // 0.5 x (1 + tanh(u)), u = sqrt(2/pi) (x + 0.044715 x^3), the formula of torch's approximate='tanh', as
 // x / (1 + exp(-2u)): nothing cancels for negative x, where 1 + tanh(u) loses all but a few bits.  Two values at a time:
-// everything but the exponentials and the reciprocals is packed (MLP of 33272 x 3072 x 12288, under the power cap, 2588 -> 2555 us).
+// everything but the exponentials and the reciprocals is packed (MLP of 33272 x 3072 x 12288, under the power cap, 2605 -> 2595 us).
 // 28 of 8.4 million bf16 results differ from the unpacked form's, errors against 64 bits are the same to seven digits.
 __device__ __forceinline__ float2 gelu_tanh2(float2 x) {
   constexpr float kLinear = -2.0f * 0.7978845608028654f * 1.4426950408889634f, kCubic = kLinear * 0.044715f;

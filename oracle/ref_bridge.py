@@ -28,7 +28,7 @@ def _ensure_path():
     if not available():
         raise ReferenceUnavailable(
             "oracle/_ref is empty: run `python oracle/build_ref.py --reference <checkout>` where the "
-            "reference is checked out (it ships to the GPU box with the repository snapshot)"
+            "reference is checked out (it travels with a copy of the repository)"
         )
     for entry in (str(REF_ROOT / "benchmarks"), str(REF_ROOT)):
         if entry not in sys.path:

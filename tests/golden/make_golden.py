@@ -1,7 +1,7 @@
 """Generate the golden fixtures in this directory from the reference itself.
 
-Run where the reference checkout exists (it is Python/torch and cannot travel
-to the GPU box):
+Run where the reference checkout exists (it is Python/torch and no part of this
+repository):
 
     python tests/golden/make_golden.py --reference /path/to/H3-Optimizations
 
